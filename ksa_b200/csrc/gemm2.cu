@@ -50,12 +50,13 @@ struct Gemm2Epilogue {
   // the epilogue, straight into that rank's memory at c_peer[owner] + (row - owner * c_shard_rows) * ldc.
   int c_shard_rows;          // 0: every row goes to `c`
   int c_world;
-  int c_tma;                 // 1: 32-row blocks that lie in one owner's rows leave through TMA stores (c_map)
+  int c_tma;                 // 1: 32-row blocks that lie in one owner's rows leave through TMA stores (a plain output
+                             // is one owner of all rows; fp32 outputs are stored or, to accumulate, reduced)
   void* c_peer[kMaxPeers];
 };
 
-// Tensor maps over the owners' output buffers ([rows of that owner, N] bf16, box 64 columns x 32 rows, 128-byte
-// swizzle) for the scattering epilogue.
+// Tensor maps over the owners' output buffers ([rows of that owner, N], box of 128 bytes x 32 rows, 128-byte swizzle)
+// for the TMA epilogue.
 struct ScatterMaps {
   CUtensorMap m[kMaxPeers];
 };
@@ -110,6 +111,12 @@ __device__ __forceinline__ void umma2_ss(uint32_t d_tmem, uint64_t adesc, uint64
       "tcgen05.mma.cta_group::2.kind::f16 [%0], %1, %2, %3, p;\n\t}"
       ::"r"(d_tmem), "l"(adesc), "l"(bdesc), "r"(idesc), "r"(accumulate)
       : "memory");
+}
+// fp32 add of a staged box into global memory (done by the memory system: nothing is read into the SM)
+__device__ __forceinline__ void tma_reduce_add_2d(const CUtensorMap* m, const void* src, int x, int y) {
+  asm volatile("cp.reduce.async.bulk.tensor.2d.global.shared::cta.add.tile.bulk_group [%0, {%2, %3}], [%1];" ::"l"(m),
+               "r"(smem_u32(src)), "r"(x), "r"(y)
+               : "memory");
 }
 // One arrival on the barrier at this shared-memory offset in BOTH CTAs of the pair once all MMAs issued so far are done.
 __device__ __forceinline__ void umma2_commit_both(uint64_t* bar) {
@@ -291,9 +298,13 @@ gemm2_bf16_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant
       const int row_w = mb * 2 * k2BM + (int)rank * k2BM + quad * 32;   // first of this warp's 32 rows
       const int row = row_w + lane;
       const uint32_t t_row = tmem_base + ((uint32_t)(quad * 32) << 16) + buf * k2BN;
-      // scattering epilogue: a 32-row block that lies in ONE owner's rows leaves through shared memory and TMA
-      // stores of 64 columns x 32 rows (128-byte rows on the wire); a block that straddles two owners' rows
-      // falls back to the per-row stores below
+      // Bound: a 256 x 256 fp32 tile at K = 2048 is 256 KB read and 256 KB written per 16k cycles of products, and 16-byte
+      // accesses at a row pitch spend the memory system on partial lines (output head, 2 x 2048 x 151936 x 2048 with fp32
+      // accumulation: 2699 us; staged and added by TMA reductions: 1888 us; weight gradients of a 2048-wide layer at 8256
+      // rows 632 -> 595 us, its bf16 products 1133 -> 1072 us).
+      // TMA epilogue: a 32-row block that lies in ONE owner's rows leaves through shared memory and TMA stores of
+      // 128 bytes x 32 rows (whole lines for the memory system, 128-byte rows on the wire); a block that straddles
+      // two owners' rows, and every block while the ring carries a gather, takes the per-row stores below
       int owner_w = 0;
       bool tma_block = false;
       if (ep.c_tma && row_w < M) {
@@ -306,10 +317,31 @@ gemm2_bf16_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant
         tmem_ld32(t_row + c * 32, r);
         tmem_wait_ld();
         const int col0 = nb * k2BN + c * 32;
+        if (tma_block && ep.out_fp32) {
+          uint8_t* stage = ring + ((warp - 2) * 2 + (c & 1)) * 4096;
+          // this buffer was read by the store issued two pieces ago; at most the newest store may be pending
+          if (lane == 0) asm volatile("cp.async.bulk.wait_group.read 1;" ::: "memory");
+          __syncwarp();
+          if (col0 < N) {
+#pragma unroll
+            for (int j = 0; j < 8; ++j)
+              *reinterpret_cast<float4*>(stage + lane * 128 + ((j ^ (lane & 7)) * 16)) =
+                  make_float4(__uint_as_float(r[4 * j]) * ep.alpha, __uint_as_float(r[4 * j + 1]) * ep.alpha,
+                              __uint_as_float(r[4 * j + 2]) * ep.alpha, __uint_as_float(r[4 * j + 3]) * ep.alpha);
+          }
+          fence_proxy_async();
+          __syncwarp();
+          if (lane == 0 && col0 < N) {
+            if (ep.accumulate) tma_reduce_add_2d(&smaps.m[owner_w], stage, col0, row_w - owner_w * ep.c_shard_rows);
+            else tma_store_2d(&smaps.m[owner_w], stage, col0, row_w - owner_w * ep.c_shard_rows);
+            tma_store_commit();
+          }
+          continue;
+        }
         if (tma_block) {
           const int piece = c >> 1, half = c & 1;                   // 64-column piece, 32-column half of it
           uint8_t* stage = ring + ((warp - 2) * 2 + (piece & 1)) * 4096;
-          const bool live = nb * k2BN + piece * 64 < N;             // N is a multiple of 64 on this path
+          const bool live = nb * k2BN + piece * 64 < N;             // columns past N are clipped by the map
           if (half == 0) {
             // this buffer was read by the store issued two pieces ago; at most the newest store may be pending
             if (lane == 0) asm volatile("cp.async.bulk.wait_group.read 1;" ::: "memory");
@@ -464,12 +496,22 @@ KSA_API int ksa_gemm2_bf16(const void* a, const void* b, void* c, int M, int N, 
   KSA_REQUIRE(!(accumulate && !out_fp32), "gemm2: accumulate needs an fp32 output");
   Gemm2Epilogue ep{};
   ep.c = c; ep.ldc = ldc; ep.out_fp32 = out_fp32; ep.accumulate = accumulate; ep.alpha = alpha;
+  ep.c_tma = 1; ep.c_shard_rows = M; ep.c_world = 1; ep.c_peer[0] = c;
+  ScatterMaps smaps{};
+  {
+    const uint64_t elem = out_fp32 ? 4 : 2;
+    uint64_t dims[2] = {(uint64_t)N, (uint64_t)M};
+    uint64_t str[2] = {elem, (uint64_t)ldc * elem};
+    uint32_t box[2] = {(uint32_t)(128 / elem), 32};
+    const int rc = make_tmap(&smaps.m[0], c, (int)elem, 2, dims, str, box, true);
+    if (rc) return rc;
+  }
   cudaStream_t st = reinterpret_cast<cudaStream_t>(stream);
   const Comm2Work none{};
-  if (!a_mn_major && !b_mn_major) return launch_gemm2<false, false>(a, b, ep, M, N, K, lda, ldb, st, none);
-  if (!a_mn_major && b_mn_major) return launch_gemm2<false, true>(a, b, ep, M, N, K, lda, ldb, st, none);
-  if (a_mn_major && !b_mn_major) return launch_gemm2<true, false>(a, b, ep, M, N, K, lda, ldb, st, none);
-  return launch_gemm2<true, true>(a, b, ep, M, N, K, lda, ldb, st, none);
+  if (!a_mn_major && !b_mn_major) return launch_gemm2<false, false>(a, b, ep, M, N, K, lda, ldb, st, none, smaps);
+  if (!a_mn_major && b_mn_major) return launch_gemm2<false, true>(a, b, ep, M, N, K, lda, ldb, st, none, smaps);
+  if (a_mn_major && !b_mn_major) return launch_gemm2<true, false>(a, b, ep, M, N, K, lda, ldb, st, none, smaps);
+  return launch_gemm2<true, true>(a, b, ep, M, N, K, lda, ldb, st, none, smaps);
 }
 
 // All-gather -> GEMM in one launch.  The GEMM arguments are those of ksa_gemm2_bf16; both operands K-major.
