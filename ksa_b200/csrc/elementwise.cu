@@ -66,53 +66,73 @@ rmsnorm_fwd_kernel(const bf16* __restrict__ x, const bf16* __restrict__ delta, c
 }
 
 // dx = rstd * (dy*w - xhat * mean(dy*w*xhat)) (+ dres); per-CTA partial dw rows in `dw_partial`.
-// NVEC 16-byte vectors per thread cover D <= NVEC * 2048; R rows are in flight per iteration so that enough
-// loads are outstanding to hide DRAM latency, and their R row reductions share one pair of barriers.
-template <int NVEC, int R>
-__global__ void __launch_bounds__(kNormThreads)
+// NVEC 16-byte vectors per thread cover D <= NVEC * 2048; R rows per iteration share one pair of barriers.  The bound is
+// the memory (three reads and one write of a row), so loads never pause for the reduction: the rows of the next iteration
+// are requested, as raw bf16 words, before the current ones are reduced (8256 x 2048 rows with a residual gradient, the pair of
+// norms of a layer: 76.8 -> 51.0 us; three CTAs per SM spill and take 79.5).
+template <int NVEC, int R, int MINB>
+__global__ void __launch_bounds__(kNormThreads, MINB)
 rmsnorm_bwd_kernel(const bf16* __restrict__ dy, const bf16* __restrict__ x, const bf16* __restrict__ w,
                    const float* __restrict__ rstd_in, const bf16* __restrict__ dres, bf16* __restrict__ dx,
                    float* __restrict__ dw_partial, int rows, int D) {
   __shared__ float red[R][8];
-  float wv[NVEC][8];
+  BF8 wv[NVEC];
   float dw[NVEC][8];
 #pragma unroll
   for (int i = 0; i < NVEC; ++i) {
     const int c = (i * kNormThreads + threadIdx.x) * 8;
 #pragma unroll
-    for (int j = 0; j < 8; ++j) { dw[i][j] = 0.f; wv[i][j] = 0.f; }
-    if (c < D) load8(w + c, wv[i]);
+    for (int j = 0; j < 8; ++j) dw[i][j] = 0.f;
+    wv[i] = BF8{{0, 0, 0, 0}};
+    if (c < D) wv[i] = *reinterpret_cast<const BF8*>(w + c);
   }
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-  for (int row0 = blockIdx.x * R; row0 < rows; row0 += gridDim.x * R) {
-    float xh[R][NVEC][8], g[R][NVEC][8];
-    BF8 rr_raw[R][NVEC];      // the residual gradient, requested with x and dy so that it arrives under the reduction
-    float dot[R];
+  BF8 nx[R][NVEC], ny[R][NVEC], nr[R][NVEC];       // x, dy and the residual gradient of the next iteration
+  float nrstd[R];
+  auto fetch = [&](int row0) {
 #pragma unroll
     for (int r = 0; r < R; ++r) {
-      dot[r] = 0.f;
       const int row = row0 + r;
-      const float rstd = row < rows ? rstd_in[row] : 0.f;
+      nrstd[r] = row < rows ? rstd_in[row] : 0.f;
 #pragma unroll
       for (int i = 0; i < NVEC; ++i) {
         const int c = (i * kNormThreads + threadIdx.x) * 8;
+        nx[r][i] = ny[r][i] = nr[r][i] = BF8{{0, 0, 0, 0}};
         if (row < rows && c < D) {
-          float xv[8], dyv[8];
-          if (dres) rr_raw[r][i] = *reinterpret_cast<const BF8*>(dres + (long long)row * D + c);
-          load8(x + (long long)row * D + c, xv);
-          load8(dy + (long long)row * D + c, dyv);
-#pragma unroll
-          for (int j = 0; j < 8; ++j) {
-            xh[r][i][j] = xv[j] * rstd;
-            g[r][i][j] = dyv[j] * wv[i][j];
-            dot[r] += g[r][i][j] * xh[r][i][j];
-            dw[i][j] += dyv[j] * xh[r][i][j];
-          }
-        } else {
-#pragma unroll
-          for (int j = 0; j < 8; ++j) { xh[r][i][j] = 0.f; g[r][i][j] = 0.f; }
+          const long long at = (long long)row * D + c;
+          nx[r][i] = *reinterpret_cast<const BF8*>(x + at);
+          ny[r][i] = *reinterpret_cast<const BF8*>(dy + at);
+          if (dres) nr[r][i] = *reinterpret_cast<const BF8*>(dres + at);
         }
       }
+    }
+  };
+  const int step = (int)gridDim.x * R;
+  fetch(blockIdx.x * R);
+  for (int row0 = blockIdx.x * R; row0 < rows; row0 += step) {
+    BF8 cx[R][NVEC], cy[R][NVEC], cr[R][NVEC];
+    float rstd[R], dot[R];
+#pragma unroll
+    for (int r = 0; r < R; ++r) {
+      rstd[r] = nrstd[r];
+#pragma unroll
+      for (int i = 0; i < NVEC; ++i) { cx[r][i] = nx[r][i]; cy[r][i] = ny[r][i]; cr[r][i] = nr[r][i]; }
+    }
+    if (row0 + step < rows) fetch(row0 + step);
+#pragma unroll
+    for (int r = 0; r < R; ++r) {
+      dot[r] = 0.f;
+#pragma unroll
+      for (int i = 0; i < NVEC; ++i)
+#pragma unroll
+        for (int j = 0; j < 4; ++j) {
+          const float2 xv = unpack_bf16x2(cx[r][i].u[j]), yv = unpack_bf16x2(cy[r][i].u[j]), ww = unpack_bf16x2(wv[i].u[j]);
+          const float h0 = xv.x * rstd[r], h1 = xv.y * rstd[r];
+          dot[r] += yv.x * ww.x * h0;
+          dot[r] += yv.y * ww.y * h1;
+          dw[i][2 * j] += yv.x * h0;
+          dw[i][2 * j + 1] += yv.y * h1;
+        }
       dot[r] = warp_sum(dot[r]);
     }
     __syncthreads();
@@ -129,21 +149,17 @@ rmsnorm_bwd_kernel(const bf16* __restrict__ dy, const bf16* __restrict__ x, cons
       const float mean = t / (float)D;
       const int row = row0 + r;
       if (row >= rows) continue;
-      const float rstd = rstd_in[row];
 #pragma unroll
       for (int i = 0; i < NVEC; ++i) {
         const int c = (i * kNormThreads + threadIdx.x) * 8;
         if (c < D) {
           float o[8];
 #pragma unroll
-          for (int j = 0; j < 8; ++j) o[j] = rstd * (g[r][i][j] - xh[r][i][j] * mean);
-          if (dres) {
-#pragma unroll
-            for (int j = 0; j < 4; ++j) {
-              const float2 t = unpack_bf16x2(rr_raw[r][i].u[j]);
-              o[2 * j] += t.x;
-              o[2 * j + 1] += t.y;
-            }
+          for (int j = 0; j < 4; ++j) {
+            const float2 xv = unpack_bf16x2(cx[r][i].u[j]), yv = unpack_bf16x2(cy[r][i].u[j]);
+            const float2 ww = unpack_bf16x2(wv[i].u[j]), rv = unpack_bf16x2(cr[r][i].u[j]);
+            o[2 * j] = rstd[r] * (yv.x * ww.x - xv.x * rstd[r] * mean) + rv.x;
+            o[2 * j + 1] = rstd[r] * (yv.y * ww.y - xv.y * rstd[r] * mean) + rv.y;
           }
           store8(dx + (long long)row * D + c, o);
         }
@@ -797,13 +813,15 @@ KSA_API int ksa_rmsnorm_fwd(const void* x, const void* delta, const void* w, voi
 // Number of partial rows the backward writes: the caller sizes `dw_partial` as [ksa_rmsnorm_bwd_parts(rows), D] fp32.
 KSA_API int ksa_rmsnorm_bwd_parts(int rows) { return rows < 592 ? (rows > 0 ? rows : 1) : 592; }
 
-template <int NVEC, int R>
+template <int NVEC, int R, int MINB>
 static int launch_rmsnorm_bwd(const void* dy, const void* x, const void* w, const void* rstd, const void* dres,
                               void* dx, void* dw_partial, int parts, int rows, int D, cudaStream_t st) {
-  int blocks = (rows + R - 1) / R;
-  if (blocks > parts) blocks = parts;
+  // as many CTAs as are resident at once, evened out over the rounds they need
+  const int groups = (rows + R - 1) / R, most = parts < 148 * MINB ? parts : 148 * MINB;
+  const int rounds = (groups + most - 1) / most;
+  const int blocks = (groups + rounds - 1) / rounds;
   // rows beyond `blocks` partial rows stay untouched; zero-fill is not needed because colsum reads `blocks` rows only
-  rmsnorm_bwd_kernel<NVEC, R><<<blocks, kNormThreads, 0, st>>>((const bf16*)dy, (const bf16*)x, (const bf16*)w,
+  rmsnorm_bwd_kernel<NVEC, R, MINB><<<blocks, kNormThreads, 0, st>>>((const bf16*)dy, (const bf16*)x, (const bf16*)w,
                                                                (const float*)rstd, (const bf16*)dres, (bf16*)dx,
                                                                (float*)dw_partial, rows, D);
   KSA_CHECK_CUDA(cudaGetLastError());
@@ -817,9 +835,9 @@ KSA_API int ksa_rmsnorm_bwd(const void* dy, const void* x, const void* w, const 
   if (rows == 0) return 0;
   const int parts = ksa_rmsnorm_bwd_parts(rows);
   int used;
-  if (D <= 2048) used = launch_rmsnorm_bwd<1, 4>(dy, x, w, rstd, dres, dx, dw_partial, parts, rows, D, ST(stream));
-  else if (D <= 4096) used = launch_rmsnorm_bwd<2, 2>(dy, x, w, rstd, dres, dx, dw_partial, parts, rows, D, ST(stream));
-  else used = launch_rmsnorm_bwd<4, 1>(dy, x, w, rstd, dres, dx, dw_partial, parts, rows, D, ST(stream));
+  if (D <= 2048) used = launch_rmsnorm_bwd<1, 2, 2>(dy, x, w, rstd, dres, dx, dw_partial, parts, rows, D, ST(stream));
+  else if (D <= 4096) used = launch_rmsnorm_bwd<2, 1, 2>(dy, x, w, rstd, dres, dx, dw_partial, parts, rows, D, ST(stream));
+  else used = launch_rmsnorm_bwd<4, 1, 1>(dy, x, w, rstd, dres, dx, dw_partial, parts, rows, D, ST(stream));
   if (used < 0) return used;
   if (dw) {
     colsum_partials_kernel<<<(D + 31) / 32, 256, 0, ST(stream)>>>((const float*)dw_partial, (float*)dw, used, D,
