@@ -3,7 +3,7 @@ import pytest
 import torch
 
 from ksa_b200 import ops
-from ksa_b200.ops import _lib
+from ksa_b200.ops import _lib, reference as ref
 
 pytestmark = pytest.mark.gpu
 DEV = "cuda"
@@ -37,3 +37,27 @@ def test_rms_norm_backward(rows, D, with_res):
     # one rounding to bf16: at most 2^-8 of every element
     assert (xs.grad.double() - want).norm() < 4e-3 * want.norm()
     assert (ws.grad.double() - wd.grad).norm() < 4e-3 * wd.grad.norm()
+
+
+@pytest.mark.parametrize("Hq,Hkv", [(1, 1), (3, 1), (5, 5), (16, 8), (32, 8)])
+@pytest.mark.parametrize("rows", [1, 9, 300])
+@pytest.mark.parametrize("interleaved", [False, True])
+def test_qk_norm_rope_head_counts(Hq, Hkv, rows, interleaved):
+    """Head counts below, at and across the number of heads that one warp takes."""
+    D, H = 128, Hq + 2 * Hkv
+    qkv, pos = bf(rows, H * D), torch.randint(0, 5000, (rows,), device=DEV)
+    wq, wk = [(1 + 0.1 * torch.randn(D, device=DEV)).bfloat16() for _ in range(2)]
+    xs, qs, ks = qkv.clone().requires_grad_(), wq.clone().requires_grad_(), wk.clone().requires_grad_()
+    out = ops.qk_norm_rope_packed(xs, qs, ks, pos, Hq, Hkv, D, 1e6, 1e-6, interleaved)
+    g = bf(*out.shape)
+    out.backward(g)
+    xf, qf, kf = [t.float().requires_grad_() for t in (qkv, wq, wk)]
+    q, k = ref.qk_norm_rope(xf[:, :Hq * D].reshape(1, rows, Hq, D), xf[:, Hq * D:(Hq + Hkv) * D].reshape(1, rows, Hkv, D),
+                            qf, kf, pos, 1e6, 1e-6, interleaved)
+    want = torch.cat([q.reshape(rows, -1), k.reshape(rows, -1), xf[:, (Hq + Hkv) * D:]], 1)
+    want.backward(g.float())
+    _lib.check_status()
+    assert (out.float() - want).norm() < 5e-3 * want.norm()
+    assert torch.equal(out[:, (Hq + Hkv) * D:], qkv[:, (Hq + Hkv) * D:])
+    for got, exp in ((xs.grad, xf.grad), (qs.grad, qf.grad), (ks.grad, kf.grad)):
+        assert (got.float() - exp).norm() < 1e-2 * exp.norm()
