@@ -215,10 +215,13 @@ __global__ void __launch_bounds__(128) summary_attn_bwd_kernel(SumAttnArgs a) {
 constexpr int kSumFwdThreads = 256;
 constexpr int kSumFwdMaxQ = 8;
 
-template <int HD>
+// NQ: queries of a group, known to the compiler for 1, 2 and 4 of them (kSumFwdMaxQ: any number up to that), so that
+// the accumulators of absent queries cost nothing (two queries, 64 chunks x 8 groups: 25.2 -> 17.1 us, backward 66.4 -> 44.2
+// us; four queries, 256 chunks: 97.1 -> 87.3 us).
+template <int HD, int NQ>
 __global__ void __launch_bounds__(kSumFwdThreads) summary_attn_fwd_fast_kernel(SumAttnArgs a, int nk_max) {
   extern __shared__ uint32_t smw[];
-  const int G = a.Hq / a.Hkv, S = a.n_sum, nq = G * S;
+  const int G = a.Hq / a.Hkv, S = a.n_sum, nq = NQ < kSumFwdMaxQ ? NQ : G * S;
   bf16* v_s = reinterpret_cast<bf16*>(smw);
   float* q_s = reinterpret_cast<float*>(v_s + (size_t)nk_max * HD);
   float* p_s = q_s + nq * HD;
@@ -266,9 +269,9 @@ __global__ void __launch_bounds__(kSumFwdThreads) summary_attn_fwd_fast_kernel(S
       uint4 u[HD / 16];
 #pragma unroll
       for (int j = 0; j < HD / 16; ++j) u[j] = valid ? *reinterpret_cast<const uint4*>(row + j * 8) : make_uint4(0, 0, 0, 0);
-      float acc[kSumFwdMaxQ];
+      float acc[NQ];
 #pragma unroll
-      for (int qi = 0; qi < kSumFwdMaxQ; ++qi) acc[qi] = 0.f;
+      for (int qi = 0; qi < NQ; ++qi) acc[qi] = 0.f;
 #pragma unroll
       for (int j = 0; j < HD / 16; ++j) {
         const uint32_t w[4] = {u[j].x, u[j].y, u[j].z, u[j].w};
@@ -277,12 +280,12 @@ __global__ void __launch_bounds__(kSumFwdThreads) summary_attn_fwd_fast_kernel(S
           const float2 f = unpack_bf16x2(w[i]);
           const int d = half * (HD / 2) + j * 8 + 2 * i;
 #pragma unroll
-          for (int qi = 0; qi < kSumFwdMaxQ; ++qi)
+          for (int qi = 0; qi < NQ; ++qi)
             if (qi < nq) acc[qi] += q_s[qi * HD + d] * f.x + q_s[qi * HD + d + 1] * f.y;
         }
       }
 #pragma unroll
-      for (int qi = 0; qi < kSumFwdMaxQ; ++qi) {
+      for (int qi = 0; qi < NQ; ++qi) {
         if (qi < nq) {
           const float sc = acc[qi] + __shfl_xor_sync(0xffffffffu, acc[qi], 1);
           // summary query j sees the chunk's text keys and summary keys 0..j
@@ -319,6 +322,7 @@ __global__ void __launch_bounds__(kSumFwdThreads) summary_attn_fwd_fast_kernel(S
     const uint32_t* vcol = reinterpret_cast<const uint32_t*>(v_s) + d2;
     const float* pr = p_s + qi * nk_max;
     float o0 = 0.f, o1 = 0.f;
+#pragma unroll 8
     for (int kk = 0; kk < nk_all; ++kk) {
       const float2 f = unpack_bf16x2(vcol[(size_t)kk * (HD / 2)]);
       o0 = fmaf(pr[kk], f.x, o0);
@@ -338,11 +342,11 @@ __global__ void __launch_bounds__(kSumFwdThreads) summary_attn_fwd_fast_kernel(S
 constexpr int kSumBwdThreads = 256;
 constexpr int kSumBwdMaxQ = 8;
 
-template <int HD>
+template <int HD, int NQ>      // NQ as in the forward kernel
 __global__ void __launch_bounds__(kSumBwdThreads) summary_attn_bwd_fast_kernel(SumAttnArgs a, int nk_max) {
   extern __shared__ uint32_t smw[];
   constexpr int kRowElems = HD + 8;                   // padded K row, bf16 elements
-  const int G = a.Hq / a.Hkv, S = a.n_sum, nq = G * S;
+  const int G = a.Hq / a.Hkv, S = a.n_sum, nq = NQ < kSumBwdMaxQ ? NQ : G * S;
   bf16* k_s = reinterpret_cast<bf16*>(smw);
   float* q_s = reinterpret_cast<float*>(k_s + (size_t)nk_max * kRowElems);
   float* do_s = q_s + nq * HD;
@@ -406,9 +410,9 @@ __global__ void __launch_bounds__(kSumBwdThreads) summary_attn_bwd_fast_kernel(S
       uint4 uv[HD / 16];
 #pragma unroll
       for (int j = 0; j < HD / 16; ++j) uv[j] = valid ? *reinterpret_cast<const uint4*>(vrow + j * 8) : make_uint4(0, 0, 0, 0);
-      float sc[kSumBwdMaxQ], dp[kSumBwdMaxQ];
+      float sc[NQ], dp[NQ];
 #pragma unroll
-      for (int qi = 0; qi < kSumBwdMaxQ; ++qi) { sc[qi] = 0.f; dp[qi] = 0.f; }
+      for (int qi = 0; qi < NQ; ++qi) { sc[qi] = 0.f; dp[qi] = 0.f; }
 #pragma unroll
       for (int j = 0; j < HD / 16; ++j) {
         const uint4 uk = *reinterpret_cast<const uint4*>(krow + j * 8);
@@ -418,7 +422,7 @@ __global__ void __launch_bounds__(kSumBwdThreads) summary_attn_bwd_fast_kernel(S
           const float2 fk = unpack_bf16x2(wk[i]), fv = unpack_bf16x2(wv[i]);
           const int d = half * (HD / 2) + j * 8 + 2 * i;
 #pragma unroll
-          for (int qi = 0; qi < kSumBwdMaxQ; ++qi)
+          for (int qi = 0; qi < NQ; ++qi)
             if (qi < nq) {
               sc[qi] += q_s[qi * HD + d] * fk.x + q_s[qi * HD + d + 1] * fk.y;
               dp[qi] += do_s[qi * HD + d] * fv.x + do_s[qi * HD + d + 1] * fv.y;
@@ -426,7 +430,7 @@ __global__ void __launch_bounds__(kSumBwdThreads) summary_attn_bwd_fast_kernel(S
         }
       }
 #pragma unroll
-      for (int qi = 0; qi < kSumBwdMaxQ; ++qi) {
+      for (int qi = 0; qi < NQ; ++qi) {
         if (qi < nq) {
           const float s2 = sc[qi] + __shfl_xor_sync(0xffffffffu, sc[qi], 1);
           const float d2 = dp[qi] + __shfl_xor_sync(0xffffffffu, dp[qi], 1);
@@ -447,6 +451,7 @@ __global__ void __launch_bounds__(kSumBwdThreads) summary_attn_bwd_fast_kernel(S
     const uint32_t* kcol = reinterpret_cast<const uint32_t*>(k_s) + d2;
     const float* dsr = ds_s + qi * nk_max;
     float g0 = 0.f, g1 = 0.f;
+#pragma unroll 8
     for (int kk = 0; kk < nk_all; ++kk) {
       const float2 f = unpack_bf16x2(kcol[(size_t)kk * (kRowElems / 2)]);
       g0 = fmaf(dsr[kk], f.x, g0);
@@ -463,7 +468,9 @@ __global__ void __launch_bounds__(kSumBwdThreads) summary_attn_bwd_fast_kernel(S
     float gk[8], gv[8];
 #pragma unroll
     for (int e = 0; e < 8; ++e) { gk[e] = 0.f; gv[e] = 0.f; }
-    for (int qi = 0; qi < nq; ++qi) {
+#pragma unroll
+    for (int qi = 0; qi < NQ; ++qi) {
+      if (qi >= nq) break;
       const float dsv = ds_s[qi * nk_max + kk], pv = p_s[qi * nk_max + kk];
 #pragma unroll
       for (int e = 0; e < 8; ++e) {
@@ -505,6 +512,32 @@ __global__ void __launch_bounds__(kSumBwdThreads) summary_attn_bwd_fast_kernel(S
   }
 }
 
+template <int NQ>
+static int launch_fwd_fast(const SumAttnArgs& a, int nk_max, size_t smem, cudaStream_t st) {
+  auto kern = summary_attn_fwd_fast_kernel<128, NQ>;
+  static bool attr = false;
+  if (!attr) {
+    KSA_CHECK_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, 100 * 1024));
+    attr = true;
+  }
+  kern<<<dim3(a.Nq / a.n_sum, a.Hkv, a.B), kSumFwdThreads, smem, st>>>(a, nk_max);
+  KSA_CHECK_CUDA(cudaGetLastError());
+  return 0;
+}
+
+template <int NQ>
+static int launch_bwd_fast(const SumAttnArgs& a, int nk_max, size_t smem, cudaStream_t st) {
+  auto kern = summary_attn_bwd_fast_kernel<128, NQ>;
+  static bool attr = false;
+  if (!attr) {
+    KSA_CHECK_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, 100 * 1024));
+    attr = true;
+  }
+  kern<<<dim3(a.Nq / a.n_sum, a.Hkv, a.B), kSumBwdThreads, smem, st>>>(a, nk_max);
+  KSA_CHECK_CUDA(cudaGetLastError());
+  return 0;
+}
+
 }  // namespace ksa
 
 using namespace ksa;
@@ -529,16 +562,11 @@ KSA_API int ksa_summary_attn_fwd(const void* qs, const void* k, const void* v, c
     const int nq = (Hq / Hkv) * n_sum, nk_max = chunk + n_sum;
     const size_t fast_smem = (size_t)nk_max * HD * sizeof(bf16) + (size_t)nq * (HD + nk_max) * sizeof(float);
     if (HD == 128 && nq <= kSumFwdMaxQ && fast_smem <= 100 * 1024 && os_rs % 2 == 0) {
-      static bool attr = false;
-      if (!attr) {
-        KSA_CHECK_CUDA(cudaFuncSetAttribute(summary_attn_fwd_fast_kernel<128>,
-                                            cudaFuncAttributeMaxDynamicSharedMemorySize, 100 * 1024));
-        attr = true;
-      }
-      dim3 fgrid(Nq / n_sum, Hkv, B);
-      summary_attn_fwd_fast_kernel<128><<<fgrid, kSumFwdThreads, fast_smem, reinterpret_cast<cudaStream_t>(stream)>>>(a, nk_max);
-      KSA_CHECK_CUDA(cudaGetLastError());
-      return 0;
+      cudaStream_t st = reinterpret_cast<cudaStream_t>(stream);
+      if (nq == 1) return launch_fwd_fast<1>(a, nk_max, fast_smem, st);
+      if (nq == 2) return launch_fwd_fast<2>(a, nk_max, fast_smem, st);
+      if (nq == 4) return launch_fwd_fast<4>(a, nk_max, fast_smem, st);
+      return launch_fwd_fast<kSumFwdMaxQ>(a, nk_max, fast_smem, st);
     }
   }
   const size_t smem = (size_t)(HD + chunk + n_sum) * sizeof(float);
@@ -578,16 +606,11 @@ KSA_API int ksa_summary_attn_bwd(const void* qs, const void* k, const void* v, c
     const int nk_max = chunk + n_sum;
     const size_t fast_smem = (size_t)nk_max * (HD + 8) * sizeof(bf16) + (size_t)nq * (2 * HD + 2 * nk_max + 2) * sizeof(float);
     if (HD == 128 && nq <= kSumBwdMaxQ && fast_smem <= 100 * 1024 && dqs_rs % 2 == 0) {
-      static bool fattr = false;
-      if (!fattr) {
-        KSA_CHECK_CUDA(cudaFuncSetAttribute(summary_attn_bwd_fast_kernel<128>,
-                                            cudaFuncAttributeMaxDynamicSharedMemorySize, 100 * 1024));
-        fattr = true;
-      }
-      dim3 fgrid(Nq / n_sum, Hkv, B);
-      summary_attn_bwd_fast_kernel<128><<<fgrid, kSumBwdThreads, fast_smem, reinterpret_cast<cudaStream_t>(stream)>>>(a, nk_max);
-      KSA_CHECK_CUDA(cudaGetLastError());
-      return 0;
+      cudaStream_t st = reinterpret_cast<cudaStream_t>(stream);
+      if (nq == 1) return launch_bwd_fast<1>(a, nk_max, fast_smem, st);
+      if (nq == 2) return launch_bwd_fast<2>(a, nk_max, fast_smem, st);
+      if (nq == 4) return launch_bwd_fast<4>(a, nk_max, fast_smem, st);
+      return launch_bwd_fast<kSumBwdMaxQ>(a, nk_max, fast_smem, st);
     }
   }
   const size_t smem = (size_t)nq * (2 * HD + 2 * (chunk + n_sum)) * sizeof(float);
