@@ -523,36 +523,48 @@ attn_bwd_fused_cp_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_c
   attn_bwd_fused_body<true>(tmQ, tmdO, cp.src.kt[1], cp.src.vt[1], cp.src.ks[0], cp.src.vs[0], tmDq, p, &cp);
 }
 
-// Preparation: one warp per (batch, head, query row of the padded length).  Writes -LSE*log2e and
-// -delta = -rowsum(O * dO) into the two planes of `stats` (rows past Lq: -inf and 0, so that P = 0 there) and
-// zeroes the row of the fp32 dQ buffer.
-__global__ void attn_bwd_prep_kernel(const bf16* __restrict__ o, const bf16* __restrict__ d_o, long long o_rs,
-                                     long long o_bs, const float* __restrict__ lse, float* __restrict__ stats,
-                                     float* __restrict__ dq32, int B, int Hq, int Lq, int lq_pad) {
-  const long long w = ((long long)blockIdx.x * blockDim.x + threadIdx.x) >> 5;
-  const int lane = threadIdx.x & 31;
+// Preparation: half a warp per (batch, query row of the padded length, head), heads of a row next to one another as they
+// lie in memory.  Writes -LSE*log2e and -delta = -rowsum(O * dO) into the two planes of `stats` (rows past Lq: -inf and
+// 0, so that P = 0 there) and zeroes the row of the fp32 dQ buffer.  Bound by the memory (134 MB at 8192 x 16 heads: 35.3 us with a warp per row
+// and 8-byte loads that walked down one head's column, 23.4 us so).
+__global__ void __launch_bounds__(256)
+attn_bwd_prep_kernel(const bf16* __restrict__ o, const bf16* __restrict__ d_o, long long o_rs, long long o_bs,
+                     const float* __restrict__ lse, float* __restrict__ stats, float* __restrict__ dq32, int B, int Hq,
+                     int Lq, int lq_pad) {
+  const long long item = ((long long)blockIdx.x * blockDim.x + threadIdx.x) >> 4;
+  const int l16 = threadIdx.x & 15;
   const long long rows = (long long)B * Hq * lq_pad;
-  if (w >= rows) return;
-  const int q = (int)(w % lq_pad);
-  const int head = (int)((w / lq_pad) % Hq);
-  const int b = (int)(w / ((long long)lq_pad * Hq));
-  float nl = -INFINITY, nd = 0.f;
-  if (q < Lq) {
-    const long long off = (long long)b * o_bs + (long long)q * o_rs + (long long)head * 128 + lane * 4;
-    const uint2 a = *reinterpret_cast<const uint2*>(o + off);
-    const uint2 g = *reinterpret_cast<const uint2*>(d_o + off);
-    const float2 a0 = unpack_bf16x2(a.x), a1 = unpack_bf16x2(a.y), g0 = unpack_bf16x2(g.x), g1 = unpack_bf16x2(g.y);
-    const float part = a0.x * g0.x + a0.y * g0.y + a1.x * g1.x + a1.y * g1.y;
-    nd = -warp_sum(part);
-    const float l = lse[((long long)b * Hq + head) * Lq + q];
-    nl = (l == -INFINITY) ? -INFINITY : -l * 1.4426950408889634f;
-    // a query row without any visible key has LSE = -inf: P must be 0, not exp2(+inf)
-    if (l == -INFINITY) nl = -INFINITY;
-    *reinterpret_cast<float4*>(dq32 + (((long long)b * Lq + q) * Hq + head) * 128 + lane * 4) = make_float4(0.f, 0.f, 0.f, 0.f);
+  const bool live = item < rows;               // the lanes of the other half still take part in the sum below
+  const long long bq = live ? item / Hq : 0;
+  const int head = live ? (int)(item - bq * Hq) : 0;
+  const int b = (int)(bq / lq_pad), q = (int)(bq - (long long)b * lq_pad);
+  float part = 0.f;
+  if (live && q < Lq) {
+    const long long off = (long long)b * o_bs + (long long)q * o_rs + (long long)head * 128 + l16 * 8;
+    const uint4 a = *reinterpret_cast<const uint4*>(o + off);
+    const uint4 g = *reinterpret_cast<const uint4*>(d_o + off);
+    const uint32_t au[4] = {a.x, a.y, a.z, a.w}, gu[4] = {g.x, g.y, g.z, g.w};
+#pragma unroll
+    for (int i = 0; i < 4; ++i) {
+      const float2 x = unpack_bf16x2(au[i]), y = unpack_bf16x2(gu[i]);
+      part += x.x * y.x + x.y * y.y;
+    }
+    float4* z = reinterpret_cast<float4*>(dq32 + (((long long)b * Lq + q) * Hq + head) * 128 + l16 * 8);
+    z[0] = make_float4(0.f, 0.f, 0.f, 0.f);
+    z[1] = make_float4(0.f, 0.f, 0.f, 0.f);
   }
-  if (lane == 0) {
-    stats[w] = nl;
-    stats[rows + w] = nd;
+#pragma unroll
+  for (int s = 8; s > 0; s >>= 1) part += __shfl_xor_sync(0xffffffffu, part, s);
+  if (live && l16 == 0) {
+    const long long at = ((long long)b * Hq + head) * lq_pad + q;
+    float nl = -INFINITY;
+    if (q < Lq) {
+      // a query row without any visible key has LSE = -inf: P must be 0, not exp2(+inf)
+      const float l = lse[((long long)b * Hq + head) * Lq + q];
+      if (l != -INFINITY) nl = -l * 1.4426950408889634f;
+    }
+    stats[at] = nl;
+    stats[rows + at] = q < Lq ? -part : 0.f;
   }
 }
 
@@ -651,9 +663,9 @@ KSA_API int ksa_attn_bwd_fused(const void* q, const void* k, const void* v, cons
     attr = true;
   }
   {
-    const long long warps = (long long)B * Hq * lq_pad;
+    const long long items = (long long)B * Hq * lq_pad;
     const int threads = 256;
-    const long long blocks = (warps * 32 + threads - 1) / threads;
+    const long long blocks = (items * 16 + threads - 1) / threads;
     attn_bwd_prep_kernel<<<(unsigned)blocks, threads, 0, st>>>((const bf16*)o, (const bf16*)d_o, o_rs, o_bs,
                                                                (const float*)lse, (float*)stats, (float*)dq32, B, Hq,
                                                                Lq, lq_pad);
@@ -764,9 +776,9 @@ KSA_API int ksa_attn_bwd_fused_cp(const void* q, const void* o, const void* d_o,
     attr = true;
   }
   {
-    const long long warps = (long long)B * Hq * lq_pad;
+    const long long items = (long long)B * Hq * lq_pad;
     const int threads = 256;
-    attn_bwd_prep_kernel<<<(unsigned)((warps * 32 + threads - 1) / threads), threads, 0, st>>>(
+    attn_bwd_prep_kernel<<<(unsigned)((items * 16 + threads - 1) / threads), threads, 0, st>>>(
         (const bf16*)o, (const bf16*)d_o, o_rs, o_bs, (const float*)lse, (float*)stats, (float*)dq32, B, Hq, Lq, lq_pad);
     KSA_CHECK_CUDA(cudaGetLastError());
   }
