@@ -1,0 +1,329 @@
+// bf16 GEMM for few activation rows: C[M, N] = X[M, K] * W^T, M from a batch of decoding sequences to some hundred rows
+// of a prompt.  Such a product has too few 128- or 256-row tiles to occupy the chip (48 x 2560 is ten tiles of 128 x 256) and is
+// bound by how many SMs stream the weights, so
+//   * the weights take the 128-row side of the MMA and the activation rows its N side: a tile is 128 weight rows by
+//     `bt` activation rows (a multiple of 16 up to 256), and nothing is staged or multiplied for absent rows;
+//   * K is split over the `split` CTAs of a cluster (1, 2, 4 or 8).  Each leaves its fp32 partial tile in its shared
+//     memory, and the cluster adds the parts in rank order (the same order every time) through distributed shared
+//     memory, each CTA a share of the rows: no workspace, no atomics, no second launch.
+// Measured against 128 x 256 tiles on single CTAs (weights from memory): 48 rows x 2560 x 9728 60.2 -> 18.1 us, 333 rows 61.3 ->
+// 29.5, 48 rows x 6144 x 2560 20.1 -> 13.7; with the activation, 48 rows x 19456 x 2560 36.2 -> 23.1 (two launches -> one).
+// The weights alone take 7.6, 7.6, 4.8 and 15.2 us at the copy bandwidth.
+// Roles per CTA (192 threads): warp 0 TMA producer, warp 1 MMA issuer, warps 2..5 move the accumulator to shared
+// memory, and all of them write the result.  One tile per CTA.  No TMA load uses multicast; every wait is bounded.
+//
+// kGlu: W holds F gate rows followed by F up rows, a tile is 64 features (64 gate rows and the matching 64 up rows) and
+// C[M, F] = silu(gate) * up, with gate and up rounded to bf16 first as separate projection and activation kernels do.
+#include "common.cuh"
+#include "host.h"
+
+namespace ksa {
+
+constexpr int kNwThreads = 192;
+constexpr int kNwBK = 64;
+constexpr int kNwWBytes = 128 * kNwBK * 2;
+constexpr int kNwMaxStages = 8;
+
+struct NarrowArgs {
+  bf16* c;
+  long long ldc;
+  int M, N, K;               // N: rows of W
+  int bt, split, stages, tiles_m, tmem_cols;
+  float alpha;
+};
+
+__device__ __forceinline__ uint32_t nw_cluster_rank() {
+  uint32_t r;
+  asm volatile("mov.u32 %0, %%cluster_ctarank;" : "=r"(r));
+  return r;
+}
+__device__ __forceinline__ void nw_cluster_sync() {
+  asm volatile("barrier.cluster.arrive.release.aligned;\n\tbarrier.cluster.wait.acquire.aligned;" ::: "memory");
+}
+__device__ __forceinline__ float4 nw_ld_cluster(uint32_t local_addr, uint32_t rank) {
+  float4 v;
+  asm volatile("{\n\t.reg .u32 a;\n\tmapa.shared::cluster.u32 a, %4, %5;\n\t"
+               "ld.shared::cluster.v4.f32 {%0, %1, %2, %3}, [a];\n\t}"
+               : "=f"(v.x), "=f"(v.y), "=f"(v.z), "=f"(v.w)
+               : "r"(local_addr), "r"(rank)
+               : "memory");
+  return v;
+}
+
+template <bool W_MN, bool kGlu>
+__global__ void __launch_bounds__(kNwThreads)
+gemm_narrow_kernel(const __grid_constant__ CUtensorMap tmW, const __grid_constant__ CUtensorMap tmX, const NarrowArgs p,
+                   int* status) {
+  extern __shared__ uint8_t smem_raw[];
+  uint8_t* smem = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~uintptr_t(1023));
+  __shared__ uint64_t full[kNwMaxStages], empty[kNwMaxStages], acc_full;
+  __shared__ uint32_t tmem_slot;
+  __shared__ int abort_word;
+
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  const int rank = (int)nw_cluster_rank();
+  const int tile = (int)blockIdx.x / p.split;
+  const int mb = tile % p.tiles_m, nb = tile / p.tiles_m;   // tiles that share weights are neighbours
+  const int m0 = mb * p.bt;
+  const int num_kb = (p.K + kNwBK - 1) / kNwBK;
+  const int kb0 = (int)((long long)num_kb * rank / p.split), kb1 = (int)((long long)num_kb * (rank + 1) / p.split);
+  const int stage_bytes = kNwWBytes + p.bt * kNwBK * 2;
+  const int n_out = kGlu ? p.N / 2 : p.N;
+  const int row0 = nb * (kGlu ? 64 : 128);                  // first weight rows of the two halves of the tile
+  const int row1 = kGlu ? n_out + row0 : row0 + 64;
+  const WaitGuard guard{&abort_word, status};
+
+  if (threadIdx.x == 0) {
+    for (int i = 0; i < p.stages; ++i) { mbar_init(&full[i], 1); mbar_init(&empty[i], 1); }
+    mbar_init(&acc_full, 1);
+    abort_word = 0;
+    fence_mbar_init();
+    tma_prefetch_desc(&tmW);
+    tma_prefetch_desc(&tmX);
+  }
+  if (warp == 2) { tmem_alloc(&tmem_slot, p.tmem_cols); tmem_relinquish(); }
+  tc_fence_before();
+  __syncthreads();
+  tc_fence_after();
+  const uint32_t tmem_base = tmem_slot;
+
+  if (warp == 0) {
+    if (lane == 0) {
+      int stage = 0;
+      uint32_t phase = 0;
+      for (int kb = kb0; kb < kb1; ++kb) {
+        if (!mbar_wait(&empty[stage], phase ^ 1, guard, kTimeoutStageEmpty)) break;
+        uint8_t* sw = smem + stage * stage_bytes;
+        mbar_expect_tx(&full[stage], stage_bytes);
+        if (!W_MN) {
+          tma_load_2d(sw, &tmW, kb * kNwBK, row0, &full[stage]);
+          tma_load_2d(sw + 8192, &tmW, kb * kNwBK, row1, &full[stage]);
+        } else {
+          tma_load_2d(sw, &tmW, row0, kb * kNwBK, &full[stage]);
+          tma_load_2d(sw + 8192, &tmW, row1, kb * kNwBK, &full[stage]);
+        }
+        tma_load_2d(sw + kNwWBytes, &tmX, kb * kNwBK, m0, &full[stage]);
+        if (++stage == p.stages) { stage = 0; phase ^= 1; }
+      }
+    }
+    __syncwarp();
+  } else if (warp == 1) {
+    if (lane == 0) {
+      const uint32_t idesc = umma_idesc_bf16(128, p.bt, W_MN ? 1 : 0, 0);
+      int stage = 0;
+      uint32_t phase = 0;
+      bool ok = true;
+      for (int kb = kb0; kb < kb1; ++kb) {
+        if (!mbar_wait(&full[stage], phase, guard, kTimeoutTmaFull)) { ok = false; break; }
+        tc_fence_after();
+        const uint32_t sw = smem_u32(smem + stage * stage_bytes), sx = sw + kNwWBytes;
+#pragma unroll
+        for (int k = 0; k < kNwBK / 16; ++k) {
+          const uint64_t dw = W_MN ? smem_desc_mnmajor_sw128(sw + k * 2048, 8192) : smem_desc_kmajor_sw128(sw + k * 32);
+          umma_ss(tmem_base, dw, smem_desc_kmajor_sw128(sx + k * 32), idesc, (kb != kb0 || k != 0) ? 1u : 0u);
+        }
+        umma_commit(&empty[stage]);
+        if (++stage == p.stages) { stage = 0; phase ^= 1; }
+      }
+      if (ok) umma_commit(&acc_full);
+    }
+    __syncwarp();
+  } else {
+    // every MMA has read its operands once acc_full completes, so the ring can hold the partial tile [bt][128]
+    const int quad = warp & 3;
+    if (mbar_wait(&acc_full, 0, guard, kTimeoutAccFull)) {
+      __syncwarp();
+      tc_fence_after();
+      float* part = reinterpret_cast<float*>(smem) + quad * 32 + lane;
+      const uint32_t t_row = tmem_base + ((uint32_t)(quad * 32) << 16);
+      for (int c = 0; c < p.bt; c += 16) {
+        uint32_t r[16];
+        tmem_ld16(t_row + c, r);
+        tmem_wait_ld();
+#pragma unroll
+        for (int j = 0; j < 16; ++j) part[(c + j) * 128] = __uint_as_float(r[j]);
+      }
+    }
+    __syncwarp();
+  }
+  tc_fence_before();
+  __syncthreads();
+  nw_cluster_sync();
+
+  // this CTA's share of the rows, the parts added in rank order
+  const int share = (p.bt + p.split - 1) / p.split;
+  const int r_lo = rank * share, r_hi = min(min(r_lo + share, p.bt), p.M - m0);
+  constexpr int kPerRow = kGlu ? 8 : 16;                    // 8 outputs per thread
+  const uint32_t part0 = smem_u32(smem);
+  for (int i = r_lo * kPerRow + (int)threadIdx.x; i < r_hi * kPerRow; i += kNwThreads) {
+    const int m = i / kPerRow, n8 = (i % kPerRow) * 8;
+    if (row0 + n8 >= n_out) continue;
+    constexpr int kVecs = kGlu ? 4 : 2;
+    float4 s[kVecs];
+#pragma unroll
+    for (int v = 0; v < kVecs; ++v) s[v] = make_float4(0.f, 0.f, 0.f, 0.f);
+    for (int r = 0; r < p.split; ++r) {
+#pragma unroll
+      for (int v = 0; v < kVecs; ++v) {
+        const float4 x = nw_ld_cluster(part0 + (m * 128 + n8 + (v >> 1) * 64 + (v & 1) * 4) * 4, r);
+        s[v].x += x.x; s[v].y += x.y; s[v].z += x.z; s[v].w += x.w;
+      }
+    }
+    float o[8] = {s[0].x, s[0].y, s[0].z, s[0].w, s[1].x, s[1].y, s[1].z, s[1].w};
+    if (kGlu) {
+      const float u[8] = {s[kVecs - 2].x, s[kVecs - 2].y, s[kVecs - 2].z, s[kVecs - 2].w,
+                          s[kVecs - 1].x, s[kVecs - 1].y, s[kVecs - 1].z, s[kVecs - 1].w};
+#pragma unroll
+      for (int j = 0; j < 8; ++j) {
+        const float g = __bfloat162float(__float2bfloat16(o[j])), up = __bfloat162float(__float2bfloat16(u[j]));
+        o[j] = g / (1.f + __expf(-g)) * up;
+      }
+    } else {
+#pragma unroll
+      for (int j = 0; j < 8; ++j) o[j] *= p.alpha;
+    }
+    uint4 v;
+    v.x = pack_bf16x2(o[0], o[1]); v.y = pack_bf16x2(o[2], o[3]);
+    v.z = pack_bf16x2(o[4], o[5]); v.w = pack_bf16x2(o[6], o[7]);
+    *reinterpret_cast<uint4*>(p.c + (long long)(m0 + m) * p.ldc + row0 + n8) = v;
+  }
+  nw_cluster_sync();          // nobody leaves while its part may still be read
+  if (warp == 2) {
+    tc_fence_after();
+    tmem_dealloc(tmem_base, p.tmem_cols);
+  }
+}
+
+// Tile height and split for a product, and its time in microseconds as modelled.  The figures were fitted to 315 measured
+// (shape, height, split) triples of 17 to 1411 rows against 4096 x 2048 .. 19456 x 2560 weights (standard deviation 5 %, the
+// choice within 3 % of the best one measured for nearly all of them):
+//   * one 64-wide step of K takes a CTA that has an SM to itself 0.32 us (the latency of its loads) and two that share
+//     one 2 x (0.142 + 0.00044 bt), so a grid should fill both slots of every SM; a ring for more than 160 rows leaves
+//     room for one CTA only;
+//   * the weights of all CTAs come through the L2 at 13.7 TB/s;
+//   * a launch costs 1.5 us, a wave of CTAs 4.6 us to start and drain, and 0.0126 + 0.0045 split per activation row to write
+//     and add up.
+constexpr int kNwSms = 148;
+constexpr int kNwMaxRows = 2048;   // the model holds near the range that it was fitted to (8000 x 128 x 2048: 27.4 against 15.3 us)
+static bool narrow_two_per_sm(int bt) { return 3 * (kNwWBytes + bt * kNwBK * 2) <= 110 * 1024; }
+static int narrow_stages(int bt) {
+  const int stages = (narrow_two_per_sm(bt) ? 110 : 220) * 1024 / (kNwWBytes + bt * kNwBK * 2);
+  return stages < kNwMaxStages ? stages : kNwMaxStages;
+}
+static double narrow_plan(int M, long long n_tiles, int K, int* bt_out, int* split_out) {
+  const int num_kb = (K + kNwBK - 1) / kNwBK, fewest = (M + 255) / 256;
+  double best = 1e30;
+  for (int tm = fewest; tm < fewest + 9; ++tm) {
+    const int bt = ((M + tm - 1) / tm + 15) / 16 * 16;
+    if (tm > fewest && bt < 48) break;
+    const int slots = kNwSms * (narrow_two_per_sm(bt) ? 2 : 1);
+    for (int split = 1; split <= 8 && split <= num_kb; split *= 2) {
+      const long long ctas = (long long)((M + bt - 1) / bt) * n_tiles * split;
+      const double steps = (num_kb + split - 1) / split;
+      auto wave = [&](long long n) {
+        if (n == 0) return 0.0;
+        const double per_sm = (double)((n + kNwSms - 1) / kNwSms);
+        double step = per_sm * (0.142 + 0.00044 * bt);
+        if (step < 0.32 + 0.00027 * bt) step = 0.32 + 0.00027 * bt;
+        if (step < n * 0.00122) step = n * 0.00122;
+        return 4.6 + steps * step + per_sm * bt * (0.0126 + (split > 1 ? 0.0045 * split : 0.0)) + (split == 8 ? 0.26 : 0.0);
+      };
+      const double t = 1.5 + (double)(ctas / slots) * wave(slots) + wave(ctas % slots);
+      if (t < best) { best = t; *bt_out = bt; *split_out = split; }
+    }
+  }
+  return best;
+}
+// The other kernels' time for the same product: 0.345 us a 64-wide step and wave of 74 CTA pairs with 256 x 256 tiles, 0.38 a
+// step and wave of 128 x 256 tiles on single CTAs, 5 us around them (17.5 us measured for 128 x 12288 x 2048, 55.3 for 1411 x 2560 x 9728,
+// 61 for 48 to 700 x 2560 x 9728 on single CTAs).
+static double tiled_time(int M, int N, int K, int pair_min_tiles) {
+  const long long num_kb = (K + 63) / 64, tn = (N + 255) / 256, pairs = (M + 255) / 256 * tn;
+  if (pair_min_tiles > 0 && pairs >= pair_min_tiles) return 5.0 + 0.345 * num_kb * ((pairs + kNwSms / 2 - 1) / (kNwSms / 2));
+  return 5.0 + 0.38 * num_kb * (((M + 127) / 128 * tn + kNwSms - 1) / kNwSms);
+}
+
+template <bool W_MN, bool kGlu>
+static int launch_narrow(const void* x, const void* w, NarrowArgs p, long long ldx, long long ldw, cudaStream_t st) {
+  CUtensorMap tmX, tmW;
+  int rc;
+  {
+    uint64_t dims[2] = {(uint64_t)p.K, (uint64_t)p.M};
+    uint64_t str[2] = {2, (uint64_t)ldx * 2};
+    uint32_t box[2] = {kNwBK, (uint32_t)p.bt};
+    if ((rc = make_tmap(&tmX, x, 2, 2, dims, str, box, true))) return rc;
+  }
+  {
+    uint64_t dims[2] = {(uint64_t)(W_MN ? p.N : p.K), (uint64_t)(W_MN ? p.K : p.N)};
+    uint64_t str[2] = {2, (uint64_t)ldw * 2};
+    uint32_t box[2] = {64, 64};
+    if ((rc = make_tmap(&tmW, w, 2, 2, dims, str, box, true))) return rc;
+  }
+  // two CTAs per SM while a ring of three stages fits half of its shared memory, else one with a deeper ring
+  p.stages = narrow_stages(p.bt);
+  const int part_bytes = p.bt * 128 * 4;
+  const int ring = p.stages * (kNwWBytes + p.bt * kNwBK * 2);
+  const int smem = (ring > part_bytes ? ring : part_bytes) + 1024;
+  p.tmem_cols = 32;
+  while (p.tmem_cols < p.bt) p.tmem_cols *= 2;
+  p.tiles_m = (p.M + p.bt - 1) / p.bt;
+  const int n_tile = kGlu ? 64 : 128, n_out = kGlu ? p.N / 2 : p.N;
+  const int tiles = p.tiles_m * ((n_out + n_tile - 1) / n_tile);
+  auto kern = gemm_narrow_kernel<W_MN, kGlu>;
+  static bool attr_set = false;
+  if (!attr_set) {
+    KSA_CHECK_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, 222 * 1024));
+    attr_set = true;
+  }
+  int* status = status_word();
+  KSA_REQUIRE(status != nullptr, "could not allocate the status word");
+  cudaLaunchConfig_t cfg = {};
+  cfg.gridDim = dim3(tiles * p.split);
+  cfg.blockDim = dim3(kNwThreads);
+  cfg.dynamicSmemBytes = smem;
+  cfg.stream = st;
+  cudaLaunchAttribute at[1];
+  at[0].id = cudaLaunchAttributeClusterDimension;
+  at[0].val.clusterDim.x = p.split;
+  at[0].val.clusterDim.y = 1;
+  at[0].val.clusterDim.z = 1;
+  cfg.attrs = at;
+  cfg.numAttrs = 1;
+  KSA_CHECK_CUDA(cudaLaunchKernelEx(&cfg, kern, tmW, tmX, p, status));
+  return 0;
+}
+
+}  // namespace ksa
+
+// C[M, N] (bf16) = alpha * X[M, K] * W^T; W is [N, K] row-major, or [K, N] with w_mn_major.  glu: W holds N/2 gate and N/2 up
+// rows (row-major only) and C[M, N/2] = silu(X gate^T) * (X up^T).  bt: activation rows per tile (multiple of 16 up to
+// 256), split: CTAs that share the reduction of a tile (1, 2, 4 or 8, at most one per 64 elements of K).
+KSA_API int ksa_gemm_narrow_bf16(const void* x, const void* w, void* c, int M, int N, int K, long long ldx, long long ldw,
+                                 long long ldc, int w_mn_major, int glu, int bt, int split, float alpha, void* stream) {
+  KSA_ENTER(x);
+  using namespace ksa;
+  KSA_REQUIRE(M > 0 && N > 0 && K > 0, "gemm_narrow: empty problem %d x %d x %d", M, N, K);
+  KSA_REQUIRE(ldx % 8 == 0 && ldw % 8 == 0, "gemm_narrow: ldx/ldw must be multiples of 8 elements (got %lld, %lld)", ldx, ldw);
+  KSA_REQUIRE(N % (glu ? 16 : 8) == 0 && ldc % 8 == 0, "gemm_narrow: N and ldc must keep 16-byte row alignment (N=%d ldc=%lld)", N, ldc);
+  KSA_REQUIRE((reinterpret_cast<uintptr_t>(c) & 15) == 0, "gemm_narrow: C must be 16-byte aligned");
+  KSA_REQUIRE(!(glu && w_mn_major), "gemm_narrow: the gated form takes row-major weights");
+  KSA_REQUIRE(bt >= 16 && bt <= 256 && bt % 16 == 0, "gemm_narrow: tile of %d rows (16 to 256, in steps of 16)", bt);
+  KSA_REQUIRE((split == 1 || split == 2 || split == 4 || split == 8) && split <= (K + kNwBK - 1) / kNwBK,
+              "gemm_narrow: K = %d in %d parts", K, split);
+  NarrowArgs p{};
+  p.c = static_cast<bf16*>(c); p.ldc = ldc; p.M = M; p.N = N; p.K = K; p.bt = bt; p.split = split; p.alpha = alpha;
+  cudaStream_t st = reinterpret_cast<cudaStream_t>(stream);
+  if (glu) return launch_narrow<false, true>(x, w, p, ldx, ldw, st);
+  return w_mn_major ? launch_narrow<true, false>(x, w, p, ldx, ldw, st) : launch_narrow<false, false>(x, w, p, ldx, ldw, st);
+}
+
+// Whether this kernel is expected to beat the tiled ones (of which CTA pairs are taken from `pair_min_tiles` 256 x 256 tiles on, 0:
+// never), by more than the model's error: bt * 16 + split for ksa_gemm_narrow_bf16, or 0.  glu: the separate activation
+// kernel, 2 us and more, counts on the other side.
+KSA_API int ksa_gemm_narrow_plan(int M, int N, int K, int glu, int pair_min_tiles) {
+  using namespace ksa;
+  if (M <= 0 || M > kNwMaxRows || N <= 0 || K <= 0) return 0;
+  int bt = 0, split = 0;
+  const double t = narrow_plan(M, glu ? (N / 2 + 63) / 64 : (N + 127) / 128, K, &bt, &split);
+  return t < 0.95 * (tiled_time(M, N, K, pair_min_tiles) + (glu ? 2.0 : 0.0)) ? bt * 16 + split : 0;
+}

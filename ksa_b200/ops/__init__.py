@@ -33,10 +33,16 @@ UNBOUNDED_WINDOW = 1 << 30
 # GEMMs with at least this many 256 x 256 tiles run on CTA pairs (tcgen05 cta_group::2, csrc/gemm2.cu; 74 pairs per
 # GPU); below that the single-CTA kernel with 128-row tiles has more CTAs to spread.  0 disables the pair kernel.
 GEMM_PAIR_MIN_TILES = int(__import__("os").environ.get("KSA_GEMM_PAIR_MIN_TILES", "32"))
-
-
 def _cuda(x: torch.Tensor) -> bool:
     return x.is_cuda
+
+
+def _narrow_swiglu(x: torch.Tensor, w13: torch.Tensor):
+    """Plan of the split-K kernel for few rows with the activation, or None.  It takes feature counts in steps of 8; tangents of
+    forward-mode differentiation, and a parameter gather that waits for a GEMM to ride in, are left to separate calls."""
+    if x.shape[0] <= 16 or w13.shape[0] % 16 != 0 or _lib.pair_gather_pending() or torch.autograd.forward_ad._current_level >= 0:
+        return None
+    return _lib.gemm_narrow_plan(x.shape[0], w13.shape[0], x.shape[1], 1, GEMM_PAIR_MIN_TILES)
 
 
 def _require_bf16(*ts):
@@ -83,6 +89,13 @@ def gemm(a: torch.Tensor, b: torch.Tensor, *, a_mn_major: bool = False, b_mn_maj
         # bandwidth-shaped kernel instead of 128-row tensor-core tiles
         _lib.call("ksa_gemv_bf16", a, b, out, M, N, K, a.stride(0), b.stride(0), out.stride(0))
         return out
+    if pair is None and sm_limit == 0 and not a_mn_major and out.dtype == torch.bfloat16 and not accumulate:
+        # too few tiles to occupy the chip: K is split as well (csrc/gemm_narrow.cu says when that is faster)
+        plan = _lib.gemm_narrow_plan(M, N, K, 0, GEMM_PAIR_MIN_TILES)
+        if plan is not None:
+            _lib.call("ksa_gemm_narrow_bf16", a, b, out, M, N, K, a.stride(0), b.stride(0), out.stride(0), int(b_mn_major), 0,
+                      plan[0], plan[1], float(alpha))
+            return out
     if pair is None:
         pair = (GEMM_PAIR_MIN_TILES > 0 and sm_limit == 0
                 and ((M + 255) // 256) * ((N + 255) // 256) >= GEMM_PAIR_MIN_TILES)
@@ -503,16 +516,22 @@ def swiglu(gate_up: torch.Tensor) -> torch.Tensor:
 
 
 def linear_swiglu(x: torch.Tensor, w13: torch.Tensor) -> torch.Tensor:
-    """``swiglu(x @ w13.T)`` with ``w13 = [gate rows | up rows]``.  For at most 16 rows on a GPU without autograd (a
-    decode step) the projection applies the activation itself (one kernel, ``ksa_gemv_swiglu_bf16``); everything else
-    is the projection followed by ``swiglu``."""
-    if (_cuda(x) and x.dim() == 2 and x.shape[0] <= 16 and x.dtype == torch.bfloat16 and w13.dtype == torch.bfloat16
+    """``swiglu(x @ w13.T)`` with ``w13 = [gate rows | up rows]``.  Without autograd on a GPU the projection of few rows (a
+    decode step, a short prompt) applies the activation itself: ``ksa_gemv_swiglu_bf16`` for at most 16 rows, the gated form of
+    ``ksa_gemm_narrow_bf16`` where ``gemm`` would take that kernel.  Everything else is the projection followed by
+    ``swiglu``."""
+    if (_cuda(x) and x.dim() == 2 and (x.shape[0] <= 16 or _narrow_swiglu(x, w13) is not None) and x.dtype == torch.bfloat16 and w13.dtype == torch.bfloat16
             and not (torch.is_grad_enabled() and (x.requires_grad or w13.requires_grad))
             and x.stride(1) == 1 and w13.stride(1) == 1 and x.shape[1] % 8 == 0 and x.stride(0) % 8 == 0
             and w13.stride(0) % 8 == 0 and w13.shape[0] % 2 == 0):
         M, K = x.shape
         N = w13.shape[0]
         out = torch.empty((M, N // 2), dtype=torch.bfloat16, device=x.device)
+        if M > 16:
+            bt, split = _narrow_swiglu(x, w13)
+            _lib.call("ksa_gemm_narrow_bf16", x, w13, out, M, N, K, x.stride(0), w13.stride(0), out.stride(0), 0, 1, bt, split,
+                      1.0)
+            return out
         _lib.call("ksa_gemv_swiglu_bf16", x, w13, out, M, N, K, x.stride(0), w13.stride(0), out.stride(0))
         return out
     return swiglu(linear(x, w13))

@@ -8,6 +8,7 @@ a machine with a GPU a missing library is an error, never a silent fallback.
 from __future__ import annotations
 
 import ctypes
+import functools
 import os
 import threading
 from pathlib import Path
@@ -26,6 +27,7 @@ _SIGNATURES: Dict[str, Sequence] = {
     "ksa_gemm2_bf16": [P, P, P, I, I, I, L, L, L, I, I, I, I, F, P],
     "ksa_gemm2_gather_bf16": [P, P, P, I, I, I, L, L, L, I, I, F, P, I, I, L, P, P, ctypes.c_uint, P, I, L, P],
     "ksa_gemm2_scatter_bf16": [P, P, I, I, I, L, L, L, P, I, I, P],
+    "ksa_gemm_narrow_bf16": [P, P, P, I, I, I, L, L, L, I, I, I, I, F, P],
     "ksa_gemv_bf16": [P, P, P, I, I, I, L, L, L, P],
     "ksa_gemv_swiglu_bf16": [P, P, P, I, I, I, L, L, L, P],
     "ksa_gemv_norm_bf16": [P, P, P, P, P, P, I, I, I, L, L, L, L, L, F, I, I, P],
@@ -95,6 +97,8 @@ def load() -> ctypes.CDLL:
     lib.ksa_rmsnorm_bwd_parts.restype = I
     lib.ksa_attn_bwd_num_segments.argtypes = [I]
     lib.ksa_attn_bwd_num_segments.restype = I
+    lib.ksa_gemm_narrow_plan.argtypes = [I] * 5
+    lib.ksa_gemm_narrow_plan.restype = I
     lib.ksa_set_dependent_launch.argtypes = [I]
     lib.ksa_set_dependent_launch.restype = I
     for name, sig in _SIGNATURES.items():
@@ -228,6 +232,13 @@ def set_dependent_launch(on: bool) -> bool:
     while its predecessor on the stream still runs and waits for it on the device) on or off; returns the previous
     setting.  The inference engine switches it on around a decode step; training leaves it off."""
     return load().ksa_set_dependent_launch(1 if on else 0) != 0
+
+
+@functools.lru_cache(maxsize=4096)
+def gemm_narrow_plan(M: int, N: int, K: int, glu: int, pair_min_tiles: int):
+    """``(activation rows per tile, split of K)`` for ``ksa_gemm_narrow_bf16``, or None where a tiled kernel is faster."""
+    plan = load().ksa_gemm_narrow_plan(M, N, K, glu, pair_min_tiles)
+    return (plan // 16, plan % 16) if plan else None
 
 
 GATHER_COUNTERS = 32   # int32 completion counters a ``ksa_gemm2_gather_bf16`` launch uses (8 shards x 4 segments)
