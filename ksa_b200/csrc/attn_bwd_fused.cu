@@ -525,8 +525,8 @@ attn_bwd_fused_cp_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_c
 
 // Preparation: half a warp per (batch, query row of the padded length, head), heads of a row next to one another as they
 // lie in memory.  Writes -LSE*log2e and -delta = -rowsum(O * dO) into the two planes of `stats` (rows past Lq: -inf and
-// 0, so that P = 0 there) and zeroes the row of the fp32 dQ buffer.  Bound by the memory (134 MB at 8192 x 16 heads: 35.3 us with a warp per row
-// and 8-byte loads that walked down one head's column, 23.4 us so).
+// 0, so that P = 0 there) and zeroes the row of the fp32 dQ buffer.  Bound by the memory (134 MB at 8192 x
+// 16 heads: 35.3 us with a warp per row and 8-byte loads that walked down one head's column, 23.4 us so).
 __global__ void __launch_bounds__(256)
 attn_bwd_prep_kernel(const bf16* __restrict__ o, const bf16* __restrict__ d_o, long long o_rs, long long o_bs,
                      const float* __restrict__ lse, float* __restrict__ stats, float* __restrict__ dq32, int B, int Hq,

@@ -125,8 +125,8 @@ class SwiGluMlp(nn.Module):
         return res, ops.linear(h, self.w2.weight)
 
     def forward(self, x, tp=None, residual_rows: Optional[int] = None):
-        if x.dim() == 2 and x.shape[0] <= 16 and (tp is None or getattr(tp, "_pending", None) is None):
-            h = ops.linear_swiglu(x, self.w13.weight)       # decode: projection and activation in one kernel
+        if tp is None or (x.dim() == 2 and x.shape[0] <= 16 and getattr(tp, "_pending", None) is None):
+            h = ops.linear_swiglu(x, self.w13.weight)       # few rows: projection and activation in one kernel
         else:
             h = ops.swiglu(_col_linear(tp, x, self.w13.weight))
         return _row_linear(tp, h, self.w2.weight, residual_rows)

@@ -37,10 +37,31 @@ def _cuda(x: torch.Tensor) -> bool:
     return x.is_cuda
 
 
+class _NoGrad:
+    """The context of a forward pass that nobody will differentiate: what it saves is dropped."""
+
+    def save_for_backward(self, *tensors):
+        pass
+
+
+def _observed() -> bool:
+    """Whether someone follows the calls themselves: forward-mode differentiation, a trace, a compiler.  They must meet the
+    autograd function (its error, or its node in their graph) and not the bare kernel call."""
+    return torch.autograd.forward_ad._current_level >= 0 or torch.jit.is_tracing() or torch.compiler.is_compiling()
+
+
+def _run(fn, *args):
+    """``fn.apply(*args)``; without autograd the forward pass alone.  The small calls of a decode step or a short prompt are bound
+    by the host, and ``apply`` is 10 of the 28 us of a projection."""
+    if _observed() or (torch.is_grad_enabled() and any(isinstance(a, torch.Tensor) and a.requires_grad for a in args)):
+        return fn.apply(*args)
+    return fn.forward(_NoGrad(), *args)
+
+
 def _narrow_swiglu(x: torch.Tensor, w13: torch.Tensor):
-    """Plan of the split-K kernel for few rows with the activation, or None.  It takes feature counts in steps of 8; tangents of
-    forward-mode differentiation, and a parameter gather that waits for a GEMM to ride in, are left to separate calls."""
-    if x.shape[0] <= 16 or w13.shape[0] % 16 != 0 or _lib.pair_gather_pending() or torch.autograd.forward_ad._current_level >= 0:
+    """Plan of the split-K kernel for few rows with the activation, or None.  It takes feature counts in steps of 8; a
+    parameter gather that waits for a GEMM to ride in, and observed calls, are left to separate calls."""
+    if x.shape[0] <= 16 or w13.shape[0] % 16 != 0 or _lib.pair_gather_pending() or _observed():
         return None
     return _lib.gemm_narrow_plan(x.shape[0], w13.shape[0], x.shape[1], 1, GEMM_PAIR_MIN_TILES)
 
@@ -184,7 +205,7 @@ def linear(x: torch.Tensor, weight: torch.Tensor, bias: Optional[torch.Tensor] =
     if not _cuda(x):
         return ref.linear(x, weight, bias)
     _require_bf16(x, weight)
-    y = _LinearFn.apply(x, weight)
+    y = _run(_LinearFn, x, weight)
     return y if bias is None else y + bias
 
 
@@ -236,7 +257,7 @@ def dual_linear(x: torch.Tensor, w_a: torch.Tensor, w_b: torch.Tensor, n_a: int)
         return torch.cat([ref.linear(x[:n_a], w_a), ref.linear(x[n_a:], w_b)], dim=0)
     _require_bf16(x, w_a, w_b)
     x = x if x.is_contiguous() else x.contiguous()
-    return _DualLinearFn.apply(x, w_a, w_b, n_a)
+    return _run(_DualLinearFn, x, w_a, w_b, n_a)
 
 
 # =============================================================================== RMSNorm
@@ -329,9 +350,9 @@ def add_rms_norm(x: torch.Tensor, delta: Optional[torch.Tensor], weight: torch.T
     _require_bf16(x, delta, weight)
     x = x if x.is_contiguous() else x.contiguous()
     if delta is None:
-        return x, _RmsNormFn.apply(x, weight, eps)
+        return x, _run(_RmsNormFn, x, weight, eps)
     delta = delta if delta.is_contiguous() else delta.contiguous()
-    return _AddRmsNormFn.apply(x, delta, weight, eps)
+    return _run(_AddRmsNormFn, x, delta, weight, eps)
 
 
 def rms_norm(x: torch.Tensor, weight: torch.Tensor, eps: float = 1e-6) -> torch.Tensor:
@@ -339,7 +360,7 @@ def rms_norm(x: torch.Tensor, weight: torch.Tensor, eps: float = 1e-6) -> torch.
         return ref.rms_norm(x, weight, eps)
     _require_bf16(x, weight)
     x = x if x.is_contiguous() else x.contiguous()
-    return _RmsNormFn.apply(x, weight, eps)
+    return _run(_RmsNormFn, x, weight, eps)
 
 
 # =============================================================================== QK-norm + RoPE
@@ -431,7 +452,7 @@ def qk_norm_rope_packed(qkv: torch.Tensor, q_w: Optional[torch.Tensor], k_w: Opt
         return torch.cat([q.reshape(T, Hq * D), k.reshape(T, Hkv * D), qkv[:, (Hq + Hkv) * D:]], dim=1)
     _require_bf16(qkv, q_w, k_w)
     assert qkv.stride(1) == 1
-    return _QkNormRopeFn.apply(qkv, q_w, k_w, pos.to(torch.int32), Hq, Hkv, D, theta, eps, interleaved)
+    return _run(_QkNormRopeFn, qkv, q_w, k_w, pos.to(torch.int32), Hq, Hkv, D, theta, eps, interleaved)
 
 
 def norm_linear(x: torch.Tensor, delta: Optional[torch.Tensor], norm_w: torch.Tensor, eps: float,
@@ -512,7 +533,7 @@ def swiglu(gate_up: torch.Tensor) -> torch.Tensor:
         return ref.swiglu(gate_up)
     _require_bf16(gate_up)
     gate_up = gate_up if gate_up.is_contiguous() else gate_up.contiguous()
-    return _SwiGluFn.apply(gate_up)
+    return _run(_SwiGluFn, gate_up)
 
 
 def linear_swiglu(x: torch.Tensor, w13: torch.Tensor) -> torch.Tensor:
@@ -583,7 +604,7 @@ def embedding(ids: torch.Tensor, table: torch.Tensor) -> torch.Tensor:
     if not _cuda(table):
         return ref.embedding(ids, table)
     _require_bf16(table)
-    return _EmbeddingFn.apply(ids, table)
+    return _run(_EmbeddingFn, ids, table)
 
 
 # =============================================================================== attention
@@ -735,12 +756,12 @@ def ksa_attention(q_t, k_t, v_t, q_s, k_s, v_s, chunk: int, n_sum: int, window: 
     _require_bf16(q_t, k_t, v_t, q_s, k_s, v_s)
     seq_len = seq_len if seq_len is not None else k_off + k_t.shape[1]
     if skip_old_summary:
-        o_t, _ = _KsaAttentionFn.apply(q_t, k_t, v_t, None, None, None, chunk, n_sum, window, 0, scale,
+        o_t, _ = _run(_KsaAttentionFn, q_t, k_t, v_t, None, None, None, chunk, n_sum, window, 0, scale,
                                        q_off, k_off, s_off, seq_len)
-        _, o_s = _KsaAttentionFn.apply(q_t[:, :0], k_t, v_t, q_s, k_s, v_s, chunk, n_sum, window, 0, scale,
+        _, o_s = _run(_KsaAttentionFn, q_t[:, :0], k_t, v_t, q_s, k_s, v_s, chunk, n_sum, window, 0, scale,
                                        q_off, k_off, s_off, seq_len)
         return o_t, o_s
-    return _KsaAttentionFn.apply(q_t, k_t, v_t, q_s, k_s, v_s, chunk, n_sum, window, 0, scale,
+    return _run(_KsaAttentionFn, q_t, k_t, v_t, q_s, k_s, v_s, chunk, n_sum, window, 0, scale,
                                  q_off, k_off, s_off, seq_len)
 
 
@@ -756,7 +777,7 @@ def causal_attention(q, k, v, scale: Optional[float] = None, window: int = -1,
     doc_start = doc_end = None
     if cu_seqlens is not None:
         doc_start, doc_end = document_bounds(cu_seqlens, q.shape[0], q.shape[1], k.shape[1], q_off)
-    o, _ = _KsaAttentionFn.apply(q, k, v, None, None, None, 128, 1, UNBOUNDED_WINDOW,
+    o, _ = _run(_KsaAttentionFn, q, k, v, None, None, None, 128, 1, UNBOUNDED_WINDOW,
                                  window if window and window > 0 else 0, scale, q_off, 0, 0, k.shape[1],
                                  doc_start, doc_end)
     return o
@@ -782,7 +803,7 @@ def shard_causal_attention(q, k, v, scale: float, tok_window: int, q_off: int, k
     """Causal attention of a sequence shard: query row ``i`` is global position ``q_off + i``, key row ``j`` is
     ``k_off + j`` (context-parallel full-attention layers stage every earlier key in front of their own)."""
     _require_bf16(q, k, v)
-    o, _ = _KsaAttentionFn.apply(q, k, v, None, None, None, 128, 1, UNBOUNDED_WINDOW,
+    o, _ = _run(_KsaAttentionFn, q, k, v, None, None, None, 128, 1, UNBOUNDED_WINDOW,
                                  tok_window if tok_window and tok_window > 0 else 0, scale, q_off, k_off, 0, seq_len)
     return o
 
@@ -897,7 +918,7 @@ def attention_packed(qkv: torch.Tensor, B: int, L: int, Ns: int, Hq: int, Hkv: i
             raise ValueError("packed documents apply to causal attention only: summary tokens are inserted without "
                              "regard to document boundaries")
         docs = document_bounds(cu_seqlens, B, L, L)
-    return _PackedAttentionFn.apply(qkv, B, L, Ns, Hq, Hkv, D, chunk, n_sum, window, tok_window, scale, *docs)
+    return _run(_PackedAttentionFn, qkv, B, L, Ns, Hq, Hkv, D, chunk, n_sum, window, tok_window, scale, *docs)
 
 
 # =============================================================================== fused linear + cross entropy
