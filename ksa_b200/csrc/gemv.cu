@@ -223,7 +223,7 @@ static int launch_gemv(const void* a, const void* b, void* c, int M, int N, int 
 }
 
 // ------------------------------------------------------------------------------------------ tensor-core variant
-// For 5..16 activation rows the SIMT kernel above is bound by its FMA issue rate, so the dot products go to the tensor
+// For 3..16 activation rows the SIMT kernel above is bound by its FMA issue rate, so the dot products go to the tensor
 // cores with warp-level mma.sync m16n8k16 (the 128-row tcgen05 tile has no use for 16 rows): a CTA owns 16 weight
 // rows, its 8 warps take the 32-wide k blocks round-robin, and the partial sums meet in shared memory.  Both operands
 // are read as 16 contiguous bytes per lane along k; a lane's 8 elements are given to the instruction as its k slots
@@ -367,7 +367,9 @@ namespace ksa {
 template <bool kGlu>
 static int gemv_dispatch(const void* a, const void* b, void* c, int M, int N, int K, long long lda, long long ldb,
                          long long ldc, cudaStream_t st, const GemvNorm& nrm = GemvNorm{}) {
-  if (M > 4 && K % 32 == 0 && nrm.w == nullptr) {
+  // three and four rows as well while 16 weight rows a CTA give every SM one (4 rows x 151936 x 2560: 173 -> 147 us, x 6144 x 2560:
+  // 16.3 -> 10.0, x 2560 x 4096: 11.9 -> 11.0; below, 4 x 2048 x 6144, 13.6 against 14.0)
+  if ((M > 4 || (M > 2 && N >= 148 * 16)) && K % 32 == 0 && nrm.w == nullptr) {
     if (N >= 16384)   // wide outputs: 32 weight rows per CTA still give every SM several CTAs
       return M <= 8 ? launch_gemv_mma<1, kGlu, 2>(a, b, c, M, N, K, lda, ldb, ldc, st)
                     : launch_gemv_mma<2, kGlu, 2>(a, b, c, M, N, K, lda, ldb, ldc, st);
