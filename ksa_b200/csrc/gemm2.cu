@@ -288,6 +288,9 @@ gemm2_bf16_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant
     const int quad = warp & 3;
     int local = 0;
     bool ok = true;
+    // Staging buffer of this warp's next store.  It flips with every store that is issued and is carried from tile to tile: pieces
+    // past N issue none, so a tile may end on either buffer, and only the newest store may still be reading its own.
+    int out_buf = 0;
     for (int tile = pair; tile < num_tiles && ok; tile += n_pairs, ++local) {
       int mb, nb;
       tile_coords(tile, mb, nb);
@@ -318,8 +321,8 @@ gemm2_bf16_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant
         tmem_wait_ld();
         const int col0 = nb * k2BN + c * 32;
         if (tma_block && ep.out_fp32) {
-          uint8_t* stage = ring + ((warp - 2) * 2 + (c & 1)) * 4096;
-          // this buffer was read by the store issued two pieces ago; at most the newest store may be pending
+          uint8_t* stage = ring + ((warp - 2) * 2 + out_buf) * 4096;
+          // this buffer was read by the last store but one; at most the newest store may be pending
           if (lane == 0) asm volatile("cp.async.bulk.wait_group.read 1;" ::: "memory");
           __syncwarp();
           if (col0 < N) {
@@ -336,14 +339,15 @@ gemm2_bf16_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant
             else tma_store_2d(&smaps.m[owner_w], stage, col0, row_w - owner_w * ep.c_shard_rows);
             tma_store_commit();
           }
+          if (col0 < N) out_buf ^= 1;
           continue;
         }
         if (tma_block) {
           const int piece = c >> 1, half = c & 1;                   // 64-column piece, 32-column half of it
-          uint8_t* stage = ring + ((warp - 2) * 2 + (piece & 1)) * 4096;
+          uint8_t* stage = ring + ((warp - 2) * 2 + out_buf) * 4096;
           const bool live = nb * k2BN + piece * 64 < N;             // columns past N are clipped by the map
           if (half == 0) {
-            // this buffer was read by the store issued two pieces ago; at most the newest store may be pending
+            // this buffer was read by the last store but one; at most the newest store may be pending
             if (lane == 0) asm volatile("cp.async.bulk.wait_group.read 1;" ::: "memory");
             __syncwarp();
           }
@@ -366,6 +370,7 @@ gemm2_bf16_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant
               tma_store_2d(&smaps.m[owner_w], stage, nb * k2BN + piece * 64, row_w - owner_w * ep.c_shard_rows);
               tma_store_commit();
             }
+            if (live) out_buf ^= 1;
           }
           continue;
         }

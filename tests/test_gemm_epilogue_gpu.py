@@ -34,3 +34,29 @@ def test_pair_gemm_stores_ragged_tiles(M, N, K, fp32):
         ops.gemm(a, b, out=out, accumulate=True, alpha=-0.5, pair=True)
         _lib.check_status()
         assert rel(out, 0.5 * want) < 1e-5 and bool(big[:, N:].isnan().all())
+
+
+# rows x columns with several tiles for every CTA pair and a last column tile that ends after 1, 2, 3, 7 pieces of 32 fp32 columns
+# or 1, 3, 4 pieces of 64 bf16 columns: the next tile's stores follow on either staging buffer
+@pytest.mark.parametrize("M,N", [(38400, 264), (8256, 2112), (16640, 2144), (8256, 2240), (8256, 2272), (9000, 2880),
+                                 (8256, 4104)])
+@pytest.mark.parametrize("K", [64, 128])
+def test_pair_gemm_staging_across_tiles(M, N, K):
+    """Short reductions, so that nothing but the staging buffers orders the stores of consecutive tiles."""
+    torch.manual_seed(N)
+    a, b = bf(M, K), bf(N, K, scale=0.1)
+    want = (a.double() @ b.double().t()).float()
+    # fp32 sums of K products of bf16 values in any order
+    bound = (K * 2.0 ** -23) * (a.float().abs() @ b.float().abs().t())
+    init = torch.randn(M, N, device=DEV)
+    for _ in range(3):
+        c = torch.full((M, N), float("nan"), device=DEV, dtype=torch.bfloat16)
+        ops.gemm(a, b, out=c, pair=True)
+        assert bool(((c.float() - want).abs() <= 2.0 ** -8 * want.abs() + bound).all())
+        c = torch.full((M, N), float("nan"), device=DEV)
+        ops.gemm(a, b, out=c, pair=True)
+        assert bool(((c - want).abs() <= bound).all())
+        c = init.clone()
+        ops.gemm(a, b, out=c, accumulate=True, pair=True)
+        assert bool(((c - (init + want)).abs() <= bound + 2.0 ** -22 * (init.abs() + want.abs())).all())
+    _lib.check_status()
