@@ -45,9 +45,11 @@ class _NoGrad:
 
 
 def _observed() -> bool:
-    """Whether someone follows the calls themselves: forward-mode differentiation, a trace, a compiler.  They must meet the
-    autograd function (its error, or its node in their graph) and not the bare kernel call."""
-    return torch.autograd.forward_ad._current_level >= 0 or torch.jit.is_tracing() or torch.compiler.is_compiling()
+    """Whether someone follows the calls themselves: a ``torch.func`` transform, forward-mode differentiation, a trace, a compiler.
+    They must meet the autograd function (its error, or its node in their graph) and not the bare kernel call, which would take
+    the wrappers' memory for that of their tensors."""
+    return (torch._C._are_functorch_transforms_active() or torch.autograd.forward_ad._current_level >= 0
+            or torch.jit.is_tracing() or torch.compiler.is_compiling())
 
 
 def _run(fn, *args):

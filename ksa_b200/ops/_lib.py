@@ -127,7 +127,11 @@ def _ptr(x):
     if isinstance(x, torch.Tensor):
         if not x.is_cuda:  # a host pointer handed to a kernel is an illegal access on the device
             raise TypeError("a CPU tensor was passed to an sm_100a kernel entry point")
-        return x.data_ptr()
+        p = x.data_ptr()
+        if p == 0 and x.numel() > 0:
+            raise RuntimeError("a tensor without memory of its own (a wrapper of a transform) was passed to an sm_100a kernel "
+                               "entry point")
+        return p
     return x
 
 

@@ -4,6 +4,7 @@ import torch
 import torch.autograd.forward_ad as fwd
 
 from ksa_b200 import ops
+from ksa_b200.ops import _lib
 
 
 class _Twice(torch.autograd.Function):
@@ -46,3 +47,77 @@ def test_a_trace_still_meets_the_function():
     with torch.no_grad():
         traced = torch.jit.trace(lambda x: ops._run(_Twice, x, 2), torch.ones(3), check_trace=False)
     assert torch.equal(traced(torch.full((3,), 5.0)), torch.full((3,), 10.0))
+
+
+# ------------------------------------------------------------------------- the framework's own calls, kernels replaced by a recorder
+def _bf(*shape):
+    return torch.ones(*shape).bfloat16()
+
+
+_W = {"w": _bf(64, 64), "n": _bf(64), "n16": _bf(16), "kv": _bf(1, 128, 1, 128)}
+_CALLS = {
+    "linear": (lambda x: ops.linear(x, _W["w"]), (32, 64)),
+    "dual_linear": (lambda x: ops.dual_linear(x, _W["w"], _W["w"], 20), (32, 64)),
+    "rms_norm": (lambda x: ops.rms_norm(x, _W["n"]), (32, 64)),
+    "add_rms_norm": (lambda x: ops.add_rms_norm(x, x, _W["n"])[1], (32, 64)),
+    "qk_norm_rope_packed": (lambda x: ops.qk_norm_rope_packed(x, _W["n16"], _W["n16"], torch.arange(32), 2, 1, 16, 1e4, 1e-6), (32, 64)),
+    "swiglu": (lambda x: ops.swiglu(x), (32, 64)),
+    "linear_swiglu": (lambda x: ops.linear_swiglu(x, _W["w"]), (32, 64)),
+    "linear_swiglu of few rows": (lambda x: ops.linear_swiglu(x, _W["w"]), (8, 64)),
+    "embedding": (lambda x: ops.embedding(torch.arange(3), x), (32, 64)),
+    "causal_attention": (lambda x: ops.causal_attention(x, _W["kv"], _W["kv"]), (1, 128, 1, 128)),
+    "ksa_attention": (lambda x: ops.ksa_attention(x, _W["kv"], _W["kv"], x[:, :1], _W["kv"][:, :1], _W["kv"][:, :1], 128, 1, 2)[0],
+                      (1, 128, 1, 128)),
+    "attention_packed": (lambda x: ops.attention_packed(x, 1, 32, 0, 2, 1, 16, 16, 1, 2), (32, 64)),
+}
+_TRANSFORMS = {
+    "functionalize": lambda f, x: torch.func.functionalize(f)(x),
+    "vmap": lambda f, x: torch.func.vmap(f)(x[None]),
+    "vmap of something else": lambda f, x: torch.func.vmap(lambda other: f(x) + other)(torch.ones(2).bfloat16()),
+    "grad": lambda f, x: torch.func.grad(lambda t: f(t).float().sum())(x),
+    "jvp": lambda f, x: torch.func.jvp(f, (x,), (x,)),
+}
+
+
+@pytest.fixture
+def recorder(monkeypatch):
+    """What reaches the kernels' entry points: the addresses of the tensors."""
+    calls = []
+    monkeypatch.setattr(ops, "_cuda", lambda x: True)
+    monkeypatch.setattr(_lib, "call", lambda name, *args: calls.append(
+        [a.data_ptr() for a in args if isinstance(a, torch.Tensor) and a.numel() > 0]))
+    monkeypatch.setattr(_lib, "gemm_narrow_plan", lambda *sizes: (32, 1))
+    return calls
+
+
+@pytest.mark.parametrize("name", list(_CALLS))
+def test_an_op_reaches_its_kernel(name, recorder):
+    f, shape = _CALLS[name]
+    f(_bf(*shape))
+    assert recorder and all(p != 0 for c in recorder for p in c)
+
+
+@pytest.mark.parametrize("transform", list(_TRANSFORMS))
+@pytest.mark.parametrize("name", [n for n in _CALLS if n != "linear_swiglu of few rows"])
+def test_an_op_is_refused_under_a_transform(name, transform, recorder):
+    """The autograd functions have no rule for transforms, and PyTorch says so; nothing of a wrapper reaches a kernel."""
+    f, shape = _CALLS[name]
+    with torch.no_grad(), pytest.raises(RuntimeError, match="functorch transforms"):
+        _TRANSFORMS[transform](f, _bf(*shape))
+    assert not recorder
+
+
+def test_a_tensor_without_memory_is_refused():
+    class OnGpu(torch.Tensor):
+        is_cuda = True
+
+    def make(t):
+        return torch.Tensor._make_subclass(OnGpu, t)
+
+    assert _lib._ptr(make(torch.ones(3))) != 0 and _lib._ptr(make(torch.empty(0))) == 0
+    hollow = torch._to_functional_tensor(torch.ones(3))
+    assert hollow.data_ptr() == 0
+    hollow = make(torch.ones(3))
+    hollow.data_ptr = lambda: 0
+    with pytest.raises(RuntimeError, match="without memory"):
+        _lib._ptr(hollow)
