@@ -127,12 +127,19 @@ def _ptr(x):
     if isinstance(x, torch.Tensor):
         if not x.is_cuda:  # a host pointer handed to a kernel is an illegal access on the device
             raise TypeError("a CPU tensor was passed to an sm_100a kernel entry point")
-        p = x.data_ptr()
-        if p == 0 and x.numel() > 0:
-            raise RuntimeError("a tensor without memory of its own (a wrapper of a transform) was passed to an sm_100a kernel "
-                               "entry point")
-        return p
+        return _address(x)
     return x
+
+
+def _address(x: torch.Tensor) -> int:
+    try:
+        p = x.data_ptr()
+    except RuntimeError:      # a wrapper: the tensor inside counts if its transform has ended, as in ``Function.apply``
+        p = torch._C._functorch.unwrap_if_dead(x).data_ptr()
+    if p == 0 and x.numel() > 0:
+        raise RuntimeError("a tensor without memory of its own (a wrapper of a transform) was passed to an sm_100a kernel "
+                           "entry point")
+    return p
 
 
 # kernels launched by one call of an entry point (default 1)

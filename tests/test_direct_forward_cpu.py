@@ -121,3 +121,22 @@ def test_a_tensor_without_memory_is_refused():
     hollow.data_ptr = lambda: 0
     with pytest.raises(RuntimeError, match="without memory"):
         _lib._ptr(hollow)
+
+
+@pytest.mark.parametrize("transform", ["jvp", "grad"])
+@pytest.mark.parametrize("call", [lambda t: ops.linear(_bf(32, 64), t), lambda t: ops.embedding(torch.arange(3), t),
+                                  lambda t: ops.linear(t, _W["w"]), lambda t: ops.rms_norm(t, _W["n"])])
+def test_a_tensor_that_outlived_its_transform(call, transform, monkeypatch):
+    """What a finished transform left behind is an ordinary tensor again."""
+    calls = []
+    monkeypatch.setattr(ops, "_cuda", lambda x: True)
+
+    def record(name, *args):
+        for a in args:
+            if isinstance(a, torch.Tensor):
+                calls.append(_lib._address(a))
+    monkeypatch.setattr(_lib, "call", record)
+    kept = []
+    _TRANSFORMS[transform](lambda t: (kept.append(t), t.float().sum())[1], _bf(64, 64))
+    call(kept[0])
+    assert calls and all(calls)
