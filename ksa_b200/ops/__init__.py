@@ -543,7 +543,9 @@ def linear_swiglu(x: torch.Tensor, w13: torch.Tensor) -> torch.Tensor:
     decode step, a short prompt) applies the activation itself: ``ksa_gemv_swiglu_bf16`` for at most 16 rows, the gated form of
     ``ksa_gemm_narrow_bf16`` where ``gemm`` would take that kernel.  Everything else is the projection followed by
     ``swiglu``."""
-    if (_cuda(x) and x.dim() == 2 and (x.shape[0] <= 16 or _narrow_swiglu(x, w13) is not None) and x.dtype == torch.bfloat16 and w13.dtype == torch.bfloat16
+    if (_cuda(x) and x.dim() == 2 and w13.dim() == 2 and x.shape[1] == w13.shape[1]
+            and (x.shape[0] <= 16 or _narrow_swiglu(x, w13) is not None)
+            and x.dtype == torch.bfloat16 and w13.dtype == torch.bfloat16
             and not (torch.is_grad_enabled() and (x.requires_grad or w13.requires_grad))
             and x.stride(1) == 1 and w13.stride(1) == 1 and x.shape[1] % 8 == 0 and x.stride(0) % 8 == 0
             and w13.stride(0) % 8 == 0 and w13.shape[0] % 2 == 0):

@@ -140,3 +140,14 @@ def test_a_tensor_that_outlived_its_transform(call, transform, monkeypatch):
     _TRANSFORMS[transform](lambda t: (kept.append(t), t.float().sum())[1], _bf(64, 64))
     call(kept[0])
     assert calls and all(calls)
+
+
+@pytest.mark.parametrize("rows", [8, 32])
+@pytest.mark.parametrize("width", [56, 72])
+def test_linear_swiglu_refuses_other_widths(rows, width, recorder):
+    """The fused kernels take the reduction length from the activations alone."""
+    with torch.no_grad(), pytest.raises(AssertionError, match="reduction mismatch"):
+        ops.linear_swiglu(_bf(rows, width), _W["w"])
+    with torch.no_grad(), pytest.raises(AssertionError):
+        ops.linear_swiglu(_bf(rows, 64), _W["w"][None])
+    assert not recorder
