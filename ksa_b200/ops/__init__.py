@@ -463,7 +463,8 @@ def norm_linear(x: torch.Tensor, delta: Optional[torch.Tensor], norm_w: torch.Te
     rows then up rows).  Returns ``(res, y)``.  For at most 4 rows on a GPU without autograd (a decode step) this is
     one launch (``ksa_gemv_norm_bf16``: every CTA normalises the few activation rows itself while it stages them);
     everything else is ``add_rms_norm`` followed by the projection."""
-    if (_cuda(x) and x.dim() == 2 and x.shape[0] <= 4 and x.dtype == torch.bfloat16 and weight.dtype == torch.bfloat16
+    if (_cuda(x) and x.dim() == 2 and weight.dim() == 2 and x.shape[1] == weight.shape[1] and x.shape[0] <= 4
+            and x.dtype == torch.bfloat16 and weight.dtype == torch.bfloat16
             and not (torch.is_grad_enabled() and (x.requires_grad or weight.requires_grad))
             and x.stride(1) == 1 and weight.stride(1) == 1 and x.shape[1] % 8 == 0 and x.stride(0) % 8 == 0
             and weight.stride(0) % 8 == 0 and (delta is None or (delta.stride(1) == 1 and delta.stride(0) % 8 == 0

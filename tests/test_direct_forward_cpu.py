@@ -151,3 +151,11 @@ def test_linear_swiglu_refuses_other_widths(rows, width, recorder):
     with torch.no_grad(), pytest.raises(AssertionError):
         ops.linear_swiglu(_bf(rows, 64), _W["w"][None])
     assert not recorder
+
+
+@pytest.mark.parametrize("width", [56, 72])
+@pytest.mark.parametrize("glu", [False, True])
+def test_norm_linear_refuses_other_widths(width, glu, recorder):
+    with torch.no_grad(), pytest.raises(AssertionError, match="reduction mismatch"):
+        ops.norm_linear(_bf(2, width), None, _bf(width), 1e-6, _W["w"], glu)
+    assert len(recorder) == 1, "the norm alone, as a call of its own"
