@@ -187,6 +187,7 @@ gemm_narrow_kernel(const __grid_constant__ CUtensorMap tmW, const __grid_constan
     v.z = pack_bf16x2(o[4], o[5]); v.w = pack_bf16x2(o[6], o[7]);
     *reinterpret_cast<uint4*>(p.c + (long long)(m0 + m) * p.ldc + row0 + n8) = v;
   }
+  __syncwarp();               // lanes leave the loop after different numbers of rows, and the barrier takes whole warps
   nw_cluster_sync();          // nobody leaves while its part may still be read
   if (warp == 2) {
     tc_fence_after();
