@@ -33,6 +33,8 @@ UNBOUNDED_WINDOW = 1 << 30
 # GEMMs with at least this many 256 x 256 tiles run on CTA pairs (tcgen05 cta_group::2, csrc/gemm2.cu; 74 pairs per
 # GPU); below that the single-CTA kernel with 128-row tiles has more CTAs to spread.  0 disables the pair kernel.
 GEMM_PAIR_MIN_TILES = int(__import__("os").environ.get("KSA_GEMM_PAIR_MIN_TILES", "32"))
+
+
 def _cuda(x: torch.Tensor) -> bool:
     return x.is_cuda
 
@@ -63,7 +65,7 @@ def _run(fn, *args):
 def _narrow_swiglu(x: torch.Tensor, w13: torch.Tensor):
     """Plan of the split-K kernel for few rows with the activation, or None.  It takes feature counts in steps of 8; a
     parameter gather that waits for a GEMM to ride in, and observed calls, are left to separate calls."""
-    if x.shape[0] <= 16 or w13.shape[0] % 16 != 0 or _lib.pair_gather_pending() or _observed():
+    if w13.shape[0] % 16 != 0 or _lib.pair_gather_pending() or _observed():
         return None
     return _lib.gemm_narrow_plan(x.shape[0], w13.shape[0], x.shape[1], 1, GEMM_PAIR_MIN_TILES)
 
@@ -545,21 +547,21 @@ def linear_swiglu(x: torch.Tensor, w13: torch.Tensor) -> torch.Tensor:
     ``ksa_gemm_narrow_bf16`` where ``gemm`` would take that kernel.  Everything else is the projection followed by
     ``swiglu``."""
     if (_cuda(x) and x.dim() == 2 and w13.dim() == 2 and x.shape[1] == w13.shape[1]
-            and (x.shape[0] <= 16 or _narrow_swiglu(x, w13) is not None)
             and x.dtype == torch.bfloat16 and w13.dtype == torch.bfloat16
             and not (torch.is_grad_enabled() and (x.requires_grad or w13.requires_grad))
             and x.stride(1) == 1 and w13.stride(1) == 1 and x.shape[1] % 8 == 0 and x.stride(0) % 8 == 0
             and w13.stride(0) % 8 == 0 and w13.shape[0] % 2 == 0):
         M, K = x.shape
         N = w13.shape[0]
-        out = torch.empty((M, N // 2), dtype=torch.bfloat16, device=x.device)
-        if M > 16:
-            bt, split = _narrow_swiglu(x, w13)
-            _lib.call("ksa_gemm_narrow_bf16", x, w13, out, M, N, K, x.stride(0), w13.stride(0), out.stride(0), 0, 1, bt, split,
-                      1.0)
+        plan = _narrow_swiglu(x, w13) if M > 16 else None
+        if M <= 16 or plan is not None:
+            out = torch.empty((M, N // 2), dtype=torch.bfloat16, device=x.device)
+            if plan is None:
+                _lib.call("ksa_gemv_swiglu_bf16", x, w13, out, M, N, K, x.stride(0), w13.stride(0), out.stride(0))
+            else:
+                _lib.call("ksa_gemm_narrow_bf16", x, w13, out, M, N, K, x.stride(0), w13.stride(0), out.stride(0), 0, 1,
+                          *plan, 1.0)
             return out
-        _lib.call("ksa_gemv_swiglu_bf16", x, w13, out, M, N, K, x.stride(0), w13.stride(0), out.stride(0))
-        return out
     return swiglu(linear(x, w13))
 
 

@@ -159,3 +159,12 @@ def test_norm_linear_refuses_other_widths(width, glu, recorder):
     with torch.no_grad(), pytest.raises(AssertionError, match="reduction mismatch"):
         ops.norm_linear(_bf(2, width), None, _bf(width), 1e-6, _W["w"], glu)
     assert len(recorder) == 1, "the norm alone, as a call of its own"
+
+
+@pytest.mark.parametrize("requires", [False, True])
+def test_linear_swiglu_asks_for_its_plan_once(requires, recorder, monkeypatch):
+    """Once where it can use the answer, not at all where the call is differentiated (the projection asks for its own)."""
+    asked = []
+    monkeypatch.setattr(_lib, "gemm_narrow_plan", lambda M, N, K, glu, tiles: asked.append(glu) or (32, 1))
+    ops.linear_swiglu(_bf(32, 64).requires_grad_(requires), _W["w"])
+    assert asked == ([0] if requires else [1])
