@@ -19,6 +19,7 @@ returned to autograd in the weight's dtype.
 """
 from __future__ import annotations
 
+import functools
 import math
 import os
 from typing import Optional, Tuple
@@ -46,12 +47,16 @@ class _NoGrad:
         pass
 
 
+# private to PyTorch: without them every call counts as observed
+_transforms_active = getattr(torch._C, "_are_functorch_transforms_active", lambda: True)
+_forward_level = functools.partial(getattr, torch.autograd.forward_ad, "_current_level", 0)
+
+
 def _observed() -> bool:
     """Whether someone follows the calls themselves: a ``torch.func`` transform, forward-mode differentiation, a trace, a compiler.
     They must meet the autograd function (its error, or its node in their graph) and not the bare kernel call, which would take
     the wrappers' memory for that of their tensors."""
-    return (torch._C._are_functorch_transforms_active() or torch.autograd.forward_ad._current_level >= 0
-            or torch.jit.is_tracing() or torch.compiler.is_compiling())
+    return _transforms_active() or _forward_level() >= 0 or torch.jit.is_tracing() or torch.compiler.is_compiling()
 
 
 def _run(fn, *args):

@@ -148,6 +148,8 @@ _launch_count = 0
 
 
 _PLAIN = (int, float, type(None))
+# private to PyTorch: without it the handle comes from a stream object
+_raw_stream = getattr(torch._C, "_cuda_getCurrentRawStream", None) or (lambda dev: torch.cuda.current_stream(dev).cuda_stream)
 
 
 def call(name: str, *args) -> None:
@@ -156,7 +158,7 @@ def call(name: str, *args) -> None:
     global _launch_count
     lib = _lib or load()
     rc = getattr(lib, name)(*[a if a.__class__ in _PLAIN else _ptr(a) for a in args],
-                            torch._C._cuda_getCurrentRawStream(torch.cuda.current_device()))
+                            _raw_stream(torch.cuda.current_device()))
     if rc != 0:
         raise RuntimeError(f"{name} failed ({rc}): {lib.ksa_last_error().decode()}")
     _launch_count += _KERNELS_PER_CALL.get(name, 1)

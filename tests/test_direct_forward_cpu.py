@@ -1,10 +1,16 @@
 """Calls without autograd skip the autograd function; whoever follows the calls still meets it."""
+import subprocess
+import sys
+from pathlib import Path
+
 import pytest
 import torch
 import torch.autograd.forward_ad as fwd
 
 from ksa_b200 import ops
 from ksa_b200.ops import _lib
+
+ROOT = Path(__file__).resolve().parents[1]
 
 
 class _Twice(torch.autograd.Function):
@@ -168,3 +174,16 @@ def test_linear_swiglu_asks_for_its_plan_once(requires, recorder, monkeypatch):
     monkeypatch.setattr(_lib, "gemm_narrow_plan", lambda M, N, K, glu, tiles: asked.append(glu) or (32, 1))
     ops.linear_swiglu(_bf(32, 64).requires_grad_(requires), _W["w"])
     assert asked == ([0] if requires else [1])
+
+
+def test_private_names_of_pytorch_are_there():
+    """The bypass works without them, but then every call takes the long way; a newer PyTorch should not do that unseen."""
+    assert hasattr(torch._C, "_are_functorch_transforms_active") and hasattr(fwd, "_current_level")
+    assert torch._C._functorch.unwrap_if_dead(torch.ones(1)) is not None
+    assert not ops._observed()
+
+
+def test_without_private_names_every_call_is_observed():
+    code = ("import torch\nimport torch.autograd.forward_ad as fwd\ndel fwd._current_level\n"
+            "from ksa_b200 import ops\nassert ops._observed()\n")
+    assert subprocess.run([sys.executable, "-c", code], cwd=ROOT).returncode == 0
