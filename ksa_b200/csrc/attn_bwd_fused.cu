@@ -625,6 +625,7 @@ KSA_API int ksa_attn_bwd_fused(const void* q, const void* k, const void* v, cons
   KSA_REQUIRE(o_rs % 8 == 0 && dq_rs % 8 == 0 && dk_rs % 8 == 0 && dv_rs % 8 == 0,
               "attn_bwd_fused: row strides must be multiples of 8");
   KSA_REQUIRE(stats != nullptr && dq32 != nullptr, "attn_bwd_fused: the stats and dq32 workspaces are required");
+  KSA_REQUIRE((reinterpret_cast<uintptr_t>(o) & 15) == 0, "attn_bwd_fused: O must be 16-byte aligned");
   if (B == 0 || Lq == 0) return 0;
   const int lq_pad = ksa_attn_bwd_fused_lq_pad(Lq);
   CUtensorMap tq, tdo, tk, tv, tks, tvs;
@@ -718,6 +719,7 @@ KSA_API int ksa_attn_bwd_fused_cp(const void* q, const void* o, const void* d_o,
   KSA_REQUIRE(n_sum_src <= 1 || nsl % 128 == 0, "attn_bwd_fused_cp: %d summary rows per rank must be a multiple of 128", nsl);
   KSA_REQUIRE(o_rs % 8 == 0 && dq_rs % 8 == 0 && dk_rs % 8 == 0 && dv_rs % 8 == 0, "attn_bwd_fused_cp: row strides must be multiples of 8");
   KSA_REQUIRE(stats != nullptr && dq32 != nullptr, "attn_bwd_fused_cp: the stats and dq32 workspaces are required");
+  KSA_REQUIRE((reinterpret_cast<uintptr_t>(o) & 15) == 0, "attn_bwd_fused_cp: O must be 16-byte aligned");
   KSA_REQUIRE(halo == 0 || ret_text != nullptr, "attn_bwd_fused_cp: a halo needs the return block of its owner");
   if (B == 0 || Lq == 0) return 0;
   const int lq_pad = ksa_attn_bwd_fused_lq_pad(Lq);

@@ -655,6 +655,8 @@ def _attn_bwd_text(q, k, v, ks, vs, o, do, lse, dq, dk, dv, dks, dvs, B, Hq, Hkv
         lq_pad = (Lq + 127) // 128 * 128
         stats = torch.empty((2, B, Hq, lq_pad), dtype=torch.float32, device=q.device)
         dq32 = torch.empty((B, Lq, Hq, D), dtype=torch.float32, device=q.device)
+        if o.data_ptr() % 16 != 0:     # a saved-tensor hook may hand back the output at any address
+            o = o.clone()
         _lib.call("ksa_attn_bwd_fused", q, k, v, ks, vs, o, do, lse, stats, dq32, dq, dk, dv, dks, dvs,
                   B, Hq, Hkv, D, Lq, Lk, Ns, *rest)
     else:

@@ -387,6 +387,8 @@ class _CpDirectAttention(torch.autograd.Function):
         dq, dk, dv = ops._packed_views(dqkv, B, Ll, Hq, Hkv, D, 0)
         dqs, dks, dvs = ops._packed_views(dqkv, B, Nsl, Hq, Hkv, D, B * Ll)
         o = out[:B * Ll].view(B, Ll, Hq, D)
+        if o.data_ptr() % 16 != 0:         # a saved-tensor hook may hand back the output at any address
+            o = o.clone()
         do = dout[:B * Ll].view(B, Ll, Hq, D)
         lq_pad = (Ll + 127) // 128 * 128
         stats = torch.empty((2, B, Hq, lq_pad), dtype=torch.float32, device=qkv.device)
