@@ -196,14 +196,22 @@ gemm_narrow_kernel(const __grid_constant__ CUtensorMap tmW, const __grid_constan
 }
 
 // Tile height and split for a product, and its time in microseconds as modelled.  The figures were fitted to 315 measured
-// (shape, height, split) triples of 17 to 1411 rows against 4096 x 2048 .. 19456 x 2560 weights (standard deviation 5 %, the
-// choice within 3 % of the best one measured for nearly all of them):
+// (shape, height, split) triples of 17 to 1411 rows against 4096 x 2048 .. 19456 x 2560 weights, the last two items to 900 shapes of
+// 17 to 2048 rows and 64 to 19456 x 64 to 12288 weights:
 //   * one 64-wide step of K takes a CTA that has an SM to itself 0.32 us (the latency of its loads) and two that share
 //     one 2 x (0.142 + 0.00044 bt), so a grid should fill both slots of every SM; a ring for more than 160 rows leaves
 //     room for one CTA only;
 //   * the weights of all CTAs come through the L2 at 13.7 TB/s;
 //   * a launch costs 1.5 us, a wave of CTAs 4.6 us to start and drain, and 0.0126 + 0.0045 split per activation row to write
-//     and add up.
+//     and add up;
+//   * clusters of 4 and 8 do not fill every SM: narrow_first and narrow_slots below;
+//   * rows that do not start on a 128-byte line take a second line for every box row: weights and activations then come
+//     through the L2 at 21 TB/s as 1.86 and 1.55 times their bytes.
+// Measured on the widths of both model presets and their transposes (16 of them, 17 to 2048 rows, 808 products): the model's
+// standard deviation is 5 %, the choice 0.6 % above the best of the plans tried on average, and no product slower than on the
+// tiled kernels.  On 497 other shapes: 10 %, 0.7 %, one of the 244 that were chosen 6 % slower (1856 x 6144 x 9728).  Without the last
+// two items 8 of those were up to 23 % slower, and of the 900 shapes 21 up to 30 % (779 x 3552 x 6008: 62.5 us on tiles of 160 rows
+// in two parts, 42.9 on CTA pairs; 193 x 4256 x 3352 30.2 on 208 rows in four parts, 21.0).
 constexpr int kNwSms = 148;
 constexpr int kNwMaxRows = 2048;   // the model holds near the range that it was fitted to (8000 x 128 x 2048: 27.4 against 15.3 us)
 static bool narrow_two_per_sm(int bt) { return 3 * (kNwWBytes + bt * kNwBK * 2) <= 110 * 1024; }
@@ -211,22 +219,36 @@ static int narrow_stages(int bt) {
   const int stages = (narrow_two_per_sm(bt) ? 110 : 220) * 1024 / (kNwWBytes + bt * kNwBK * 2);
   return stages < kNwMaxStages ? stages : kNwMaxStages;
 }
-static double narrow_plan(int M, long long n_tiles, int K, int* bt_out, int* split_out) {
+// CTAs that run with an SM to themselves, and CTAs resident at once.  A cluster stays within one group of SMs, and the groups' sizes
+// are no multiples of 4 and 8: 33 clusters of 4 and 15 of 8 with one CTA per SM (the occupancy query's answer and the
+// grids at which the time jumps), 70 and 33 with two (the grids at which it jumps).
+static int narrow_first(int split) { return split <= 2 ? kNwSms : split == 4 ? 132 : 120; }
+static int narrow_slots(int bt, int split) {
+  if (!narrow_two_per_sm(bt)) return narrow_first(split);
+  return split <= 2 ? 2 * kNwSms : split == 4 ? 280 : 264;
+}
+static double narrow_plan(int M, long long n_tiles, int K, bool ragged_x, bool ragged_w, int* bt_out, int* split_out) {
   const int num_kb = (K + kNwBK - 1) / kNwBK, fewest = (M + 255) / 256;
   double best = 1e30;
   for (int tm = fewest; tm < fewest + 9; ++tm) {
     const int bt = ((M + tm - 1) / tm + 15) / 16 * 16;
     if (tm > fewest && bt < 48) break;
-    const int slots = kNwSms * (narrow_two_per_sm(bt) ? 2 : 1);
+    const int per_sm_most = narrow_two_per_sm(bt) ? 2 : 1;
     for (int split = 1; split <= 8 && split <= num_kb; split *= 2) {
       const long long ctas = (long long)((M + bt - 1) / bt) * n_tiles * split;
       const double steps = (num_kb + split - 1) / split;
+      const int slots = narrow_slots(bt, split), first = narrow_first(split);
       auto wave = [&](long long n) {
         if (n == 0) return 0.0;
-        const double per_sm = (double)((n + kNwSms - 1) / kNwSms);
+        const long long rounds = (n + first - 1) / first;
+        const double per_sm = (double)(rounds < per_sm_most ? rounds : per_sm_most);
         double step = per_sm * (0.142 + 0.00044 * bt);
         if (step < 0.32 + 0.00027 * bt) step = 0.32 + 0.00027 * bt;
         if (step < n * 0.00122) step = n * 0.00122;
+        if (ragged_x || ragged_w) {
+          const double bytes = kNwWBytes * (ragged_w ? 1.86 : 1.0) + bt * kNwBK * 2 * (ragged_x ? 1.55 : 1.0);
+          if (step < n * bytes / 21e6) step = n * bytes / 21e6;
+        }
         return 4.6 + steps * step + per_sm * bt * (0.0126 + (split > 1 ? 0.0045 * split : 0.0)) + (split == 8 ? 0.26 : 0.0);
       };
       const double t = 1.5 + (double)(ctas / slots) * wave(slots) + wave(ctas % slots);
@@ -320,11 +342,12 @@ KSA_API int ksa_gemm_narrow_bf16(const void* x, const void* w, void* c, int M, i
 
 // Whether this kernel is expected to beat the tiled ones (of which CTA pairs are taken from `pair_min_tiles` 256 x 256 tiles on, 0:
 // never), by more than the model's error: bt * 16 + split for ksa_gemm_narrow_bf16, or 0.  glu: the separate activation
-// kernel, 2 us and more, counts on the other side.
-KSA_API int ksa_gemm_narrow_plan(int M, int N, int K, int glu, int pair_min_tiles) {
+// kernel, 2 us and more, counts on the other side.  ragged: bit 0, the activations' rows do not all start on a 128-byte line (their
+// pitch is no multiple of 64 elements); bit 1, those of the weights as they lie in memory.
+KSA_API int ksa_gemm_narrow_plan(int M, int N, int K, int glu, int pair_min_tiles, int ragged) {
   using namespace ksa;
   if (M <= 0 || M > kNwMaxRows || N <= 0 || K <= 0) return 0;
   int bt = 0, split = 0;
-  const double t = narrow_plan(M, glu ? (N / 2 + 63) / 64 : (N + 127) / 128, K, &bt, &split);
+  const double t = narrow_plan(M, glu ? (N / 2 + 63) / 64 : (N + 127) / 128, K, (ragged & 1) != 0, (ragged & 2) != 0, &bt, &split);
   return t < 0.95 * (tiled_time(M, N, K, pair_min_tiles) + (glu ? 2.0 : 0.0)) ? bt * 16 + split : 0;
 }

@@ -67,12 +67,17 @@ def _run(fn, *args):
     return fn.forward(_NoGrad(), *args)
 
 
+def _ragged(x: torch.Tensor, w: torch.Tensor) -> int:
+    """Which operands' rows do not all start on a 128-byte line (bit 0: ``x``, bit 1: ``w``)."""
+    return (x.stride(0) % 64 != 0) + 2 * (w.stride(0) % 64 != 0)
+
+
 def _narrow_swiglu(x: torch.Tensor, w13: torch.Tensor):
     """Plan of the split-K kernel for few rows with the activation, or None.  It takes feature counts in steps of 8; a
     parameter gather that waits for a GEMM to ride in, and observed calls, are left to separate calls."""
     if w13.shape[0] % 16 != 0 or _lib.pair_gather_pending() or _observed():
         return None
-    return _lib.gemm_narrow_plan(x.shape[0], w13.shape[0], x.shape[1], 1, GEMM_PAIR_MIN_TILES)
+    return _lib.gemm_narrow_plan(x.shape[0], w13.shape[0], x.shape[1], 1, GEMM_PAIR_MIN_TILES, _ragged(x, w13))
 
 
 def _require_bf16(*ts):
@@ -121,7 +126,7 @@ def gemm(a: torch.Tensor, b: torch.Tensor, *, a_mn_major: bool = False, b_mn_maj
         return out
     if pair is None and sm_limit == 0 and not a_mn_major and out.dtype == torch.bfloat16 and not accumulate:
         # too few tiles to occupy the chip: K is split as well (csrc/gemm_narrow.cu says when that is faster)
-        plan = _lib.gemm_narrow_plan(M, N, K, 0, GEMM_PAIR_MIN_TILES)
+        plan = _lib.gemm_narrow_plan(M, N, K, 0, GEMM_PAIR_MIN_TILES, _ragged(a, b))
         if plan is not None:
             _lib.call("ksa_gemm_narrow_bf16", a, b, out, M, N, K, a.stride(0), b.stride(0), out.stride(0), int(b_mn_major), 0,
                       plan[0], plan[1], float(alpha))

@@ -97,7 +97,7 @@ def load() -> ctypes.CDLL:
     lib.ksa_rmsnorm_bwd_parts.restype = I
     lib.ksa_attn_bwd_num_segments.argtypes = [I]
     lib.ksa_attn_bwd_num_segments.restype = I
-    lib.ksa_gemm_narrow_plan.argtypes = [I] * 5
+    lib.ksa_gemm_narrow_plan.argtypes = [I] * 6
     lib.ksa_gemm_narrow_plan.restype = I
     lib.ksa_set_dependent_launch.argtypes = [I]
     lib.ksa_set_dependent_launch.restype = I
@@ -251,9 +251,10 @@ def set_dependent_launch(on: bool) -> bool:
 
 
 @functools.lru_cache(maxsize=4096)
-def gemm_narrow_plan(M: int, N: int, K: int, glu: int, pair_min_tiles: int):
-    """``(activation rows per tile, split of K)`` for ``ksa_gemm_narrow_bf16``, or None where a tiled kernel is faster."""
-    plan = load().ksa_gemm_narrow_plan(M, N, K, glu, pair_min_tiles)
+def gemm_narrow_plan(M: int, N: int, K: int, glu: int, pair_min_tiles: int, ragged: int = 0):
+    """``(activation rows per tile, split of K)`` for ``ksa_gemm_narrow_bf16``, or None where a tiled kernel is faster.
+    ``ragged``: bit 0 for activations, bit 1 for weights whose row pitch is no multiple of 64 elements."""
+    plan = load().ksa_gemm_narrow_plan(M, N, K, glu, pair_min_tiles, ragged)
     return (plan // 16, plan % 16) if plan else None
 
 

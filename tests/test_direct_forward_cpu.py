@@ -171,7 +171,7 @@ def test_norm_linear_refuses_other_widths(width, glu, recorder):
 def test_linear_swiglu_asks_for_its_plan_once(requires, recorder, monkeypatch):
     """Once where it can use the answer, not at all where the call is differentiated (the projection asks for its own)."""
     asked = []
-    monkeypatch.setattr(_lib, "gemm_narrow_plan", lambda M, N, K, glu, tiles: asked.append(glu) or (32, 1))
+    monkeypatch.setattr(_lib, "gemm_narrow_plan", lambda M, N, K, glu, *rest: asked.append(glu) or (32, 1))
     ops.linear_swiglu(_bf(32, 64).requires_grad_(requires), _W["w"])
     assert asked == ([0] if requires else [1])
 
