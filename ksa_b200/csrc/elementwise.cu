@@ -353,7 +353,10 @@ __global__ void __launch_bounds__(256) qknorm_rope_bwd_kernel(QkRopeBwdArgs b) {
 
 // ---- head_dim 128: in the forward direction a warp takes kRopeHeads heads of a row, all requested at once (a row's 24 to
 // 48 heads in one warp are a serial chain of load, reduction and store that leaves the memory idle; the sines and
-// cosines are cheap to work out again: 1411 rows x 32 heads 13.8 -> 9.3 us, 8256 rows 41.0 -> 36.6 us).  The backward
+// cosines are cheap to work out again: 1411 rows x 32 heads 13.8 -> 9.3 us, 8256 rows 41.0 -> 36.6 us).  A row of up to four
+// heads (a rank of a tensor-parallel group) takes four requests: eight cost 2.7 us at 500 rows x 3 heads and 6.5 at 8256, four 2.3
+// and 5.5 (a warp per row in batches of four 2.5 and 5.8).  One size is slower than a warp per row: 9 to 12 heads at some 3300
+// rows, whose second half a wave starts late (8.0 -> 8.6 us).  The backward
 // kernel, whose warps carry weight-gradient sums from row to row, walks whole rows (cut the same way it was slower, 52.1
 // against 55.7 us at 8256 rows).  A lane owns two 32-bit words A and B of every head
 // (half-split rotary: elements {2l, 2l+1} and {2l+64, 2l+65}; interleaved: {4l, 4l+1} and {4l+2, 4l+3}), i.e. the
@@ -398,32 +401,32 @@ __device__ __forceinline__ void rope_pair_idx(int p, int& i1, int& i2) {
   else { i1 = p; i2 = p + 2; }
 }
 
-template <bool IL>
+template <bool IL, int NH>      // NH: heads of a row that a warp takes
 __global__ void __launch_bounds__(256) qknorm_rope_fwd128_kernel(QkRopeArgs a) {
   grid_dependency_launch();   // a dependent-launched successor may start (the skinny GEMM: its weight loads)
   grid_dependency_wait();     // launched dependently itself: the previous kernel's results are complete from here on
   const int lane = threadIdx.x & 31;
   const int H = a.Hq + a.Hkv;
   const int Hall = H + (a.copy_v ? a.Hkv : 0);
-  const int groups = rope_groups(Hall);
+  const int groups = NH < kRopeHeads ? 1 : rope_groups(Hall);      // fewer only where they are the whole row
   const long long item = (long long)blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5);
   if (item >= (long long)a.rows * groups) return;
-  const int row = (int)(item / groups), head0 = (int)(item - (long long)row * groups) * kRopeHeads;
-  const int head1 = min(head0 + kRopeHeads, Hall);
+  const int row = (int)(item / groups), head0 = (int)(item - (long long)row * groups) * NH;
+  const int head1 = min(head0 + NH, Hall);
   const RopeLane r = rope_lane_setup(a, row, lane);
   const uint32_t* src = reinterpret_cast<const uint32_t*>(a.qkv + (long long)row * a.in_stride);
   uint32_t* dst = reinterpret_cast<uint32_t*>(a.out + (long long)row * a.out_stride);
   {
     const int h0 = head0;
-    uint32_t ua[kRopeHeads], ub[kRopeHeads];
+    uint32_t ua[NH], ub[NH];
 #pragma unroll
-    for (int u = 0; u < kRopeHeads; ++u) {
+    for (int u = 0; u < NH; ++u) {
       const int head = min(h0 + u, Hall - 1);
       ua[u] = src[head * 64 + r.offA];
       ub[u] = src[head * 64 + r.offB];
     }
 #pragma unroll
-    for (int u = 0; u < kRopeHeads; ++u) {
+    for (int u = 0; u < NH; ++u) {
       const int head = h0 + u;
       if (head >= head1) break;
       if (head >= H) {      // v head: plain copy
@@ -867,14 +870,17 @@ KSA_API int ksa_qknorm_rope_fwd(const void* qkv, void* out, const void* q_w, con
                in_stride, out_stride, rows, Hq, Hkv, D, log2f(theta), eps, interleaved, copy_v};
   const long long warps = (long long)rows * (Hq + Hkv + (copy_v ? Hkv : 0));
   const int blocks = (int)((warps + 7) / 8);
-  const int blocks128 = (int)(((long long)rows * rope_groups(Hq + Hkv + (copy_v ? Hkv : 0)) + 7) / 8);
+  const int heads = Hq + Hkv + (copy_v ? Hkv : 0);
+  const int blocks128 = (int)(((long long)rows * rope_groups(heads) + 7) / 8);
   const bool dep = dependent_launch_enabled();
-  if (D == 128 && interleaved)
-    KSA_CHECK_CUDA(launch_kernel(dep, qknorm_rope_fwd128_kernel<true>, dim3(blocks128), dim3(256), 0, ST(stream), a));
-  else if (D == 128)
-    KSA_CHECK_CUDA(launch_kernel(dep, qknorm_rope_fwd128_kernel<false>, dim3(blocks128), dim3(256), 0, ST(stream), a));
-  else
+  const bool few = heads <= 4;
+  if (D == 128) {
+    auto kern = interleaved ? (few ? qknorm_rope_fwd128_kernel<true, 4> : qknorm_rope_fwd128_kernel<true, kRopeHeads>)
+                            : (few ? qknorm_rope_fwd128_kernel<false, 4> : qknorm_rope_fwd128_kernel<false, kRopeHeads>);
+    KSA_CHECK_CUDA(launch_kernel(dep, kern, dim3(blocks128), dim3(256), 0, ST(stream), a));
+  } else {
     KSA_CHECK_CUDA(launch_kernel(dep, qknorm_rope_fwd_kernel<64>, dim3(blocks), dim3(256), 0, ST(stream), a));
+  }
   return 0;
 }
 

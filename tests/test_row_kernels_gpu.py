@@ -61,3 +61,21 @@ def test_qk_norm_rope_head_counts(Hq, Hkv, rows, interleaved):
     assert torch.equal(out[:, (Hq + Hkv) * D:], qkv[:, (Hq + Hkv) * D:])
     for got, exp in ((xs.grad, xf.grad), (qs.grad, qf.grad), (ks.grad, kf.grad)):
         assert (got.float() - exp).norm() < 1e-2 * exp.norm()
+
+
+@pytest.mark.parametrize("Hq,Hkv", [(1, 1), (2, 1), (3, 1), (2, 2)])
+@pytest.mark.parametrize("rows", [1, 9, 300])
+@pytest.mark.parametrize("interleaved", [False, True])
+def test_rope_of_few_heads(Hq, Hkv, rows, interleaved):
+    """Rows of up to four heads have a kernel of their own: a head's result is that of the same head in a wide row."""
+    D = 128
+    wide, pos = bf(rows, 16 * D), torch.randint(0, 5000, (rows,), device=DEV)           # 8 q heads, 4 k heads, 4 v heads
+    wq, wk = [(1 + 0.1 * torch.randn(D, device=DEV)).bfloat16() for _ in range(2)]
+
+    def few(t):
+        return torch.cat([t[:, :Hq * D], t[:, 8 * D:(8 + Hkv) * D], t[:, 12 * D:(12 + Hkv) * D]], 1)
+
+    want = ops.qk_norm_rope_packed(wide, wq, wk, pos, 8, 4, D, 1e6, 1e-6, interleaved)
+    got = ops.qk_norm_rope_packed(few(wide), wq, wk, pos, Hq, Hkv, D, 1e6, 1e-6, interleaved)
+    _lib.check_status()
+    assert torch.equal(got, few(want))
