@@ -79,3 +79,10 @@ def test_rope_of_few_heads(Hq, Hkv, rows, interleaved):
     got = ops.qk_norm_rope_packed(few(wide), wq, wk, pos, Hq, Hkv, D, 1e6, 1e-6, interleaved)
     _lib.check_status()
     assert torch.equal(got, few(want))
+
+
+@pytest.mark.parametrize("rows", [148, 149, 295, 296, 297, 592, 593])
+@pytest.mark.parametrize("D", [2048, 2560])
+def test_rms_norm_backward_rounds(rows, D):
+    """Row counts at which the number of CTAs and of their rounds changes."""
+    test_rms_norm_backward(rows, D, True)
