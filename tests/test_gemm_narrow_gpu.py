@@ -96,3 +96,32 @@ def test_plans_that_were_slower_than_tiles(M, N, K, ragged, slow):
         w = (torch.randn(N, K, device="cuda") * 0.1).bfloat16()
         _check(ops.gemm(x, w), x, w)
         _lib.check_status()
+
+
+@pytest.mark.parametrize("M,N,K,fused", [(48, 19456, 2560, True), (333, 1040, 1032, True), (129, 272, 2048, True),
+                                         (48, 272, 64, False), (2047, 12288, 2048, False), (2049, 256, 2048, False)])
+def test_linear_swiglu_takes_the_gated_kernel(M, N, K, fused):
+    """One launch where there is a plan for the gated form, the projection and the activation where there is none (too little
+    or too much work, too many rows)."""
+    torch.manual_seed(M)
+    x = torch.randn(M, K, device="cuda").bfloat16()
+    w = (torch.randn(N, K, device="cuda") * 0.1).bfloat16()
+    plan = _lib.gemm_narrow_plan(M, N, K, 1, ops.GEMM_PAIR_MIN_TILES, 3 * (K % 64 != 0))
+    assert (plan is not None) == fused
+    with torch.no_grad():
+        before = _lib.launch_count()
+        h = ops.linear_swiglu(x, w)
+        assert _lib.launch_count() - before == (1 if fused else 2)
+    _lib.check_status()
+    _check(h, x, w, glu=True)
+
+
+@pytest.mark.parametrize("N,ldc,w_mn,glu,offset", [(132, 136, 0, 0, 0), (128, 132, 0, 0, 0), (136, 136, 0, 1, 0),
+                                                   (128, 128, 1, 1, 0), (128, 128, 0, 0, 4)])
+def test_rejects_bad_outputs_and_layouts(N, ldc, w_mn, glu, offset):
+    """Rows of C off 16 bytes, feature counts the gated form does not pair, gated weights in the other layout."""
+    x = torch.zeros(32, 64, device="cuda", dtype=torch.bfloat16)
+    w = torch.zeros(144, 144, device="cuda", dtype=torch.bfloat16)
+    c = torch.empty(32 * 144 + 8, device="cuda", dtype=torch.bfloat16)[offset:]
+    with pytest.raises(RuntimeError, match="gemm_narrow"):
+        _lib.call("ksa_gemm_narrow_bf16", x, w, c, 32, N, 64, 64, 144, ldc, w_mn, glu, 32, 1, 1.0)
