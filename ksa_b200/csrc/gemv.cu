@@ -367,8 +367,11 @@ namespace ksa {
 template <bool kGlu>
 static int gemv_dispatch(const void* a, const void* b, void* c, int M, int N, int K, long long lda, long long ldb,
                          long long ldc, cudaStream_t st, const GemvNorm& nrm = GemvNorm{}) {
-  // three and four rows as well while 16 weight rows a CTA give every SM one (4 rows x 151936 x 2560: 173 -> 147 us, x 6144 x 2560:
-  // 16.3 -> 10.0, x 2560 x 4096: 11.9 -> 11.0; below, 4 x 2048 x 6144, 13.6 against 14.0)
+  // Three and four rows as well while 16 weight rows a CTA give every SM one.  Scalar and tensor-core times in us at three and at
+  // four rows: 151936 x 2560 172 / 134, 173 / 141; 19456 x 2560 30.4 / 24.8, 30.5 / 25.4; 6144 x 2560 16.1 / 9.9, 16.3 / 9.9;
+  // 2560 x 4096 11.6 / 10.3, 11.9 / 10.5; at the line, 2368 x 2560, 7.6 / 7.0, 7.8 / 7.1.  Below it, 2048 x 6144, 13.2 and 13.6
+  // against 14.0.  One and two rows stay scalar (two rows x 6144 x 2560 11.5).  The error against 64 bits is that of the one
+  // rounding to bf16 in both (0.00166 over ten seeds, 3 and 4 rows x 6144 x 2560).
   if ((M > 4 || (M > 2 && N >= 148 * 16)) && K % 32 == 0 && nrm.w == nullptr) {
     if (N >= 16384)   // wide outputs: 32 weight rows per CTA still give every SM several CTAs
       return M <= 8 ? launch_gemv_mma<1, kGlu, 2>(a, b, c, M, N, K, lda, ldb, ldc, st)

@@ -121,7 +121,9 @@ def gemm(a: torch.Tensor, b: torch.Tensor, *, a_mn_major: bool = False, b_mn_maj
     if (M <= 16 and not a_mn_major and not b_mn_major and out.dtype == torch.bfloat16 and not accumulate
             and alpha == 1.0 and K % 8 == 0):
         # decoding: a few activation rows against a whole weight matrix is a stream of the weights, served by the
-        # bandwidth-shaped kernel instead of 128-row tensor-core tiles
+        # bandwidth-shaped kernel instead of 128-row tensor-core tiles.  16 rows is where that kernel ends and not where the split-K
+        # kernel below starts to pay: 16 rows x 6144 x 2560 take 15.7 us here and 11.9 there, x 2560 x 9728 25.1 and 15.4, x 19456 x
+        # 2560 37.1 and 22.3; but 8 rows x 6144 x 2560 10.6 and 11.5, 16 x 4096 x 2048 7.8 and 9.2, x 2048 x 2048 5.9 and 8.5
         _lib.call("ksa_gemv_bf16", a, b, out, M, N, K, a.stride(0), b.stride(0), out.stride(0))
         return out
     if pair is None and sm_limit == 0 and not a_mn_major and out.dtype == torch.bfloat16 and not accumulate:
