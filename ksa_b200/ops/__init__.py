@@ -50,13 +50,14 @@ class _NoGrad:
 # private to PyTorch: without them every call counts as observed
 _transforms_active = getattr(torch._C, "_are_functorch_transforms_active", lambda: True)
 _forward_level = functools.partial(getattr, torch.autograd.forward_ad, "_current_level", 0)
+_is_tracing, _is_compiling = torch.jit.is_tracing, torch.compiler.is_compiling
 
 
 def _observed() -> bool:
     """Whether someone follows the calls themselves: a ``torch.func`` transform, forward-mode differentiation, a trace, a compiler.
     They must meet the autograd function (its error, or its node in their graph) and not the bare kernel call, which would take
     the wrappers' memory for that of their tensors."""
-    return _transforms_active() or _forward_level() >= 0 or torch.jit.is_tracing() or torch.compiler.is_compiling()
+    return _transforms_active() or _forward_level() >= 0 or _is_tracing() or _is_compiling()
 
 
 def _run(fn, *args):
@@ -67,17 +68,13 @@ def _run(fn, *args):
     return fn.forward(_NoGrad(), *args)
 
 
-def _ragged(x: torch.Tensor, w: torch.Tensor) -> int:
-    """Which operands' rows do not all start on a 128-byte line (bit 0: ``x``, bit 1: ``w``)."""
-    return (x.stride(0) % 64 != 0) + 2 * (w.stride(0) % 64 != 0)
-
-
 def _narrow_swiglu(x: torch.Tensor, w13: torch.Tensor):
     """Plan of the split-K kernel for few rows with the activation, or None.  It takes feature counts in steps of 8; a
     parameter gather that waits for a GEMM to ride in, and observed calls, are left to separate calls."""
     if w13.shape[0] % 16 != 0 or _lib.pair_gather_pending() or _observed():
         return None
-    return _lib.gemm_narrow_plan(x.shape[0], w13.shape[0], x.shape[1], 1, GEMM_PAIR_MIN_TILES, _ragged(x, w13))
+    return _lib.gemm_narrow_plan(x.shape[0], w13.shape[0], x.shape[1], 1, GEMM_PAIR_MIN_TILES,
+                                 (x.stride(0) % 64 != 0) + 2 * (w13.stride(0) % 64 != 0))
 
 
 def _require_bf16(*ts):
@@ -128,10 +125,11 @@ def gemm(a: torch.Tensor, b: torch.Tensor, *, a_mn_major: bool = False, b_mn_maj
         return out
     if pair is None and sm_limit == 0 and not a_mn_major and out.dtype == torch.bfloat16 and not accumulate:
         # too few tiles to occupy the chip: K is split as well (csrc/gemm_narrow.cu says when that is faster)
-        plan = _lib.gemm_narrow_plan(M, N, K, 0, GEMM_PAIR_MIN_TILES, _ragged(a, b))
+        lda, ldb = a.stride(0), b.stride(0)
+        plan = _lib.gemm_narrow_plan(M, N, K, 0, GEMM_PAIR_MIN_TILES, (lda % 64 != 0) + 2 * (ldb % 64 != 0))
         if plan is not None:
-            _lib.call("ksa_gemm_narrow_bf16", a, b, out, M, N, K, a.stride(0), b.stride(0), out.stride(0), int(b_mn_major), 0,
-                      plan[0], plan[1], float(alpha))
+            _lib.call("ksa_gemm_narrow_bf16", a, b, out, M, N, K, lda, ldb, out.stride(0), int(b_mn_major), 0, *plan,
+                      float(alpha))
             return out
     if pair is None:
         pair = (GEMM_PAIR_MIN_TILES > 0 and sm_limit == 0

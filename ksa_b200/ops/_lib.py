@@ -122,16 +122,21 @@ _STATUS_TEXT = {
 
 
 def _ptr(x):
-    if x is None:
-        return None
     if isinstance(x, torch.Tensor):
         if not x.is_cuda:  # a host pointer handed to a kernel is an illegal access on the device
             raise TypeError("a CPU tensor was passed to an sm_100a kernel entry point")
+        try:
+            p = x.data_ptr()
+            if p:
+                return p
+        except RuntimeError:
+            pass
         return _address(x)
     return x
 
 
 def _address(x: torch.Tensor) -> int:
+    """The address of ``x`` where it is not simply ``x.data_ptr()``."""
     try:
         p = x.data_ptr()
     except RuntimeError:      # a wrapper: the tensor inside counts if its transform has ended, as in ``Function.apply``
