@@ -3,7 +3,8 @@
 ``python -m ksa_b200.csrc.build`` compiles every ``.cu`` next to this file for
 ``compute_100a/sm_100a`` and links ``ksa_b200/_lib/libksa_b200.so``.  Objects are
 rebuilt only when a source or header is newer.  The library exposes plain C
-entry points; ``ksa_b200.ops._lib`` binds them with ctypes.
+entry points; ``ksa_b200.ops._lib`` binds them with ctypes.  ``native.cpp`` (the ordinary operator calls, on top of those
+entry points) is compiled by the host compiler into ``ksa_b200/_lib/ksa_native.so``.
 """
 from __future__ import annotations
 
@@ -64,6 +65,35 @@ def _compile(src: Path, force: bool, verbose: bool) -> Path:
     return obj
 
 
+def _compile_native(force: bool) -> Path:
+    """The operator calls in native code: the one file that knows torch, linked to the kernel library beside it."""
+    import sysconfig
+
+    import torch
+
+    src, out = CSRC / "native.cpp", LIB_DIR / "ksa_native.so"
+    stamp = OBJ_DIR / "native.txt"
+    built_for = f"{torch.__version__} {sys.version}"
+    if (not force and out.exists() and out.stat().st_mtime >= src.stat().st_mtime and stamp.exists()
+            and stamp.read_text() == built_for):
+        return out
+    lib = Path(torch.__file__).parent / "lib"
+    inc = Path(torch.__file__).parent / "include"
+    cuda = Path(_nvcc()).resolve().parents[1]
+    tmp = out.with_suffix(".so.tmp")
+    cmd = [os.environ.get("CXX") or "g++", "-O2", "-std=c++17", "-fPIC", "-shared", "-fvisibility=hidden", "-Wall",
+           f"-D_GLIBCXX_USE_CXX11_ABI={int(torch.compiled_with_cxx11_abi())}", "-isystem", str(inc),
+           "-isystem", str(inc / "torch" / "csrc" / "api" / "include"), "-isystem", str(cuda / "include"),
+           "-isystem", sysconfig.get_paths()["include"], str(src), "-o", str(tmp), str(LIB_PATH), f"-L{lib}",
+           "-ltorch_python", "-ltorch", "-ltorch_cpu", "-ltorch_cuda", "-lc10", "-lc10_cuda", "-Wl,-rpath,$ORIGIN"]
+    r = subprocess.run(cmd, capture_output=True, text=True)
+    if r.returncode != 0:
+        raise RuntimeError(f"{cmd[0]} failed on {src.name}:\n{r.stdout}\n{r.stderr}")
+    os.replace(tmp, out)
+    stamp.write_text(built_for)
+    return out
+
+
 def build(force: bool = False, verbose: bool = False) -> Path:
     OBJ_DIR.mkdir(exist_ok=True)
     LIB_DIR.mkdir(exist_ok=True)
@@ -79,11 +109,12 @@ def build(force: bool = False, verbose: bool = False) -> Path:
     newest_obj = max(o.stat().st_mtime for o in objs)
     if force or not LIB_PATH.exists() or LIB_PATH.stat().st_mtime < newest_obj:
         tmp = LIB_PATH.with_suffix(".so.tmp")
-        cmd = [_nvcc(), "-shared", "-o", str(tmp), *map(str, objs)]
+        cmd = [_nvcc(), "-shared", "-Xlinker", f"-soname={LIB_PATH.name}", "-o", str(tmp), *map(str, objs)]
         r = subprocess.run(cmd, capture_output=True, text=True)
         if r.returncode != 0:
             raise RuntimeError(f"link failed:\n{r.stdout}\n{r.stderr}")
         os.replace(tmp, LIB_PATH)
+    _compile_native(force)
     return LIB_PATH
 
 

@@ -28,6 +28,7 @@ import torch
 
 from . import reference as ref
 from . import _lib
+from ._lib import native as _native
 from .layout import SummaryLayout, get_layout
 
 UNBOUNDED_WINDOW = 1 << 30
@@ -94,6 +95,11 @@ def gemm(a: torch.Tensor, b: torch.Tensor, *, a_mn_major: bool = False, b_mn_maj
     ``[K,N]`` when ``b_mn_major``).  Row strides may exceed the row length
     (views of packed buffers); the last dimension must be contiguous.
     """
+    if pair is None and sm_limit == 0 and alpha == 1.0 and not _lib.pair_gather_pending():
+        c = _native.gemm(a, b, out, (out_dtype if out is None else out.dtype) == torch.float32, a_mn_major, b_mn_major,
+                         accumulate, GEMM_PAIR_MIN_TILES)
+        if c is not None:
+            return c
     _require_bf16(a, b)
     assert a.dim() == 2 and b.dim() == 2 and a.stride(1) == 1 and b.stride(1) == 1
     M, K = (a.shape[1], a.shape[0]) if a_mn_major else (a.shape[0], a.shape[1])
@@ -185,15 +191,29 @@ def _weight_grad(weight: torch.Tensor, compute):
     return compute(None, False)
 
 
+def _linear_weight_grad(weight: torch.Tensor, dy: torch.Tensor, x: torch.Tensor, lo: int, hi: int):
+    """The gradient of ``weight`` in ``x[lo:hi] @ weight.T``, routed by :func:`_weight_grad`."""
+    def compute(out, acc):
+        dw = _native.linear_dw(dy, x, lo, hi, out, acc, GEMM_PAIR_MIN_TILES)
+        if dw is not None:
+            return dw
+        return gemm(dy[lo:hi], x[lo:hi], a_mn_major=True, b_mn_major=True, out=out, accumulate=acc)
+    return _weight_grad(weight, compute)
+
+
 class _LinearFn(torch.autograd.Function):
     @staticmethod
     def forward(ctx, x, weight):
+        ctx.x_shape = x.shape
+        y = None if _lib.pair_gather_pending() else _native.linear(x, weight, GEMM_PAIR_MIN_TILES)
+        if y is not None:
+            ctx.save_for_backward(x if x.dim() == 2 else x.reshape(-1, x.shape[-1]), weight)
+            return y
         x2 = x.reshape(-1, x.shape[-1])
         if x2.stride(1) != 1:
             x2 = x2.contiguous()
         y = gemm(x2, weight)
         ctx.save_for_backward(x2, weight)
-        ctx.x_shape = x.shape
         return y.view(*x.shape[:-1], weight.shape[0])
 
     @staticmethod
@@ -206,11 +226,7 @@ class _LinearFn(torch.autograd.Function):
         if ctx.needs_input_grad[0]:
             dx = gemm(dy2, weight, b_mn_major=True).view(ctx.x_shape)
         if ctx.needs_input_grad[1]:
-            def compute(out, acc):
-                if out is None:
-                    return gemm(dy2, x2, a_mn_major=True, b_mn_major=True)
-                gemm(dy2, x2, a_mn_major=True, b_mn_major=True, out=out, accumulate=acc)
-            dw = _weight_grad(weight, compute)
+            dw = _linear_weight_grad(weight, dy2, x2, 0, x2.shape[0])
         return dx, dw
 
 
@@ -218,6 +234,10 @@ def linear(x: torch.Tensor, weight: torch.Tensor, bias: Optional[torch.Tensor] =
     """``x @ weight.T (+ bias)``; the CUDA path is the tcgen05 GEMM for forward, dX and dW."""
     if not _cuda(x):
         return ref.linear(x, weight, bias)
+    if not _observed() and not _lib.pair_gather_pending():       # nobody differentiates it: one call
+        y = _native.linear(x, weight, GEMM_PAIR_MIN_TILES)
+        if y is not None:
+            return y if bias is None else y + bias
     _require_bf16(x, weight)
     y = _run(_LinearFn, x, weight)
     return y if bias is None else y + bias
@@ -229,11 +249,13 @@ class _DualLinearFn(torch.autograd.Function):
     @staticmethod
     def forward(ctx, x, w_a, w_b, n_a):
         R = x.shape[0]
-        y = torch.empty((R, w_a.shape[0]), dtype=x.dtype, device=x.device)
-        if n_a > 0:
-            gemm(x[:n_a], w_a, out=y[:n_a])
-        if R > n_a:
-            gemm(x[n_a:], w_b, out=y[n_a:])
+        y = None if _lib.pair_gather_pending() else _native.dual_linear(x, w_a, w_b, n_a, 0, GEMM_PAIR_MIN_TILES)
+        if y is None:
+            y = torch.empty((R, w_a.shape[0]), dtype=x.dtype, device=x.device)
+            if n_a > 0:
+                gemm(x[:n_a], w_a, out=y[:n_a])
+            if R > n_a:
+                gemm(x[n_a:], w_b, out=y[n_a:])
         ctx.save_for_backward(x, w_a, w_b)
         ctx.n_a = n_a
         return y
@@ -245,23 +267,19 @@ class _DualLinearFn(torch.autograd.Function):
         dy = dy if dy.is_contiguous() else dy.contiguous()
         dx = None
         if ctx.needs_input_grad[0]:
-            dx = torch.empty_like(x)
-            if n_a > 0:
-                gemm(dy[:n_a], w_a, b_mn_major=True, out=dx[:n_a])
-            if R > n_a:
-                gemm(dy[n_a:], w_b, b_mn_major=True, out=dx[n_a:])
+            dx = _native.dual_linear(dy, w_a, w_b, n_a, 1, GEMM_PAIR_MIN_TILES)
+            if dx is None:
+                dx = torch.empty_like(x)
+                if n_a > 0:
+                    gemm(dy[:n_a], w_a, b_mn_major=True, out=dx[:n_a])
+                if R > n_a:
+                    gemm(dy[n_a:], w_b, b_mn_major=True, out=dx[n_a:])
         grads = []
         for need, w, lo, hi in ((ctx.needs_input_grad[1], w_a, 0, n_a), (ctx.needs_input_grad[2], w_b, n_a, R)):
             if not need or hi <= lo:
                 grads.append(None)
                 continue
-            dys, xs = dy[lo:hi], x[lo:hi]
-
-            def compute(out, acc, dys=dys, xs=xs):
-                if out is None:
-                    return gemm(dys, xs, a_mn_major=True, b_mn_major=True)
-                gemm(dys, xs, a_mn_major=True, b_mn_major=True, out=out, accumulate=acc)
-            grads.append(_weight_grad(w, compute))
+            grads.append(_linear_weight_grad(w, dy, x, lo, hi))
         return dx, grads[0], grads[1], None
 
 
@@ -276,6 +294,12 @@ def dual_linear(x: torch.Tensor, w_a: torch.Tensor, w_b: torch.Tensor, n_a: int)
 
 # =============================================================================== RMSNorm
 def _rmsnorm_backward(res, weight, rstd, dy, dres, shape):
+    mg = getattr(weight, "main_grad", None)
+    if mg is not None:
+        dx = _native.rms_norm_bwd(dy, res, weight, rstd, dres, mg, getattr(weight, "_grad_written", False))
+        if dx is not None:
+            weight._grad_written = True
+            return dx.view(shape), None
     rows, D = res.shape
     dy2 = dy.reshape(-1, D)
     dy2 = dy2 if dy2.is_contiguous() else dy2.contiguous()
@@ -303,6 +327,13 @@ class _AddRmsNormFn(torch.autograd.Function):
 
     @staticmethod
     def forward(ctx, x, delta, weight, eps):
+        ctx.shape = x.shape
+        ctx.delta_shape = delta.shape
+        made = _native.rms_norm(x, delta, weight, eps)
+        if made is not None:
+            res, y, rstd = made
+            ctx.save_for_backward(res, weight, rstd)
+            return res.view(x.shape), y
         D = x.shape[-1]
         x2 = x.reshape(-1, D)
         rows = x2.shape[0]
@@ -312,8 +343,6 @@ class _AddRmsNormFn(torch.autograd.Function):
         d2 = delta.reshape(-1, D)
         _lib.call("ksa_rmsnorm_fwd", x2, d2, weight, res, y, rstd, rows, D, float(eps), d2.shape[0])
         ctx.save_for_backward(res, weight, rstd)
-        ctx.shape = x.shape
-        ctx.delta_shape = delta.shape
         return res.view(x.shape), y.view(x.shape)
 
     @staticmethod
@@ -332,6 +361,12 @@ class _AddRmsNormFn(torch.autograd.Function):
 class _RmsNormFn(torch.autograd.Function):
     @staticmethod
     def forward(ctx, x, weight, eps):
+        made = _native.rms_norm(x, None, weight, eps)
+        if made is not None:
+            y, rstd = made
+            ctx.save_for_backward(x, weight, rstd)
+            ctx.shape = x.shape
+            return y
         D = x.shape[-1]
         x2 = x.reshape(-1, D)
         rows = x2.shape[0]
@@ -383,11 +418,15 @@ class _QkNormRopeFn(torch.autograd.Function):
 
     @staticmethod
     def forward(ctx, qkv, q_w, k_w, pos, Hq, Hkv, D, theta, eps, interleaved):
-        T = qkv.shape[0]
-        out = torch.empty((T, (Hq + 2 * Hkv) * D), dtype=qkv.dtype, device=qkv.device)
-        rstd = torch.empty((T, Hq + Hkv), dtype=torch.float32, device=qkv.device)
-        _lib.call("ksa_qknorm_rope_fwd", qkv, out, q_w, k_w, pos, rstd, qkv.stride(0), out.stride(0), T, Hq, Hkv, D,
-                  float(theta), float(eps), int(interleaved), 1)
+        made = _native.qk_norm_rope(qkv, q_w, k_w, pos, Hq, Hkv, D, theta, eps, interleaved)
+        if made is not None:
+            out, rstd = made
+        else:
+            T = qkv.shape[0]
+            out = torch.empty((T, (Hq + 2 * Hkv) * D), dtype=qkv.dtype, device=qkv.device)
+            rstd = torch.empty((T, Hq + Hkv), dtype=torch.float32, device=qkv.device)
+            _lib.call("ksa_qknorm_rope_fwd", qkv, out, q_w, k_w, pos, rstd, qkv.stride(0), out.stride(0), T, Hq, Hkv, D,
+                      float(theta), float(eps), int(interleaved), 1)
         ctx.save_for_backward(qkv, q_w, k_w, pos, rstd)
         ctx.cfg = (Hq, Hkv, D, theta, eps, interleaved)
         return out
@@ -398,7 +437,6 @@ class _QkNormRopeFn(torch.autograd.Function):
         Hq, Hkv, D, theta, eps, interleaved = ctx.cfg
         T = qkv.shape[0]
         d_out = d_out if d_out.is_contiguous() else d_out.contiguous()
-        d_qkv = torch.empty_like(qkv)
         targets = []
         for w in (q_w, k_w):
             if w is None:
@@ -415,8 +453,11 @@ class _QkNormRopeFn(torch.autograd.Function):
         sinks = targets
         if _deterministic:     # the kernel's weight gradients are fp32 atomics: let them land in scratch vectors
             sinks = [None if t is None else torch.zeros(D, dtype=torch.float32, device=qkv.device) for t in targets]
-        _lib.call("ksa_qknorm_rope_bwd", qkv, d_out, d_qkv, q_w, k_w, pos, rstd, sinks[0], sinks[1],
-                  qkv.stride(0), d_out.stride(0), T, Hq, Hkv, D, float(theta), float(eps), int(interleaved), 1)
+        d_qkv = _native.qk_norm_rope_bwd(qkv, d_out, q_w, k_w, pos, rstd, sinks[0], sinks[1], Hq, Hkv, D, theta, eps, interleaved)
+        if d_qkv is None:
+            d_qkv = torch.empty_like(qkv)
+            _lib.call("ksa_qknorm_rope_bwd", qkv, d_out, d_qkv, q_w, k_w, pos, rstd, sinks[0], sinks[1],
+                      qkv.stride(0), d_out.stride(0), T, Hq, Hkv, D, float(theta), float(eps), int(interleaved), 1)
         if _deterministic:
             for t, g in zip(targets, _qk_norm_weight_grads(qkv, d_out, q_w, k_w, pos, *ctx.cfg)):
                 if t is not None:
@@ -475,6 +516,10 @@ def norm_linear(x: torch.Tensor, delta: Optional[torch.Tensor], norm_w: torch.Te
     rows then up rows).  Returns ``(res, y)``.  For at most 4 rows on a GPU without autograd (a decode step) this is
     one launch (``ksa_gemv_norm_bf16``: every CTA normalises the few activation rows itself while it stages them);
     everything else is ``add_rms_norm`` followed by the projection."""
+    if x.shape[0] <= 4 and _cuda(x) and not _observed():
+        made = _native.norm_linear(x, delta, norm_w, eps, weight, glu)
+        if made is not None:
+            return made
     if (_cuda(x) and x.dim() == 2 and weight.dim() == 2 and x.shape[1] == weight.shape[1] and x.shape[0] <= 4
             and x.dtype == torch.bfloat16 and weight.dtype == torch.bfloat16
             and not (torch.is_grad_enabled() and (x.requires_grad or weight.requires_grad))
@@ -524,6 +569,11 @@ def qk_norm_rope_decode(qkv: torch.Tensor, q_w: Optional[torch.Tensor], k_w: Opt
 class _SwiGluFn(torch.autograd.Function):
     @staticmethod
     def forward(ctx, gu):
+        out = _native.swiglu(gu)
+        if out is not None:
+            ctx.save_for_backward(gu if gu.dim() == 2 else gu.reshape(-1, gu.shape[-1]))
+            ctx.shape = gu.shape
+            return out
         F2 = gu.shape[-1]
         g2 = gu.reshape(-1, F2)
         out = torch.empty((g2.shape[0], F2 // 2), dtype=gu.dtype, device=gu.device)
@@ -535,6 +585,9 @@ class _SwiGluFn(torch.autograd.Function):
     @staticmethod
     def backward(ctx, dout):
         (g2,) = ctx.saved_tensors
+        dgu = _native.swiglu_bwd(g2, dout)
+        if dgu is not None:
+            return dgu.view(ctx.shape)
         d2 = dout.reshape(-1, dout.shape[-1])
         d2 = d2 if d2.is_contiguous() else d2.contiguous()
         dgu = torch.empty_like(g2)
@@ -556,6 +609,10 @@ def linear_swiglu(x: torch.Tensor, w13: torch.Tensor) -> torch.Tensor:
     decode step, a short prompt) applies the activation itself: ``ksa_gemv_swiglu_bf16`` for at most 16 rows, the gated form of
     ``ksa_gemm_narrow_bf16`` where ``gemm`` would take that kernel.  Everything else is the projection followed by
     ``swiglu``."""
+    if _cuda(x) and not _observed() and not _lib.pair_gather_pending():
+        out = _native.linear_swiglu(x, w13, GEMM_PAIR_MIN_TILES)
+        if out is not None:
+            return out
     if (_cuda(x) and x.dim() == 2 and w13.dim() == 2 and x.shape[1] == w13.shape[1]
             and x.dtype == torch.bfloat16 and w13.dtype == torch.bfloat16
             and not (torch.is_grad_enabled() and (x.requires_grad or w13.requires_grad))
@@ -846,6 +903,14 @@ class _PackedAttentionFn(torch.autograd.Function):
 
     @staticmethod
     def forward(ctx, qkv, B, L, Ns, Hq, Hkv, D, chunk, n_sum, window, tok_window, scale, doc_start=None, doc_end=None):
+        if doc_start is None and doc_end is None:
+            made = _native.attention(qkv, B, L, Ns, Hq, Hkv, D, chunk, n_sum, window, tok_window, scale)
+            if made is not None:
+                out, lse, lse_s = made
+                ctx.save_for_backward(qkv, out, lse, lse_s)
+                ctx.cfg = (B, L, Ns, Hq, Hkv, D, chunk, n_sum, window, tok_window, scale)
+                ctx.docs = (None, None)
+                return out
         R = B * (L + Ns)
         assert qkv.shape[0] == R and qkv.stride(1) == 1
         q, k, v = _packed_views(qkv, B, L, Hq, Hkv, D, 0)
@@ -877,6 +942,10 @@ class _PackedAttentionFn(torch.autograd.Function):
         qkv, out, lse, lse_s = ctx.saved_tensors
         B, L, Ns, Hq, Hkv, D, chunk, n_sum, window, tok_window, scale = ctx.cfg
         dout = dout if dout.is_contiguous() else dout.contiguous()
+        if not _deterministic and ctx.docs == (None, None):
+            dqkv = _native.attention_bwd(qkv, out, lse, lse_s, dout, B, L, Ns, Hq, Hkv, D, chunk, n_sum, window, tok_window, scale)
+            if dqkv is not None:
+                return (dqkv,) + (None,) * 13
         dqkv = torch.empty_like(qkv)
         rs, drs = qkv.stride(0), dqkv.stride(0)
         q, k, v = _packed_views(qkv, B, L, Hq, Hkv, D, 0)

@@ -9,8 +9,11 @@ from __future__ import annotations
 
 import ctypes
 import functools
+import importlib.machinery
+import importlib.util
 import os
 import threading
+import warnings
 from pathlib import Path
 from typing import Dict, Optional, Sequence
 
@@ -109,6 +112,30 @@ def load() -> ctypes.CDLL:
     _lib = lib
     return lib
 
+
+class NotBuilt:
+    """In the place of the native calls where they are not built: every one declines, and the operators go their general way."""
+
+    def __getattr__(self, name):
+        return lambda *args: None
+
+
+def _load_native():
+    """The ordinary operator calls in native code (``csrc/native.cpp``): each returns None for what it leaves to Python."""
+    path = _LIB_PATH.with_name("ksa_native.so")
+    if not path.exists():
+        return NotBuilt()
+    loader = importlib.machinery.ExtensionFileLoader("ksa_native", str(path))
+    try:
+        module = importlib.util.module_from_spec(importlib.util.spec_from_loader("ksa_native", loader))
+        loader.exec_module(module)
+    except ImportError as e:     # built against another PyTorch or Python
+        warnings.warn(f"{path} does not load ({e}); rebuild it with `python -m ksa_b200.csrc.build`")
+        return NotBuilt()
+    return module
+
+
+native = _load_native()
 
 _STATUS_TEXT = {
     1: "a consumer timed out waiting for a TMA-filled stage",
@@ -216,14 +243,14 @@ def flush_pair_gather() -> None:
 
 def launch_count() -> int:
     """Kernels of this library launched (or captured into a graph) so far in this process."""
-    return _launch_count
+    return _launch_count + (native.launches() or 0)
 
 
 def count_launches(fn) -> int:
     """Run ``fn()`` and return how many kernels of this library it launched."""
-    before = _launch_count
+    before = launch_count()
     fn()
-    return _launch_count - before
+    return launch_count() - before
 
 
 def call_on(name: str, stream: int, *args) -> None:
