@@ -436,6 +436,7 @@ class _QkNormRopeFn(torch.autograd.Function):
         qkv, q_w, k_w, pos, rstd = ctx.saved_tensors
         Hq, Hkv, D, theta, eps, interleaved = ctx.cfg
         T = qkv.shape[0]
+        qkv = qkv if qkv.is_contiguous() else qkv.contiguous()     # the kernel writes the gradient at the pitch of the rows it reads
         d_out = d_out if d_out.is_contiguous() else d_out.contiguous()
         targets = []
         for w in (q_w, k_w):

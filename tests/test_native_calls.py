@@ -79,6 +79,9 @@ def _case(name, rows, main_grad):
     if name == "qk_norm_rope":
         q, k, y = _weight(128, 0, main_grad), _weight(128, 0, main_grad), _n(rows, 4 * 128)
         return lambda: ops.qk_norm_rope_packed(y, q, k, pos, 2, 1, 128, 1e4), [y, q, k]
+    if name == "qk_norm_rope of rows with a pitch, without norms":
+        y = _n(rows, 640)
+        return lambda: ops.qk_norm_rope_packed(y[:, :512], None, None, pos, 2, 1, 128, 1e4), [y]
     if name == "attention":
         y = _n(rows, 4 * 128)
         return lambda: ops.attention_packed(y, 1, rows, 0, 2, 1, 128), [y]
@@ -87,7 +90,8 @@ def _case(name, rows, main_grad):
 
 
 _NAMES = ["linear", "linear of rows with a pitch", "linear of three dimensions", "linear of columns", "dual_linear", "add_rms_norm",
-          "rms_norm of three dimensions", "swiglu", "qk_norm_rope", "attention", "summary attention"]
+          "rms_norm of three dimensions", "swiglu", "qk_norm_rope", "qk_norm_rope of rows with a pitch, without norms", "attention",
+          "summary attention"]
 
 
 def _run(name, rows, main_grad, monkeypatch, native):
