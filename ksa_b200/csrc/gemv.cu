@@ -1,19 +1,396 @@
 // Skinny GEMM for decoding: C[M, N] = A[M, K] * B[N, K]^T with M <= 16 rows (one token per sequence of the batch).
-// The work is a stream of the weight matrix B, so the kernel is laid out for memory bandwidth, not for the tensor
-// cores: every CTA owns a slab of output columns small enough that the grid covers all SMs several times (a 128-row
-// MMA tile would leave N/256 = 10 CTAs busy for a 2560-wide projection), each warp streams whole weight rows with
-// 16-byte loads, the activation rows sit in shared memory, and the dot products are accumulated in fp32.
+// The work is a stream of the weight matrix B, and what bounds it is how early and how steadily every SM asks for its share:
+//   * one CTA per SM, and each owns the same number of weight rows (+-1) whatever N is, so no last wave is left over;
+//   * a producer thread brings the rows in as TMA boxes of 64 columns through a ring of some 90 KB of shared memory, so a CTA keeps
+//     its share of the memory system busy from its first cycle to its last; the activations of the same columns travel in
+//     the same stages;
+//   * eight warps split the 16-wide steps of K of a stage among themselves and multiply with mma.sync m16n8k16 (16 weight rows by
+//     8 or 16 activation rows; a 128-row tcgen05 tile would leave most SMs without a tile), and their partial sums meet in shared
+//     memory once per group of at most 32 rows.
+// (Untiled bulk copies of whole row segments to rows padded by 16 bytes reached 11 GB/s an SM, a quarter of its share: a destination
+// off the 128-byte lines is written 16 bytes at a time.  The boxes' 128-byte swizzle serves ldmatrix as well.)
+//
+// Measured against scalar products (up to 4 rows with a norm) and mma.sync on register tiles with a barrier every 1024 columns,
+// weights from memory, us: 4 rows x 2560 x 9728 21.5 -> 12.5 (the weights alone take 7.6 at the copy bandwidth), 16 rows 24.5 -> 12.3,
+// 16 x 6144 x 2560 15.1 -> 9.3, 16 x 151936 x 2560 208 -> 118; with the norm, 4 x 6144 x 2560 25.4 -> 10.8, 4 x 19456 x 2560 with
+// SwiGLU 41.6 -> 22.7.  Integer divisions by the number of stages in the producer's loop alone had cost 0.4 us a stage.
 //
 // A decode step is a chain of such kernels, each a few microseconds long, so the engine switches dependent launches
-// on (host.h): a CTA may then start while the previous kernel of the stream is still running, asks for its first
-// weight bytes (which no earlier kernel writes), and only then waits for the previous kernel (griddepcontrol.wait)
-// before it reads the activations.  The gate/up projection can apply SwiGLU itself (kGlu): a
-// warp (a CTA in the tensor-core variant) then owns matching gate and up rows and writes silu(gate) * up.
+// on (host.h): a CTA may then start beside the CTA of the previous kernel of the stream (both fit one SM), fill its whole ring with
+// weights, which no earlier kernel writes, and only then waits for the previous kernel (griddepcontrol.wait) before it
+// reads the activations.  The gate/up projection can apply SwiGLU itself (kGlu): a group then holds matching gate and up
+// rows and the CTA writes silu(gate) * up.  Every wait is bounded; no TMA load uses multicast.
 #include "common.cuh"
 #include "host.h"
 
 namespace ksa {
 
+constexpr int kStWarps = 8;                        // warps that multiply
+constexpr int kStThreads = kStWarps * 32;
+constexpr int kStMaxStages = 16;
+constexpr int kStBlocks = 2;                       // 16-row blocks of a group
+constexpr int kStBarrierBytes = 2 * kStMaxStages * 8 + 64;
+constexpr int kStBoxes = 8;                        // boxes of 64 columns a stage at most
+constexpr int kStSmemMost = 225 * 1024;
+
+// kGlu: B holds N/2 gate rows followed by N/2 up rows; C[m, f] = silu(gate) * up has N/2 columns.
+// Optional residual add + RMSNorm in front of the projection (a decode step's `x + delta -> norm -> projection`): the
+// activation rows are then A = bf16(rms_norm(bf16(A + delta)) * w), computed by every CTA and kept in its shared memory (the
+// rows are a few kilobytes), and CTA 0 also writes the new residual stream bf16(A + delta) to `res_out`.
+struct GemvNorm {
+  const bf16* delta;     // [delta_rows, K] or null
+  const bf16* w;         // [K] norm weight; null: no norm, A is used as it is
+  bf16* res_out;         // [M, K] or null
+  long long ld_delta, ld_res;
+  float eps;
+  int delta_rows;
+};
+
+struct StreamArgs {
+  const bf16* A;         // read directly for the norm only
+  bf16* C;
+  long long lda, ldc;
+  int M, N, K;
+  int groups, per_group; // row groups of a CTA, and their output columns
+  int boxes;             // boxes of 64 columns of a stage
+  int ragged;            // K is no multiple of 64: one load per box, which fills the columns past K with zeros
+  int w_rows, x_rows;    // rows of a box in shared memory (weights, activations): those loaded, for `ragged` in whole swizzle atoms
+  int stages, stage_bytes;
+  GemvNorm nrm;
+};
+
+__device__ __forceinline__ void mma_bf16_16x8x16(float (&c)[4], uint32_t a0, uint32_t a1, uint32_t a2, uint32_t a3,
+                                                 uint32_t b0, uint32_t b1) {
+  asm volatile("mma.sync.aligned.m16n8k16.row.col.f32.bf16.bf16.f32 {%0, %1, %2, %3}, {%4, %5, %6, %7}, {%8, %9}, "
+               "{%0, %1, %2, %3};"
+               : "+f"(c[0]), "+f"(c[1]), "+f"(c[2]), "+f"(c[3])
+               : "r"(a0), "r"(a1), "r"(a2), "r"(a3), "r"(b0), "r"(b1));
+}
+__device__ __forceinline__ void ldmatrix4(uint32_t (&r)[4], uint32_t addr) {
+  asm volatile("ldmatrix.sync.aligned.m8n8.x4.shared.b16 {%0, %1, %2, %3}, [%4];"
+               : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]) : "r"(addr) : "memory");
+}
+__device__ __forceinline__ void multiply_sync() { asm volatile("bar.sync 1, %0;" ::"n"(kStThreads) : "memory"); }
+
+// byte offset of columns 8 q .. 8 q + 7 (q < 8) of row r in a box of 128-byte rows with the 128-byte swizzle
+__device__ __forceinline__ uint32_t swizzled(int r, int q) { return (uint32_t)(r * 128 + ((q ^ (r & 7)) << 4)); }
+
+template <int NB, bool kGlu, bool kNorm>   // NB: batch blocks of 8 rows, 1 (M <= 8) or 2 (M <= 16)
+__global__ void __launch_bounds__(kStThreads + 32, 2)
+stream_gemm_kernel(const __grid_constant__ CUtensorMap tmB, const __grid_constant__ CUtensorMap tmA, const StreamArgs p,
+                   int* status) {
+  extern __shared__ uint8_t st_raw[];
+  uint8_t* ring = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(st_raw) + 1023) & ~uintptr_t(1023));
+  uint64_t* full = reinterpret_cast<uint64_t*>(ring + p.stages * p.stage_bytes);
+  uint64_t* empty = full + kStMaxStages;
+  volatile int* abort_flag = reinterpret_cast<volatile int*>(empty + kStMaxStages);
+  float* part = reinterpret_cast<float*>(reinterpret_cast<uint8_t*>(full) + kStBarrierBytes);   // [warps][NB * 8][part_pitch]
+  const int half_rows = (p.per_group + 15) / 16 * 16;               // rows of a half (gate, up), in whole blocks
+  const int part_pitch = half_rows * (kGlu ? 2 : 1) + 4;     // 4 modulo 16: the fragments' stores and the sums' loads both miss no bank twice
+  uint8_t* xres = reinterpret_cast<uint8_t*>(part + kStWarps * NB * 8 * part_pitch);    // kNorm: [M][K] + 16 to 32 bytes a row
+  const int xpitch = (p.K + 15) / 16 * 32 + 16;
+  __shared__ float s_red[kStWarps][4], s_rstd[4];
+
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  const WaitGuard guard{abort_flag, status};
+  const int n_out = kGlu ? p.N / 2 : p.N;
+  const int c0 = (int)blockIdx.x * p.groups * p.per_group;           // first output column of this CTA
+  const int groups = min(p.groups, (n_out - c0 + p.per_group - 1) / p.per_group);
+  const int num_kb = (p.K + 63) / 64, nk = (num_kb + p.boxes - 1) / p.boxes;
+  const int n_items = groups * nk;
+  const int w_bytes = (p.boxes * p.w_rows + 7) / 8 * 1024;        // a box of weights (of the gate or the up half)
+  const int x_off = w_bytes * (kGlu ? 2 : 1);                        // the activations' box follows the weights'
+
+  if (threadIdx.x == 0) {
+    for (int i = 0; i < p.stages; ++i) { mbar_init(&full[i], 1); mbar_init(&empty[i], kStWarps); }
+    *abort_flag = 0;
+    fence_mbar_init();
+    tma_prefetch_desc(&tmB);
+    if (!kNorm) tma_prefetch_desc(&tmA);
+  }
+  __syncthreads();
+  grid_dependency_launch();
+
+  if (warp == kStWarps) {
+    // ------------------------------------------------------------ producer: lane 0, or for `ragged` a lane per box
+    // position in the ring and in the matrix, carried along: a division a stage costs more than its loads
+    struct Cursor {
+      int stage = 0, kb = 0, row;
+      uint32_t phase = 1;
+    } w, x;
+    w.row = c0;
+    auto next = [&](Cursor& c) {
+      if (++c.stage == p.stages) { c.stage = 0; c.phase ^= 1; }
+      if ((c.kb += p.boxes) >= num_kb) { c.kb = 0; c.row += p.per_group; }
+    };
+    const uint32_t bytes = p.boxes * 128 * (p.per_group * (kGlu ? 2 : 1) + (kNorm ? 0 : p.M));     // also past the matrix's edges
+    auto load_weights = [&]() {
+      uint8_t* dst = ring + w.stage * p.stage_bytes;
+      if (lane == 0) mbar_expect_tx(&full[w.stage], bytes);
+      __syncwarp();
+      if (lane < (p.ragged ? p.boxes : 1)) {
+        const int col = p.ragged ? (w.kb + lane) * 64 : 0, kb = p.ragged ? 0 : w.kb;
+        dst += lane * p.w_rows * 128;
+        tma_load_3d(dst, &tmB, col, w.row, kb, &full[w.stage]);
+        if (kGlu) tma_load_3d(dst + w_bytes, &tmB, col, n_out + w.row, kb, &full[w.stage]);
+      }
+      next(w);
+    };
+    auto load_acts = [&]() {
+      if (kNorm) return;
+      if (lane < (p.ragged ? p.boxes : 1))
+        tma_load_3d(ring + x.stage * p.stage_bytes + x_off + lane * p.x_rows * 128, &tmA, p.ragged ? (x.kb + lane) * 64 : 0, 0,
+                    p.ragged ? 0 : x.kb, &full[x.stage]);
+      next(x);
+    };
+    // weights do not depend on the previous kernel; the activations do
+    const int ahead = min(p.stages, n_items);
+    for (int it = 0; it < ahead; ++it) load_weights();
+    grid_dependency_wait();
+    for (int it = 0; it < ahead; ++it) load_acts();
+    for (int it = ahead; it < n_items; ++it) {
+      if (!__all_sync(0xffffffffu, mbar_wait(&empty[w.stage], w.phase, guard, kTimeoutStageEmpty))) break;
+      load_weights();
+      load_acts();
+    }
+    return;
+  }
+
+  // -------------------------------------------------------------- the eight warps that multiply
+  grid_dependency_wait();     // also for the outputs: an earlier kernel may still read their memory
+  if (kNorm) {
+    float ss[4] = {0.f, 0.f, 0.f, 0.f};
+    for (int c = threadIdx.x * 8; c < p.K; c += kStThreads * 8) {
+      uint4 xv[4], dv[4];
+#pragma unroll
+      for (int m = 0; m < 4; ++m) {
+        xv[m] = dv[m] = make_uint4(0, 0, 0, 0);
+        if (m < p.M) {
+          xv[m] = *reinterpret_cast<const uint4*>(p.A + m * p.lda + c);
+          if (m < p.nrm.delta_rows) dv[m] = *reinterpret_cast<const uint4*>(p.nrm.delta + m * p.nrm.ld_delta + c);
+        }
+      }
+#pragma unroll
+      for (int m = 0; m < 4; ++m) {
+        if (m >= p.M) break;
+        const uint32_t xu[4] = {xv[m].x, xv[m].y, xv[m].z, xv[m].w}, du[4] = {dv[m].x, dv[m].y, dv[m].z, dv[m].w};
+        uint32_t o[4];
+#pragma unroll
+        for (int q = 0; q < 4; ++q) {
+          float2 f = unpack_bf16x2(xu[q]);
+          if (m < p.nrm.delta_rows) {
+            const float2 d = unpack_bf16x2(du[q]);
+            f.x = __bfloat162float(__float2bfloat16(f.x + d.x));
+            f.y = __bfloat162float(__float2bfloat16(f.y + d.y));
+          }
+          ss[m] += f.x * f.x + f.y * f.y;
+          o[q] = pack_bf16x2(f.x, f.y);
+        }
+        const uint4 r = make_uint4(o[0], o[1], o[2], o[3]);
+        *reinterpret_cast<uint4*>(xres + m * xpitch + c * 2) = r;
+        if (blockIdx.x == 0 && p.nrm.res_out != nullptr)
+          *reinterpret_cast<uint4*>(p.nrm.res_out + m * p.nrm.ld_res + c) = r;
+      }
+    }
+#pragma unroll
+    for (int m = 0; m < 4; ++m) {
+      ss[m] = warp_sum(ss[m]);
+      if (lane == 0) s_red[warp][m] = ss[m];
+    }
+    if (p.K % 16 != 0 && threadIdx.x < p.M)               // columns K .. K + 7 take part in the last step, against zeros
+      *reinterpret_cast<uint4*>(xres + threadIdx.x * xpitch + p.K * 2) = make_uint4(0, 0, 0, 0);
+    multiply_sync();
+    if (threadIdx.x < 4) {
+      float t = 0.f;
+#pragma unroll
+      for (int k = 0; k < kStWarps; ++k) t += s_red[k][threadIdx.x];
+      s_rstd[threadIdx.x] = rsqrtf(t / (float)p.K + p.nrm.eps);
+    }
+    multiply_sync();
+    for (int c = threadIdx.x * 8; c < p.K; c += kStThreads * 8) {      // a thread's own columns again
+      const uint4 wv = *reinterpret_cast<const uint4*>(p.nrm.w + c);
+      const uint32_t wu[4] = {wv.x, wv.y, wv.z, wv.w};
+      for (int m = 0; m < p.M; ++m) {
+        uint4* at = reinterpret_cast<uint4*>(xres + m * xpitch + c * 2);
+        const uint4 xv = *at;
+        const uint32_t xu[4] = {xv.x, xv.y, xv.z, xv.w};
+        const float rstd = s_rstd[m];
+        uint32_t o[4];
+#pragma unroll
+        for (int q = 0; q < 4; ++q) {
+          const float2 x = unpack_bf16x2(xu[q]), f = unpack_bf16x2(wu[q]);
+          o[q] = pack_bf16x2(x.x * rstd * f.x, x.y * rstd * f.y);
+        }
+        *at = make_uint4(o[0], o[1], o[2], o[3]);
+      }
+    }
+    multiply_sync();
+  }
+
+  bool ok = true;
+  int stage = 0;
+  uint32_t phase = 0;
+  for (int g = 0; g < groups; ++g) {
+    const int f0 = c0 + g * p.per_group, nf = min(p.per_group, n_out - f0);
+    const int nblk = (nf + 15) / 16;                 // blocks in use: of the gate and of the up half each for kGlu
+    constexpr int kHalf = kGlu ? kStBlocks / 2 : kStBlocks;
+    // this lane's row of every block (rows past the end repeat the last one; their sums are dropped) ..
+    int row[kStBlocks];
+#pragma unroll
+    for (int b = 0; b < kStBlocks; ++b) row[b] = min((b % kHalf) * 16 + (lane & 15), nf - 1);
+    // .. and of the activations: lanes 0-7 / 8-15 rows 0-7 at k and k + 8, lanes 16-31 the same of rows 8-15
+    const int xrow = min((lane & 7) + (NB == 2 ? (lane >> 4) * 8 : 0), p.M - 1), xq = (lane >> 3) & 1;
+    float acc[kStBlocks][NB][4];
+#pragma unroll
+    for (int b = 0; b < kStBlocks; ++b)
+#pragma unroll
+      for (int n = 0; n < NB; ++n)
+#pragma unroll
+        for (int i = 0; i < 4; ++i) acc[b][n][i] = 0.f;
+
+    for (int kb = 0; kb < num_kb; kb += p.boxes) {
+      if (ok) ok = mbar_wait(&full[stage], phase, guard, kTimeoutTmaFull);
+      if (ok) {
+        // steps of 16 columns, four to a box; columns past K are zeros in both operands
+        const int steps = min(p.boxes * 4, (p.K - kb * 64 + 15) / 16);
+        const uint32_t sw = smem_u32(ring + stage * p.stage_bytes);
+        const uint32_t sx = kNorm ? smem_u32(xres) + xrow * xpitch + kb * 128 + xq * 16 : sw + x_off;
+#pragma unroll
+        for (int u = 0; u < kStBoxes * 4 / kStWarps; ++u) {
+          const int s = u * kStWarps + warp, box = s >> 2, q = (s & 3) * 2;
+          if (s >= steps) break;
+          uint32_t x[4];                              // NB == 1: lanes 16-31 repeat lanes 0-15, x[2] and x[3] are not used
+          ldmatrix4(x, kNorm ? sx + s * 32 : sx + swizzled(box * p.x_rows + xrow, q + xq));
+#pragma unroll
+          for (int b = 0; b < kStBlocks; ++b) {
+            if (b % kHalf >= nblk) continue;
+            uint32_t w[4];
+            ldmatrix4(w, sw + (b >= kHalf ? w_bytes : 0) + swizzled(box * p.w_rows + row[b], q + (lane >> 4)));
+#pragma unroll
+            for (int n = 0; n < NB; ++n) mma_bf16_16x8x16(acc[b][n], w[0], w[1], w[2], w[3], x[2 * n], x[2 * n + 1]);
+          }
+        }
+      }
+      __syncwarp();
+      if (lane == 0) mbar_arrive(&empty[stage]);
+      if (++stage == p.stages) { stage = 0; phase ^= 1; }
+    }
+    // acc[b][n] = {D[gr][2t], D[gr][2t + 1], D[gr + 8][2t], D[gr + 8][2t + 1]}: rows of the block by activation rows 8 n + ..
+    {
+      const int gr = lane >> 2, t = lane & 3;
+      float* dst = part + warp * NB * 8 * part_pitch;
+#pragma unroll
+      for (int b = 0; b < kStBlocks; ++b) {
+        if (b % kHalf >= nblk) continue;
+        const int r = (b % kHalf) * 16 + gr + (b >= kHalf ? half_rows : 0);
+#pragma unroll
+        for (int n = 0; n < NB; ++n) {
+          float* at = dst + (n * 8 + 2 * t) * part_pitch + r;
+          at[0] = acc[b][n][0];
+          at[part_pitch] = acc[b][n][1];
+          at[8] = acc[b][n][2];
+          at[part_pitch + 8] = acc[b][n][3];
+        }
+      }
+      multiply_sync();
+      if (ok) {
+        for (int i = threadIdx.x; i < nf * p.M; i += kStThreads) {
+          const int f = i % nf, m = i / nf;            // consecutive threads -> consecutive outputs
+          float v = 0.f, u = 0.f;
+#pragma unroll
+          for (int w = 0; w < kStWarps; ++w) {
+            const float* src = part + (w * NB * 8 + m) * part_pitch + f;
+            v += src[0];
+            if (kGlu) u += src[half_rows];
+          }
+          if (kGlu) {
+            // gate and up are rounded to bf16 first, as the separate projection + SwiGLU kernels do
+            const float gt = __bfloat162float(__float2bfloat16(v)), up = __bfloat162float(__float2bfloat16(u));
+            v = gt / (1.f + __expf(-gt)) * up;
+          }
+          p.C[(long long)m * p.ldc + f0 + f] = __float2bfloat16(v);
+        }
+      }
+      multiply_sync();        // the next group's partial sums overwrite these
+    }
+  }
+}
+
+static int stream_sms() {
+  static int sms = 0;
+  if (sms == 0) {
+    int dev = 0, n = 0;
+    if (cudaGetDevice(&dev) != cudaSuccess) return 0;
+    if (cudaDeviceGetAttribute(&n, cudaDevAttrMultiProcessorCount, dev) != cudaSuccess) return 0;
+    sms = n;
+  }
+  return sms;
+}
+
+template <int NB, bool kGlu, bool kNorm>
+static int launch_stream(StreamArgs p, const void* b, long long ldb, cudaStream_t st) {
+  const int sms = stream_sms();
+  KSA_REQUIRE(sms > 0, "gemv: no device");
+  int* status = status_word();
+  KSA_REQUIRE(status != nullptr, "could not allocate the status word");
+  const int n_out = kGlu ? p.N / 2 : p.N;
+  const int most = (n_out + sms - 1) / sms;                       // output columns of a CTA
+  constexpr int kCap = kStBlocks * 16 / (kGlu ? 2 : 1);
+  p.groups = (most + kCap - 1) / kCap;
+  p.per_group = (most + p.groups - 1) / p.groups;
+  const int grid = (n_out + p.groups * p.per_group - 1) / (p.groups * p.per_group);
+  const int num_kb = (p.K + 63) / 64;
+  p.ragged = p.K % 64 != 0;
+  p.w_rows = p.ragged ? (p.per_group + 7) / 8 * 8 : p.per_group;
+  p.x_rows = p.ragged ? NB * 8 : p.M;
+  p.boxes = kStBoxes;
+  if (p.boxes > num_kb) p.boxes = num_kb;
+  p.stage_bytes = (p.boxes * p.w_rows + 7) / 8 * 1024 * (kGlu ? 2 : 1) + (kNorm ? 0 : (p.boxes * p.x_rows + 7) / 8 * 1024);
+  const int part_pitch = (p.per_group + 15) / 16 * 16 * (kGlu ? 2 : 1) + 4;
+  const int fixed = 1024 + kStBarrierBytes + kStWarps * NB * 8 * part_pitch * 4 + (kNorm ? p.M * ((p.K + 15) / 16 * 32 + 16) : 0);
+  const int n_items = p.groups * ((num_kb + p.boxes - 1) / p.boxes);
+  // Both limits together leave room for this kernel and its neighbour in a decode step on one SM.  A ring of two stages, or of
+  // less than 64 KB, does not hide the memory's latency: the ring is then as large as it can be (4 x 151936 x 2560 with two stages of
+  // 36 KB 132 us, with five 117).
+  const int beside = (kNorm ? 130 : 96) * 1024, ring = beside - fixed;
+  const int limit = ring < 3 * p.stage_bytes || ring < 64 * 1024 ? kStSmemMost : beside;
+  p.stages = (limit - fixed) / p.stage_bytes;
+  if (p.stages > kStMaxStages) p.stages = kStMaxStages;
+  if (p.stages > n_items) p.stages = n_items;
+  KSA_REQUIRE(p.stages >= 1, "gemv: %d rows of %d columns do not fit shared memory", p.M, p.K);
+  const int smem = fixed + p.stages * p.stage_bytes;
+  CUtensorMap tmB, tmA;
+  int rc;
+  {
+    uint64_t dims[3] = {(uint64_t)(p.ragged ? p.K : 64), (uint64_t)p.N, (uint64_t)(p.ragged ? 1 : num_kb)};
+    uint64_t str[3] = {2, (uint64_t)(p.N == 1 ? p.K : ldb) * 2, 128};       // one row: its pitch may be anything
+    uint32_t box[3] = {64, (uint32_t)p.per_group, (uint32_t)(p.ragged ? 1 : p.boxes)};
+    if ((rc = make_tmap(&tmB, b, 2, 3, dims, str, box, true))) return rc;
+  }
+  if (kNorm) {
+    tmA = tmB;       // not used
+  } else {
+    uint64_t dims[3] = {(uint64_t)(p.ragged ? p.K : 64), (uint64_t)p.M, (uint64_t)(p.ragged ? 1 : num_kb)};
+    uint64_t str[3] = {2, (uint64_t)(p.M == 1 ? p.K : p.lda) * 2, 128};
+    uint32_t box[3] = {64, (uint32_t)p.M, (uint32_t)(p.ragged ? 1 : p.boxes)};
+    if ((rc = make_tmap(&tmA, p.A, 2, 3, dims, str, box, true))) return rc;
+  }
+  auto kern = stream_gemm_kernel<NB, kGlu, kNorm>;
+  static bool attr = false;
+  if (!attr) {
+    KSA_CHECK_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, kStSmemMost));
+    attr = true;
+  }
+  KSA_CHECK_CUDA(launch_kernel(dependent_launch_enabled(), kern, dim3(grid), dim3(kStThreads + 32), (size_t)smem, st, tmB, tmA,
+                              p, status));
+  return 0;
+}
+
+// ------------------------------------------------------------------------------------------ one and two rows
+// Each warp streams whole weight rows with 16-byte loads and multiplies on the FMA units; the activation rows sit in shared memory.
+// No ring to set up and as many CTAs as there are rows for, which the hardware deals out as SMs become free: launched by itself it
+// starts 0.7 us earlier than the ring and ends more evenly (one row x 2560 x 4096 6.4 against 7.1 us, x 151936 x 2560 108 against 115).
+// kGlu: weight row r of a warp is gate row f for even r and up row f for odd r (f = first feature + r / 2).
 constexpr int kGemvThreads = 256;
 constexpr int kGemvKTile = 2048;   // activation columns staged in shared memory per pass
 
@@ -25,28 +402,12 @@ __device__ __forceinline__ uint4 ld_stream_16(const void* p) {
   return v;
 }
 
-// kGlu: B holds N/2 gate rows followed by N/2 up rows; weight row r of a warp is gate row f for even r and up row f
-// for odd r (f = first feature + r / 2), and C[m, f] = silu(gate) * up has N/2 columns.
-// Optional residual add + RMSNorm in front of the projection (a decode step's `x + delta -> norm -> projection`): the
-// activation rows are then A = bf16(rms_norm(bf16(A + delta)) * w), computed by every CTA while it stages them (the
-// rows are a few kilobytes), and CTA 0 also writes the new residual stream bf16(A + delta) to `res_out`.
-struct GemvNorm {
-  const bf16* delta;     // [delta_rows, K] or null
-  const bf16* w;         // [K] norm weight; null: no norm, A is used as it is
-  bf16* res_out;         // [M, K] or null
-  long long ld_delta, ld_res;
-  float eps;
-  int delta_rows;
-};
-
 template <int MT, int R, bool kGlu>
 __global__ void __launch_bounds__(kGemvThreads)
 gemv_kernel(const bf16* __restrict__ A, const bf16* __restrict__ B, bf16* __restrict__ C, int M, int N, int K,
-            long long lda, long long ldb, long long ldc, GemvNorm nrm) {
+            long long lda, long long ldb, long long ldc) {
   extern __shared__ __align__(16) uint8_t gemv_smem[];
   bf16* sA = reinterpret_cast<bf16*>(gemv_smem);           // [MT][kGemvKTile]
-  __shared__ float s_rstd[MT];
-  __shared__ float s_red[kGemvThreads / 32];
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   const int n0 = (blockIdx.x * (kGemvThreads / 32) + warp) * (kGlu ? R / 2 : R);   // first row / first feature
   const int n_out = kGlu ? N / 2 : N;
@@ -81,77 +442,13 @@ gemv_kernel(const bf16* __restrict__ A, const bf16* __restrict__ B, bf16* __rest
   grid_dependency_wait();
   grid_dependency_launch();
 
-  // eight elements of the (residual-added, bf16-rounded) activation row m at column c
-  auto load_row8 = [&](int m, int c, float (&v)[8]) {
-    const uint4 u = *reinterpret_cast<const uint4*>(A + (long long)m * lda + c);
-    const uint32_t uu[4] = {u.x, u.y, u.z, u.w};
-#pragma unroll
-    for (int q = 0; q < 4; ++q) { const float2 f = unpack_bf16x2(uu[q]); v[2 * q] = f.x; v[2 * q + 1] = f.y; }
-    if (nrm.delta != nullptr && m < nrm.delta_rows) {
-      const uint4 d = *reinterpret_cast<const uint4*>(nrm.delta + (long long)m * nrm.ld_delta + c);
-      const uint32_t du[4] = {d.x, d.y, d.z, d.w};
-#pragma unroll
-      for (int q = 0; q < 4; ++q) {
-        const float2 f = unpack_bf16x2(du[q]);
-        v[2 * q] = __bfloat162float(__float2bfloat16(v[2 * q] + f.x));
-        v[2 * q + 1] = __bfloat162float(__float2bfloat16(v[2 * q + 1] + f.y));
-      }
-    }
-  };
-  if (nrm.w != nullptr) {
-    for (int m = 0; m < MT; ++m) {
-      float ss = 0.f;
-      if (m < M) {
-        for (int c = threadIdx.x * 8; c < K; c += kGemvThreads * 8) {
-          float v[8];
-          load_row8(m, c, v);
-#pragma unroll
-          for (int q = 0; q < 8; ++q) ss += v[q] * v[q];
-          if (blockIdx.x == 0 && nrm.res_out != nullptr) {
-            uint4 o;
-            o.x = pack_bf16x2(v[0], v[1]); o.y = pack_bf16x2(v[2], v[3]);
-            o.z = pack_bf16x2(v[4], v[5]); o.w = pack_bf16x2(v[6], v[7]);
-            *reinterpret_cast<uint4*>(nrm.res_out + (long long)m * nrm.ld_res + c) = o;
-          }
-        }
-      }
-      ss = warp_sum(ss);
-      __syncthreads();
-      if (lane == 0) s_red[warp] = ss;
-      __syncthreads();
-      if (threadIdx.x == 0) {
-        float t = 0.f;
-#pragma unroll
-        for (int k = 0; k < kGemvThreads / 32; ++k) t += s_red[k];
-        s_rstd[m] = rsqrtf(t / (float)K + nrm.eps);
-      }
-    }
-  }
-
   for (int k0 = 0; k0 < K; k0 += kGemvKTile) {
     const int kt = min(kGemvKTile, K - k0);          // multiple of 8
     __syncthreads();
     for (int i = threadIdx.x; i < MT * (kGemvKTile / 8); i += kGemvThreads) {
       const int m = i / (kGemvKTile / 8), c = (i % (kGemvKTile / 8)) * 8;
       uint4 v = make_uint4(0, 0, 0, 0);
-      if (m < M && c < kt) {
-        if (nrm.w == nullptr) {
-          v = *reinterpret_cast<const uint4*>(A + (long long)m * lda + k0 + c);
-        } else {
-          float x[8];
-          load_row8(m, k0 + c, x);
-          const uint4 wv = *reinterpret_cast<const uint4*>(nrm.w + k0 + c);
-          const uint32_t wu[4] = {wv.x, wv.y, wv.z, wv.w};
-          const float rstd = s_rstd[m];
-          uint32_t o[4];
-#pragma unroll
-          for (int q = 0; q < 4; ++q) {
-            const float2 f = unpack_bf16x2(wu[q]);
-            o[q] = pack_bf16x2(x[2 * q] * rstd * f.x, x[2 * q + 1] * rstd * f.y);
-          }
-          v = make_uint4(o[0], o[1], o[2], o[3]);
-        }
-      }
+      if (m < M && c < kt) v = *reinterpret_cast<const uint4*>(A + (long long)m * lda + k0 + c);
       *reinterpret_cast<uint4*>(sA + m * kGemvKTile + c) = v;
     }
     __syncthreads();
@@ -206,188 +503,40 @@ gemv_kernel(const bf16* __restrict__ A, const bf16* __restrict__ B, bf16* __rest
 
 template <int MT, int R, bool kGlu>
 static int launch_gemv(const void* a, const void* b, void* c, int M, int N, int K, long long lda, long long ldb,
-                       long long ldc, cudaStream_t st, const GemvNorm& nrm = GemvNorm{}) {
+                       long long ldc, cudaStream_t st) {
   const int per_cta = (kGemvThreads / 32) * (kGlu ? R / 2 : R);      // output columns per CTA
   const int n_out = kGlu ? N / 2 : N;
   const size_t smem = (size_t)MT * kGemvKTile * sizeof(bf16);
   auto kern = gemv_kernel<MT, R, kGlu>;
-  static bool attr = false;
-  if (!attr && smem > 48 * 1024) {
-    KSA_CHECK_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
-    attr = true;
-  }
   KSA_CHECK_CUDA(launch_kernel(dependent_launch_enabled(), kern, dim3((n_out + per_cta - 1) / per_cta),
                               dim3(kGemvThreads), smem, st, (const bf16*)a, (const bf16*)b, (bf16*)c, M, N, K, lda, ldb,
-                              ldc, nrm));
+                              ldc));
   return 0;
 }
 
-// ------------------------------------------------------------------------------------------ tensor-core variant
-// For 3..16 activation rows the SIMT kernel above is bound by its FMA issue rate, so the dot products go to the tensor
-// cores with warp-level mma.sync m16n8k16 (the 128-row tcgen05 tile has no use for 16 rows): a CTA owns 16 weight
-// rows, its 8 warps take the 32-wide k blocks round-robin, and the partial sums meet in shared memory.  Both operands
-// are read as 16 contiguous bytes per lane along k; a lane's 8 elements are given to the instruction as its k slots
-// {2t, 2t+1, 2t+8, 2t+9} of two MMAs.  That permutes k inside a 32-block, identically for weights and activations,
-// which a dot product does not see.
-constexpr int kMmaKTile = 1024;               // activation columns staged per pass (32 blocks of 32)
-constexpr int kMmaRowStride = kMmaKTile + 32;  // +64 bytes: the two row groups of a quarter warp hit different banks
-
-__device__ __forceinline__ void mma_bf16_16x8x16(float (&c)[4], uint32_t a0, uint32_t a1, uint32_t a2, uint32_t a3,
-                                                 uint32_t b0, uint32_t b1) {
-  asm volatile("mma.sync.aligned.m16n8k16.row.col.f32.bf16.bf16.f32 {%0, %1, %2, %3}, {%4, %5, %6, %7}, {%8, %9}, "
-               "{%0, %1, %2, %3};"
-               : "+f"(c[0]), "+f"(c[1]), "+f"(c[2]), "+f"(c[3])
-               : "r"(a0), "r"(a1), "r"(a2), "r"(a3), "r"(b0), "r"(b1));
-}
-
-// A CTA owns RB blocks of 16 weight rows and stages the activations once for all of them (RB = 2 for wide outputs:
-// the activation tile is as large as 16 weight rows, so with one block a CTA would read as many activation bytes
-// from L2 as weight bytes from HBM).  kGlu: a block is 8 features, rows 0-7 their gate rows and rows 8-15 their up
-// rows.
-template <int NB, bool kGlu, int RB>   // NB: batch blocks of 8 rows, 1 (M <= 8) or 2 (M <= 16)
-__global__ void __launch_bounds__(kGemvThreads, 2)
-gemv_mma_kernel(const bf16* __restrict__ A, const bf16* __restrict__ B, bf16* __restrict__ C, int M, int N, int K,
-                long long lda, long long ldb, long long ldc) {
-  extern __shared__ __align__(16) uint8_t gemv_smem[];
-  bf16* sX = reinterpret_cast<bf16*>(gemv_smem);                       // [NB*8][kMmaRowStride]
-  float* sRed = reinterpret_cast<float*>(gemv_smem);                   // reused after the k loop: [8 warps][RB*16][NB*8]
-  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-  const int g = lane >> 2, t = lane & 3;
-  const int n_out = kGlu ? N / 2 : N;
-  constexpr int kBlockOut = kGlu ? 8 : 16;                              // output columns per row block
-  const int n0 = blockIdx.x * kBlockOut * RB;
-  int r0[RB], r1[RB];                                                   // clamped: rows past the end are never written
-#pragma unroll
-  for (int rb = 0; rb < RB; ++rb) {
-    r0[rb] = min(n0 + rb * kBlockOut + g, n_out - 1);
-    r1[rb] = kGlu ? n_out + r0[rb] : min(n0 + rb * 16 + g + 8, N - 1);
-  }
-  float acc[RB][NB][4];
-#pragma unroll
-  for (int rb = 0; rb < RB; ++rb)
-#pragma unroll
-    for (int b = 0; b < NB; ++b)
-#pragma unroll
-      for (int i = 0; i < 4; ++i) acc[rb][b][i] = 0.f;
-
-  // this warp's 32-wide blocks of a tile: warp, warp + 8, warp + 16, warp + 24; all weight loads first
-  uint4 w0[RB][4], w1[RB][4];
-  auto load_w = [&](int k0, int kt) {
-#pragma unroll
-    for (int rb = 0; rb < RB; ++rb)
-#pragma unroll
-      for (int u = 0; u < 4; ++u) {
-        const int c = (warp + 8 * u) * 32 + t * 8;
-        w0[rb][u] = make_uint4(0, 0, 0, 0);
-        w1[rb][u] = make_uint4(0, 0, 0, 0);
-        if (c < kt) {
-          w0[rb][u] = ld_stream_16(B + (long long)r0[rb] * ldb + k0 + c);
-          w1[rb][u] = ld_stream_16(B + (long long)r1[rb] * ldb + k0 + c);
-        }
-      }
-  };
-  load_w(0, min(kMmaKTile, K));     // weights do not depend on the previous kernel; the activations do
-  grid_dependency_wait();
-  grid_dependency_launch();
-
-  for (int k0 = 0; k0 < K; k0 += kMmaKTile) {
-    const int kt = min(kMmaKTile, K - k0);   // multiple of 32
-    __syncthreads();
-    for (int i = threadIdx.x; i < NB * 8 * (kMmaKTile / 8); i += kGemvThreads) {
-      const int m = i / (kMmaKTile / 8), c = (i % (kMmaKTile / 8)) * 8;
-      uint4 v = make_uint4(0, 0, 0, 0);
-      if (m < M && c < kt) v = *reinterpret_cast<const uint4*>(A + (long long)m * lda + k0 + c);
-      *reinterpret_cast<uint4*>(sX + m * kMmaRowStride + c) = v;
-    }
-    __syncthreads();
-    if (k0 != 0) load_w(k0, kt);
-#pragma unroll
-    for (int u = 0; u < 4; ++u) {
-      const int c = (warp + 8 * u) * 32 + t * 8;
-      if (c >= kt) break;
-#pragma unroll
-      for (int b = 0; b < NB; ++b) {
-        const uint4 x = *reinterpret_cast<const uint4*>(sX + (b * 8 + g) * kMmaRowStride + c);
-#pragma unroll
-        for (int rb = 0; rb < RB; ++rb) {
-          mma_bf16_16x8x16(acc[rb][b], w0[rb][u].x, w1[rb][u].x, w0[rb][u].y, w1[rb][u].y, x.x, x.y);
-          mma_bf16_16x8x16(acc[rb][b], w0[rb][u].z, w1[rb][u].z, w0[rb][u].w, w1[rb][u].w, x.z, x.w);
-        }
-      }
-    }
-  }
-  // acc[rb][b] = {C[g][2t], C[g][2t+1], C[g+8][2t], C[g+8][2t+1]}: rows = weight rows of block rb, columns = batch
-  __syncthreads();
-  constexpr int NBATCH = NB * 8;
-  constexpr int kRows = RB * 16;
-#pragma unroll
-  for (int rb = 0; rb < RB; ++rb)
-#pragma unroll
-    for (int b = 0; b < NB; ++b) {
-      float* dst = sRed + (warp * kRows + rb * 16) * NBATCH;
-      dst[g * NBATCH + b * 8 + 2 * t] = acc[rb][b][0];
-      dst[g * NBATCH + b * 8 + 2 * t + 1] = acc[rb][b][1];
-      dst[(g + 8) * NBATCH + b * 8 + 2 * t] = acc[rb][b][2];
-      dst[(g + 8) * NBATCH + b * 8 + 2 * t + 1] = acc[rb][b][3];
-    }
-  __syncthreads();
-  for (int i = threadIdx.x; i < RB * kBlockOut * NBATCH; i += kGemvThreads) {
-    const int col = i % (RB * kBlockOut), m = i / (RB * kBlockOut);   // consecutive threads -> consecutive outputs
-    const int rb = col / kBlockOut, row = rb * 16 + col % kBlockOut;    // row inside the CTA's RB * 16 weight rows
-    float v = 0.f, u = 0.f;
-#pragma unroll
-    for (int w = 0; w < kGemvThreads / 32; ++w) {
-      v += sRed[(w * kRows + row) * NBATCH + m];
-      if (kGlu) u += sRed[(w * kRows + row + 8) * NBATCH + m];
-    }
-    if (kGlu) {
-      const float gt = __bfloat162float(__float2bfloat16(v)), up = __bfloat162float(__float2bfloat16(u));
-      v = gt / (1.f + __expf(-gt)) * up;
-    }
-    if (m < M && n0 + col < n_out) C[(long long)m * ldc + n0 + col] = __float2bfloat16(v);
-  }
-}
-
-template <int NB, bool kGlu, int RB>
-static int launch_gemv_mma(const void* a, const void* b, void* c, int M, int N, int K, long long lda, long long ldb,
-                           long long ldc, cudaStream_t st) {
-  // the activation tile, reused for the final reduction [8 warps][RB * 16][NB * 8] floats
-  const size_t x_bytes = (size_t)NB * 8 * kMmaRowStride * sizeof(bf16), red_bytes = (size_t)8 * RB * 16 * NB * 8 * 4;
-  const size_t smem = x_bytes > red_bytes ? x_bytes : red_bytes;
-  const int per_cta = (kGlu ? 8 : 16) * RB, n_out = kGlu ? N / 2 : N;
-  KSA_CHECK_CUDA(launch_kernel(dependent_launch_enabled(), gemv_mma_kernel<NB, kGlu, RB>,
-                              dim3((n_out + per_cta - 1) / per_cta), dim3(kGemvThreads), smem, st, (const bf16*)a,
-                              (const bf16*)b, (bf16*)c, M, N, K, lda, ldb, ldc));
-  return 0;
-}
-
-}  // namespace ksa
-
-namespace ksa {
 template <bool kGlu>
 static int gemv_dispatch(const void* a, const void* b, void* c, int M, int N, int K, long long lda, long long ldb,
                          long long ldc, cudaStream_t st, const GemvNorm& nrm = GemvNorm{}) {
-  // Three and four rows as well while 16 weight rows a CTA give every SM one.  Scalar and tensor-core times in us at three and at
-  // four rows: 151936 x 2560 172 / 134, 173 / 141; 19456 x 2560 30.4 / 24.8, 30.5 / 25.4; 6144 x 2560 16.1 / 9.9, 16.3 / 9.9;
-  // 2560 x 4096 11.6 / 10.3, 11.9 / 10.5; at the line, 2368 x 2560, 7.6 / 7.0, 7.8 / 7.1.  Below it, 2048 x 6144, 13.2 and 13.6
-  // against 14.0.  One and two rows stay scalar (two rows x 6144 x 2560 11.5).  The error against 64 bits is that of the one
-  // rounding to bf16 in both (0.00166 over ten seeds, 3 and 4 rows x 6144 x 2560).
-  if ((M > 4 || (M > 2 && N >= 148 * 16)) && K % 32 == 0 && nrm.w == nullptr) {
-    if (N >= 16384)   // wide outputs: 32 weight rows per CTA still give every SM several CTAs
-      return M <= 8 ? launch_gemv_mma<1, kGlu, 2>(a, b, c, M, N, K, lda, ldb, ldc, st)
-                    : launch_gemv_mma<2, kGlu, 2>(a, b, c, M, N, K, lda, ldb, ldc, st);
-    return M <= 8 ? launch_gemv_mma<1, kGlu, 1>(a, b, c, M, N, K, lda, ldb, ldc, st)
-                  : launch_gemv_mma<2, kGlu, 1>(a, b, c, M, N, K, lda, ldb, ldc, st);
+  KSA_REQUIRE(((reinterpret_cast<uintptr_t>(a) | reinterpret_cast<uintptr_t>(b) | reinterpret_cast<uintptr_t>(nrm.delta) |
+                reinterpret_cast<uintptr_t>(nrm.w) | reinterpret_cast<uintptr_t>(nrm.res_out)) & 15) == 0,
+              "gemv: the operands must be 16-byte aligned");
+  StreamArgs p{};
+  p.A = (const bf16*)a; p.C = (bf16*)c;
+  p.lda = lda; p.ldc = ldc; p.M = M; p.N = N; p.K = K;
+  p.nrm = nrm;
+  if (nrm.w != nullptr) return launch_stream<1, kGlu, true>(p, b, ldb, st);
+  // In a chain of dependent launches the ring is filled while the previous kernel runs (one row x 2560 x 9728 10.4 against 11.9 us, x
+  // 4096 x 2048 4.4 against 5.4, x 2560 x 4096 6.2 both); the output head is long enough not to need that.
+  if (M <= 2 && !(dependent_launch_enabled() && N <= 32768)) {
+    // rows per warp: fewer for narrow outputs so that the grid still covers every SM a few times (with SwiGLU a warp
+    // needs at least one gate row and one up row)
+    constexpr int R1 = kGlu ? 2 : 1;
+    if (M == 1) return N <= 8192 ? launch_gemv<1, R1, kGlu>(a, b, c, M, N, K, lda, ldb, ldc, st)
+                                 : launch_gemv<1, 4, kGlu>(a, b, c, M, N, K, lda, ldb, ldc, st);
+    return N <= 8192 ? launch_gemv<2, R1, kGlu>(a, b, c, M, N, K, lda, ldb, ldc, st)
+                     : launch_gemv<2, 4, kGlu>(a, b, c, M, N, K, lda, ldb, ldc, st);
   }
-  // rows per warp: fewer for narrow outputs so that the grid still covers every SM a few times (with SwiGLU a warp
-  // needs at least one gate row and one up row)
-  const bool narrow = N <= 8192;
-  constexpr int R1 = kGlu ? 2 : 1;
-  if (M == 1) return narrow ? launch_gemv<1, R1, kGlu>(a, b, c, M, N, K, lda, ldb, ldc, st, nrm) : launch_gemv<1, 4, kGlu>(a, b, c, M, N, K, lda, ldb, ldc, st, nrm);
-  if (M <= 2) return narrow ? launch_gemv<2, R1, kGlu>(a, b, c, M, N, K, lda, ldb, ldc, st, nrm) : launch_gemv<2, 4, kGlu>(a, b, c, M, N, K, lda, ldb, ldc, st, nrm);
-  if (M <= 4) return narrow ? launch_gemv<4, R1, kGlu>(a, b, c, M, N, K, lda, ldb, ldc, st, nrm) : launch_gemv<4, 4, kGlu>(a, b, c, M, N, K, lda, ldb, ldc, st, nrm);
-  if (M <= 8) return narrow ? launch_gemv<8, R1, kGlu>(a, b, c, M, N, K, lda, ldb, ldc, st) : launch_gemv<8, 2, kGlu>(a, b, c, M, N, K, lda, ldb, ldc, st);
-  return narrow ? launch_gemv<16, R1, kGlu>(a, b, c, M, N, K, lda, ldb, ldc, st) : launch_gemv<16, 2, kGlu>(a, b, c, M, N, K, lda, ldb, ldc, st);
+  return M <= 8 ? launch_stream<1, kGlu, false>(p, b, ldb, st) : launch_stream<2, kGlu, false>(p, b, ldb, st);
 }
 }  // namespace ksa
 

@@ -102,8 +102,18 @@ int* status_word() {
   std::lock_guard<std::mutex> lk(g_status_mu);
   if (!g_status[dev]) {
     int* p = nullptr;
+    // the first kernel of a process may be launched into a capture: the word is then set up beside it, on a stream of its own
+    struct Relaxed {
+      cudaStreamCaptureMode mode = cudaStreamCaptureModeRelaxed;
+      cudaStream_t st = nullptr;
+      Relaxed() { cudaThreadExchangeStreamCaptureMode(&mode); }
+      ~Relaxed() {
+        if (st) cudaStreamDestroy(st);
+        cudaThreadExchangeStreamCaptureMode(&mode);
+      }
+    } relaxed;
     if (cudaMalloc(&p, 256) != cudaSuccess) return nullptr;
-    cudaMemset(p, 0, 256);
+    if (cudaStreamCreateWithFlags(&relaxed.st, cudaStreamNonBlocking) != cudaSuccess) return nullptr;
     // word 1: limit of waits on flags written by OTHER GPUs, in units of 2^20 clock cycles (0 = the built-in limit).
     // Ranks drift apart on the host (graph capture, a slow data loader), so this limit is longer than the one of the
     // waits inside a kernel; KSA_PEER_WAIT_MS overrides it, ksa_set_peer_wait_ms changes it at run time.
@@ -112,7 +122,10 @@ int* status_word() {
       const long long ms = atoll(e);
       if (ms > 0) units = (int)(ms * 2000LL / 1049 + 1);
     }
-    cudaMemcpy(p + 1, &units, sizeof(int), cudaMemcpyHostToDevice);
+    int words[64] = {0, units};
+    if (cudaMemcpyAsync(p, words, sizeof(words), cudaMemcpyHostToDevice, relaxed.st) != cudaSuccess ||
+        cudaStreamSynchronize(relaxed.st) != cudaSuccess)
+      return nullptr;
     g_status[dev] = p;
   }
   return g_status[dev];

@@ -143,7 +143,7 @@ struct Args {
   }
 };
 
-bool rows2d(const Tensor* t) { return t->dim() == 2 && t->stride(1) == 1; }      // rows with any pitch
+bool rows2d(const Tensor* t) { return t->dim() == 2 && t->stride(1) == 1 && t->stride(0) > 0; }      // rows with any pitch
 bool packed2d(const Tensor* t) { return t->dim() == 2 && t->is_contiguous(); }
 bool vector(const Tensor* t, long long n) { return t->dim() == 1 && t->size(0) == n && t->is_contiguous(); }
 bool fits(long long x) { return x > 0 && x <= INT_MAX; }
@@ -471,7 +471,7 @@ PyObject* py_norm_linear(PyObject*, PyObject* const* v, Py_ssize_t n) {
   const float eps = a.real();
   const Tensor* w = a.tensor();
   const int glu = a.integer() != 0;
-  if (!a.ok() || !rows2d(x) || !rows2d(w) || x->size(0) > 4 || x->size(1) != w->size(1) || !vector(nw, x->size(1)) || !fits(w->size(0)) ||
+  if (!a.ok() || !rows2d(x) || !rows2d(w) || x->size(0) > 4 || x->numel() > 81920 || x->size(1) != w->size(1) || !vector(nw, x->size(1)) || !fits(w->size(0)) ||
       !fits(x->size(1)) || x->size(1) % 8 != 0 || x->stride(0) % 8 != 0 || w->stride(0) % 8 != 0 || (glu && w->size(0) % 2 != 0))
     return none();
   if (d && !(rows2d(d) && d->size(1) == x->size(1) && d->size(0) <= x->size(0) && d->stride(0) % 8 == 0)) return none();

@@ -124,9 +124,10 @@ def gemm(a: torch.Tensor, b: torch.Tensor, *, a_mn_major: bool = False, b_mn_maj
     if (M <= 16 and not a_mn_major and not b_mn_major and out.dtype == torch.bfloat16 and not accumulate
             and alpha == 1.0 and K % 8 == 0):
         # decoding: a few activation rows against a whole weight matrix is a stream of the weights, served by the
-        # bandwidth-shaped kernel instead of 128-row tensor-core tiles.  16 rows is where that kernel ends and not where the split-K
-        # kernel below starts to pay: 16 rows x 6144 x 2560 take 15.7 us here and 11.9 there, x 2560 x 9728 25.1 and 15.4, x 19456 x
-        # 2560 37.1 and 22.3; but 8 rows x 6144 x 2560 10.6 and 11.5, 16 x 4096 x 2048 7.8 and 9.2, x 2048 x 2048 5.9 and 8.5
+        # bandwidth-shaped kernel instead of 128-row tensor-core tiles: at 16 rows, where it ends, 6144 x 2560 take 9.3 us there and
+        # 11.9 on the split-K kernel below, 2560 x 9728 12.3 and 15.4
+        # (its tensor maps take no pitch of zero: expanded rows are written out first)
+        a, b = (t if t.stride(0) > 0 or t.shape[0] == 1 else t.contiguous() for t in (a, b))
         _lib.call("ksa_gemv_bf16", a, b, out, M, N, K, a.stride(0), b.stride(0), out.stride(0))
         return out
     if pair is None and sm_limit == 0 and not a_mn_major and out.dtype == torch.bfloat16 and not accumulate:
@@ -515,8 +516,8 @@ def norm_linear(x: torch.Tensor, delta: Optional[torch.Tensor], norm_w: torch.Te
                 weight: torch.Tensor, glu: bool = False):
     """``res = x + delta``; ``y = rms_norm(res, norm_w) @ weight.T`` (with ``glu``: ``swiglu`` of it, ``weight`` = gate
     rows then up rows).  Returns ``(res, y)``.  For at most 4 rows on a GPU without autograd (a decode step) this is
-    one launch (``ksa_gemv_norm_bf16``: every CTA normalises the few activation rows itself while it stages them);
-    everything else is ``add_rms_norm`` followed by the projection."""
+    one launch (``ksa_gemv_norm_bf16``: every CTA normalises the few activation rows itself and keeps them in shared memory, up
+    to 160 KB of them); everything else is ``add_rms_norm`` followed by the projection."""
     if x.shape[0] <= 4 and _cuda(x) and not _observed():
         made = _native.norm_linear(x, delta, norm_w, eps, weight, glu)
         if made is not None:
@@ -525,11 +526,15 @@ def norm_linear(x: torch.Tensor, delta: Optional[torch.Tensor], norm_w: torch.Te
             and x.dtype == torch.bfloat16 and weight.dtype == torch.bfloat16
             and not (torch.is_grad_enabled() and (x.requires_grad or weight.requires_grad))
             and x.stride(1) == 1 and weight.stride(1) == 1 and x.shape[1] % 8 == 0 and x.stride(0) % 8 == 0
-            and weight.stride(0) % 8 == 0 and (delta is None or (delta.stride(1) == 1 and delta.stride(0) % 8 == 0
+            and weight.stride(0) % 8 == 0 and weight.stride(0) > 0 and (delta is None or (delta.stride(1) == 1 and delta.stride(0) % 8 == 0
                                                                   and delta.dtype == torch.bfloat16))
-            and (not glu or weight.shape[0] % 2 == 0)):
+            and (not glu or weight.shape[0] % 2 == 0) and (x.numel() <= 81920 or x.shape[0] > 1)):
         M, K = x.shape
         N = weight.shape[0]
+        if x.numel() > 81920:              # more than a CTA keeps in shared memory beside its ring: row by row
+            parts = [norm_linear(x[i:i + 1], None if delta is None or i >= delta.shape[0] else delta[i:i + 1], norm_w, eps, weight, glu)
+                     for i in range(M)]
+            return x if delta is None else torch.cat([r for r, _ in parts]), torch.cat([y for _, y in parts])
         res = torch.empty((M, K), dtype=torch.bfloat16, device=x.device) if delta is not None else x
         out = torch.empty((M, N // 2 if glu else N), dtype=torch.bfloat16, device=x.device)
         _lib.call("ksa_gemv_norm_bf16", x, delta, norm_w, res if delta is not None else None, weight, out, M, N, K,
@@ -618,7 +623,7 @@ def linear_swiglu(x: torch.Tensor, w13: torch.Tensor) -> torch.Tensor:
             and x.dtype == torch.bfloat16 and w13.dtype == torch.bfloat16
             and not (torch.is_grad_enabled() and (x.requires_grad or w13.requires_grad))
             and x.stride(1) == 1 and w13.stride(1) == 1 and x.shape[1] % 8 == 0 and x.stride(0) % 8 == 0
-            and w13.stride(0) % 8 == 0 and w13.shape[0] % 2 == 0):
+            and w13.stride(0) % 8 == 0 and min(x.stride(0), w13.stride(0)) > 0 and w13.shape[0] % 2 == 0):
         M, K = x.shape
         N = w13.shape[0]
         plan = _narrow_swiglu(x, w13) if M > 16 else None
