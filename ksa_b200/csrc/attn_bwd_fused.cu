@@ -226,6 +226,7 @@ __device__ __forceinline__ void attn_bwd_fused_body(const CUtensorMap& tmQ, cons
   __syncthreads();
   tc_fence_after();
   const uint32_t tmem_base = *tmem_slot;
+  grid_dependency_enter();
   const uint32_t tS = tmem_base, tdP = tmem_base + 128, tdV = tmem_base + 256, tdK = tmem_base + 384;
 
   if (warp == 0) {
@@ -531,6 +532,7 @@ __global__ void __launch_bounds__(256)
 attn_bwd_prep_kernel(const bf16* __restrict__ o, const bf16* __restrict__ d_o, long long o_rs, long long o_bs,
                      const float* __restrict__ lse, float* __restrict__ stats, float* __restrict__ dq32, int B, int Hq,
                      int Lq, int lq_pad) {
+  grid_dependency_enter();
   const long long item = ((long long)blockIdx.x * blockDim.x + threadIdx.x) >> 4;
   const int l16 = threadIdx.x & 15;
   const long long rows = (long long)B * Hq * lq_pad;
@@ -571,6 +573,7 @@ attn_bwd_prep_kernel(const bf16* __restrict__ o, const bf16* __restrict__ d_o, l
 // Conversion: dq = bf16(dq32 * scale).  One thread per 8 elements.
 __global__ void attn_bwd_dq_convert_kernel(const float* __restrict__ dq32, bf16* __restrict__ dq, long long dq_rs,
                                            long long dq_bs, int B, int Lq, int Hq, float scale) {
+  grid_dependency_enter();
   const long long idx = (long long)blockIdx.x * blockDim.x + threadIdx.x;   // over B * Lq * Hq * 16
   const long long n = (long long)B * Lq * Hq * 16;
   if (idx >= n) return;
@@ -667,10 +670,9 @@ KSA_API int ksa_attn_bwd_fused(const void* q, const void* k, const void* v, cons
     const long long items = (long long)B * Hq * lq_pad;
     const int threads = 256;
     const long long blocks = (items * 16 + threads - 1) / threads;
-    attn_bwd_prep_kernel<<<(unsigned)blocks, threads, 0, st>>>((const bf16*)o, (const bf16*)d_o, o_rs, o_bs,
-                                                               (const float*)lse, (float*)stats, (float*)dq32, B, Hq,
-                                                               Lq, lq_pad);
-    KSA_CHECK_CUDA(cudaGetLastError());
+    KSA_CHECK_CUDA(launch_stream_kernel(items * 1024, attn_bwd_prep_kernel, dim3((unsigned)blocks), dim3(threads), 0, st,
+                                        (const bf16*)o, (const bf16*)d_o, o_rs, o_bs, (const float*)lse, (float*)stats,
+                                        (float*)dq32, B, Hq, Lq, lq_pad));
   }
   CUtensorMap tdq;
   {
@@ -680,14 +682,14 @@ KSA_API int ksa_attn_bwd_fused(const void* q, const void* k, const void* v, cons
     if ((rc = make_tmap(&tdq, dq32, 4, 4, dims, str, box, false))) return rc;
   }
   dim3 grid((Lk + 127) / 128 + ((Ns + 127) / 128) * p.n_seg, Hkv, B);
-  attn_bwd_fused_kernel<<<grid, kFbThreads, FbSmem::kTotal, st>>>(tq, tdo, tk, tv, tks, tvs, tdq, p);
-  KSA_CHECK_CUDA(cudaGetLastError());
+  KSA_CHECK_CUDA(launch_kernel(attn_bwd_fused_kernel, grid, dim3(kFbThreads), (size_t)FbSmem::kTotal, st, tq, tdo, tk, tv,
+                               tks, tvs, tdq, p));
   {
     const long long n = (long long)B * Lq * Hq * 16;
     const int threads = 256;
-    attn_bwd_dq_convert_kernel<<<(unsigned)((n + threads - 1) / threads), threads, 0, st>>>(
-        (const float*)dq32, (bf16*)dq, dq_rs, dq_bs, B, Lq, Hq, scale);
-    KSA_CHECK_CUDA(cudaGetLastError());
+    KSA_CHECK_CUDA(launch_stream_kernel(n * 48, attn_bwd_dq_convert_kernel, dim3((unsigned)((n + threads - 1) / threads)),
+                                        dim3(threads), 0, st, (const float*)dq32, (bf16*)dq, dq_rs, dq_bs, B, Lq, Hq,
+                                        scale));
   }
   return 0;
 }

@@ -121,6 +121,7 @@ __device__ __forceinline__ void attn_fwd_body(const CUtensorMap& tmQ, const CUte
   __syncthreads();
   tc_fence_after();
   const uint32_t tmem_base = *tmem_slot;
+  grid_dependency_enter();
 
   if (warp >= 8) {
     asm volatile("setmaxnreg.dec.sync.aligned.u32 56;");
@@ -461,8 +462,7 @@ static int launch_fwd(const CUtensorMap& tq, const CUtensorMap& tk, const CUtens
   int sms = sm_count();
   if (sms <= 0) return 1;
   dim3 grid(items < sms ? items : sms);
-  kern<<<grid, kFwdThreads, FwdSmem<HD>::kTotal, st>>>(tq, tk, tv, tks, tvs, p);
-  KSA_CHECK_CUDA(cudaGetLastError());
+  KSA_CHECK_CUDA(launch_kernel(kern, grid, dim3(kFwdThreads), (size_t)FwdSmem<HD>::kTotal, st, tq, tk, tv, tks, tvs, p));
   return 0;
 }
 

@@ -70,6 +70,7 @@ __device__ __forceinline__ const bf16* key_row(const bf16* text, long long t_rs,
 
 // grid (local chunks, Hq, B), 128 threads, dynamic smem = (HD + C + S) floats
 __global__ void __launch_bounds__(128) summary_attn_fwd_kernel(SumAttnArgs a) {
+  grid_dependency_enter();
   extern __shared__ float sm[];
   __shared__ float red[4];
   float* q_s = sm;
@@ -120,6 +121,7 @@ __global__ void __launch_bounds__(128) summary_attn_fwd_kernel(SumAttnArgs a) {
 // dynamic smem: nq * (2*HD + 2*(C+S)) floats with nq = (Hq/Hkv) * S queries per block.
 // dK/dV of the chunk's text keys and summary keys are ADDED to what the text-query backward wrote.
 __global__ void __launch_bounds__(128) summary_attn_bwd_kernel(SumAttnArgs a) {
+  grid_dependency_enter();
   extern __shared__ float sm[];
   __shared__ float red[4];
   const int G = a.Hq / a.Hkv, S = a.n_sum, HD = a.HD;
@@ -220,6 +222,7 @@ constexpr int kSumFwdMaxQ = 8;
 // us; four queries, 256 chunks: 97.1 -> 87.3 us).
 template <int HD, int NQ>
 __global__ void __launch_bounds__(kSumFwdThreads) summary_attn_fwd_fast_kernel(SumAttnArgs a, int nk_max) {
+  grid_dependency_enter();
   extern __shared__ uint32_t smw[];
   const int G = a.Hq / a.Hkv, S = a.n_sum, nq = NQ < kSumFwdMaxQ ? NQ : G * S;
   bf16* v_s = reinterpret_cast<bf16*>(smw);
@@ -344,6 +347,7 @@ constexpr int kSumBwdMaxQ = 8;
 
 template <int HD, int NQ>      // NQ as in the forward kernel
 __global__ void __launch_bounds__(kSumBwdThreads) summary_attn_bwd_fast_kernel(SumAttnArgs a, int nk_max) {
+  grid_dependency_enter();
   extern __shared__ uint32_t smw[];
   constexpr int kRowElems = HD + 8;                   // padded K row, bf16 elements
   const int G = a.Hq / a.Hkv, S = a.n_sum, nq = NQ < kSumBwdMaxQ ? NQ : G * S;
@@ -520,8 +524,8 @@ static int launch_fwd_fast(const SumAttnArgs& a, int nk_max, size_t smem, cudaSt
     KSA_CHECK_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, 100 * 1024));
     attr = true;
   }
-  kern<<<dim3(a.Nq / a.n_sum, a.Hkv, a.B), kSumFwdThreads, smem, st>>>(a, nk_max);
-  KSA_CHECK_CUDA(cudaGetLastError());
+  KSA_CHECK_CUDA(launch_stream_kernel((long long)a.B * a.Hkv * (a.Nq / a.n_sum) * nk_max * 512, kern, dim3(a.Nq / a.n_sum,
+                                      a.Hkv, a.B), dim3(kSumFwdThreads), smem, st, a, nk_max));
   return 0;
 }
 
@@ -533,8 +537,8 @@ static int launch_bwd_fast(const SumAttnArgs& a, int nk_max, size_t smem, cudaSt
     KSA_CHECK_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, 100 * 1024));
     attr = true;
   }
-  kern<<<dim3(a.Nq / a.n_sum, a.Hkv, a.B), kSumBwdThreads, smem, st>>>(a, nk_max);
-  KSA_CHECK_CUDA(cudaGetLastError());
+  KSA_CHECK_CUDA(launch_stream_kernel((long long)a.B * a.Hkv * (a.Nq / a.n_sum) * nk_max * 512, kern, dim3(a.Nq / a.n_sum,
+                                      a.Hkv, a.B), dim3(kSumBwdThreads), smem, st, a, nk_max));
   return 0;
 }
 
@@ -572,8 +576,7 @@ KSA_API int ksa_summary_attn_fwd(const void* qs, const void* k, const void* v, c
   const size_t smem = (size_t)(HD + chunk + n_sum) * sizeof(float);
   KSA_REQUIRE(smem <= 48 * 1024, "summary_attn_fwd: chunk %d too large for the SIMT kernel", chunk);
   dim3 grid(Nq / n_sum, Hq, B);
-  summary_attn_fwd_kernel<<<grid, 128, smem, reinterpret_cast<cudaStream_t>(stream)>>>(a);
-  KSA_CHECK_CUDA(cudaGetLastError());
+  KSA_CHECK_CUDA(launch_kernel(summary_attn_fwd_kernel, grid, dim3(128), smem, reinterpret_cast<cudaStream_t>(stream), a));
   return 0;
 }
 
@@ -622,7 +625,6 @@ KSA_API int ksa_summary_attn_bwd(const void* qs, const void* k, const void* v, c
     attr = true;
   }
   dim3 grid(Nq / n_sum, Hkv, B);
-  summary_attn_bwd_kernel<<<grid, 128, smem, reinterpret_cast<cudaStream_t>(stream)>>>(a);
-  KSA_CHECK_CUDA(cudaGetLastError());
+  KSA_CHECK_CUDA(launch_kernel(summary_attn_bwd_kernel, grid, dim3(128), smem, reinterpret_cast<cudaStream_t>(stream), a));
   return 0;
 }

@@ -299,6 +299,14 @@ __host__ __device__ constexpr uint32_t umma_idesc_bf16(int m, int n, int a_mn_ma
 __device__ __forceinline__ void grid_dependency_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
 __device__ __forceinline__ void grid_dependency_launch() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
 
+// The first thing a kernel does with memory that others write, or before it writes memory that others read: everything up to here
+// (barriers, tensor memory, address arithmetic) may run while the previous kernel of the stream still does.  Its own successor may
+// start from now on, so a kernel that only waits here overlaps at most its immediate predecessor.
+__device__ __forceinline__ void grid_dependency_enter() {
+  grid_dependency_wait();
+  grid_dependency_launch();
+}
+
 // ----------------------------------------------------------------- small helpers
 __device__ __forceinline__ uint32_t pack_bf16x2(float lo, float hi) {
   __nv_bfloat162 v = __floats2bfloat162_rn(lo, hi);

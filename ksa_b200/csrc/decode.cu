@@ -491,12 +491,11 @@ KSA_API int ksa_decode_attn(const void* q, const void* k_cache, const void* v_ca
   dim3 grid(splits, Hkv, B);
   cudaStream_t st = reinterpret_cast<cudaStream_t>(stream);
   const int nq = (Hq / Hkv) * Tq;
-  const bool dep = dependent_launch_enabled();
-  if (D == 128 && nq <= 4) KSA_CHECK_CUDA(launch_kernel(dep, decode_attn_mma_kernel<4>, grid, dim3(kDecThreads), 0, st, a));
-  else if (D == 128 && nq <= 8) KSA_CHECK_CUDA(launch_kernel(dep, decode_attn_mma_kernel<8>, grid, dim3(kDecThreads), 0, st, a));
-  else if (D == 128) KSA_CHECK_CUDA(launch_kernel(dep, decode_attn_mma_kernel<16>, grid, dim3(kDecThreads), 0, st, a));
-  else KSA_CHECK_CUDA(launch_kernel(dep, decode_attn_kernel<64>, grid, dim3(kDecThreads), 0, st, a));
-  if (counters == nullptr) KSA_CHECK_CUDA(launch_kernel(dep, decode_combine_kernel, dim3(B * Tq * Hq), dim3(128), 0, st, a));
+  if (D == 128 && nq <= 4) KSA_CHECK_CUDA(launch_kernel(decode_attn_mma_kernel<4>, grid, dim3(kDecThreads), 0, st, a));
+  else if (D == 128 && nq <= 8) KSA_CHECK_CUDA(launch_kernel(decode_attn_mma_kernel<8>, grid, dim3(kDecThreads), 0, st, a));
+  else if (D == 128) KSA_CHECK_CUDA(launch_kernel(decode_attn_mma_kernel<16>, grid, dim3(kDecThreads), 0, st, a));
+  else KSA_CHECK_CUDA(launch_kernel(decode_attn_kernel<64>, grid, dim3(kDecThreads), 0, st, a));
+  if (counters == nullptr) KSA_CHECK_CUDA(launch_kernel(decode_combine_kernel, dim3(B * Tq * Hq), dim3(128), 0, st, a));
   return 0;
 }
 
@@ -507,7 +506,7 @@ KSA_API int ksa_kv_cache_append(const void* k_new, const void* v_new, void* k_ca
   KSA_REQUIRE(D % 8 == 0, "kv_cache_append: head_dim must be a multiple of 8");
   const long long n = (long long)B * T * H * (D / 8);
   if (n == 0) return 0;
-  KSA_CHECK_CUDA(launch_kernel(dependent_launch_enabled(), kv_cache_append_kernel, dim3((unsigned)((n + 255) / 256)),
+  KSA_CHECK_CUDA(launch_kernel(kv_cache_append_kernel, dim3((unsigned)((n + 255) / 256)),
                               dim3(256), 0, reinterpret_cast<cudaStream_t>(stream), (const bf16*)k_new,
                               (const bf16*)v_new, (bf16*)k_cache, (bf16*)v_cache, (const int*)slots, B, T, H, D, cap,
                               src_row_stride, src_batch_stride));
@@ -519,7 +518,7 @@ KSA_API int ksa_kv_cache_move(void* k_cache, void* v_cache, const void* src, con
   KSA_ENTER(k_cache);
   const long long n = (long long)B * H * rows * (D / 8);
   if (n == 0) return 0;
-  KSA_CHECK_CUDA(launch_kernel(dependent_launch_enabled(), kv_cache_move_kernel, dim3((unsigned)((n + 255) / 256)),
+  KSA_CHECK_CUDA(launch_kernel(kv_cache_move_kernel, dim3((unsigned)((n + 255) / 256)),
                               dim3(256), 0, reinterpret_cast<cudaStream_t>(stream), (bf16*)k_cache, (bf16*)v_cache,
                               (const int*)src, (const int*)dst, (const int*)enable, B, H, D, cap, rows));
   return 0;

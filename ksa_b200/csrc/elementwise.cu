@@ -21,8 +21,7 @@ __global__ void __launch_bounds__(kNormThreads)
 rmsnorm_fwd_kernel(const bf16* __restrict__ x, const bf16* __restrict__ delta, const bf16* __restrict__ w,
                    bf16* __restrict__ res_out, bf16* __restrict__ y, float* __restrict__ rstd_out, int rows, int D,
                    float eps, int delta_rows) {
-  grid_dependency_launch();   // a dependent-launched successor may start (the skinny GEMM: its weight loads)
-  grid_dependency_wait();     // launched dependently itself: the previous kernel's results are complete from here on
+  grid_dependency_enter();
   __shared__ float red[32];
   const int row = blockIdx.x;
   if (row >= rows) return;
@@ -75,6 +74,7 @@ __global__ void __launch_bounds__(kNormThreads, MINB)
 rmsnorm_bwd_kernel(const bf16* __restrict__ dy, const bf16* __restrict__ x, const bf16* __restrict__ w,
                    const float* __restrict__ rstd_in, const bf16* __restrict__ dres, bf16* __restrict__ dx,
                    float* __restrict__ dw_partial, int rows, int D) {
+  grid_dependency_enter();
   __shared__ float red[R][8];
   BF8 wv[NVEC];
   float dw[NVEC][8];
@@ -180,6 +180,7 @@ rmsnorm_bwd_kernel(const bf16* __restrict__ dy, const bf16* __restrict__ x, cons
 // dw[c] (+)= sum over partial rows.  Block = 32 columns x 8 row groups.
 __global__ void __launch_bounds__(256)
 colsum_partials_kernel(const float* __restrict__ partial, float* __restrict__ dw, int nparts, int D, int accumulate) {
+  grid_dependency_enter();
   __shared__ float red[8][33];
   const int tx = threadIdx.x & 31, ty = threadIdx.x >> 5;
   const int c = blockIdx.x * 32 + tx;
@@ -215,8 +216,7 @@ struct QkRopeArgs {
 
 template <int D>
 __global__ void __launch_bounds__(256) qknorm_rope_fwd_kernel(QkRopeArgs a) {
-  grid_dependency_launch();   // a dependent-launched successor may start (the skinny GEMM: its weight loads)
-  grid_dependency_wait();     // launched dependently itself: the previous kernel's results are complete from here on
+  grid_dependency_enter();
   constexpr int PAIRS = D / 64;  // rotary pairs per lane
   const int warp_global = blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5);
   const int lane = threadIdx.x & 31;
@@ -279,6 +279,7 @@ struct QkRopeBwdArgs {
 
 template <int D>
 __global__ void __launch_bounds__(256) qknorm_rope_bwd_kernel(QkRopeBwdArgs b) {
+  grid_dependency_enter();
   constexpr int PAIRS = D / 64;
   const QkRopeArgs& a = b.f;
   __shared__ float s_dw[2][D];
@@ -403,8 +404,7 @@ __device__ __forceinline__ void rope_pair_idx(int p, int& i1, int& i2) {
 
 template <bool IL, int NH>      // NH: heads of a row that a warp takes
 __global__ void __launch_bounds__(256) qknorm_rope_fwd128_kernel(QkRopeArgs a) {
-  grid_dependency_launch();   // a dependent-launched successor may start (the skinny GEMM: its weight loads)
-  grid_dependency_wait();     // launched dependently itself: the previous kernel's results are complete from here on
+  grid_dependency_enter();
   const int lane = threadIdx.x & 31;
   const int H = a.Hq + a.Hkv;
   const int Hall = H + (a.copy_v ? a.Hkv : 0);
@@ -527,6 +527,7 @@ __global__ void __launch_bounds__(256) qknorm_rope_decode128_kernel(QkRopeArgs a
 
 template <bool IL>
 __global__ void __launch_bounds__(256) qknorm_rope_bwd128_kernel(QkRopeBwdArgs b) {
+  grid_dependency_enter();
   const QkRopeArgs& a = b.f;
   __shared__ float s_dw[2][128];
   for (int i = threadIdx.x; i < 256; i += blockDim.x) (&s_dw[0][0])[i] = 0.f;
@@ -616,8 +617,7 @@ __global__ void __launch_bounds__(256) qknorm_rope_bwd128_kernel(QkRopeBwdArgs b
 // gate_up is [rows, 2F] = [gate | up]; out is [rows, F].
 __global__ void __launch_bounds__(256)
 swiglu_fwd_kernel(const bf16* __restrict__ gu, bf16* __restrict__ out, long long rows, int F) {
-  grid_dependency_launch();   // a dependent-launched successor may start (the skinny GEMM: its weight loads)
-  grid_dependency_wait();     // launched dependently itself: the previous kernel's results are complete from here on
+  grid_dependency_enter();
   const long long vec = (long long)blockIdx.x * blockDim.x + threadIdx.x;
   const int per_row = F / 8;
   if (vec >= rows * per_row) return;
@@ -633,6 +633,7 @@ swiglu_fwd_kernel(const bf16* __restrict__ gu, bf16* __restrict__ out, long long
 __global__ void __launch_bounds__(256)
 swiglu_bwd_kernel(const bf16* __restrict__ gu, const bf16* __restrict__ dout, bf16* __restrict__ dgu, long long rows,
                   int F) {
+  grid_dependency_enter();
   const long long vec = (long long)blockIdx.x * blockDim.x + threadIdx.x;
   const int per_row = F / 8;
   if (vec >= rows * per_row) return;
@@ -657,8 +658,7 @@ swiglu_bwd_kernel(const bf16* __restrict__ gu, const bf16* __restrict__ dout, bf
 __global__ void __launch_bounds__(256)
 embedding_fwd_kernel(const long long* __restrict__ ids, const bf16* __restrict__ table, bf16* __restrict__ out,
                      long long rows, int D, long long vocab) {
-  grid_dependency_launch();   // a dependent-launched successor may start (the skinny GEMM: its weight loads)
-  grid_dependency_wait();     // launched dependently itself: the previous kernel's results are complete from here on
+  grid_dependency_enter();
   const long long vec = (long long)blockIdx.x * blockDim.x + threadIdx.x;
   const int per_row = D / 8;
   if (vec >= rows * per_row) return;
@@ -671,6 +671,7 @@ embedding_fwd_kernel(const long long* __restrict__ ids, const bf16* __restrict__
 __global__ void __launch_bounds__(256)
 embedding_bwd_kernel(const long long* __restrict__ ids, const bf16* __restrict__ dout, float* __restrict__ dtable,
                      long long rows, int D, long long vocab) {
+  grid_dependency_enter();
   const long long vec = (long long)blockIdx.x * blockDim.x + threadIdx.x;
   const int per_row = D / 8;
   if (vec >= rows * per_row) return;
@@ -692,6 +693,7 @@ constexpr int kCeThreads = 512;
 __global__ void __launch_bounds__(kCeThreads)
 cross_entropy_kernel(bf16* __restrict__ logits, const long long* __restrict__ labels, float* __restrict__ row_loss,
                      const float* __restrict__ grad_scale, int V, long long ld, int ignore_index, int write_grad) {
+  grid_dependency_enter();
   __shared__ float red[32];
   const long long row = blockIdx.x;
   bf16* lg = logits + row * ld;
@@ -744,6 +746,7 @@ cross_entropy_kernel(bf16* __restrict__ logits, const long long* __restrict__ la
 // n_valid and 1/n_valid (times an extra scale) on the device: no host sync in the step.
 __global__ void count_valid_kernel(const long long* __restrict__ labels, long long n, int ignore_index, float extra_scale,
                                    float* __restrict__ out /* [0]=count, [1]=extra/count */) {
+  grid_dependency_enter();
   __shared__ float red[32];
   float c = 0.f;
   for (long long i = threadIdx.x; i < n; i += blockDim.x) c += (labels[i] != ignore_index) ? 1.f : 0.f;
@@ -761,6 +764,7 @@ __global__ void __launch_bounds__(256)
 adamw_kernel(float* __restrict__ master, const float* __restrict__ grad, float* __restrict__ m, float* __restrict__ v,
              bf16* __restrict__ out_bf16, long long n, const float* __restrict__ hyper, float beta1, float beta2,
              float eps, float weight_decay, float clip_value, float* __restrict__ sumsq) {
+  grid_dependency_wait();     // and no early successor: this kernel writes weights
   __shared__ float red[32];
   const float lr = hyper[0], bc1 = hyper[1], bc2 = hyper[2], gscale = hyper[3];
   float sq = 0.f;
@@ -798,6 +802,7 @@ adamw_kernel(float* __restrict__ master, const float* __restrict__ grad, float* 
 
 // fp32 -> bf16 cast (flat), used to refresh compute weights from master weights.
 __global__ void __launch_bounds__(256) cast_f32_bf16_kernel(const float* __restrict__ src, bf16* __restrict__ dst, long long n) {
+  grid_dependency_wait();     // and no early successor: the copies may be weights
   const long long nvec = n / 4;
   for (long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x; i < nvec; i += (long long)gridDim.x * blockDim.x) {
     float4 a = reinterpret_cast<const float4*>(src)[i];
@@ -817,9 +822,9 @@ KSA_API int ksa_rmsnorm_fwd(const void* x, const void* delta, const void* w, voi
   KSA_REQUIRE(D % 8 == 0 && D <= kNormThreads * 8 * kNormMaxVec, "rmsnorm: D=%d must be a multiple of 8 and <= %d", D,
               kNormThreads * 8 * kNormMaxVec);
   if (rows == 0) return 0;
-  KSA_CHECK_CUDA(launch_kernel(dependent_launch_enabled(), rmsnorm_fwd_kernel, dim3(rows), dim3(kNormThreads), 0,
-                              ST(stream), (const bf16*)x, (const bf16*)delta, (const bf16*)w, (bf16*)res_out, (bf16*)y,
-                              (float*)rstd, rows, D, eps, delta_rows));
+  KSA_CHECK_CUDA(launch_stream_kernel(8LL * rows * D, rmsnorm_fwd_kernel, dim3(rows), dim3(kNormThreads), 0, ST(stream),
+                                      (const bf16*)x, (const bf16*)delta, (const bf16*)w, (bf16*)res_out, (bf16*)y,
+                                      (float*)rstd, rows, D, eps, delta_rows));
   return 0;
 }
 
@@ -836,10 +841,9 @@ static int launch_rmsnorm_bwd(const void* dy, const void* x, const void* w, cons
   const int rounds = (groups + most - 1) / most;
   const int blocks = (groups + rounds - 1) / rounds;
   // rows beyond `blocks` partial rows stay untouched; zero-fill is not needed because colsum reads `blocks` rows only
-  rmsnorm_bwd_kernel<NVEC, R, MINB><<<blocks, kNormThreads, 0, st>>>((const bf16*)dy, (const bf16*)x, (const bf16*)w,
-                                                               (const float*)rstd, (const bf16*)dres, (bf16*)dx,
-                                                               (float*)dw_partial, rows, D);
-  KSA_CHECK_CUDA(cudaGetLastError());
+  KSA_CHECK_CUDA(launch_stream_kernel(8LL * rows * D, rmsnorm_bwd_kernel<NVEC, R, MINB>, dim3(blocks), dim3(kNormThreads),
+                                      0, st, (const bf16*)dy, (const bf16*)x, (const bf16*)w, (const float*)rstd,
+                                      (const bf16*)dres, (bf16*)dx, (float*)dw_partial, rows, D));
   return blocks;
 }
 
@@ -855,9 +859,8 @@ KSA_API int ksa_rmsnorm_bwd(const void* dy, const void* x, const void* w, const 
   else used = launch_rmsnorm_bwd<4, 1, 1>(dy, x, w, rstd, dres, dx, dw_partial, parts, rows, D, ST(stream));
   if (used < 0) return used;
   if (dw) {
-    colsum_partials_kernel<<<(D + 31) / 32, 256, 0, ST(stream)>>>((const float*)dw_partial, (float*)dw, used, D,
-                                                                  accumulate_dw);
-    KSA_CHECK_CUDA(cudaGetLastError());
+    KSA_CHECK_CUDA(launch_kernel(colsum_partials_kernel, dim3((D + 31) / 32), dim3(256), 0, ST(stream),
+                                 (const float*)dw_partial, (float*)dw, used, D, accumulate_dw));
   }
   return 0;
 }
@@ -874,14 +877,15 @@ KSA_API int ksa_qknorm_rope_fwd(const void* qkv, void* out, const void* q_w, con
   const int blocks = (int)((warps + 7) / 8);
   const int heads = Hq + Hkv + (copy_v ? Hkv : 0);
   const int blocks128 = (int)(((long long)rows * rope_groups(heads) + 7) / 8);
-  const bool dep = dependent_launch_enabled();
   const bool few = heads <= 4;
   if (D == 128) {
     auto kern = interleaved ? (few ? qknorm_rope_fwd128_kernel<true, 4> : qknorm_rope_fwd128_kernel<true, kRopeHeads>)
                             : (few ? qknorm_rope_fwd128_kernel<false, 4> : qknorm_rope_fwd128_kernel<false, kRopeHeads>);
-    KSA_CHECK_CUDA(launch_kernel(dep, kern, dim3(blocks128), dim3(256), 0, ST(stream), a));
+    KSA_CHECK_CUDA(launch_stream_kernel(4LL * rows * (Hq + 2 * Hkv) * D, kern, dim3(blocks128), dim3(256), 0, ST(stream),
+                                        a));
   } else {
-    KSA_CHECK_CUDA(launch_kernel(dep, qknorm_rope_fwd_kernel<64>, dim3(blocks), dim3(256), 0, ST(stream), a));
+    KSA_CHECK_CUDA(launch_stream_kernel(4LL * rows * (Hq + 2 * Hkv) * D, qknorm_rope_fwd_kernel<64>, dim3(blocks),
+                                        dim3(256), 0, ST(stream), a));
   }
   return 0;
 }
@@ -901,11 +905,12 @@ KSA_API int ksa_qknorm_rope_decode(const void* qkv, void* out, const void* q_w, 
                in_stride, out_stride, rows, Hq, Hkv, D, log2f(theta), eps, interleaved, 1};
   QkRopeCacheArgs c{(bf16*)k_cache, (bf16*)v_cache, (const int*)slots, cache_rows, cap};
   const int warps = rows * (Hq + 2 * Hkv);
-  const bool dep = dependent_launch_enabled();
   if (interleaved)
-    KSA_CHECK_CUDA(launch_kernel(dep, qknorm_rope_decode128_kernel<true>, dim3((warps + 7) / 8), dim3(256), 0, ST(stream), a, c));
+    KSA_CHECK_CUDA(launch_kernel(qknorm_rope_decode128_kernel<true>, dim3((warps + 7) / 8), dim3(256), 0, ST(stream), a,
+                                 c));
   else
-    KSA_CHECK_CUDA(launch_kernel(dep, qknorm_rope_decode128_kernel<false>, dim3((warps + 7) / 8), dim3(256), 0, ST(stream), a, c));
+    KSA_CHECK_CUDA(launch_kernel(qknorm_rope_decode128_kernel<false>, dim3((warps + 7) / 8), dim3(256), 0, ST(stream), a,
+                                 c));
   return 0;
 }
 
@@ -925,10 +930,13 @@ KSA_API int ksa_qknorm_rope_bwd(const void* qkv, const void* d_out, void* d_qkv,
   if (D == 128) {
     int rb = (rows + 7) / 8;
     if (rb > 148 * 8) rb = 148 * 8;
-    if (interleaved) qknorm_rope_bwd128_kernel<true><<<rb, 256, 0, ST(stream)>>>(b);
-    else qknorm_rope_bwd128_kernel<false><<<rb, 256, 0, ST(stream)>>>(b);
+    if (interleaved) KSA_CHECK_CUDA(launch_stream_kernel(6LL * rows * (Hq + 2 * Hkv) * D, qknorm_rope_bwd128_kernel<true>,
+                                                         dim3(rb), dim3(256), 0, ST(stream), b));
+    else KSA_CHECK_CUDA(launch_stream_kernel(6LL * rows * (Hq + 2 * Hkv) * D, qknorm_rope_bwd128_kernel<false>, dim3(rb),
+                                             dim3(256), 0, ST(stream), b));
   } else {
-    qknorm_rope_bwd_kernel<64><<<(int)blocks, 256, 0, ST(stream)>>>(b);
+    KSA_CHECK_CUDA(launch_stream_kernel(6LL * rows * (Hq + 2 * Hkv) * D, qknorm_rope_bwd_kernel<64>, dim3((int)blocks),
+                                        dim3(256), 0, ST(stream), b));
   }
   KSA_CHECK_CUDA(cudaGetLastError());
   return 0;
@@ -939,8 +947,8 @@ KSA_API int ksa_swiglu_fwd(const void* gu, void* out, long long rows, int F, voi
   KSA_REQUIRE(F % 8 == 0, "swiglu: F=%d must be a multiple of 8", F);
   const long long n = rows * (F / 8);
   if (n == 0) return 0;
-  KSA_CHECK_CUDA(launch_kernel(dependent_launch_enabled(), swiglu_fwd_kernel, dim3((unsigned)((n + 255) / 256)), dim3(256),
-                              0, ST(stream), (const bf16*)gu, (bf16*)out, rows, F));
+  KSA_CHECK_CUDA(launch_stream_kernel(6LL * rows * F, swiglu_fwd_kernel, dim3((unsigned)((n + 255) / 256)), dim3(256), 0,
+                                      ST(stream), (const bf16*)gu, (bf16*)out, rows, F));
   return 0;
 }
 KSA_API int ksa_swiglu_bwd(const void* gu, const void* dout, void* dgu, long long rows, int F, void* stream) {
@@ -948,9 +956,8 @@ KSA_API int ksa_swiglu_bwd(const void* gu, const void* dout, void* dgu, long lon
   KSA_REQUIRE(F % 8 == 0, "swiglu: F=%d must be a multiple of 8", F);
   const long long n = rows * (F / 8);
   if (n == 0) return 0;
-  swiglu_bwd_kernel<<<(unsigned)((n + 255) / 256), 256, 0, ST(stream)>>>((const bf16*)gu, (const bf16*)dout, (bf16*)dgu,
-                                                                        rows, F);
-  KSA_CHECK_CUDA(cudaGetLastError());
+  KSA_CHECK_CUDA(launch_stream_kernel(10LL * rows * F, swiglu_bwd_kernel, dim3((unsigned)((n + 255) / 256)), dim3(256), 0,
+                                      ST(stream), (const bf16*)gu, (const bf16*)dout, (bf16*)dgu, rows, F));
   return 0;
 }
 
@@ -960,9 +967,8 @@ KSA_API int ksa_embedding_fwd(const void* ids, const void* table, void* out, lon
   KSA_REQUIRE(D % 8 == 0, "embedding: D=%d must be a multiple of 8", D);
   const long long n = rows * (D / 8);
   if (n == 0) return 0;
-  KSA_CHECK_CUDA(launch_kernel(dependent_launch_enabled(), embedding_fwd_kernel, dim3((unsigned)((n + 255) / 256)),
-                              dim3(256), 0, ST(stream), (const long long*)ids, (const bf16*)table, (bf16*)out, rows, D,
-                              vocab));
+  KSA_CHECK_CUDA(launch_stream_kernel(4LL * rows * D, embedding_fwd_kernel, dim3((unsigned)((n + 255) / 256)), dim3(256), 0,
+                                      ST(stream), (const long long*)ids, (const bf16*)table, (bf16*)out, rows, D, vocab));
   return 0;
 }
 KSA_API int ksa_embedding_bwd(const void* ids, const void* dout, void* dtable_f32, long long rows, int D,
@@ -971,17 +977,17 @@ KSA_API int ksa_embedding_bwd(const void* ids, const void* dout, void* dtable_f3
   KSA_REQUIRE(D % 8 == 0, "embedding: D=%d must be a multiple of 8", D);
   const long long n = rows * (D / 8);
   if (n == 0) return 0;
-  embedding_bwd_kernel<<<(unsigned)((n + 255) / 256), 256, 0, ST(stream)>>>((const long long*)ids, (const bf16*)dout,
-                                                                           (float*)dtable_f32, rows, D, vocab);
-  KSA_CHECK_CUDA(cudaGetLastError());
+  KSA_CHECK_CUDA(launch_stream_kernel(6LL * rows * D, embedding_bwd_kernel, dim3((unsigned)((n + 255) / 256)), dim3(256), 0,
+                                      ST(stream), (const long long*)ids, (const bf16*)dout, (float*)dtable_f32, rows, D,
+                                      vocab));
   return 0;
 }
 
 KSA_API int ksa_count_valid(const void* labels, long long n, int ignore_index, float extra_scale, void* out2,
                             void* stream) {
   KSA_ENTER(labels);
-  count_valid_kernel<<<1, 1024, 0, ST(stream)>>>((const long long*)labels, n, ignore_index, extra_scale, (float*)out2);
-  KSA_CHECK_CUDA(cudaGetLastError());
+  KSA_CHECK_CUDA(launch_kernel(count_valid_kernel, dim3(1), dim3(1024), 0, ST(stream), (const long long*)labels, n,
+                               ignore_index, extra_scale, (float*)out2));
   return 0;
 }
 
@@ -990,10 +996,9 @@ KSA_API int ksa_cross_entropy(void* logits, const void* labels, void* row_loss, 
   KSA_ENTER(logits);
   KSA_REQUIRE(V % 8 == 0 && ld % 8 == 0, "cross_entropy: V=%d and ld=%lld must be multiples of 8", V, ld);
   if (rows == 0) return 0;
-  cross_entropy_kernel<<<(unsigned)rows, kCeThreads, 0, ST(stream)>>>((bf16*)logits, (const long long*)labels,
-                                                                     (float*)row_loss, (const float*)grad_scale, V, ld,
-                                                                     ignore_index, write_grad);
-  KSA_CHECK_CUDA(cudaGetLastError());
+  KSA_CHECK_CUDA(launch_stream_kernel(6LL * rows * V, cross_entropy_kernel, dim3((unsigned)rows), dim3(kCeThreads), 0,
+                                      ST(stream), (bf16*)logits, (const long long*)labels, (float*)row_loss,
+                                      (const float*)grad_scale, V, ld, ignore_index, write_grad));
   return 0;
 }
 
@@ -1005,10 +1010,9 @@ KSA_API int ksa_adamw(void* master, const void* grad, void* m, void* v, void* ou
   if (n == 0) return 0;
   long long blocks = (n / 4 + 255) / 256;
   if (blocks > 148 * 16) blocks = 148 * 16;
-  adamw_kernel<<<(unsigned)blocks, 256, 0, ST(stream)>>>((float*)master, (const float*)grad, (float*)m, (float*)v,
-                                                        (bf16*)out_bf16, n, (const float*)hyper, beta1, beta2, eps,
-                                                        weight_decay, clip_value, (float*)sumsq);
-  KSA_CHECK_CUDA(cudaGetLastError());
+  KSA_CHECK_CUDA(launch_stream_kernel(30LL * n, adamw_kernel, dim3((unsigned)blocks), dim3(256), 0, ST(stream),
+                                      (float*)master, (const float*)grad, (float*)m, (float*)v, (bf16*)out_bf16, n,
+                                      (const float*)hyper, beta1, beta2, eps, weight_decay, clip_value, (float*)sumsq));
   return 0;
 }
 
@@ -1018,7 +1022,7 @@ KSA_API int ksa_cast_f32_bf16(const void* src, void* dst, long long n, void* str
   if (n == 0) return 0;
   long long blocks = (n / 4 + 255) / 256;
   if (blocks > 148 * 16) blocks = 148 * 16;
-  cast_f32_bf16_kernel<<<(unsigned)blocks, 256, 0, ST(stream)>>>((const float*)src, (bf16*)dst, n);
-  KSA_CHECK_CUDA(cudaGetLastError());
+  KSA_CHECK_CUDA(launch_stream_kernel(6LL * n, cast_f32_bf16_kernel, dim3((unsigned)blocks), dim3(256), 0, ST(stream),
+                                      (const float*)src, (bf16*)dst, n));
   return 0;
 }

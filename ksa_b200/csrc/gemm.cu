@@ -89,6 +89,7 @@ gemm_bf16_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant_
   __syncthreads();
   tc_fence_after();
   const uint32_t tmem_base = *tmem_slot;
+  grid_dependency_enter();
 
   auto tile_coords = [&](int tile, int& mb, int& nb) {
     const int per_group = kGroupM * tiles_n;
@@ -280,8 +281,7 @@ static int launch_gemm(const void* a, const void* b, const GemmEpilogue& ep, int
   if (tiles < ctas) ctas = tiles;
   int* status = status_word();
   KSA_REQUIRE(status != nullptr, "could not allocate the status word");
-  kern<<<ctas, kGemmThreads, S::kTotal, stream>>>(tmA, tmB, ep, M, N, K, status);
-  KSA_CHECK_CUDA(cudaGetLastError());
+  KSA_CHECK_CUDA(launch_kernel(kern, dim3(ctas), dim3(kGemmThreads), S::kTotal, stream, tmA, tmB, ep, M, N, K, status));
   return kErrNone;
 }
 

@@ -168,6 +168,7 @@ gemm2_bf16_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant
   cluster_sync_all();          // both CTAs' barriers are initialised before any remote arrival
   tc_fence_after();
   const uint32_t tmem_base = *tmem_slot;
+  grid_dependency_enter();     // (returns at once in the ordinary launches of the communication forms)
 
   auto tile_coords = [&](int tile, int& mb, int& nb) {
     const int per_group = k2GroupM * tiles_n;
@@ -481,8 +482,13 @@ static int launch_gemm2(const void* a, const void* b, const Gemm2Epilogue& ep, i
   if (tiles < pairs) pairs = tiles;
   int* status = status_word();
   KSA_REQUIRE(status != nullptr, "could not allocate the status word");
-  kern<<<2 * pairs, k2Threads, k2SmemTotal, stream>>>(tmA, tmB, ep, M, N, K, status, comm, smaps);
-  KSA_CHECK_CUDA(cudaGetLastError());
+  if (comm.active || ep.c_world > 1) {
+    kern<<<2 * pairs, k2Threads, k2SmemTotal, stream>>>(tmA, tmB, ep, M, N, K, status, comm, smaps);
+    KSA_CHECK_CUDA(cudaGetLastError());
+    return 0;
+  }
+  KSA_CHECK_CUDA(launch_kernel(kern, dim3(2 * pairs), dim3(k2Threads), (size_t)k2SmemTotal, stream, tmA, tmB, ep, M, N, K, status, comm,
+                              smaps));
   return 0;
 }
 

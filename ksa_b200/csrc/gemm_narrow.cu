@@ -86,6 +86,7 @@ gemm_narrow_kernel(const __grid_constant__ CUtensorMap tmW, const __grid_constan
   __syncthreads();
   tc_fence_after();
   const uint32_t tmem_base = tmem_slot;
+  grid_dependency_enter();
 
   if (warp == 0) {
     if (lane == 0) {
@@ -305,13 +306,15 @@ static int launch_narrow(const void* x, const void* w, NarrowArgs p, long long l
   cfg.blockDim = dim3(kNwThreads);
   cfg.dynamicSmemBytes = smem;
   cfg.stream = st;
-  cudaLaunchAttribute at[1];
+  cudaLaunchAttribute at[2];
   at[0].id = cudaLaunchAttributeClusterDimension;
   at[0].val.clusterDim.x = p.split;
   at[0].val.clusterDim.y = 1;
   at[0].val.clusterDim.z = 1;
+  at[1].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+  at[1].val.programmaticStreamSerializationAllowed = 1;
   cfg.attrs = at;
-  cfg.numAttrs = 1;
+  cfg.numAttrs = 2;
   KSA_CHECK_CUDA(cudaLaunchKernelEx(&cfg, kern, tmW, tmX, p, status));
   return 0;
 }

@@ -56,6 +56,7 @@ struct StreamArgs {
   int ragged;            // K is no multiple of 64: one load per box, which fills the columns past K with zeros
   int w_rows, x_rows;    // rows of a box in shared memory (weights, activations): those loaded, for `ragged` in whole swizzle atoms
   int stages, stage_bytes;
+  int early;             // dependent launches are on: the weights are read before the previous kernel has ended
   GemvNorm nrm;
 };
 
@@ -143,7 +144,8 @@ stream_gemm_kernel(const __grid_constant__ CUtensorMap tmB, const __grid_constan
                     p.ragged ? 0 : x.kb, &full[x.stage]);
       next(x);
     };
-    // weights do not depend on the previous kernel; the activations do
+    // in a decode step weights do not depend on the previous kernel; the activations do
+    if (!p.early) grid_dependency_wait();
     const int ahead = min(p.stages, n_items);
     for (int it = 0; it < ahead; ++it) load_weights();
     grid_dependency_wait();
@@ -381,7 +383,7 @@ static int launch_stream(StreamArgs p, const void* b, long long ldb, cudaStream_
     KSA_CHECK_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, kStSmemMost));
     attr = true;
   }
-  KSA_CHECK_CUDA(launch_kernel(dependent_launch_enabled(), kern, dim3(grid), dim3(kStThreads + 32), (size_t)smem, st, tmB, tmA,
+  KSA_CHECK_CUDA(launch_kernel(kern, dim3(grid), dim3(kStThreads + 32), (size_t)smem, st, tmB, tmA,
                               p, status));
   return 0;
 }
@@ -405,7 +407,7 @@ __device__ __forceinline__ uint4 ld_stream_16(const void* p) {
 template <int MT, int R, bool kGlu>
 __global__ void __launch_bounds__(kGemvThreads)
 gemv_kernel(const bf16* __restrict__ A, const bf16* __restrict__ B, bf16* __restrict__ C, int M, int N, int K,
-            long long lda, long long ldb, long long ldc) {
+            long long lda, long long ldb, long long ldc, int early) {
   extern __shared__ __align__(16) uint8_t gemv_smem[];
   bf16* sA = reinterpret_cast<bf16*>(gemv_smem);           // [MT][kGemvKTile]
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
@@ -436,8 +438,9 @@ gemv_kernel(const bf16* __restrict__ A, const bf16* __restrict__ B, bf16* __rest
         if (c < kt && row_of[r] >= 0) w[u][r] = ld_stream_16(B + row_of[r] * ldb + k0 + c);
       }
   };
-  // weights are never written by an earlier kernel of the stream: ask for the first chunks, then wait for the
+  // in a decode step weights are not written by an earlier kernel of the stream: ask for the first chunks, then wait for the
   // kernel that produces the activations
+  if (!early) grid_dependency_wait();
   load_w(0, min(kGemvKTile, K), lane * 8);
   grid_dependency_wait();
   grid_dependency_launch();
@@ -508,9 +511,9 @@ static int launch_gemv(const void* a, const void* b, void* c, int M, int N, int 
   const int n_out = kGlu ? N / 2 : N;
   const size_t smem = (size_t)MT * kGemvKTile * sizeof(bf16);
   auto kern = gemv_kernel<MT, R, kGlu>;
-  KSA_CHECK_CUDA(launch_kernel(dependent_launch_enabled(), kern, dim3((n_out + per_cta - 1) / per_cta),
+  KSA_CHECK_CUDA(launch_kernel(kern, dim3((n_out + per_cta - 1) / per_cta),
                               dim3(kGemvThreads), smem, st, (const bf16*)a, (const bf16*)b, (bf16*)c, M, N, K, lda, ldb,
-                              ldc));
+                              ldc, (int)dependent_launch_enabled()));
   return 0;
 }
 
@@ -524,6 +527,7 @@ static int gemv_dispatch(const void* a, const void* b, void* c, int M, int N, in
   p.A = (const bf16*)a; p.C = (bf16*)c;
   p.lda = lda; p.ldc = ldc; p.M = M; p.N = N; p.K = K;
   p.nrm = nrm;
+  p.early = dependent_launch_enabled();
   if (nrm.w != nullptr) return launch_stream<1, kGlu, true>(p, b, ldb, st);
   // In a chain of dependent launches the ring is filled while the previous kernel runs (one row x 2560 x 9728 10.4 against 11.9 us, x
   // 4096 x 2048 4.4 against 5.4, x 2560 x 4096 6.2 both); the output head is long enough not to need that.
