@@ -529,8 +529,8 @@ attn_bwd_fused_cp_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_c
 // 0, so that P = 0 there) and zeroes the row of the fp32 dQ buffer.  Bound by the memory (134 MB at 8192 x
 // 16 heads: 35.3 us with a warp per row and 8-byte loads that walked down one head's column, 23.4 us so).
 __global__ void __launch_bounds__(256)
-attn_bwd_prep_kernel(const bf16* __restrict__ o, const bf16* __restrict__ d_o, long long o_rs, long long o_bs,
-                     const float* __restrict__ lse, float* __restrict__ stats, float* __restrict__ dq32, int B, int Hq,
+attn_bwd_prep_kernel(const bf16* o, const bf16* d_o, long long o_rs, long long o_bs,
+                     const float* lse, float* stats, float* dq32, int B, int Hq,
                      int Lq, int lq_pad) {
   grid_dependency_enter();
   const long long item = ((long long)blockIdx.x * blockDim.x + threadIdx.x) >> 4;
@@ -571,7 +571,7 @@ attn_bwd_prep_kernel(const bf16* __restrict__ o, const bf16* __restrict__ d_o, l
 }
 
 // Conversion: dq = bf16(dq32 * scale).  One thread per 8 elements.
-__global__ void attn_bwd_dq_convert_kernel(const float* __restrict__ dq32, bf16* __restrict__ dq, long long dq_rs,
+__global__ void attn_bwd_dq_convert_kernel(const float* dq32, bf16* dq, long long dq_rs,
                                            long long dq_bs, int B, int Lq, int Hq, float scale) {
   grid_dependency_enter();
   const long long idx = (long long)blockIdx.x * blockDim.x + threadIdx.x;   // over B * Lq * Hq * 16

@@ -426,8 +426,8 @@ __global__ void __launch_bounds__(128) decode_combine_kernel(DecodeArgs a) {
 
 // cache[b, h, slot[b, t], :] = src[b, t, h, :] for slot >= 0 (K and V together)
 __global__ void __launch_bounds__(256)
-kv_cache_append_kernel(const bf16* __restrict__ k_new, const bf16* __restrict__ v_new, bf16* __restrict__ k_cache,
-                       bf16* __restrict__ v_cache, const int* __restrict__ slots, int B, int T, int H, int D, int cap,
+kv_cache_append_kernel(const bf16* k_new, const bf16* v_new, bf16* k_cache,
+                       bf16* v_cache, const int* slots, int B, int T, int H, int D, int cap,
                        long long src_row_stride, long long src_batch_stride) {
   grid_dependency_launch();   // a dependent-launched successor may start (the skinny GEMM: its weight loads)
   grid_dependency_wait();     // launched dependently itself: the previous kernel's results are complete from here on
@@ -448,8 +448,8 @@ kv_cache_append_kernel(const bf16* __restrict__ k_new, const bf16* __restrict__ 
 
 // cache[b, h, dst[b] + r, :] = cache[b, h, src[b] + r, :] for r < rows, for sequences with enable[b] != 0
 __global__ void __launch_bounds__(256)
-kv_cache_move_kernel(bf16* __restrict__ k_cache, bf16* __restrict__ v_cache, const int* __restrict__ src,
-                     const int* __restrict__ dst, const int* __restrict__ enable, int B, int H, int D, int cap,
+kv_cache_move_kernel(bf16* k_cache, bf16* v_cache, const int* src,
+                     const int* dst, const int* enable, int B, int H, int D, int cap,
                      int rows) {
   grid_dependency_launch();   // a dependent-launched successor may start (the skinny GEMM: its weight loads)
   grid_dependency_wait();     // launched dependently itself: the previous kernel's results are complete from here on

@@ -18,8 +18,8 @@ constexpr int kNormThreads = 256;
 constexpr int kNormMaxVec = 4;  // D up to 8192
 
 __global__ void __launch_bounds__(kNormThreads)
-rmsnorm_fwd_kernel(const bf16* __restrict__ x, const bf16* __restrict__ delta, const bf16* __restrict__ w,
-                   bf16* __restrict__ res_out, bf16* __restrict__ y, float* __restrict__ rstd_out, int rows, int D,
+rmsnorm_fwd_kernel(const bf16* x, const bf16* delta, const bf16* w,
+                   bf16* res_out, bf16* y, float* rstd_out, int rows, int D,
                    float eps, int delta_rows) {
   grid_dependency_enter();
   __shared__ float red[32];
@@ -71,9 +71,9 @@ rmsnorm_fwd_kernel(const bf16* __restrict__ x, const bf16* __restrict__ delta, c
 // norms of a layer: 76.8 -> 51.0 us; three CTAs per SM spill and take 79.5).
 template <int NVEC, int R, int MINB>
 __global__ void __launch_bounds__(kNormThreads, MINB)
-rmsnorm_bwd_kernel(const bf16* __restrict__ dy, const bf16* __restrict__ x, const bf16* __restrict__ w,
-                   const float* __restrict__ rstd_in, const bf16* __restrict__ dres, bf16* __restrict__ dx,
-                   float* __restrict__ dw_partial, int rows, int D) {
+rmsnorm_bwd_kernel(const bf16* dy, const bf16* x, const bf16* w,
+                   const float* rstd_in, const bf16* dres, bf16* dx,
+                   float* dw_partial, int rows, int D) {
   grid_dependency_enter();
   __shared__ float red[R][8];
   BF8 wv[NVEC];
@@ -179,7 +179,7 @@ rmsnorm_bwd_kernel(const bf16* __restrict__ dy, const bf16* __restrict__ x, cons
 
 // dw[c] (+)= sum over partial rows.  Block = 32 columns x 8 row groups.
 __global__ void __launch_bounds__(256)
-colsum_partials_kernel(const float* __restrict__ partial, float* __restrict__ dw, int nparts, int D, int accumulate) {
+colsum_partials_kernel(const float* partial, float* dw, int nparts, int D, int accumulate) {
   grid_dependency_enter();
   __shared__ float red[8][33];
   const int tx = threadIdx.x & 31, ty = threadIdx.x >> 5;
@@ -616,7 +616,7 @@ __global__ void __launch_bounds__(256) qknorm_rope_bwd128_kernel(QkRopeBwdArgs b
 // ------------------------------------------------------------------------------ SwiGLU
 // gate_up is [rows, 2F] = [gate | up]; out is [rows, F].
 __global__ void __launch_bounds__(256)
-swiglu_fwd_kernel(const bf16* __restrict__ gu, bf16* __restrict__ out, long long rows, int F) {
+swiglu_fwd_kernel(const bf16* gu, bf16* out, long long rows, int F) {
   grid_dependency_enter();
   const long long vec = (long long)blockIdx.x * blockDim.x + threadIdx.x;
   const int per_row = F / 8;
@@ -631,7 +631,7 @@ swiglu_fwd_kernel(const bf16* __restrict__ gu, bf16* __restrict__ out, long long
   store8(out + row * F + c, o);
 }
 __global__ void __launch_bounds__(256)
-swiglu_bwd_kernel(const bf16* __restrict__ gu, const bf16* __restrict__ dout, bf16* __restrict__ dgu, long long rows,
+swiglu_bwd_kernel(const bf16* gu, const bf16* dout, bf16* dgu, long long rows,
                   int F) {
   grid_dependency_enter();
   const long long vec = (long long)blockIdx.x * blockDim.x + threadIdx.x;
@@ -656,7 +656,7 @@ swiglu_bwd_kernel(const bf16* __restrict__ gu, const bf16* __restrict__ dout, bf
 
 // ------------------------------------------------------------------------------ embedding
 __global__ void __launch_bounds__(256)
-embedding_fwd_kernel(const long long* __restrict__ ids, const bf16* __restrict__ table, bf16* __restrict__ out,
+embedding_fwd_kernel(const long long* ids, const bf16* table, bf16* out,
                      long long rows, int D, long long vocab) {
   grid_dependency_enter();
   const long long vec = (long long)blockIdx.x * blockDim.x + threadIdx.x;
@@ -669,7 +669,7 @@ embedding_fwd_kernel(const long long* __restrict__ ids, const bf16* __restrict__
   *reinterpret_cast<BF8*>(out + row * D + c) = *reinterpret_cast<const BF8*>(table + id * D + c);
 }
 __global__ void __launch_bounds__(256)
-embedding_bwd_kernel(const long long* __restrict__ ids, const bf16* __restrict__ dout, float* __restrict__ dtable,
+embedding_bwd_kernel(const long long* ids, const bf16* dout, float* dtable,
                      long long rows, int D, long long vocab) {
   grid_dependency_enter();
   const long long vec = (long long)blockIdx.x * blockDim.x + threadIdx.x;
@@ -691,8 +691,8 @@ embedding_bwd_kernel(const long long* __restrict__ ids, const bf16* __restrict__
 // logits into d(loss)/d(logits) * (*grad_scale) in place.
 constexpr int kCeThreads = 512;
 __global__ void __launch_bounds__(kCeThreads)
-cross_entropy_kernel(bf16* __restrict__ logits, const long long* __restrict__ labels, float* __restrict__ row_loss,
-                     const float* __restrict__ grad_scale, int V, long long ld, int ignore_index, int write_grad) {
+cross_entropy_kernel(bf16* logits, const long long* labels, float* row_loss,
+                     const float* grad_scale, int V, long long ld, int ignore_index, int write_grad) {
   grid_dependency_enter();
   __shared__ float red[32];
   const long long row = blockIdx.x;
@@ -744,8 +744,8 @@ cross_entropy_kernel(bf16* __restrict__ logits, const long long* __restrict__ la
 }
 
 // n_valid and 1/n_valid (times an extra scale) on the device: no host sync in the step.
-__global__ void count_valid_kernel(const long long* __restrict__ labels, long long n, int ignore_index, float extra_scale,
-                                   float* __restrict__ out /* [0]=count, [1]=extra/count */) {
+__global__ void count_valid_kernel(const long long* labels, long long n, int ignore_index, float extra_scale,
+                                   float* out /* [0]=count, [1]=extra/count */) {
   grid_dependency_enter();
   __shared__ float red[32];
   float c = 0.f;
@@ -764,7 +764,6 @@ __global__ void __launch_bounds__(256)
 adamw_kernel(float* __restrict__ master, const float* __restrict__ grad, float* __restrict__ m, float* __restrict__ v,
              bf16* __restrict__ out_bf16, long long n, const float* __restrict__ hyper, float beta1, float beta2,
              float eps, float weight_decay, float clip_value, float* __restrict__ sumsq) {
-  grid_dependency_wait();     // and no early successor: this kernel writes weights
   __shared__ float red[32];
   const float lr = hyper[0], bc1 = hyper[1], bc2 = hyper[2], gscale = hyper[3];
   float sq = 0.f;
@@ -802,7 +801,6 @@ adamw_kernel(float* __restrict__ master, const float* __restrict__ grad, float* 
 
 // fp32 -> bf16 cast (flat), used to refresh compute weights from master weights.
 __global__ void __launch_bounds__(256) cast_f32_bf16_kernel(const float* __restrict__ src, bf16* __restrict__ dst, long long n) {
-  grid_dependency_wait();     // and no early successor: the copies may be weights
   const long long nvec = n / 4;
   for (long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x; i < nvec; i += (long long)gridDim.x * blockDim.x) {
     float4 a = reinterpret_cast<const float4*>(src)[i];
@@ -1010,7 +1008,7 @@ KSA_API int ksa_adamw(void* master, const void* grad, void* m, void* v, void* ou
   if (n == 0) return 0;
   long long blocks = (n / 4 + 255) / 256;
   if (blocks > 148 * 16) blocks = 148 * 16;
-  KSA_CHECK_CUDA(launch_stream_kernel(30LL * n, adamw_kernel, dim3((unsigned)blocks), dim3(256), 0, ST(stream),
+  KSA_CHECK_CUDA(launch_kernel_if(false, adamw_kernel, dim3((unsigned)blocks), dim3(256), 0, ST(stream),
                                       (float*)master, (const float*)grad, (float*)m, (float*)v, (bf16*)out_bf16, n,
                                       (const float*)hyper, beta1, beta2, eps, weight_decay, clip_value, (float*)sumsq));
   return 0;
@@ -1022,7 +1020,7 @@ KSA_API int ksa_cast_f32_bf16(const void* src, void* dst, long long n, void* str
   if (n == 0) return 0;
   long long blocks = (n / 4 + 255) / 256;
   if (blocks > 148 * 16) blocks = 148 * 16;
-  KSA_CHECK_CUDA(launch_stream_kernel(6LL * n, cast_f32_bf16_kernel, dim3((unsigned)blocks), dim3(256), 0, ST(stream),
+  KSA_CHECK_CUDA(launch_kernel_if(false, cast_f32_bf16_kernel, dim3((unsigned)blocks), dim3(256), 0, ST(stream),
                                       (const float*)src, (bf16*)dst, n));
   return 0;
 }

@@ -396,17 +396,17 @@ static int launch_stream(StreamArgs p, const void* b, long long ldb, cudaStream_
 constexpr int kGemvThreads = 256;
 constexpr int kGemvKTile = 2048;   // activation columns staged in shared memory per pass
 
-// 16-byte read-only load that does not pollute L1: every weight byte is used once per step
+// 16-byte load that does not pollute L1: every weight byte is used once per step
 __device__ __forceinline__ uint4 ld_stream_16(const void* p) {
   uint4 v;
-  asm volatile("ld.global.nc.L1::no_allocate.v4.u32 {%0, %1, %2, %3}, [%4];"
-               : "=r"(v.x), "=r"(v.y), "=r"(v.z), "=r"(v.w) : "l"(p));
+  asm volatile("ld.global.L1::no_allocate.v4.u32 {%0, %1, %2, %3}, [%4];"
+               : "=r"(v.x), "=r"(v.y), "=r"(v.z), "=r"(v.w) : "l"(p) : "memory");
   return v;
 }
 
 template <int MT, int R, bool kGlu>
 __global__ void __launch_bounds__(kGemvThreads)
-gemv_kernel(const bf16* __restrict__ A, const bf16* __restrict__ B, bf16* __restrict__ C, int M, int N, int K,
+gemv_kernel(const bf16* A, const bf16* B, bf16* C, int M, int N, int K,
             long long lda, long long ldb, long long ldc, int early) {
   extern __shared__ __align__(16) uint8_t gemv_smem[];
   bf16* sA = reinterpret_cast<bf16*>(gemv_smem);           // [MT][kGemvKTile]

@@ -57,7 +57,7 @@ int ensure_device(const void* device_ptr);
 
 // Dependent launches (programmatic stream serialization).  Most kernels are launched so that each may start while its predecessor on the
 // stream still runs, and wait for it on the device before they touch memory (grid_dependency_enter): the launch and the set-up of
-// one kernel lie under the end of the one before.  Kernels that write weights (the optimizer) do not let their successor start early.
+// one kernel lie under the end of the one before.  Kernels that write weights (the optimizer) are launched the ordinary way.
 // While the switch is on (ksa_set_dependent_launch; the inference engine's decode step), the weight-streaming products also
 // read their weights before they wait: no kernel of such a chain writes weights.
 bool dependent_launch_enabled();
