@@ -31,6 +31,8 @@ int ksa_gemm2_bf16(const void* a, const void* b, void* c, int M, int N, int K, l
                    int a_mn_major, int b_mn_major, int out_fp32, int accumulate, float alpha, void* stream);
 int ksa_gemm_narrow_bf16(const void* x, const void* w, void* c, int M, int N, int K, long long ldx, long long ldw, long long ldc,
                          int w_mn_major, int glu, int bt, int split, float alpha, void* stream);
+int ksa_gemm2_swiglu_bf16(const void* a, const void* b, void* gu, void* h, int M, int F, int K, long long lda, long long ldb,
+                          long long ld_gu, long long ld_h, void* stream);
 int ksa_gemv_bf16(const void* a, const void* b, void* c, int M, int N, int K, long long lda, long long ldb, long long ldc,
                   void* stream);
 int ksa_gemv_swiglu_bf16(const void* a, const void* b, void* c, int M, int N, int K, long long lda, long long ldb, long long ldc,
@@ -462,6 +464,32 @@ PyObject* py_linear_swiglu(PyObject*, PyObject* const* v, Py_ssize_t n) {
   END_HANDLE_TH_ERRORS
 }
 
+// gemm_swiglu(x, w13, pair_min) -> (silu(gate) * up, gate | up) from one launch of the CTA-pair kernel where `gemm` would
+// take it for the projection, else None
+PyObject* py_gemm_swiglu(PyObject*, PyObject* const* v, Py_ssize_t n) {
+  HANDLE_TH_ERRORS
+  Args a(v, n);
+  const Tensor *x = a.tensor(), *w = a.tensor();
+  const int pair_min = (int)a.integer();
+  if (!a.ok() || !rows2d(x) || !rows2d(w) || x->size(1) != w->size(1) || w->size(0) % 128 != 0 || !fits(x->size(0)) || !fits(w->size(0)) ||
+      !fits(x->size(1)) || x->stride(0) % 8 != 0 || w->stride(0) % 8 != 0 || x->size(0) <= 16)
+    return none();
+  const int M = (int)x->size(0), F = (int)(w->size(0) / 2), K = (int)x->size(1);
+  if (pair_min <= 0 || (long long)((M + 255) / 256) * ((F + 127) / 128) < pair_min ||
+      ksa_gemm_narrow_plan(M, 2 * F, K, 0, pair_min, (x->stride(0) % 64 != 0) + 2 * (w->stride(0) % 64 != 0)) != 0)
+    return none();
+  Tensor h, gu;
+  {
+    pybind11::gil_scoped_release no_gil;
+    h = a.empty({M, F});
+    gu = a.empty({M, 2LL * F});
+    LAUNCH(ksa_gemm2_swiglu_bf16, x->const_data_ptr(), w->const_data_ptr(), gu.mutable_data_ptr(), h.mutable_data_ptr(), M, F, K, x->stride(0),
+           w->stride(0), 2LL * F, F, a.stream());
+  }
+  return wrap(h, gu);
+  END_HANDLE_TH_ERRORS
+}
+
 // norm_linear(x, delta | None, norm_w, eps, w, glu) -> (x + delta, product of the normalised rows), at most four rows, no gradients
 PyObject* py_norm_linear(PyObject*, PyObject* const* v, Py_ssize_t n) {
   HANDLE_TH_ERRORS
@@ -593,7 +621,7 @@ PyObject* py_launches(PyObject*, PyObject* const*, Py_ssize_t) { return PyLong_F
 
 #define FN(name) {#name, reinterpret_cast<PyCFunction>(reinterpret_cast<void (*)()>(py_##name)), METH_FASTCALL, nullptr}
 PyMethodDef g_methods[] = {FN(gemm), FN(linear), FN(linear_dw), FN(dual_linear), FN(rms_norm), FN(rms_norm_bwd), FN(qk_norm_rope),
-                           FN(qk_norm_rope_bwd), FN(swiglu), FN(swiglu_bwd), FN(linear_swiglu), FN(norm_linear), FN(attention),
+                           FN(qk_norm_rope_bwd), FN(swiglu), FN(swiglu_bwd), FN(linear_swiglu), FN(gemm_swiglu), FN(norm_linear), FN(attention),
                            FN(attention_bwd), FN(launches), {nullptr, nullptr, 0, nullptr}};
 PyModuleDef g_module = {PyModuleDef_HEAD_INIT, "ksa_native", nullptr, -1, g_methods, nullptr, nullptr, nullptr, nullptr};
 

@@ -591,14 +591,19 @@ class _SwiGluFn(torch.autograd.Function):
     @staticmethod
     def backward(ctx, dout):
         (g2,) = ctx.saved_tensors
-        dgu = _native.swiglu_bwd(g2, dout)
-        if dgu is not None:
-            return dgu.view(ctx.shape)
-        d2 = dout.reshape(-1, dout.shape[-1])
-        d2 = d2 if d2.is_contiguous() else d2.contiguous()
-        dgu = torch.empty_like(g2)
-        _lib.call("ksa_swiglu_bwd", g2, d2, dgu, g2.shape[0], g2.shape[1] // 2)
-        return dgu.view(ctx.shape)
+        return _swiglu_backward(g2, dout).view(ctx.shape)
+
+
+def _swiglu_backward(gu, dout):
+    """The gradient of ``gu`` ``[rows, 2 F]`` in ``swiglu(gu)``."""
+    dgu = _native.swiglu_bwd(gu, dout)
+    if dgu is not None:
+        return dgu
+    d2 = dout.reshape(-1, dout.shape[-1])
+    d2 = d2 if d2.is_contiguous() else d2.contiguous()
+    dgu = torch.empty_like(gu)
+    _lib.call("ksa_swiglu_bwd", gu, d2, dgu, gu.shape[0], gu.shape[1] // 2)
+    return dgu
 
 
 def swiglu(gate_up: torch.Tensor) -> torch.Tensor:
@@ -610,11 +615,34 @@ def swiglu(gate_up: torch.Tensor) -> torch.Tensor:
     return _run(_SwiGluFn, gate_up)
 
 
+class _LinearSwiGluFn(torch.autograd.Function):
+    """``swiglu(x @ w13.T)`` of two-dimensional ``x``, differentiated; one launch where the projection goes to the CTA-pair kernel."""
+
+    @staticmethod
+    def forward(ctx, x, w13):
+        made = None if _lib.pair_gather_pending() else _native.gemm_swiglu(x, w13, GEMM_PAIR_MIN_TILES)
+        if made is not None:
+            out, gu = made
+        else:
+            x = x if x.stride(1) == 1 else x.contiguous()
+            gu = gemm(x, w13)
+            out = _SwiGluFn.forward(_NoGrad(), gu)
+        ctx.save_for_backward(x, w13, gu)
+        return out
+
+    @staticmethod
+    def backward(ctx, dout):
+        x, w13, gu = ctx.saved_tensors
+        dgu = _swiglu_backward(gu, dout)
+        dx = gemm(dgu, w13, b_mn_major=True) if ctx.needs_input_grad[0] else None
+        return dx, _linear_weight_grad(w13, dgu, x, 0, x.shape[0]) if ctx.needs_input_grad[1] else None
+
+
 def linear_swiglu(x: torch.Tensor, w13: torch.Tensor) -> torch.Tensor:
     """``swiglu(x @ w13.T)`` with ``w13 = [gate rows | up rows]``.  Without autograd on a GPU the projection of few rows (a
     decode step, a short prompt) applies the activation itself: ``ksa_gemv_swiglu_bf16`` for at most 16 rows, the gated form of
-    ``ksa_gemm_narrow_bf16`` where ``gemm`` would take that kernel.  Everything else is the projection followed by
-    ``swiglu``."""
+    ``ksa_gemm_narrow_bf16`` where ``gemm`` would take that kernel; in a differentiated call the CTA-pair kernel does so
+    and leaves the projection for the backward pass (``ksa_gemm2_swiglu_bf16``).  Everything else is the projection followed by ``swiglu``."""
     if _cuda(x) and not _observed() and not _lib.pair_gather_pending():
         out = _native.linear_swiglu(x, w13, GEMM_PAIR_MIN_TILES)
         if out is not None:
@@ -635,6 +663,10 @@ def linear_swiglu(x: torch.Tensor, w13: torch.Tensor) -> torch.Tensor:
                 _lib.call("ksa_gemm_narrow_bf16", x, w13, out, M, N, K, x.stride(0), w13.stride(0), out.stride(0), 0, 1,
                           *plan, 1.0)
             return out
+    if (_cuda(x) and x.dim() == 2 and w13.dim() == 2 and w13.shape[0] % 2 == 0 and torch.is_grad_enabled()
+            and (x.requires_grad or w13.requires_grad)):
+        _require_bf16(x, w13)
+        return _run(_LinearSwiGluFn, x, w13)
     return swiglu(linear(x, w13))
 
 

@@ -30,6 +30,7 @@ _SIGNATURES: Dict[str, Sequence] = {
     "ksa_gemm2_bf16": [P, P, P, I, I, I, L, L, L, I, I, I, I, F, P],
     "ksa_gemm2_gather_bf16": [P, P, P, I, I, I, L, L, L, I, I, F, P, I, I, L, P, P, ctypes.c_uint, P, I, L, P],
     "ksa_gemm2_scatter_bf16": [P, P, I, I, I, L, L, L, P, I, I, P],
+    "ksa_gemm2_swiglu_bf16": [P, P, P, P, I, I, I, L, L, L, L, P],
     "ksa_gemm_narrow_bf16": [P, P, P, I, I, I, L, L, L, I, I, I, I, F, P],
     "ksa_gemv_bf16": [P, P, P, I, I, I, L, L, L, P],
     "ksa_gemv_swiglu_bf16": [P, P, P, I, I, I, L, L, L, P],
