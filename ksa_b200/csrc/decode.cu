@@ -23,7 +23,7 @@ constexpr int kDecMaxQ = 16;       // queries (G * Tq) served per CTA
 constexpr int kDecMaxSplits = 64;  // splits of the key range when the last split merges them itself
 
 struct DecodeArgs {
-  const bf16* q;        // [B, Tq, Hq, D]
+  const bf16* q;        // [B, Tq] rows of Hq heads, `q_rs` elements apart
   const bf16* k_cache;  // [B, Hkv, cap, D]
   const bf16* v_cache;
   const int* start;     // [B, Tq]
@@ -33,6 +33,7 @@ struct DecodeArgs {
   bf16* out;            // [B, Tq, Hq, D]
   int B, Tq, Hq, Hkv, D, cap, splits, keys_per_split;
   float scale;
+  long long q_rs;
   int* counters;        // [B * Hkv] zeros, or null: with counters the last split of a KV group to finish merges the
                         // splits itself (and puts the counter back to zero); without, decode_combine_kernel does
 };
@@ -76,21 +77,35 @@ __device__ __forceinline__ void combine_if_last(const DecodeArgs& a, int b, int 
     for (int sp = 0; sp < S; ++sp) s_w[q][sp] *= inv;
   }
   __syncthreads();
-  for (int i = threadIdx.x; i < nq * D; i += blockDim.x) {
-    const int q = i / D, d = i - q * D;
-    const long long row = ((long long)b * a.Tq + q / G) * a.Hq + kvh * G + q % G;
-    const float* po = a.part_o + row * S * D + d;
-    float o = 0.f;
-    int sp = 0;
-    for (; sp + 8 <= S; sp += 8) {
-      float v[8];
+  // a thread takes one head dimension of four queries at once and asks for sixteen partial results before it adds any: the merge is a
+  // chain of loads from other SMs' writes, and with one query at a time it was half of a short slice's time
+  constexpr int QB = 4, SB = 4;
+  for (int d = threadIdx.x; d < D; d += blockDim.x) {
+    for (int q0 = 0; q0 < nq; q0 += QB) {
+      long long row[QB];
+      float o[QB];
 #pragma unroll
-      for (int u = 0; u < 8; ++u) v[u] = __ldcg(po + (long long)(sp + u) * D);
+      for (int u = 0; u < QB; ++u) {
+        const int q = min(q0 + u, nq - 1);
+        row[u] = ((long long)b * a.Tq + q / G) * a.Hq + kvh * G + q % G;
+        o[u] = 0.f;
+      }
+      for (int sp = 0; sp < S; sp += SB) {
+        float v[QB][SB];
 #pragma unroll
-      for (int u = 0; u < 8; ++u) o = fmaf(v[u], s_w[q][sp + u], o);
+        for (int u = 0; u < QB; ++u)
+#pragma unroll
+          for (int w = 0; w < SB; ++w) v[u][w] = sp + w < S ? __ldcg(a.part_o + (row[u] * S + sp + w) * D + d) : 0.f;
+#pragma unroll
+        for (int u = 0; u < QB; ++u)
+#pragma unroll
+          for (int w = 0; w < SB; ++w)
+            if (sp + w < S) o[u] = fmaf(v[u][w], s_w[min(q0 + u, nq - 1)][sp + w], o[u]);
+      }
+#pragma unroll
+      for (int u = 0; u < QB; ++u)
+        if (q0 + u < nq) a.out[row[u] * D + d] = __float2bfloat16(o[u]);
     }
-    for (; sp < S; ++sp) o = fmaf(__ldcg(po + (long long)sp * D), s_w[q][sp], o);
-    a.out[row * D + d] = __float2bfloat16(o);
   }
 }
 
@@ -111,7 +126,7 @@ __global__ void __launch_bounds__(kDecThreads) decode_attn_kernel(DecodeArgs a) 
   const int tid = threadIdx.x;
   for (int i = tid; i < nq * D; i += kDecThreads) {
     const int qi = i / D, d = i % D, t = qi / G, g = qi % G;
-    q_s[i] = __bfloat162float(a.q[(((long long)b * a.Tq + t) * a.Hq + kvh * G + g) * D + d]) * a.scale;
+    q_s[i] = __bfloat162float(a.q[((long long)b * a.Tq + t) * a.q_rs + (kvh * G + g) * D + d]) * a.scale;
   }
   if (tid < nq) {
     const int t = tid / G;
@@ -271,11 +286,11 @@ __global__ void __launch_bounds__(kDecThreads) decode_attn_mma_kernel(DecodeArgs
     qb[blk] = make_uint4(0, 0, 0, 0);
     if (g < nq) {
       const int tq = g / G, gg = g % G;
-      qa[blk] = *reinterpret_cast<const uint4*>(a.q + (((long long)b * a.Tq + tq) * a.Hq + kvh * G + gg) * D + blk * 32 + t * 8);
+      qa[blk] = *reinterpret_cast<const uint4*>(a.q + ((long long)b * a.Tq + tq) * a.q_rs + (kvh * G + gg) * D + blk * 32 + t * 8);
     }
     if (NQ > 8 && g + 8 < nq) {
       const int tq = (g + 8) / G, gg = (g + 8) % G;
-      qb[blk] = *reinterpret_cast<const uint4*>(a.q + (((long long)b * a.Tq + tq) * a.Hq + kvh * G + gg) * D + blk * 32 + t * 8);
+      qb[blk] = *reinterpret_cast<const uint4*>(a.q + ((long long)b * a.Tq + tq) * a.q_rs + (kvh * G + gg) * D + blk * 32 + t * 8);
     }
   }
   const bf16* kb = a.k_cache + ((long long)b * a.Hkv + kvh) * a.cap * D;
@@ -471,22 +486,23 @@ kv_cache_move_kernel(bf16* k_cache, bf16* v_cache, const int* src,
 
 using namespace ksa;
 
-// Scratch sizes the caller allocates: part_o [B*Tq*Hq*splits*D] fp32, part_ml [B*Tq*Hq*splits*2] fp32.
+// q_rs: elements from one (sequence, query) row of q to the next.  Scratch sizes the caller allocates: part_o [B*Tq*Hq*splits*D] fp32, part_ml [B*Tq*Hq*splits*2] fp32.
 // counters: B*Hkv int32 zeros that launches on one stream may share (each launch leaves them zero), or null for a
 // separate merge kernel.
 KSA_API int ksa_decode_attn(const void* q, const void* k_cache, const void* v_cache, const void* start, const void* len,
                             void* part_o, void* part_ml, void* out, int B, int Tq, int Hq, int Hkv, int D, int cap,
-                            int splits, int keys_per_split, float scale, void* counters, void* stream) {
+                            int splits, int keys_per_split, long long q_rs, float scale, void* counters, void* stream) {
   KSA_ENTER(q);
   KSA_REQUIRE(D == 128 || D == 64, "decode_attn: head_dim %d unsupported (64 or 128)", D);
   KSA_REQUIRE(Hq % Hkv == 0 && (Hq / Hkv) * Tq <= kDecMaxQ, "decode_attn: (Hq/Hkv) * Tq = %d exceeds %d queries per CTA",
               (Hq / Hkv) * Tq, kDecMaxQ);
+  KSA_REQUIRE(q_rs % 8 == 0 && (reinterpret_cast<uintptr_t>(q) & 15) == 0, "decode_attn: query rows must be 16-byte aligned");
   KSA_REQUIRE(splits >= 1 && keys_per_split >= 1, "decode_attn: bad split configuration");
   KSA_REQUIRE(counters == nullptr || splits <= kDecMaxSplits, "decode_attn: %d splits (at most %d with counters)", splits,
               kDecMaxSplits);
   if (B == 0) return 0;
   DecodeArgs a{(const bf16*)q, (const bf16*)k_cache, (const bf16*)v_cache, (const int*)start, (const int*)len,
-               (float*)part_o, (float*)part_ml, (bf16*)out, B, Tq, Hq, Hkv, D, cap, splits, keys_per_split, scale,
+               (float*)part_o, (float*)part_ml, (bf16*)out, B, Tq, Hq, Hkv, D, cap, splits, keys_per_split, scale, q_rs,
                (int*)counters};
   dim3 grid(splits, Hkv, B);
   cudaStream_t st = reinterpret_cast<cudaStream_t>(stream);
@@ -521,5 +537,51 @@ KSA_API int ksa_kv_cache_move(void* k_cache, void* v_cache, const void* src, con
   KSA_CHECK_CUDA(launch_kernel(kv_cache_move_kernel, dim3((unsigned)((n + 255) / 256)),
                               dim3(256), 0, reinterpret_cast<cudaStream_t>(stream), (bf16*)k_cache, (bf16*)v_cache,
                               (const int*)src, (const int*)dst, (const int*)enable, B, H, D, cap, rows));
+  return 0;
+}
+
+namespace ksa {
+// The slices of a step's text tokens on a ring-buffer cache (inference/cache.py), one thread per sequence: what PyTorch takes ten
+// kernels of a microsecond and a half for, none of which the next one may overlap.
+__global__ void decode_step_slices_kernel(const int* __restrict__ text_len, const int* __restrict__ cbl, const int* __restrict__ chunks,
+                                          int* __restrict__ out, int B, int n_sum, int chunk, int window, int text0, int sum0) {
+  grid_dependency_launch();
+  grid_dependency_wait();
+  const int b = blockIdx.x * blockDim.x + threadIdx.x;
+  if (b >= B) return;
+  const int done = chunks[b], slot = n_sum + chunk - 1 - cbl[b];
+  const int end = done >= window ? sum0 + (done - window) * n_sum : text0 + done * chunk;
+  out[b] = slot;
+  out[B + b] = end - slot;
+  out[2 * B + b] = text_len[b] + 1;
+}
+// The counters after an ordinary step.
+__global__ void decode_advance_kernel(int* __restrict__ text_len, int* __restrict__ cbl, int B) {
+  grid_dependency_launch();
+  grid_dependency_wait();
+  const int b = blockIdx.x * blockDim.x + threadIdx.x;
+  if (b >= B) return;
+  text_len[b] += 1;
+  if (cbl != nullptr) cbl[b] += 1;
+}
+}  // namespace ksa
+
+// out [3, B] int32: write slot (also the start of the slice), slice length, text length with the new token.
+KSA_API int ksa_decode_step_slices(const void* text_len, const void* cbl, const void* chunks, void* out, int B, int n_sum, int chunk,
+                                   int window, int text0, int sum0, void* stream) {
+  KSA_ENTER(text_len);
+  if (B == 0) return 0;
+  KSA_CHECK_CUDA(launch_kernel(decode_step_slices_kernel, dim3((B + 127) / 128), dim3(128), 0, reinterpret_cast<cudaStream_t>(stream),
+                               (const int*)text_len, (const int*)cbl, (const int*)chunks, (int*)out, B, n_sum, chunk, window, text0,
+                               sum0));
+  return 0;
+}
+
+// text_len += 1, and cbl += 1 unless null.
+KSA_API int ksa_decode_advance(void* text_len, void* cbl, int B, void* stream) {
+  KSA_ENTER(text_len);
+  if (B == 0) return 0;
+  KSA_CHECK_CUDA(launch_kernel(decode_advance_kernel, dim3((B + 127) / 128), dim3(128), 0, reinterpret_cast<cudaStream_t>(stream),
+                               (int*)text_len, (int*)cbl, B));
   return 0;
 }

@@ -40,13 +40,20 @@ def _decode_attention(q, k_cache, v_cache, start, length, scale, counters=None):
     keys_per_split = ((cap + splits - 1) // splits + 63) // 64 * 64
     part_o = torch.empty((B, Tq, Hq, splits, D), dtype=torch.float32, device=q.device)
     part_ml = torch.empty((B, Tq, Hq, splits, 2), dtype=torch.float32, device=q.device)
-    out = torch.empty_like(q)
+    out = torch.empty((B, Tq, Hq, D), dtype=q.dtype, device=q.device)
+    # rows of heads at any pitch are read as they are (the query columns of packed projection rows)
+    if q.stride(3) != 1 or q.stride(2) != D or (Tq > 1 and q.stride(0) != Tq * q.stride(1)):
+        q = q.contiguous()
+    q_rs = q.stride(0) if Tq == 1 else q.stride(1)
+    if B * Tq == 1 or q_rs % 8 != 0 or q.data_ptr() % 16 != 0:
+        q, q_rs = q.contiguous(), Hq * D
+        q = q if q.data_ptr() % 16 == 0 else q.clone()
     # the split that finishes last merges the splits itself and puts its counter back to zero, so launches that
     # follow one another on a stream can share ``counters`` (``[B * Hkv]`` int32 zeros; a fresh array when not given)
     if counters is None:
         counters = torch.zeros(B * Hkv, dtype=torch.int32, device=q.device)
-    _lib.call("ksa_decode_attn", q.contiguous(), k_cache, v_cache, start.contiguous(), length.contiguous(), part_o,
-              part_ml, out, B, Tq, Hq, Hkv, D, cap, splits, keys_per_split, float(scale), counters)
+    _lib.call("ksa_decode_attn", q, k_cache, v_cache, start.contiguous(), length.contiguous(), part_o,
+              part_ml, out, B, Tq, Hq, Hkv, D, cap, splits, keys_per_split, q_rs, float(scale), counters)
     return out
 
 
@@ -80,6 +87,17 @@ def _cache_move(k_cache, v_cache, src, dst, enable, rows):
     B, H, cap, D = k_cache.shape
     _lib.call("ksa_kv_cache_move", k_cache, v_cache, src.contiguous(), dst.contiguous(), enable.contiguous(), B, H, D,
               cap, rows)
+
+
+def _step_slices(spec: CacheSpec, st: CacheState):
+    """``text_step_slices`` (write slot, start, length of every sequence's text token), in one launch on a GPU."""
+    if not st.cbl.is_cuda:
+        return text_step_slices(spec, st)
+    B = st.cbl.numel()
+    out = torch.empty((3, B), dtype=torch.int32, device=st.cbl.device)
+    _lib.call("ksa_decode_step_slices", st.text_len, st.cbl, st.chunks, out, B, spec.n_sum, spec.chunk, spec.window, spec.text0,
+              spec.sum0)
+    return out[0], out[0], out[1]
 
 
 class KsaInferenceEngine:
@@ -117,6 +135,7 @@ class KsaInferenceEngine:
         self.host_len = [0] * batch
         self._boundary_dev = torch.zeros(batch, dtype=torch.int32, device=self.device)
         self._merge_counters = torch.zeros(batch * Hkv, dtype=torch.int32, device=self.device)
+        self._zero_starts = torch.zeros(batch, 1, dtype=torch.int32, device=self.device)     # of full-attention slices
 
     def reserve(self, max_len: int) -> None:
         """Grow every layer's cache so that sequences may reach ``max_len`` tokens; contents are kept.  The cache layout
@@ -247,10 +266,10 @@ class KsaInferenceEngine:
         if anyb:
             self._boundary_dev.copy_(torch.tensor(boundary_host, dtype=torch.int32), non_blocking=False)
         if not graphable:
-            logits = self._decode_impl(tokens, anyb)
+            logits = self._decode_impl(tokens, anyb).float()
         elif anyb not in self._graphs and self._plain_steps[anyb] == 0:
             self._plain_steps[anyb] += 1    # first-call set-up of the kernels happens outside a capture
-            logits = self._decode_impl(tokens, anyb)
+            logits = self._decode_impl(tokens, anyb).float()
         else:
             if self._graph_tokens is None:
                 self._graph_tokens = tokens.reshape(self.batch).clone()
@@ -263,16 +282,17 @@ class KsaInferenceEngine:
             graph, out = self._graphs[anyb]
             self._graph_tokens.copy_(tokens.reshape(self.batch))
             graph.replay()
-            logits = out.clone() if head_in_graph else self._head(out)
+            # another tensor: the graph's own output is used again
+            logits = (out if head_in_graph else self._logits(out)).to(torch.float32, copy=True)
         self.host_len = [l + 1 for l in self.host_len]
         return logits
 
-    def _head(self, hidden: torch.Tensor) -> torch.Tensor:
+    def _logits(self, hidden: torch.Tensor) -> torch.Tensor:
         model, tp = self.model, getattr(self.model, "tp", None)
         logits = ops.linear(hidden, model.lm_head_weight)
         if tp is not None and logits.shape[-1] != self.cfg.vocab_size:
             logits = tp.gather_logits(logits)
-        return logits.float()
+        return logits
 
     def _decode_impl(self, tokens: torch.Tensor, any_boundary: bool, with_head: bool = True) -> torch.Tensor:
         """Device work of one decode step (launches only; the host mirror of the lengths is advanced by the caller).
@@ -295,7 +315,7 @@ class KsaInferenceEngine:
         scale = Dh ** -0.5
         st = self.state
         dev = self.device
-        pos_t = st.text_len.clone()                              # position of the new text token
+        pos_t = st.text_len                                      # position of the new text token; advanced when the step is done
         x = ops.embedding(tokens.reshape(B), model.tok_embeddings.weight)      # [B, D]
         if any_boundary:
             boundary = self._boundary_dev
@@ -316,6 +336,7 @@ class KsaInferenceEngine:
             pos_all = pos_all.clone()
             pos_all[:B] = st.cbl
         delta = None
+        full_len = None     # slice lengths of the full-attention layers
         slices_of = {}      # layers with the same cache geometry share the step's slot / slice tensors
         # ordinary steps without tensor parallelism: residual add + norm live inside the projection that follows them
         fuse_norm = tp is None and not any_boundary and B <= 4
@@ -340,7 +361,7 @@ class KsaInferenceEngine:
                     qkv = ops.linear(h, a.wqkv.weight)
                 skey = (spec.chunk, spec.n_sum, spec.window, spec.max_chunks)
                 if skey not in slices_of:
-                    slot_t, start_t, len_t = text_step_slices(spec, st)
+                    slot_t, start_t, len_t = _step_slices(spec, st)
                     slices_of[skey] = (slot_t.view(B, 1).to(torch.int32).contiguous(),
                                        start_t.view(B, 1).to(torch.int32).contiguous(),
                                        len_t.view(B, 1).to(torch.int32).contiguous(), start_t, len_t)
@@ -384,25 +405,33 @@ class KsaInferenceEngine:
                                               cfg.rope_base, cfg.norm_eps, cfg.rope_impl == "llama", cache.k, cache.v,
                                               st.text_len)
                 q_t = qkv[:, :Hq * Dh].view(B, 1, Hq, Dh)
-                zeros = torch.zeros(B, 1, dtype=torch.int32, device=dev)
-                att = _decode_attention(q_t, cache.k, cache.v, zeros, (st.text_len + 1).view(B, 1).to(torch.int32),
-                                        scale, self._merge_counters).reshape(B, Hq * Dh)
+                if full_len is None:
+                    full_len = (st.text_len + 1).view(B, 1).to(torch.int32)
+                att = _decode_attention(q_t, cache.k, cache.v, self._zero_starts, full_len, scale,
+                                        self._merge_counters).reshape(B, Hq * Dh)
                 attn_out = _row_linear(tp, att, a.output_proj.weight)
                 if fuse_norm:
                     x, delta = layer.mlp.forward_after_norm(x, attn_out, layer.mlp_norm.scale, cfg.norm_eps)
                 else:
                     x, h2 = _add_norm(tp, x, attn_out, layer.mlp_norm.scale, cfg.norm_eps)
                     delta = layer.mlp(h2[:B], tp)
-        _, hN = _add_norm(tp, x[:B], delta[:B], model.norm.scale, cfg.norm_eps)
+        if fuse_norm and with_head:
+            out = ops.norm_linear(x, delta, model.norm.scale, cfg.norm_eps, model.lm_head_weight)[1]
+        else:
+            _, out = _add_norm(tp, x[:B], delta[:B], model.norm.scale, cfg.norm_eps)
+            out = self._logits(out) if with_head else out
         # advance the counters
-        st.text_len += 1
-        if S > 0:
-            if any_boundary:
-                st.chunks += boundary
-                st.cbl.copy_(torch.where(boundary > 0, torch.zeros_like(st.cbl), st.cbl + 1))
-            else:
+        if S > 0 and any_boundary:
+            st.text_len += 1
+            st.chunks += boundary
+            st.cbl.copy_(torch.where(boundary > 0, torch.zeros_like(st.cbl), st.cbl + 1))
+        elif st.text_len.is_cuda:
+            _lib.call("ksa_decode_advance", st.text_len, st.cbl if S > 0 else None, B)
+        else:
+            st.text_len += 1
+            if S > 0:
                 st.cbl += 1
-        return self._head(hN) if with_head else hN
+        return out
 
     @torch.no_grad()
     def generate(self, prompt: torch.Tensor, max_new_tokens: int, eos_id: Optional[int] = None,
