@@ -64,6 +64,71 @@ rmsnorm_fwd_kernel(const bf16* x, const bf16* delta, const bf16* w,
   }
 }
 
+// The same with a warp per row, for up to 2560 columns: a lane requests its NV vectors of both inputs before it uses any, and nothing
+// waits at a barrier, so an SM has some 100 KB in flight where a CTA per row (half of its threads without a vector at 1024 columns)
+// had less than half of that.  With residual and its write, CTA per row -> warp per row: 8256 x 1024 26.7 -> 14.4 us, 8256 x 2048
+// 32.8 -> 26.4, 33024 x 2560 165.6 -> 104.2 (103.4 at the copy bandwidth).
+template <int NV>
+__global__ void __launch_bounds__(128)
+rmsnorm_fwd_warp_kernel(const bf16* x, const bf16* delta, const bf16* w,
+                        bf16* res_out, bf16* y, float* rstd_out, int rows, int D, float eps,
+                        int delta_rows) {
+  grid_dependency_enter();
+  const int row = blockIdx.x * 4 + (threadIdx.x >> 5), lane = threadIdx.x & 31;
+  if (row >= rows) return;
+  const bool has_delta = delta != nullptr && row < delta_rows;
+  const long long base = (long long)row * D;
+  BF8 v[NV], d[NV];
+#pragma unroll
+  for (int i = 0; i < NV; ++i) {
+    const int c = (i * 32 + lane) * 8;
+    v[i] = d[i] = BF8{{0, 0, 0, 0}};
+    if (c < D) v[i] = *reinterpret_cast<const BF8*>(x + base + c);
+  }
+  if (has_delta) {
+#pragma unroll
+    for (int i = 0; i < NV; ++i) {
+      const int c = (i * 32 + lane) * 8;
+      if (c < D) d[i] = *reinterpret_cast<const BF8*>(delta + base + c);
+    }
+#pragma unroll
+    for (int i = 0; i < NV; ++i)
+#pragma unroll
+      for (int j = 0; j < 4; ++j) {
+        const float2 a = unpack_bf16x2(v[i].u[j]), b = unpack_bf16x2(d[i].u[j]);
+        v[i].u[j] = pack_bf16x2(a.x + b.x, a.y + b.y);       // the residual stream in bf16, so that norm and stream agree
+      }
+  }
+  float ss = 0.f;
+#pragma unroll
+  for (int i = 0; i < NV; ++i) {
+    const int c = (i * 32 + lane) * 8;
+    if (res_out && c < D) *reinterpret_cast<BF8*>(res_out + base + c) = v[i];
+#pragma unroll
+    for (int j = 0; j < 4; ++j) {
+      const float2 a = unpack_bf16x2(v[i].u[j]);
+      ss += a.x * a.x + a.y * a.y;
+    }
+  }
+  ss = warp_sum(ss);
+  const float rstd = rsqrtf(ss / (float)D + eps);
+  if (lane == 0 && rstd_out) rstd_out[row] = rstd;
+#pragma unroll
+  for (int i = 0; i < NV; ++i) {
+    const int c = (i * 32 + lane) * 8;
+    if (c < D) {
+      const BF8 wv = *reinterpret_cast<const BF8*>(w + c);
+      BF8 o;
+#pragma unroll
+      for (int j = 0; j < 4; ++j) {
+        const float2 a = unpack_bf16x2(v[i].u[j]), b = unpack_bf16x2(wv.u[j]);
+        o.u[j] = pack_bf16x2(a.x * rstd * b.x, a.y * rstd * b.y);
+      }
+      *reinterpret_cast<BF8*>(y + base + c) = o;
+    }
+  }
+}
+
 // dx = rstd * (dy*w - xhat * mean(dy*w*xhat)) (+ dres); per-CTA partial dw rows in `dw_partial`.
 // NVEC 16-byte vectors per thread cover D <= NVEC * 2048; R rows per iteration share one pair of barriers.  The bound is
 // the memory (three reads and one write of a row), so loads never pause for the reduction: the rows of the next iteration
@@ -820,6 +885,16 @@ KSA_API int ksa_rmsnorm_fwd(const void* x, const void* delta, const void* w, voi
   KSA_REQUIRE(D % 8 == 0 && D <= kNormThreads * 8 * kNormMaxVec, "rmsnorm: D=%d must be a multiple of 8 and <= %d", D,
               kNormThreads * 8 * kNormMaxVec);
   if (rows == 0) return 0;
+  // A warp per row from 1024 rows on, about 7 warps an SM: 1024 x 2560 10.1 -> 6.7 us, 1411 x 1024 8.0 -> 4.6.  256 and 512 rows take 5 to
+  // 9 us back to back in both forms, most of it the launch, and stay with the wider CTA.  The vectors of both inputs have to fit a
+  // lane's registers, 10 of each, so rows above 2560 columns keep the CTA as well.
+  if (rows >= 1024 && D <= 2560) {
+    auto kern = D <= 1024 ? rmsnorm_fwd_warp_kernel<4> : D <= 2048 ? rmsnorm_fwd_warp_kernel<8> : rmsnorm_fwd_warp_kernel<10>;
+    KSA_CHECK_CUDA(launch_stream_kernel(8LL * rows * D, kern, dim3((rows + 3) / 4), dim3(128), 0, ST(stream), (const bf16*)x,
+                                        (const bf16*)delta, (const bf16*)w, (bf16*)res_out, (bf16*)y, (float*)rstd, rows, D, eps,
+                                        delta_rows));
+    return 0;
+  }
   KSA_CHECK_CUDA(launch_stream_kernel(8LL * rows * D, rmsnorm_fwd_kernel, dim3(rows), dim3(kNormThreads), 0, ST(stream),
                                       (const bf16*)x, (const bf16*)delta, (const bf16*)w, (bf16*)res_out, (bf16*)y,
                                       (float*)rstd, rows, D, eps, delta_rows));
