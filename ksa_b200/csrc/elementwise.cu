@@ -751,63 +751,6 @@ embedding_bwd_kernel(const long long* ids, const bf16* dout, float* dtable,
   for (int j = 0; j < 8; ++j) atomicAdd(dst + j, g[j]);
 }
 
-// ------------------------------------------------------------------------------ cross entropy
-// One CTA per row of bf16 logits [rows, V].  Writes per-row loss (0 for ignored rows) and turns the
-// logits into d(loss)/d(logits) * (*grad_scale) in place.
-constexpr int kCeThreads = 512;
-__global__ void __launch_bounds__(kCeThreads)
-cross_entropy_kernel(bf16* logits, const long long* labels, float* row_loss,
-                     const float* grad_scale, int V, long long ld, int ignore_index, int write_grad) {
-  grid_dependency_enter();
-  __shared__ float red[32];
-  const long long row = blockIdx.x;
-  bf16* lg = logits + row * ld;
-  const long long label = labels[row];
-  const bool ignored = (label == ignore_index) || label < 0 || label >= V;
-  const int nvec = V / 8;
-  if (ignored) {
-    if (threadIdx.x == 0) row_loss[row] = 0.f;
-    if (write_grad) {
-      BF8 z{{0, 0, 0, 0}};
-      for (int i = threadIdx.x; i < nvec; i += kCeThreads) *reinterpret_cast<BF8*>(lg + i * 8) = z;
-    }
-    return;
-  }
-  float mx = -INFINITY;
-  for (int i = threadIdx.x; i < nvec; i += kCeThreads) {
-    float f[8];
-    load8(lg + i * 8, f);
-#pragma unroll
-    for (int j = 0; j < 8; ++j) mx = fmaxf(mx, f[j]);
-  }
-  mx = block_max<kCeThreads>(mx, red);
-  float sum = 0.f;
-  for (int i = threadIdx.x; i < nvec; i += kCeThreads) {
-    float f[8];
-    load8(lg + i * 8, f);
-#pragma unroll
-    for (int j = 0; j < 8; ++j) sum += __expf(f[j] - mx);
-  }
-  sum = block_sum<kCeThreads>(sum, red);
-  const float lse = mx + __logf(sum);
-  if (threadIdx.x == 0) row_loss[row] = lse - __bfloat162float(lg[label]);
-  if (!write_grad) return;
-  __syncthreads();
-  const float gs = *grad_scale;
-  const float inv = 1.f / sum;
-  for (int i = threadIdx.x; i < nvec; i += kCeThreads) {
-    float f[8];
-    load8(lg + i * 8, f);
-#pragma unroll
-    for (int j = 0; j < 8; ++j) {
-      float p = __expf(f[j] - mx) * inv;
-      if ((long long)i * 8 + j == label) p -= 1.f;
-      f[j] = p * gs;
-    }
-    store8(lg + i * 8, f);
-  }
-}
-
 // n_valid and 1/n_valid (times an extra scale) on the device: no host sync in the step.
 __global__ void count_valid_kernel(const long long* labels, long long n, int ignore_index, float extra_scale,
                                    float* out /* [0]=count, [1]=extra/count */) {
@@ -1061,17 +1004,6 @@ KSA_API int ksa_count_valid(const void* labels, long long n, int ignore_index, f
   KSA_ENTER(labels);
   KSA_CHECK_CUDA(launch_kernel(count_valid_kernel, dim3(1), dim3(1024), 0, ST(stream), (const long long*)labels, n,
                                ignore_index, extra_scale, (float*)out2));
-  return 0;
-}
-
-KSA_API int ksa_cross_entropy(void* logits, const void* labels, void* row_loss, const void* grad_scale, long long rows,
-                              int V, long long ld, int ignore_index, int write_grad, void* stream) {
-  KSA_ENTER(logits);
-  KSA_REQUIRE(V % 8 == 0 && ld % 8 == 0, "cross_entropy: V=%d and ld=%lld must be multiples of 8", V, ld);
-  if (rows == 0) return 0;
-  KSA_CHECK_CUDA(launch_stream_kernel(6LL * rows * V, cross_entropy_kernel, dim3((unsigned)rows), dim3(kCeThreads), 0,
-                                      ST(stream), (bf16*)logits, (const long long*)labels, (float*)row_loss,
-                                      (const float*)grad_scale, V, ld, ignore_index, write_grad));
   return 0;
 }
 
