@@ -267,6 +267,10 @@ static double tiled_time(int M, int N, int K, int pair_min_tiles) {
   return 5.0 + 0.38 * num_kb * (((M + 127) / 128 * tn + kNwSms - 1) / kNwSms);
 }
 
+static long long tiled_waves(int M, int N, int rows, int slots) {
+  return ((long long)((M + rows - 1) / rows) * ((N + 255) / 256) + slots - 1) / slots;
+}
+
 template <bool W_MN, bool kGlu>
 static int launch_narrow(const void* x, const void* w, NarrowArgs p, long long ldx, long long ldw, cudaStream_t st) {
   CUtensorMap tmX, tmW;
@@ -341,6 +345,18 @@ KSA_API int ksa_gemm_narrow_bf16(const void* x, const void* w, void* c, int M, i
   cudaStream_t st = reinterpret_cast<cudaStream_t>(stream);
   if (glu) return launch_narrow<false, true>(x, w, p, ldx, ldw, st);
   return w_mn_major ? launch_narrow<true, false>(x, w, p, ldx, ldw, st) : launch_narrow<false, false>(x, w, p, ldx, ldw, st);
+}
+
+// Whether the CTA pairs of ksa_gemm2_bf16 serve an M x N product (from `pair_min_tiles` 256 x 256 tiles on, 0: never) or the single CTAs of
+// ksa_gemm_bf16: a tile of 256 rows on a pair takes 0.75 to 0.95 of the time of two tiles of 128 rows, but rows that end
+// in the first half of a tile and a last wave of a few tiles can cost pairs a whole wave more.  Pairs unless they take half as many waves
+// again: 333 x 19456 x 2560 3 waves against 2, 44.0 us on pairs and 41.0 on single CTAs; 333 x 12288 x 2048 2 against 1, 28.7 and 21.9;
+// 1152 x 4096 x 2048 2 against 1, 26.0 and 18.0 (fp32 from transposed operands 29.1 and 22.5).  At 4 against 3 both are within 6 %
+// (513 x 19456 x 2560 59.3 and 57.5, fp32 at 1152 x 12288 x 2048 53.3 and 61.1), at 6 against 5 pairs are 5 to 15 % faster.
+KSA_API int ksa_gemm_on_pairs(int M, int N, int pair_min_tiles) {
+  using namespace ksa;
+  if (pair_min_tiles <= 0 || (long long)((M + 255) / 256) * ((N + 255) / 256) < pair_min_tiles) return 0;
+  return 2 * tiled_waves(M, N, 256, kNwSms / 2) < 3 * tiled_waves(M, N, 128, kNwSms);
 }
 
 // Whether this kernel is expected to beat the tiled ones (of which CTA pairs are taken from `pair_min_tiles` 256 x 256 tiles on, 0:

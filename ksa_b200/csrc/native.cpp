@@ -22,6 +22,7 @@
 
 extern "C" {
 const char* ksa_last_error();
+int ksa_gemm_on_pairs(int M, int N, int pair_min_tiles);
 int ksa_gemm_narrow_plan(int M, int N, int K, int glu, int pair_min_tiles, int ragged);
 int ksa_rmsnorm_bwd_parts(int rows);
 int ksa_attn_bwd_num_segments(int lq);
@@ -181,7 +182,7 @@ void gemm(const Product& p, int pair_min, void* st) {
       return;
     }
   }
-  if (pair_min > 0 && (p.M + 255) / 256 * ((p.N + 255) / 256) >= pair_min)
+  if (ksa_gemm_on_pairs(M, N, pair_min))
     LAUNCH(ksa_gemm2_bf16, p.a, p.b, p.c, M, N, K, p.lda, p.ldb, p.ldc, p.a_mn, p.b_mn, p.fp32, p.accumulate, 1.f, st);
   else
     LAUNCH(ksa_gemm_bf16, p.a, p.b, p.c, M, N, K, p.lda, p.ldb, p.ldc, p.a_mn, p.b_mn, p.fp32, p.accumulate, 1.f, 0, st);
@@ -464,8 +465,8 @@ PyObject* py_linear_swiglu(PyObject*, PyObject* const* v, Py_ssize_t n) {
   END_HANDLE_TH_ERRORS
 }
 
-// gemm_swiglu(x, w13, pair_min) -> (silu(gate) * up, gate | up) from one launch of the CTA-pair kernel where `gemm` would
-// take it for the projection, else None
+// gemm_swiglu(x, w13, pair_min) -> (silu(gate) * up, gate | up) from one launch of the CTA-pair kernel from `pair_min`
+// tiles on where the split-K kernel is no faster, else None
 PyObject* py_gemm_swiglu(PyObject*, PyObject* const* v, Py_ssize_t n) {
   HANDLE_TH_ERRORS
   Args a(v, n);

@@ -32,8 +32,9 @@ from ._lib import native as _native
 from .layout import SummaryLayout, get_layout
 
 UNBOUNDED_WINDOW = 1 << 30
-# GEMMs with at least this many 256 x 256 tiles run on CTA pairs (tcgen05 cta_group::2, csrc/gemm2.cu; 74 pairs per
-# GPU); below that the single-CTA kernel with 128-row tiles has more CTAs to spread.  0 disables the pair kernel.
+# GEMMs with at least this many 256 x 256 tiles may run on CTA pairs (tcgen05 cta_group::2, csrc/gemm2.cu; 74 pairs per
+# GPU); below that, and where they would take 1.5 times the waves of 128-row tiles on single CTAs (``ksa_gemm_on_pairs``
+# in csrc/gemm_narrow.cu), the single-CTA kernel has more CTAs to spread.  0 disables the pair kernel.
 GEMM_PAIR_MIN_TILES = int(__import__("os").environ.get("KSA_GEMM_PAIR_MIN_TILES", "32"))
 
 
@@ -139,8 +140,7 @@ def gemm(a: torch.Tensor, b: torch.Tensor, *, a_mn_major: bool = False, b_mn_maj
                       float(alpha))
             return out
     if pair is None:
-        pair = (GEMM_PAIR_MIN_TILES > 0 and sm_limit == 0
-                and ((M + 255) // 256) * ((N + 255) // 256) >= GEMM_PAIR_MIN_TILES)
+        pair = sm_limit == 0 and _lib.gemm_on_pairs(M, N, GEMM_PAIR_MIN_TILES)
     if pair:
         _lib.call("ksa_gemm2_bf16", a, b, out, M, N, K, a.stride(0), b.stride(0), out.stride(0),
                   int(a_mn_major), int(b_mn_major), int(out.dtype == torch.float32), int(accumulate), float(alpha))

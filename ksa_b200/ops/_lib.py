@@ -103,6 +103,8 @@ def load() -> ctypes.CDLL:
     lib.ksa_rmsnorm_bwd_parts.restype = I
     lib.ksa_attn_bwd_num_segments.argtypes = [I]
     lib.ksa_attn_bwd_num_segments.restype = I
+    lib.ksa_gemm_on_pairs.argtypes = [I] * 3
+    lib.ksa_gemm_on_pairs.restype = I
     lib.ksa_gemm_narrow_plan.argtypes = [I] * 6
     lib.ksa_gemm_narrow_plan.restype = I
     lib.ksa_set_dependent_launch.argtypes = [I]
@@ -283,6 +285,11 @@ def set_dependent_launch(on: bool) -> bool:
     while its predecessor on the stream still runs and waits for it on the device) on or off; returns the previous
     setting.  The inference engine switches it on around a decode step; training leaves it off."""
     return load().ksa_set_dependent_launch(1 if on else 0) != 0
+
+
+def gemm_on_pairs(M: int, N: int, pair_min_tiles: int) -> bool:
+    """Whether the CTA-pair kernel serves an M x N product, or the kernel of single CTAs."""
+    return load().ksa_gemm_on_pairs(M, N, pair_min_tiles) != 0
 
 
 @functools.lru_cache(maxsize=4096)
