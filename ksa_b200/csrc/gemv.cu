@@ -15,9 +15,9 @@
 // 16 x 6144 x 2560 15.1 -> 9.3, 16 x 151936 x 2560 208 -> 118; with the norm, 4 x 6144 x 2560 25.4 -> 10.8, 4 x 19456 x 2560 with
 // SwiGLU 41.6 -> 22.7.  Integer divisions by the number of stages in the producer's loop alone had cost 0.4 us a stage.
 //
-// A decode step is a chain of such kernels, each a few microseconds long, so the engine switches dependent launches
-// on (host.h): a CTA may then start beside the CTA of the previous kernel of the stream (both fit one SM), fill its whole ring with
-// weights, which no earlier kernel writes, and only then waits for the previous kernel (griddepcontrol.wait) before it
+// A decode step is a chain of such kernels, each a few microseconds long, so the engine switches early weights on for its
+// thread (host.h): a CTA that starts beside the CTA of the previous kernel of the stream (both fit one SM) then fills its whole ring
+// with weights, which no earlier kernel writes, and only after that waits for the previous kernel (griddepcontrol.wait) and
 // reads the activations.  The gate/up projection can apply SwiGLU itself (kGlu): a group then holds matching gate and up
 // rows and the CTA writes silu(gate) * up.  Every wait is bounded; no TMA load uses multicast.
 #include "common.cuh"
@@ -56,7 +56,7 @@ struct StreamArgs {
   int ragged;            // K is no multiple of 64: one load per box, which fills the columns past K with zeros
   int w_rows, x_rows;    // rows of a box in shared memory (weights, activations): those loaded, for `ragged` in whole swizzle atoms
   int stages, stage_bytes;
-  int early;             // dependent launches are on: the weights are read before the previous kernel has ended
+  int early;             // weights_early(): the weights are read before the previous kernel has ended
   GemvNorm nrm;
 };
 
@@ -513,7 +513,7 @@ static int launch_gemv(const void* a, const void* b, void* c, int M, int N, int 
   auto kern = gemv_kernel<MT, R, kGlu>;
   KSA_CHECK_CUDA(launch_kernel(kern, dim3((n_out + per_cta - 1) / per_cta),
                               dim3(kGemvThreads), smem, st, (const bf16*)a, (const bf16*)b, (bf16*)c, M, N, K, lda, ldb,
-                              ldc, (int)dependent_launch_enabled()));
+                              ldc, (int)weights_early()));
   return 0;
 }
 
@@ -527,11 +527,11 @@ static int gemv_dispatch(const void* a, const void* b, void* c, int M, int N, in
   p.A = (const bf16*)a; p.C = (bf16*)c;
   p.lda = lda; p.ldc = ldc; p.M = M; p.N = N; p.K = K;
   p.nrm = nrm;
-  p.early = dependent_launch_enabled();
+  p.early = weights_early();
   if (nrm.w != nullptr) return launch_stream<1, kGlu, true>(p, b, ldb, st);
-  // In a chain of dependent launches the ring is filled while the previous kernel runs (one row x 2560 x 9728 10.4 against 11.9 us, x
+  // In a decode step the ring is filled while the previous kernel runs (one row x 2560 x 9728 10.4 against 11.9 us, x
   // 4096 x 2048 4.4 against 5.4, x 2560 x 4096 6.2 both); the output head is long enough not to need that.
-  if (M <= 2 && !(dependent_launch_enabled() && N <= 32768)) {
+  if (M <= 2 && !(weights_early() && N <= 32768)) {
     // rows per warp: fewer for narrow outputs so that the grid still covers every SM a few times (with SwiGLU a warp
     // needs at least one gate row and one up row)
     constexpr int R1 = kGlu ? 2 : 1;

@@ -157,14 +157,17 @@ KSA_API int ksa_set_peer_wait_ms(int ms) {
 }
 
 namespace ksa {
-static bool g_dependent_launch = false;
-bool dependent_launch_enabled() { return g_dependent_launch; }
+// Of the calling thread alone: a product that another thread issues meanwhile must not read its weights early, and two threads
+// that each save and restore the setting would leave it on.
+static thread_local bool t_weights_early = false;
+bool weights_early() { return t_weights_early; }
 }  // namespace ksa
 
-// Switch dependent launches of the decode-step kernels on (1) or off (0); returns the previous setting.
+// Whether the weight-streaming products that the calling thread launches from here on are part of a decode step, in which no kernel
+// writes weights: they then read them before the previous kernel has ended.  Returns the thread's previous setting.
 KSA_API int ksa_set_dependent_launch(int on) {
-  const int before = ksa::g_dependent_launch ? 1 : 0;
-  ksa::g_dependent_launch = on != 0;
+  const int before = ksa::t_weights_early ? 1 : 0;
+  ksa::t_weights_early = on != 0;
   return before;
 }
 

@@ -58,9 +58,9 @@ int ensure_device(const void* device_ptr);
 // Dependent launches (programmatic stream serialization).  Most kernels are launched so that each may start while its predecessor on the
 // stream still runs, and wait for it on the device before they touch memory (grid_dependency_enter): the launch and the set-up of
 // one kernel lie under the end of the one before.  Kernels that write weights (the optimizer) are launched the ordinary way.
-// While the switch is on (ksa_set_dependent_launch; the inference engine's decode step), the weight-streaming products also
-// read their weights before they wait: no kernel of such a chain writes weights.
-bool dependent_launch_enabled();
+// While a thread has its switch on (ksa_set_dependent_launch; the inference engine's decode step), the weight-streaming products
+// that it launches also read their weights before they wait: no kernel of such a chain writes weights.
+bool weights_early();
 
 template <typename Kern, typename... Args>
 inline cudaError_t launch_kernel_if(bool dependent, Kern kern, dim3 grid, dim3 block, size_t smem, cudaStream_t st, Args... args) {

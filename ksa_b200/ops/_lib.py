@@ -281,9 +281,9 @@ def set_peer_wait_ms(ms: int) -> None:
 
 
 def set_dependent_launch(on: bool) -> bool:
-    """Switch dependent launches of the decode-step kernels (programmatic stream serialization: a kernel may start
-    while its predecessor on the stream still runs and waits for it on the device) on or off; returns the previous
-    setting.  The inference engine switches it on around a decode step; training leaves it off."""
+    """Whether the weight-streaming products that THIS THREAD launches may read their weights before the previous kernel of the
+    stream has ended; returns the thread's previous setting.  The inference engine switches it on around a decode step, in
+    which no kernel writes weights.  (That kernels start while their predecessor still runs is not switched here.)"""
     return load().ksa_set_dependent_launch(1 if on else 0) != 0
 
 
