@@ -221,7 +221,7 @@ KSA_API int ksa_cross_entropy(void* logits, const void* labels, void* row_loss, 
     at[1].id = cudaLaunchAttributeProgrammaticStreamSerialization;
     at[1].val.programmaticStreamSerializationAllowed = 1;
     cfg.attrs = at;
-    cfg.numAttrs = 2;
+    cfg.numAttrs = dependent_launches() ? 2 : 1;
     KSA_CHECK_CUDA(cudaLaunchKernelEx(&cfg, cross_entropy_cluster_kernel, (bf16*)logits, (const long long*)labels, (float*)row_loss,
                                       (const float*)grad_scale, V, ld, ignore_index, write_grad, ctas, part, status));
     return 0;

@@ -318,7 +318,7 @@ static int launch_narrow(const void* x, const void* w, NarrowArgs p, long long l
   at[1].id = cudaLaunchAttributeProgrammaticStreamSerialization;
   at[1].val.programmaticStreamSerializationAllowed = 1;
   cfg.attrs = at;
-  cfg.numAttrs = 2;
+  cfg.numAttrs = dependent_launches() ? 2 : 1;
   KSA_CHECK_CUDA(cudaLaunchKernelEx(&cfg, kern, tmW, tmX, p, status));
   return 0;
 }

@@ -157,17 +157,24 @@ KSA_API int ksa_set_peer_wait_ms(int ms) {
 }
 
 namespace ksa {
-// Of the calling thread alone: a product that another thread issues meanwhile must not read its weights early, and two threads
-// that each save and restore the setting would leave it on.
-static thread_local bool t_weights_early = false;
-bool weights_early() { return t_weights_early; }
+// How the calling thread launches (host.h).  Of the thread alone: a product that another thread issues meanwhile must not read its
+// weights early, and two threads that each save and restore the setting would leave it on.
+static int first_launch_mode() {
+  static const int mode = [] {
+    const char* e = getenv("KSA_DEPENDENT_LAUNCH");
+    return e != nullptr && strcmp(e, "0") == 0 ? kLaunchOrdinary : kLaunchDependent;
+  }();
+  return mode;
+}
+static thread_local int t_launch_mode = first_launch_mode();
+int launch_mode() { return t_launch_mode; }
 }  // namespace ksa
 
-// Whether the weight-streaming products that the calling thread launches from here on are part of a decode step, in which no kernel
-// writes weights: they then read them before the previous kernel has ended.  Returns the thread's previous setting.
-KSA_API int ksa_set_dependent_launch(int on) {
-  const int before = ksa::t_weights_early ? 1 : 0;
-  ksa::t_weights_early = on != 0;
+// Sets the calling thread's launch mode (below zero: ordinary, 0: dependent, above: dependent with early weights) and returns the
+// one it had.
+KSA_API int ksa_set_dependent_launch(int mode) {
+  const int before = ksa::t_launch_mode;
+  ksa::t_launch_mode = mode < 0 ? ksa::kLaunchOrdinary : mode > 0 ? ksa::kLaunchEarlyWeights : ksa::kLaunchDependent;
   return before;
 }
 

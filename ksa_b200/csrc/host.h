@@ -58,9 +58,13 @@ int ensure_device(const void* device_ptr);
 // Dependent launches (programmatic stream serialization).  Most kernels are launched so that each may start while its predecessor on the
 // stream still runs, and wait for it on the device before they touch memory (grid_dependency_enter): the launch and the set-up of
 // one kernel lie under the end of the one before.  Kernels that write weights (the optimizer) are launched the ordinary way.
-// While a thread has its switch on (ksa_set_dependent_launch; the inference engine's decode step), the weight-streaming products
-// that it launches also read their weights before they wait: no kernel of such a chain writes weights.
-bool weights_early();
+// A thread launches in one of three modes (ksa_set_dependent_launch): as described, or with early weights (the inference engine's
+// decode step), in which the weight-streaming products also read their weights before they wait, since no kernel of such a chain
+// writes weights, or the ordinary way (KSA_DEPENDENT_LAUNCH=0).
+enum LaunchMode : int { kLaunchOrdinary = -1, kLaunchDependent = 0, kLaunchEarlyWeights = 1 };
+int launch_mode();
+inline bool dependent_launches() { return launch_mode() != kLaunchOrdinary; }
+inline bool weights_early() { return launch_mode() == kLaunchEarlyWeights; }
 
 template <typename Kern, typename... Args>
 inline cudaError_t launch_kernel_if(bool dependent, Kern kern, dim3 grid, dim3 block, size_t smem, cudaStream_t st, Args... args) {
@@ -73,7 +77,7 @@ inline cudaError_t launch_kernel_if(bool dependent, Kern kern, dim3 grid, dim3 b
   at[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
   at[0].val.programmaticStreamSerializationAllowed = 1;
   cfg.attrs = at;
-  cfg.numAttrs = dependent ? 1 : 0;
+  cfg.numAttrs = dependent && dependent_launches() ? 1 : 0;
   return cudaLaunchKernelEx(&cfg, kern, args...);
 }
 // Kernels that bring their data in by TMA, and short ones.

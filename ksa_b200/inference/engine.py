@@ -297,11 +297,11 @@ class KsaInferenceEngine:
     def _decode_impl(self, tokens: torch.Tensor, any_boundary: bool, with_head: bool = True) -> torch.Tensor:
         """Device work of one decode step (launches only; the host mirror of the lengths is advanced by the caller).
         ``any_boundary``: some sequence closes a chunk in this step; which ones is read from ``_boundary_dev``."""
-        if not tokens.is_cuda or os.environ.get("KSA_DEPENDENT_LAUNCH", "1") == "0":
+        if not tokens.is_cuda:
             return self._decode_body(tokens, any_boundary, with_head)
-        # a step is a chain of some four hundred kernels of a few microseconds each: launched dependently, each may
-        # start (and the projections fetch their first weights) while its predecessor is still running
-        before = _lib.set_dependent_launch(True)
+        # a step is a chain of some four hundred kernels of a few microseconds each: while a kernel's predecessor still runs, it
+        # may start, and a projection may fetch its first weights
+        before = _lib.set_dependent_launch(_lib.ORDINARY if os.environ.get("KSA_DEPENDENT_LAUNCH", "1") == "0" else _lib.EARLY_WEIGHTS)
         try:
             return self._decode_body(tokens, any_boundary, with_head)
         finally:

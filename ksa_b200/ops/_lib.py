@@ -280,11 +280,15 @@ def set_peer_wait_ms(ms: int) -> None:
         raise RuntimeError("could not set the peer wait limit")
 
 
-def set_dependent_launch(on: bool) -> bool:
-    """Whether the weight-streaming products that THIS THREAD launches may read their weights before the previous kernel of the
-    stream has ended; returns the thread's previous setting.  The inference engine switches it on around a decode step, in
-    which no kernel writes weights.  (That kernels start while their predecessor still runs is not switched here.)"""
-    return load().ksa_set_dependent_launch(1 if on else 0) != 0
+ORDINARY, DEPENDENT, EARLY_WEIGHTS = -1, 0, 1
+
+
+def set_dependent_launch(mode: int) -> int:
+    """How THIS THREAD launches kernels from here on; returns how it did before.  ``DEPENDENT`` (or False): a kernel may start while
+    its predecessor on the stream still runs, and waits for it on the device before it touches memory.  ``EARLY_WEIGHTS`` (or
+    True): the products that stream weights also read them before they wait; for chains in which no kernel writes weights (the
+    inference engine's decode step).  ``ORDINARY``: one after the other; where a thread starts with ``KSA_DEPENDENT_LAUNCH=0``."""
+    return load().ksa_set_dependent_launch(int(mode))
 
 
 def gemm_on_pairs(M: int, N: int, pair_min_tiles: int) -> bool:
