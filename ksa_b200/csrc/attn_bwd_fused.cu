@@ -226,7 +226,7 @@ __device__ __forceinline__ void attn_bwd_fused_body(const CUtensorMap& tmQ, cons
   __syncthreads();
   tc_fence_after();
   const uint32_t tmem_base = *tmem_slot;
-  grid_dependency_enter();
+  if (!kCp) grid_dependency_enter();     // the context-parallel form waits for other GPUs: see grid_dependency_enter
   const uint32_t tS = tmem_base, tdP = tmem_base + 128, tdV = tmem_base + 256, tdK = tmem_base + 384;
 
   if (warp == 0) {

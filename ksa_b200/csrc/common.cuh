@@ -302,6 +302,8 @@ __device__ __forceinline__ void grid_dependency_launch() { asm volatile("griddep
 // The first thing a kernel does with memory that others write, or before it writes memory that others read: everything up to here
 // (barriers, tensor memory, address arithmetic) may run while the previous kernel of the stream still does.  Its own successor may
 // start from now on, so a kernel that only waits here overlaps at most its immediate predecessor.
+// A kernel that waits for other GPUs is launched the ordinary way and lets no successor start: CTAs of a successor would sit on the SMs
+// for as long as the peers take, in the places of the side stream's kernels that the peers may be waiting for.
 // What the predecessor writes changes while such a kernel is already running, so its parameters are not `const __restrict__` and its
 // loads not `ld.global.nc`: both promise memory that stays the same for the whole kernel, may be moved ahead of the wait and may hit
 // lines that an SM kept from before.

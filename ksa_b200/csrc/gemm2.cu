@@ -173,7 +173,7 @@ gemm2_bf16_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant
   cluster_sync_all();          // both CTAs' barriers are initialised before any remote arrival
   tc_fence_after();
   const uint32_t tmem_base = *tmem_slot;
-  grid_dependency_enter();     // (returns at once in the ordinary launches of the communication forms)
+  if (!comm.active && ep.c_world <= 1) grid_dependency_enter();     // not in the communicating forms: see there
 
   auto tile_coords = [&](int tile, int& mb, int& nb) {
     const int per_group = k2GroupM * tiles_n;

@@ -24,6 +24,7 @@ struct TpReduceArgs {
   uint32_t* done;                  // CTAs of this launch that have finished (the last one advances *epoch)
   int row_lo, row_hi;              // rows reduced by this rank (all of them, or its shard in the two-phase form)
   uint32_t* notify[kMaxPeers];     // two-phase form: flag2[rank] on every rank, raised when the shard is written
+  int release_successor;           // the next kernel may start while this one waits
 };
 
 constexpr int kTpThreads = 256;
@@ -79,8 +80,9 @@ __device__ __forceinline__ void tp_reduce_rows(const TpReduceArgs& a, float* red
 }
 
 __global__ void __launch_bounds__(kTpThreads) tp_allreduce_add_rmsnorm_kernel(TpReduceArgs a, int* status) {
-  grid_dependency_launch();   // a dependent-launched successor may start (the skinny GEMM: its weight loads)
-  grid_dependency_wait();     // launched dependently itself: the previous kernel's results are complete from here on
+  // In a decode step the projection that follows may start and fetch its weights; elsewhere nothing may while this kernel waits for
+  // other GPUs (see grid_dependency_enter).  The kernel itself is launched the ordinary way.
+  if (a.release_successor) grid_dependency_launch();
   __shared__ float red[32];
   __shared__ int s_ok;
   if (threadIdx.x == 0) s_ok = 1;
@@ -140,6 +142,7 @@ static int tp_launch(const void* x, const void* const* partial_ptrs, const void*
   a.rows_x = rows_x; a.delta_rows = delta_rows; a.D = D; a.eps = eps;
   a.epoch = static_cast<const uint32_t*>(epoch); a.done = static_cast<uint32_t*>(done);
   a.row_lo = row_lo; a.row_hi = row_hi;
+  a.release_successor = weights_early();
   KSA_REQUIRE(a.epoch != nullptr && a.done != nullptr, "tp all-reduce: epoch and done counters are required");
   // every CTA must be resident while it waits for the peers: at most 4 CTAs of 256 threads per SM are launched
   int sms = 148;

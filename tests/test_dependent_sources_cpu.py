@@ -1,0 +1,33 @@
+"""Rules for kernels that start while their predecessor still runs, held against the sources."""
+import re
+from pathlib import Path
+
+CSRC = Path(__file__).resolve().parents[1] / "ksa_b200" / "csrc"
+
+
+def _functions(text):
+    """(header, body) of every device function and kernel."""
+    text = re.sub(r"//[^\n]*", "", text)
+    for m in re.finditer(r"(?:__global__|__device__)[^;{}()]*(?:\([^(){};]*\)[^;{}()]*)*?\b\w+\s*\(([^{};]*?)\)\s*\{", text):
+        depth, at = 1, m.end()
+        while depth:
+            depth += {"{": 1, "}": -1}.get(text[at], 0)
+            at += 1
+        yield m.group(0), text[m.end():at]
+
+
+SOURCES = [(f.name, *fn) for f in sorted(CSRC.glob("*.cu")) for fn in _functions(f.read_text())]
+WAITS_FOR_PEERS = re.compile(r"flag_wait_ge\(")
+
+
+def test_what_waits_for_other_gpus_lets_no_successor_start():
+    """Its successors, always launched dependently, would hold SMs for as long as the peers take."""
+    checked = 0
+    for name, header, body in SOURCES:
+        if not WAITS_FOR_PEERS.search(body):
+            continue
+        checked += 1
+        for line in body.split("\n"):
+            if re.search(r"grid_dependency_(enter|launch)\(", line):
+                assert re.search(r"\bif \(", line), (name, header[-120:], line)
+    assert checked >= 4
