@@ -543,8 +543,8 @@ KSA_API int ksa_kv_cache_move(void* k_cache, void* v_cache, const void* src, con
 namespace ksa {
 // The slices of a step's text tokens on a ring-buffer cache (inference/cache.py), one thread per sequence: what PyTorch takes ten
 // kernels of a microsecond and a half for, none of which the next one may overlap.
-__global__ void decode_step_slices_kernel(const int* __restrict__ text_len, const int* __restrict__ cbl, const int* __restrict__ chunks,
-                                          int* __restrict__ out, int B, int n_sum, int chunk, int window, int text0, int sum0) {
+__global__ void decode_step_slices_kernel(const int* cbl, const int* chunks, int* out, int B, int n_sum, int chunk, int window, int text0,
+                                          int sum0) {
   grid_dependency_launch();
   grid_dependency_wait();
   const int b = blockIdx.x * blockDim.x + threadIdx.x;
@@ -553,10 +553,9 @@ __global__ void decode_step_slices_kernel(const int* __restrict__ text_len, cons
   const int end = done >= window ? sum0 + (done - window) * n_sum : text0 + done * chunk;
   out[b] = slot;
   out[B + b] = end - slot;
-  out[2 * B + b] = text_len[b] + 1;
 }
 // The counters after an ordinary step.
-__global__ void decode_advance_kernel(int* __restrict__ text_len, int* __restrict__ cbl, int B) {
+__global__ void decode_advance_kernel(int* text_len, int* cbl, int B) {
   grid_dependency_launch();
   grid_dependency_wait();
   const int b = blockIdx.x * blockDim.x + threadIdx.x;
@@ -566,14 +565,13 @@ __global__ void decode_advance_kernel(int* __restrict__ text_len, int* __restric
 }
 }  // namespace ksa
 
-// out [3, B] int32: write slot (also the start of the slice), slice length, text length with the new token.
-KSA_API int ksa_decode_step_slices(const void* text_len, const void* cbl, const void* chunks, void* out, int B, int n_sum, int chunk,
-                                   int window, int text0, int sum0, void* stream) {
-  KSA_ENTER(text_len);
+// out [2, B] int32: write slot (also the start of the slice), slice length.
+KSA_API int ksa_decode_step_slices(const void* cbl, const void* chunks, void* out, int B, int n_sum, int chunk, int window, int text0,
+                                   int sum0, void* stream) {
+  KSA_ENTER(cbl);
   if (B == 0) return 0;
   KSA_CHECK_CUDA(launch_kernel(decode_step_slices_kernel, dim3((B + 127) / 128), dim3(128), 0, reinterpret_cast<cudaStream_t>(stream),
-                               (const int*)text_len, (const int*)cbl, (const int*)chunks, (int*)out, B, n_sum, chunk, window, text0,
-                               sum0));
+                               (const int*)cbl, (const int*)chunks, (int*)out, B, n_sum, chunk, window, text0, sum0));
   return 0;
 }
 

@@ -94,8 +94,8 @@ def _step_slices(spec: CacheSpec, st: CacheState):
     if not st.cbl.is_cuda:
         return text_step_slices(spec, st)
     B = st.cbl.numel()
-    out = torch.empty((3, B), dtype=torch.int32, device=st.cbl.device)
-    _lib.call("ksa_decode_step_slices", st.text_len, st.cbl, st.chunks, out, B, spec.n_sum, spec.chunk, spec.window, spec.text0,
+    out = torch.empty((2, B), dtype=torch.int32, device=st.cbl.device)
+    _lib.call("ksa_decode_step_slices", st.cbl, st.chunks, out, B, spec.n_sum, spec.chunk, spec.window, spec.text0,
               spec.sum0)
     return out[0], out[0], out[1]
 

@@ -58,7 +58,7 @@ _SIGNATURES: Dict[str, Sequence] = {
     "ksa_summary_attn_fwd": [P] * 7 + [I] * 6 + [L] * 12 + [I] * 5 + [F, P],
     "ksa_summary_attn_bwd": [P] * 13 + [I] * 6 + [L] * 22 + [I] * 5 + [F, P, P, I, P],
     "ksa_decode_attn": [P] * 8 + [I] * 8 + [L, F, P, P],
-    "ksa_decode_step_slices": [P, P, P, P, I, I, I, I, I, I, P],
+    "ksa_decode_step_slices": [P, P, P, I, I, I, I, I, I, P],
     "ksa_decode_advance": [P, P, I, P],
     "ksa_kv_cache_append": [P] * 5 + [I] * 5 + [L, L, P],
     "ksa_kv_cache_move": [P] * 5 + [I] * 5 + [P],

@@ -31,3 +31,10 @@ def test_what_waits_for_other_gpus_lets_no_successor_start():
             if re.search(r"grid_dependency_(enter|launch)\(", line):
                 assert re.search(r"\bif \(", line), (name, header[-120:], line)
     assert checked >= 4
+
+
+def test_kernels_that_start_early_promise_nothing_about_their_memory():
+    """``const __restrict__`` lets loads move ahead of the wait or hit lines that an SM kept from before."""
+    kernels = [(n, h) for n, h, body in SOURCES if "__global__" in h and "grid_dependency_" in body]
+    assert len(kernels) >= 25
+    assert not [(n, h) for n, h in kernels if "__restrict__" in h]
