@@ -526,11 +526,18 @@ def norm_linear(x: torch.Tensor, delta: Optional[torch.Tensor], norm_w: torch.Te
             and x.dtype == torch.bfloat16 and weight.dtype == torch.bfloat16
             and not (torch.is_grad_enabled() and (x.requires_grad or weight.requires_grad))
             and x.stride(1) == 1 and weight.stride(1) == 1 and x.shape[1] % 8 == 0 and x.stride(0) % 8 == 0
-            and weight.stride(0) % 8 == 0 and weight.stride(0) > 0 and (delta is None or (delta.stride(1) == 1 and delta.stride(0) % 8 == 0
+            and weight.stride(0) % 8 == 0 and (delta is None or (delta.stride(1) == 1 and delta.stride(0) % 8 == 0
                                                                   and delta.dtype == torch.bfloat16))
-            and (not glu or weight.shape[0] % 2 == 0) and (x.numel() <= 81920 or x.shape[0] > 1)):
+            and (not glu or weight.shape[0] % 2 == 0)):
         M, K = x.shape
         N = weight.shape[0]
+        if weight.stride(0) == 0:          # (its tensor map takes no pitch of zero)
+            weight = weight.contiguous()
+        if K > 81920:                      # wider than any kernel's norm: a few rows of a few hundred kilobytes beside all their weights
+            n = 0 if delta is None else delta.shape[0]
+            res = x if delta is None else torch.cat([(x[:n].float() + delta.float()).to(x.dtype), x[n:]])
+            h = ref.rms_norm(res, norm_w, eps)
+            return res, (linear_swiglu(h, weight) if glu else linear(h, weight))
         if x.numel() > 81920:              # more than a CTA keeps in shared memory beside its ring: row by row
             parts = [norm_linear(x[i:i + 1], None if delta is None or i >= delta.shape[0] else delta[i:i + 1], norm_w, eps, weight, glu)
                      for i in range(M)]

@@ -96,6 +96,37 @@ def test_norm_and_product_of_long_rows(rows, k):
     _lib.check_status()
 
 
+@pytest.mark.parametrize("rows, delta_rows", [(1, None), (1, 1), (4, 3), (3, None)])
+@pytest.mark.parametrize("glu", [False, True])
+def test_rows_wider_than_any_norm_kernel(rows, delta_rows, glu):
+    k = 81928
+    x, nw = torch.randn(rows, k, device="cuda").bfloat16(), (1 + 0.1 * torch.randn(k, device="cuda")).bfloat16()
+    d = None if delta_rows is None else torch.randn(delta_rows, k, device="cuda").bfloat16()
+    w = (torch.randn(64, k, device="cuda") * k ** -0.5).bfloat16()
+    with torch.no_grad():
+        res, y = ops.norm_linear(x, d, nw, 1e-6, w, glu)
+    want_res = x.clone()
+    if d is not None:
+        want_res[:delta_rows] += d
+    h = want_res.float()
+    want = (h * torch.rsqrt(h.square().mean(-1, keepdim=True) + 1e-6) * nw.float()).bfloat16().float() @ w.float().t()
+    if glu:
+        gate, up = want.bfloat16().float().chunk(2, -1)
+        want = torch.nn.functional.silu(gate) * up
+    assert torch.equal(res, want_res)
+    assert float((y.float() - want).norm()) <= 2.0 ** -6 * float(want.norm())      # a rounding of gate, up and result each, 2^-8
+    _lib.check_status()
+
+
+def test_norm_and_product_with_expanded_weights():
+    """Long rows, so that no other way is open."""
+    x, nw = torch.randn(2, 16384, device="cuda").bfloat16(), torch.ones(16384, device="cuda").bfloat16()
+    w = torch.randn(1, 16384, device="cuda").bfloat16()
+    with torch.no_grad():
+        assert torch.equal(ops.norm_linear(x, None, nw, 1e-6, w.expand(40, -1))[1], ops.norm_linear(x, None, nw, 1e-6, w.repeat(40, 1))[1])
+    _lib.check_status()
+
+
 def test_operands_off_16_bytes_are_refused():
     w, x = torch.zeros(300 * 64 + 4, device="cuda").bfloat16(), torch.zeros(3, 64, device="cuda").bfloat16()
     with pytest.raises(RuntimeError, match="aligned"):
