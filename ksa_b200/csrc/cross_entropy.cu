@@ -198,12 +198,13 @@ KSA_API int ksa_cross_entropy(void* logits, const void* labels, void* row_loss, 
                               int V, long long ld, int ignore_index, int write_grad, void* stream) {
   KSA_ENTER(logits);
   KSA_REQUIRE(V % 8 == 0 && ld % 8 == 0, "cross_entropy: V=%d and ld=%lld must be multiples of 8", V, ld);
+  KSA_REQUIRE((reinterpret_cast<uintptr_t>(logits) & 15) == 0, "cross_entropy: the logits must be 16-byte aligned");
   if (rows == 0) return 0;
   cudaStream_t st = reinterpret_cast<cudaStream_t>(stream);
   int ctas = 1;
   while (ctas < 8 && ((V / 8 + ctas - 1) / ctas) * 16 > kCeMostBytes) ctas *= 2;
   const int part = (V / 8 + ctas - 1) / ctas;
-  if (V > 0 && part * 16 <= kCeMostBytes && (reinterpret_cast<uintptr_t>(logits) & 15) == 0) {
+  if (V > 0 && part * 16 <= kCeMostBytes) {
     // (per device, so on each call)
     KSA_CHECK_CUDA(cudaFuncSetAttribute(cross_entropy_cluster_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, kCeMostBytes));
     int* status = status_word();

@@ -39,3 +39,13 @@ def test_rows(V, grad):
     err = (y[:6, :V].double() - g[:6]).abs()
     # one rounding to bf16, half of 2^-7, of a p with less than 2^-17 (arguments of __expf down to -40), and (p - 1) / 4 with p's 2^-19
     assert bool((err <= (2.0 ** -8 + 2.0 ** -16) * g[:6].abs() + 2.0 ** -21).all()), float(err.max())
+
+
+@pytest.mark.parametrize("V", [4096, 327688])
+def test_logits_off_16_bytes_are_refused(V):
+    """Both kernels read and write 16 bytes at a time."""
+    x = torch.zeros(2 * V + 8, device="cuda").bfloat16()[4:4 + 2 * V].view(2, V)
+    loss, labels = torch.zeros(2, device="cuda"), torch.zeros(2, dtype=torch.int64, device="cuda")
+    with pytest.raises(RuntimeError, match="aligned"):
+        _lib.call("ksa_cross_entropy", x, labels, loss, loss, 2, V, V, -100, 1)
+    _lib.check_status()
