@@ -576,12 +576,9 @@ static int launch_bwd(const CUtensorMap& tq, const CUtensorMap& tdo, const CUten
                       const CUtensorMap& tks, const CUtensorMap& tvs, const BwdParams& p, cudaStream_t st) {
   auto k1 = attn_bwd_dq_kernel<HD>;
   auto k2 = attn_bwd_dkv_kernel<HD>;
-  static bool attr = false;
-  if (!attr) {
-    KSA_CHECK_CUDA(cudaFuncSetAttribute(k1, cudaFuncAttributeMaxDynamicSharedMemorySize, BwdSmem<HD>::kTotal));
-    KSA_CHECK_CUDA(cudaFuncSetAttribute(k2, cudaFuncAttributeMaxDynamicSharedMemorySize, BwdSmem<HD>::kTotal));
-    attr = true;
-  }
+  static PerDevice raised1, raised2;
+  KSA_CHECK_CUDA(raise_smem_limit(raised1, k1, BwdSmem<HD>::kTotal));
+  KSA_CHECK_CUDA(raise_smem_limit(raised2, k2, BwdSmem<HD>::kTotal));
   dim3 g1((p.s.Lq + 127) / 128, p.s.Hq, p.s.B);
   k1<<<g1, kBwdThreads, BwdSmem<HD>::kTotal, st>>>(tq, tdo, tk, tv, tks, tvs, p);
   KSA_CHECK_CUDA(cudaGetLastError());

@@ -661,11 +661,8 @@ KSA_API int ksa_attn_bwd_fused(const void* q, const void* k, const void* v, cons
   p.status = status_word();
   KSA_REQUIRE(p.status != nullptr, "could not allocate the status word");
   cudaStream_t st = reinterpret_cast<cudaStream_t>(stream);
-  static bool attr = false;
-  if (!attr) {
-    KSA_CHECK_CUDA(cudaFuncSetAttribute(attn_bwd_fused_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, FbSmem::kTotal));
-    attr = true;
-  }
+  static PerDevice raised;
+  KSA_CHECK_CUDA(raise_smem_limit(raised, attn_bwd_fused_kernel, FbSmem::kTotal));
   {
     const long long items = (long long)B * Hq * lq_pad;
     const int threads = 256;
@@ -774,11 +771,8 @@ KSA_API int ksa_attn_bwd_fused_cp(const void* q, const void* o, const void* d_o,
   p.status = status_word();
   KSA_REQUIRE(p.status != nullptr, "could not allocate the status word");
   cudaStream_t st = reinterpret_cast<cudaStream_t>(stream);
-  static bool attr = false;
-  if (!attr) {
-    KSA_CHECK_CUDA(cudaFuncSetAttribute(attn_bwd_fused_cp_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, FbSmem::kTotal));
-    attr = true;
-  }
+  static PerDevice raised;
+  KSA_CHECK_CUDA(raise_smem_limit(raised, attn_bwd_fused_cp_kernel, FbSmem::kTotal));
   {
     const long long items = (long long)B * Hq * lq_pad;
     const int threads = 256;

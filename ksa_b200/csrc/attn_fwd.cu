@@ -439,25 +439,12 @@ static int make_head_tmap(CUtensorMap* m, const void* base, int HD, long long T,
   return make_tmap(m, base, 2, 4, dims, str, box, true);
 }
 
-static int sm_count() {
-  static int num_sms = 0;
-  if (num_sms == 0) {
-    int dev = 0;
-    if (cudaGetDevice(&dev) != cudaSuccess) return 0;
-    if (cudaDeviceGetAttribute(&num_sms, cudaDevAttrMultiProcessorCount, dev) != cudaSuccess) return 0;
-  }
-  return num_sms;
-}
-
 template <int HD>
 static int launch_fwd(const CUtensorMap& tq, const CUtensorMap& tk, const CUtensorMap& tv, const CUtensorMap& tks,
                       const CUtensorMap& tvs, const FwdParams& p, cudaStream_t st) {
   auto kern = attn_fwd_kernel<HD>;
-  static bool attr = false;
-  if (!attr) {
-    KSA_CHECK_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, FwdSmem<HD>::kTotal));
-    attr = true;
-  }
+  static PerDevice raised;
+  KSA_CHECK_CUDA(raise_smem_limit(raised, kern, FwdSmem<HD>::kTotal));
   const int items = ((p.s.Lq + 127) / 128) * (p.s.Hq / p.nslot) * p.s.B;
   int sms = sm_count();
   if (sms <= 0) return 1;
@@ -469,11 +456,8 @@ static int launch_fwd(const CUtensorMap& tq, const CUtensorMap& tk, const CUtens
 template <int HD>
 static int launch_fwd_cp(const CUtensorMap& tq, const CpSources& cps, const FwdParams& p, cudaStream_t st) {
   auto kern = attn_fwd_cp_kernel<HD>;
-  static bool attr = false;
-  if (!attr) {
-    KSA_CHECK_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, FwdSmem<HD>::kTotal));
-    attr = true;
-  }
+  static PerDevice raised;
+  KSA_CHECK_CUDA(raise_smem_limit(raised, kern, FwdSmem<HD>::kTotal));
   const int items = ((p.s.Lq + 127) / 128) * (p.s.Hq / p.nslot) * p.s.B;
   int sms = sm_count();
   if (sms <= 0) return 1;

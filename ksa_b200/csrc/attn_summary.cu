@@ -519,11 +519,8 @@ __global__ void __launch_bounds__(kSumBwdThreads) summary_attn_bwd_fast_kernel(S
 template <int NQ>
 static int launch_fwd_fast(const SumAttnArgs& a, int nk_max, size_t smem, cudaStream_t st) {
   auto kern = summary_attn_fwd_fast_kernel<128, NQ>;
-  static bool attr = false;
-  if (!attr) {
-    KSA_CHECK_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, 100 * 1024));
-    attr = true;
-  }
+  static PerDevice raised;
+  KSA_CHECK_CUDA(raise_smem_limit(raised, kern, 100 * 1024));
   KSA_CHECK_CUDA(launch_stream_kernel((long long)a.B * a.Hkv * (a.Nq / a.n_sum) * nk_max * 512, kern, dim3(a.Nq / a.n_sum,
                                       a.Hkv, a.B), dim3(kSumFwdThreads), smem, st, a, nk_max));
   return 0;
@@ -532,11 +529,8 @@ static int launch_fwd_fast(const SumAttnArgs& a, int nk_max, size_t smem, cudaSt
 template <int NQ>
 static int launch_bwd_fast(const SumAttnArgs& a, int nk_max, size_t smem, cudaStream_t st) {
   auto kern = summary_attn_bwd_fast_kernel<128, NQ>;
-  static bool attr = false;
-  if (!attr) {
-    KSA_CHECK_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, 100 * 1024));
-    attr = true;
-  }
+  static PerDevice raised;
+  KSA_CHECK_CUDA(raise_smem_limit(raised, kern, 100 * 1024));
   KSA_CHECK_CUDA(launch_stream_kernel((long long)a.B * a.Hkv * (a.Nq / a.n_sum) * nk_max * 512, kern, dim3(a.Nq / a.n_sum,
                                       a.Hkv, a.B), dim3(kSumBwdThreads), smem, st, a, nk_max));
   return 0;
@@ -619,11 +613,8 @@ KSA_API int ksa_summary_attn_bwd(const void* qs, const void* k, const void* v, c
   const size_t smem = (size_t)nq * (2 * HD + 2 * (chunk + n_sum)) * sizeof(float);
   KSA_REQUIRE(smem <= 200 * 1024, "summary_attn_bwd: %zu bytes of shared memory needed (chunk %d, %d queries)", smem,
               chunk, nq);
-  static bool attr = false;
-  if (!attr) {
-    KSA_CHECK_CUDA(cudaFuncSetAttribute(summary_attn_bwd_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, 200 * 1024));
-    attr = true;
-  }
+  static PerDevice raised;
+  KSA_CHECK_CUDA(raise_smem_limit(raised, summary_attn_bwd_kernel, 200 * 1024));
   dim3 grid(Nq / n_sum, Hkv, B);
   KSA_CHECK_CUDA(launch_kernel(summary_attn_bwd_kernel, grid, dim3(128), smem, reinterpret_cast<cudaStream_t>(stream), a));
   return 0;

@@ -205,8 +205,8 @@ KSA_API int ksa_cross_entropy(void* logits, const void* labels, void* row_loss, 
   while (ctas < 8 && ((V / 8 + ctas - 1) / ctas) * 16 > kCeMostBytes) ctas *= 2;
   const int part = (V / 8 + ctas - 1) / ctas;
   if (V > 0 && part * 16 <= kCeMostBytes) {
-    // (per device, so on each call)
-    KSA_CHECK_CUDA(cudaFuncSetAttribute(cross_entropy_cluster_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, kCeMostBytes));
+    static PerDevice raised;
+    KSA_CHECK_CUDA(raise_smem_limit(raised, cross_entropy_cluster_kernel, kCeMostBytes));
     int* status = status_word();
     KSA_REQUIRE(status != nullptr, "could not allocate the status word");
     cudaLaunchConfig_t cfg = {};

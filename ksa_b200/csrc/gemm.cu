@@ -263,18 +263,11 @@ static int launch_gemm(const void* a, const void* b, const GemmEpilogue& ep, int
   }
   if (rc) return rc;
 
-  static int num_sms = 0;
-  if (num_sms == 0) {
-    int dev = 0;
-    KSA_CHECK_CUDA(cudaGetDevice(&dev));
-    KSA_CHECK_CUDA(cudaDeviceGetAttribute(&num_sms, cudaDevAttrMultiProcessorCount, dev));
-  }
+  const int num_sms = sm_count();
+  KSA_REQUIRE(num_sms > 0, "no device");
   auto kern = gemm_bf16_kernel<BN, A_MN, B_MN>;
-  static bool attr_set = false;
-  if (!attr_set) {
-    KSA_CHECK_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, S::kTotal));
-    attr_set = true;
-  }
+  static PerDevice raised;
+  KSA_CHECK_CUDA(raise_smem_limit(raised, kern, S::kTotal));
   const int tiles = ((M + kBM - 1) / kBM) * ((N + BN - 1) / BN);
   int ctas = num_sms;
   if (sm_limit > 0 && sm_limit < ctas) ctas = sm_limit;

@@ -513,18 +513,11 @@ static int launch_gemm2(const void* a, const void* b, const Gemm2Epilogue& ep, i
     rc = make_tmap(&tmB, b, 2, 2, dims, str, box, true);
   }
   if (rc) return rc;
-  static int num_sms = 0;
-  if (num_sms == 0) {
-    int dev = 0;
-    KSA_CHECK_CUDA(cudaGetDevice(&dev));
-    KSA_CHECK_CUDA(cudaDeviceGetAttribute(&num_sms, cudaDevAttrMultiProcessorCount, dev));
-  }
+  const int num_sms = sm_count();
+  KSA_REQUIRE(num_sms > 0, "no device");
   auto kern = gemm2_bf16_kernel<A_MN, B_MN, kGlu>;
-  static bool attr_set = false;
-  if (!attr_set) {
-    KSA_CHECK_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, k2SmemTotal));
-    attr_set = true;
-  }
+  static PerDevice raised;
+  KSA_CHECK_CUDA(raise_smem_limit(raised, kern, k2SmemTotal));
   const int tiles = ((M + 2 * k2BM - 1) / (2 * k2BM)) * (kGlu ? (N / 2 + k2BNh - 1) / k2BNh : (N + k2BN - 1) / k2BN);
   int pairs = num_sms / 2;
   if (tiles < pairs) pairs = tiles;

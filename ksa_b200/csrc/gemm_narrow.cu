@@ -298,11 +298,8 @@ static int launch_narrow(const void* x, const void* w, NarrowArgs p, long long l
   const int n_tile = kGlu ? 64 : 128, n_out = kGlu ? p.N / 2 : p.N;
   const int tiles = p.tiles_m * ((n_out + n_tile - 1) / n_tile);
   auto kern = gemm_narrow_kernel<W_MN, kGlu>;
-  static bool attr_set = false;
-  if (!attr_set) {
-    KSA_CHECK_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, 222 * 1024));
-    attr_set = true;
-  }
+  static PerDevice raised;
+  KSA_CHECK_CUDA(raise_smem_limit(raised, kern, 222 * 1024));
   int* status = status_word();
   KSA_REQUIRE(status != nullptr, "could not allocate the status word");
   cudaLaunchConfig_t cfg = {};

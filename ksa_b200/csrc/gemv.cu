@@ -318,20 +318,9 @@ stream_gemm_kernel(const __grid_constant__ CUtensorMap tmB, const __grid_constan
   }
 }
 
-static int stream_sms() {
-  static int sms = 0;
-  if (sms == 0) {
-    int dev = 0, n = 0;
-    if (cudaGetDevice(&dev) != cudaSuccess) return 0;
-    if (cudaDeviceGetAttribute(&n, cudaDevAttrMultiProcessorCount, dev) != cudaSuccess) return 0;
-    sms = n;
-  }
-  return sms;
-}
-
 template <int NB, bool kGlu, bool kNorm>
 static int launch_stream(StreamArgs p, const void* b, long long ldb, cudaStream_t st) {
-  const int sms = stream_sms();
+  const int sms = sm_count();
   KSA_REQUIRE(sms > 0, "gemv: no device");
   int* status = status_word();
   KSA_REQUIRE(status != nullptr, "could not allocate the status word");
@@ -378,11 +367,8 @@ static int launch_stream(StreamArgs p, const void* b, long long ldb, cudaStream_
     if ((rc = make_tmap(&tmA, p.A, 2, 3, dims, str, box, true))) return rc;
   }
   auto kern = stream_gemm_kernel<NB, kGlu, kNorm>;
-  static bool attr = false;
-  if (!attr) {
-    KSA_CHECK_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, kStSmemMost));
-    attr = true;
-  }
+  static PerDevice raised;
+  KSA_CHECK_CUDA(raise_smem_limit(raised, kern, kStSmemMost));
   KSA_CHECK_CUDA(launch_kernel(kern, dim3(grid), dim3(kStThreads + 32), (size_t)smem, st, tmB, tmA,
                               p, status));
   return 0;

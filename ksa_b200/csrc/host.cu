@@ -92,6 +92,16 @@ int ensure_device(const void* device_ptr) {
   return kErrNone;
 }
 
+int sm_count() {
+  static std::atomic<int> counts[64];
+  int dev = 0, n = 0;
+  if (cudaGetDevice(&dev) != cudaSuccess) return 0;
+  if (dev < 64 && (n = counts[dev].load(std::memory_order_relaxed)) > 0) return n;
+  if (cudaDeviceGetAttribute(&n, cudaDevAttrMultiProcessorCount, dev) != cudaSuccess) return 0;
+  if (dev < 64) counts[dev].store(n, std::memory_order_relaxed);
+  return n;
+}
+
 constexpr long long kDefaultPeerWaitMs = 10000;   // 10 s
 static int* g_status[64] = {nullptr};
 static std::mutex g_status_mu;

@@ -5,6 +5,7 @@
 
 #include <cuda.h>
 #include <cuda_runtime.h>
+#include <atomic>
 #include <stdint.h>
 #include <stdio.h>
 
@@ -34,6 +35,25 @@ int make_tmap(CUtensorMap* out, const void* base, int elem_bytes, int rank, cons
 
 // Device status word for the current device (allocated once per device on first use).
 int* status_word();
+
+// SMs of the current device, or 0.
+int sm_count();
+
+// What has been done once on every device (a process may use several, from several threads).
+struct PerDevice {
+  std::atomic<uint64_t> done{0};
+};
+// The limit of a kernel's dynamic shared memory belongs to the kernel on one device.
+template <typename Kern>
+inline cudaError_t raise_smem_limit(PerDevice& raised, Kern kern, size_t bytes) {
+  int dev = 0;
+  if (const cudaError_t e = cudaGetDevice(&dev)) return e;
+  const uint64_t bit = dev < 64 ? 1ull << dev : 0;
+  if (raised.done.load(std::memory_order_acquire) & bit) return cudaSuccess;
+  const cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)bytes);
+  if (e == cudaSuccess) raised.done.fetch_or(bit, std::memory_order_release);
+  return e;
+}
 
 // Make the device that owns `device_ptr` current on the calling thread.  Callers may arrive on threads that have
 // never touched CUDA through this library's runtime (autograd worker threads): without this, descriptor encoding

@@ -145,9 +145,8 @@ static int tp_launch(const void* x, const void* const* partial_ptrs, const void*
   a.release_successor = weights_early();
   KSA_REQUIRE(a.epoch != nullptr && a.done != nullptr, "tp all-reduce: epoch and done counters are required");
   // every CTA must be resident while it waits for the peers: at most 4 CTAs of 256 threads per SM are launched
-  int sms = 148;
-  int dev = 0;
-  if (cudaGetDevice(&dev) == cudaSuccess) cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
+  const int sms = sm_count();
+  KSA_REQUIRE(sms > 0, "no device");
   int rows = row_hi - row_lo;
   int grid = rows < sms * 4 ? (rows > 0 ? rows : 1) : sms * 4;
   tp_allreduce_add_rmsnorm_kernel<<<grid, kTpThreads, 0, reinterpret_cast<cudaStream_t>(stream)>>>(a, status);
