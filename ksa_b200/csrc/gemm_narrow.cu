@@ -258,17 +258,29 @@ static double narrow_plan(int M, long long n_tiles, int K, bool ragged_x, bool r
   }
   return best;
 }
-// The other kernels' time for the same product: 0.345 us a 64-wide step and wave of 74 CTA pairs with 256 x 256 tiles, 0.38 a
-// step and wave of 128 x 256 tiles on single CTAs, 5 us around them (17.5 us measured for 128 x 12288 x 2048, 55.3 for 1411 x 2560 x 9728,
-// 61 for 48 to 700 x 2560 x 9728 on single CTAs).
-static double tiled_time(int M, int N, int K, int pair_min_tiles) {
-  const long long num_kb = (K + 63) / 64, tn = (N + 255) / 256, pairs = (M + 255) / 256 * tn;
-  if (pair_min_tiles > 0 && pairs >= pair_min_tiles) return 5.0 + 0.345 * num_kb * ((pairs + kNwSms / 2 - 1) / (kNwSms / 2));
-  return 5.0 + 0.38 * num_kb * (((M + 127) / 128 * tn + kNwSms - 1) / kNwSms);
-}
-
 static long long tiled_waves(int M, int N, int rows, int slots) {
   return ((long long)((M + rows - 1) / rows) * ((N + 255) / 256) + slots - 1) / slots;
+}
+static bool enough_for_pairs(int M, int N, int pair_min_tiles) {
+  return pair_min_tiles > 0 && (long long)((M + 255) / 256) * ((N + 255) / 256) >= pair_min_tiles;
+}
+static bool on_pairs(int M, int N, int pair_min_tiles) {
+  return enough_for_pairs(M, N, pair_min_tiles) && 2 * tiled_waves(M, N, 256, kNwSms / 2) < 3 * tiled_waves(M, N, 128, kNwSms);
+}
+// The time of the tiled kernel that serves the same product otherwise: 0.345 us a 64-wide step and wave of 74 CTA pairs with 256 x 256
+// tiles, 5 us around them.  Single CTAs with 128 x 256 tiles take 0.38 a step and wave and 5 around them where there are too few tiles for
+// pairs (17.5 us measured for 128 x 12288 x 2048, 55.3 for 1411 x 2560 x 9728, 61 for 48 to 700 x 2560 x 9728).  Where they are
+// taken for their fewer waves, most SMs have a tile: 6.5 us and, a step and wave, 0.38 and 0.05 for every megabyte of weights that the
+// step's tiles read: 1152 x 4096 x 2048 17.4 us (0.5 MB), 333 x 12288 x 2048 21.2 (1.6 MB), 128 x 19456 x 2560 26.2 (2.5 MB).
+// glu: and of the separate activation kernel, 2 us and more, 2.8 to 3.7 behind the products of the last kind.
+static double tiled_time(int M, int N, int K, bool glu, int pair_min_tiles) {
+  const long long num_kb = (K + 63) / 64;
+  const double act = glu ? 2.0 : 0.0;
+  if (on_pairs(M, N, pair_min_tiles)) return act + 5.0 + 0.345 * num_kb * tiled_waves(M, N, 256, kNwSms / 2);
+  const double steps = (double)(num_kb * tiled_waves(M, N, 128, kNwSms));
+  if (!enough_for_pairs(M, N, pair_min_tiles)) return act + 5.0 + 0.38 * steps;
+  const long long tm = (M + 127) / 128, tn = (N + 255) / 256, abreast = (kNwSms + tm - 1) / tm;      // tiles of a row in one wave
+  return (glu ? 3.5 : 0.0) + 6.5 + (0.38 + 0.05 * (tn < abreast ? tn : abreast) * 256 * kNwBK * 2 / 1e6) * steps;
 }
 
 template <bool W_MN, bool kGlu>
@@ -350,20 +362,20 @@ KSA_API int ksa_gemm_narrow_bf16(const void* x, const void* w, void* c, int M, i
 // again: 333 x 19456 x 2560 3 waves against 2, 44.0 us on pairs and 41.0 on single CTAs; 333 x 12288 x 2048 2 against 1, 28.7 and 21.9;
 // 1152 x 4096 x 2048 2 against 1, 26.0 and 18.0 (fp32 from transposed operands 29.1 and 22.5).  At 4 against 3 both are within 6 %
 // (513 x 19456 x 2560 59.3 and 57.5, fp32 at 1152 x 12288 x 2048 53.3 and 61.1), at 6 against 5 pairs are 5 to 15 % faster.
+// Waves count 128 x 256 tiles; the 128 x 128 tiles that ksa_gemm_bf16 takes for a ragged N of few tiles take about as long together
+// (100 x 19320 x 2560 34.5 us on pairs and 32.5 there).
 KSA_API int ksa_gemm_on_pairs(int M, int N, int pair_min_tiles) {
-  using namespace ksa;
-  if (pair_min_tiles <= 0 || (long long)((M + 255) / 256) * ((N + 255) / 256) < pair_min_tiles) return 0;
-  return 2 * tiled_waves(M, N, 256, kNwSms / 2) < 3 * tiled_waves(M, N, 128, kNwSms);
+  return ksa::on_pairs(M, N, pair_min_tiles);
 }
 
 // Whether this kernel is expected to beat the tiled ones (of which CTA pairs are taken from `pair_min_tiles` 256 x 256 tiles on, 0:
 // never), by more than the model's error: bt * 16 + split for ksa_gemm_narrow_bf16, or 0.  glu: the separate activation
-// kernel, 2 us and more, counts on the other side.  ragged: bit 0, the activations' rows do not all start on a 128-byte line (their
+// kernel counts on the other side.  ragged: bit 0, the activations' rows do not all start on a 128-byte line (their
 // pitch is no multiple of 64 elements); bit 1, those of the weights as they lie in memory.
 KSA_API int ksa_gemm_narrow_plan(int M, int N, int K, int glu, int pair_min_tiles, int ragged) {
   using namespace ksa;
   if (M <= 0 || M > kNwMaxRows || N <= 0 || K <= 0) return 0;
   int bt = 0, split = 0;
   const double t = narrow_plan(M, glu ? (N / 2 + 63) / 64 : (N + 127) / 128, K, (ragged & 1) != 0, (ragged & 2) != 0, &bt, &split);
-  return t < 0.95 * (tiled_time(M, N, K, pair_min_tiles) + (glu ? 2.0 : 0.0)) ? bt * 16 + split : 0;
+  return t < 0.95 * tiled_time(M, N, K, glu != 0, pair_min_tiles) ? bt * 16 + split : 0;
 }

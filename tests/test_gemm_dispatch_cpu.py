@@ -72,3 +72,14 @@ def test_short_gemms_do_not_take_the_gather_and_flush_runs_it_alone(calls):
     n = len(calls)
     _lib.attach_pair_gather(_job(unit))
     assert len(calls) == n + 1 and calls[-1][0] == "ksa_peer_gather"
+
+
+@pytest.mark.parametrize("M, N, K, kernel", [
+    (333, 12288, 2048, "ksa_gemm_bf16"), (1152, 4096, 2048, "ksa_gemm_bf16"), (333, 19456, 2560, "ksa_gemm_bf16"),   # half the waves of pairs
+    (24, 19456, 2560, "ksa_gemm_narrow_bf16"), (64, 19456, 2560, "ksa_gemm_narrow_bf16"),     # and still longer than the split-K kernel
+    (160, 12288, 2048, "ksa_gemm2_bf16"), (1411, 12288, 2048, "ksa_gemm2_bf16"), (8192, 6144, 2048, "ksa_gemm2_bf16"),
+    (333, 2560, 4096, "ksa_gemm_narrow_bf16"), (16, 6144, 2560, "ksa_gemv_bf16")])
+def test_the_kernel_of_a_product(calls, M, N, K, kernel):
+    """The whole dispatch: the split-K kernel is weighed against the tiled kernel that the rule for CTA pairs leaves."""
+    ops.gemm(torch.empty(M, K, dtype=torch.bfloat16), torch.empty(N, K, dtype=torch.bfloat16))
+    assert calls[-1][0] == kernel

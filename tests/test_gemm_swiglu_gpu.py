@@ -51,3 +51,12 @@ def test_the_operator(rows, fused, main_grad):
     with torch.no_grad():
         assert (ops.linear_swiglu(x, w).float() - results[0][0].float()).abs().max() < 0.1
     _lib.check_status()
+
+
+@pytest.mark.parametrize("rows, F, launches", [(333, 6144, 2), (640, 6144, 1), (336, 9728, 2)])
+def test_the_fused_form_goes_by_the_rule_for_pairs(rows, F, launches):
+    """Where single CTAs take fewer waves, they and a separate activation are faster than the activation on pairs."""
+    x, w = torch.randn(rows, 512, device="cuda").bfloat16(), torch.randn(2 * F, 512, device="cuda").bfloat16().requires_grad_()
+    assert _lib.count_launches(lambda: ops.linear_swiglu(x, w)) == launches
+    assert _lib.gemm_on_pairs(rows, 2 * F, ops.GEMM_PAIR_MIN_TILES) == (launches == 1)
+    _lib.check_status()
