@@ -111,8 +111,8 @@ __device__ __forceinline__ void combine_if_last(const DecodeArgs& a, int b, int 
 
 template <int D>
 __global__ void __launch_bounds__(kDecThreads) decode_attn_kernel(DecodeArgs a) {
-  grid_dependency_launch();   // a dependent-launched successor may start (the skinny GEMM: its weight loads)
-  grid_dependency_wait();     // launched dependently itself: the previous kernel's results are complete from here on
+  grid_dependency_launch();   // the successor may start now: in a decode step it is a projection that reads its weights first
+  grid_dependency_wait();     // the previous kernel's results are complete from here on
   constexpr int ROW_W = D / 2 + 1;  // 32-bit words per padded row
   __shared__ uint32_t k_s[kDecTile * ROW_W];
   __shared__ uint32_t v_s[kDecTile * ROW_W];
@@ -257,8 +257,8 @@ __device__ __forceinline__ void mma_qk(float (&c)[4], uint32_t a0, uint32_t a1, 
 
 template <int NQ>   // queries served per CTA, padded: 4, 8 or 16
 __global__ void __launch_bounds__(kDecThreads) decode_attn_mma_kernel(DecodeArgs a) {
-  grid_dependency_launch();   // a dependent-launched successor may start (the skinny GEMM: its weight loads)
-  grid_dependency_wait();     // launched dependently itself: the previous kernel's results are complete from here on
+  grid_dependency_launch();   // the successor may start now: in a decode step it is a projection that reads its weights first
+  grid_dependency_wait();     // the previous kernel's results are complete from here on
   constexpr int D = 128, KPI = 16;                 // keys per warp iteration
   __shared__ __align__(16) float s_p[4][KPI][NQ];  // per warp: probabilities, [key][query]
   __shared__ float s_m[4][NQ], s_l[4][NQ];
@@ -420,8 +420,8 @@ __global__ void __launch_bounds__(kDecThreads) decode_attn_mma_kernel(DecodeArgs
 
 // one CTA per (b, t, head): merge the splits
 __global__ void __launch_bounds__(128) decode_combine_kernel(DecodeArgs a) {
-  grid_dependency_launch();   // a dependent-launched successor may start (the skinny GEMM: its weight loads)
-  grid_dependency_wait();     // launched dependently itself: the previous kernel's results are complete from here on
+  grid_dependency_launch();   // the successor may start now: in a decode step it is a projection that reads its weights first
+  grid_dependency_wait();     // the previous kernel's results are complete from here on
   const long long row = blockIdx.x;  // (b * Tq + t) * Hq + h
   const float* ml = a.part_ml + row * a.splits * 2;
   float m = -INFINITY;
@@ -444,8 +444,8 @@ __global__ void __launch_bounds__(256)
 kv_cache_append_kernel(const bf16* k_new, const bf16* v_new, bf16* k_cache,
                        bf16* v_cache, const int* slots, int B, int T, int H, int D, int cap,
                        long long src_row_stride, long long src_batch_stride) {
-  grid_dependency_launch();   // a dependent-launched successor may start (the skinny GEMM: its weight loads)
-  grid_dependency_wait();     // launched dependently itself: the previous kernel's results are complete from here on
+  grid_dependency_launch();   // the successor may start now: in a decode step it is a projection that reads its weights first
+  grid_dependency_wait();     // the previous kernel's results are complete from here on
   const long long vec = (long long)blockIdx.x * blockDim.x + threadIdx.x;
   const int per = D / 8;
   if (vec >= (long long)B * T * H * per) return;
@@ -466,8 +466,8 @@ __global__ void __launch_bounds__(256)
 kv_cache_move_kernel(bf16* k_cache, bf16* v_cache, const int* src,
                      const int* dst, const int* enable, int B, int H, int D, int cap,
                      int rows) {
-  grid_dependency_launch();   // a dependent-launched successor may start (the skinny GEMM: its weight loads)
-  grid_dependency_wait();     // launched dependently itself: the previous kernel's results are complete from here on
+  grid_dependency_launch();   // the successor may start now: in a decode step it is a projection that reads its weights first
+  grid_dependency_wait();     // the previous kernel's results are complete from here on
   const long long vec = (long long)blockIdx.x * blockDim.x + threadIdx.x;
   const int per = D / 8;
   if (vec >= (long long)B * H * rows * per) return;

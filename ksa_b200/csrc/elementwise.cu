@@ -829,8 +829,8 @@ KSA_API int ksa_rmsnorm_fwd(const void* x, const void* delta, const void* w, voi
               kNormThreads * 8 * kNormMaxVec);
   if (rows == 0) return 0;
   // A warp per row from 1024 rows on, about 7 warps an SM: 1024 x 2560 10.1 -> 6.7 us, 1411 x 1024 8.0 -> 4.6.  256 and 512 rows take 5 to
-  // 9 us back to back in both forms, most of it the launch, and stay with the wider CTA.  The vectors of both inputs have to fit a
-  // lane's registers, 10 of each, so rows above 2560 columns keep the CTA as well.
+  // 9 us back to back in both forms, most of it the launch, and stay with the wider CTA.  A lane holds the vectors of both inputs,
+  // 10 of each at 2560 columns (100 registers, no spills); a wider form was not measured, so wider rows keep the CTA as well.
   if (rows >= 1024 && D <= 2560) {
     auto kern = D <= 1024 ? rmsnorm_fwd_warp_kernel<4> : D <= 2048 ? rmsnorm_fwd_warp_kernel<8> : rmsnorm_fwd_warp_kernel<10>;
     KSA_CHECK_CUDA(launch_stream_kernel(8LL * rows * D, kern, dim3((rows + 3) / 4), dim3(128), 0, ST(stream), (const bf16*)x,
