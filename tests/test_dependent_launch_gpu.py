@@ -1,4 +1,6 @@
 """Kernels start while their predecessor on the stream still runs: whatever one writes, the next one reads, weights included."""
+import threading
+
 import pytest
 import torch
 
@@ -81,4 +83,26 @@ def test_a_decode_step_sees_the_weights_of_the_kernel_before(writer):
         want = steps(torch.cuda.synchronize)
         for _ in range(3):
             assert torch.equal(steps(lambda: None), want)
+    _lib.check_status()
+
+
+def test_products_beside_a_decode_step_wait_for_their_weights():
+    """Early weights belong to the thread that runs a decode step: products of other threads, of up to 16 rows as well, wait."""
+    with torch.no_grad():
+        x, a, b, norm = _n(3, 512), _n(8, 512, 512, std=0.05), _n(512, 512, std=0.05), _n(512)
+        want = _chain(x, a, b, norm, torch.cuda.synchronize)
+        got = []
+
+        def other():
+            with torch.no_grad():
+                got.extend(_chain(x, a, b, norm, lambda: None) for _ in range(5))
+        before = _lib.set_dependent_launch(_lib.EARLY_WEIGHTS)
+        try:
+            t = threading.Thread(target=other)
+            t.start()
+            t.join()
+        finally:
+            _lib.set_dependent_launch(before)
+        torch.cuda.synchronize()
+        assert len(got) == 5 and all(torch.equal(g, w) for run in got for g, w in zip(run, want))
     _lib.check_status()
