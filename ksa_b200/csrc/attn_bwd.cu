@@ -131,7 +131,7 @@ attn_bwd_dq_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constan
   const uint32_t tS = tmem_base, tdP = tmem_base + 128, tdQ = tmem_base + 256;
 
   if (warp == 0) {
-    if (lane == 0) {
+    if (elect_one()) {
       mbar_expect_tx(q_full, 2 * S::kTile);
       load_tile_b<HD>(sQ, &tmQ, q_tile * 128, head, b, q_full);
       load_tile_b<HD>(sdO, &tmdO, q_tile * 128, head, b, q_full);
@@ -148,7 +148,7 @@ attn_bwd_dq_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constan
       }
     }
   } else if (warp == 1) {
-    if (lane == 0) {
+    if (elect_one()) {
       // The 128 keys of a tile are handled as two halves of 64 (one per softmax warpgroup), software-pipelined:
       // while a warpgroup turns the scores of its half into dS, the tensor pipe runs the other half's dQ update and
       // the next tile's S / dP for the half that has just been consumed.  tcgen05 MMAs issued by one thread execute
@@ -354,7 +354,7 @@ attn_bwd_dkv_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_consta
   const uint32_t tS = tmem_base, tdP = tmem_base + 128, tdV = tmem_base + 256, tdK = tmem_base + 256 + HD;
 
   if (warp == 0) {
-    if (lane == 0 && total > 0) {
+    if (total > 0 && elect_one()) {
       mbar_expect_tx(kv_full, 2 * S::kTile);
       load_tile_b<HD>(sK, is_sum ? &tmKs : &tmK, kt * 128, kv_head, b, kv_full);
       load_tile_b<HD>(sV, is_sum ? &tmVs : &tmV, kt * 128, kv_head, b, kv_full);
@@ -369,7 +369,7 @@ attn_bwd_dkv_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_consta
       }
     }
   } else if (warp == 1) {
-    if (lane == 0 && total > 0) {
+    if (total > 0 && elect_one()) {
       // Same software pipeline as the dQ kernel, over the two halves of 64 query columns: warpgroup h turns
       // S^T / dP^T of its half into P^T / dS^T while the tensor pipe updates dV / dK with the other half and computes
       // the next step's scores for the half that has just been consumed.

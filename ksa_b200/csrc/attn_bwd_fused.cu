@@ -231,7 +231,7 @@ __device__ __forceinline__ void attn_bwd_fused_body(const CUtensorMap& tmQ, cons
 
   if (warp == 0) {
     // ------------------------------------------------------------------ TMA producer
-    if (lane == 0 && total > 0) {
+    if (total > 0 && elect_one()) {
       const CUtensorMap* mk = is_sum ? &tmKs : &tmK;
       const CUtensorMap* mv = is_sum ? &tmVs : &tmV;
       bool src_ok = true;
@@ -268,7 +268,7 @@ __device__ __forceinline__ void attn_bwd_fused_body(const CUtensorMap& tmQ, cons
     }
   } else if (warp == 1) {
     // ------------------------------------------------------------------ MMA issuer
-    if (lane == 0 && total > 0) {
+    if (total > 0 && elect_one()) {
       constexpr uint32_t idesc_s = umma_idesc_bf16(128, 128, 0, 0);    // S^T, dP^T: all 128 queries of the step at once
       constexpr uint32_t idesc_acc = umma_idesc_bf16(128, 128, 0, 1);  // dV, dK: A from TMEM, B MN-major
       constexpr uint32_t idesc_dq = umma_idesc_bf16(128, 64, 1, 1);    // dQ^T_h: A = K^T, B = dS^T_h, both MN-major

@@ -127,7 +127,7 @@ __device__ __forceinline__ void attn_fwd_body(const CUtensorMap& tmQ, const CUte
     asm volatile("setmaxnreg.dec.sync.aligned.u32 56;");
     if (warp == 8) {
       // -------------------------------------------------------------- TMA producer
-      if (lane == 0) {
+      if (elect_one()) {
         int n = 0, it = 0;
         bool ok = true;
         uint32_t waited = 0;   // context parallel: sources whose flag has been seen (bit s: text, bit 2 + s: summary)
@@ -188,7 +188,7 @@ __device__ __forceinline__ void attn_fwd_body(const CUtensorMap& tmQ, const CUte
       }
     } else if (warp == 9) {
       // -------------------------------------------------------------- MMA issuer
-      if (lane == 0) {
+      if (elect_one()) {
         constexpr uint32_t idesc_s = umma_idesc_bf16(128, 128, 0, 0);
         constexpr uint32_t idesc_o = umma_idesc_bf16(128, HD, 0, 1);
         auto issue_s = [&](int t, int stage) {

@@ -89,7 +89,7 @@ gemm_narrow_kernel(const __grid_constant__ CUtensorMap tmW, const __grid_constan
   grid_dependency_enter();
 
   if (warp == 0) {
-    if (lane == 0) {
+    if (elect_one()) {
       int stage = 0;
       uint32_t phase = 0;
       for (int kb = kb0; kb < kb1; ++kb) {
@@ -109,7 +109,7 @@ gemm_narrow_kernel(const __grid_constant__ CUtensorMap tmW, const __grid_constan
     }
     __syncwarp();
   } else if (warp == 1) {
-    if (lane == 0) {
+    if (elect_one()) {
       const uint32_t idesc = umma_idesc_bf16(128, p.bt, W_MN ? 1 : 0, 0);
       int stage = 0;
       uint32_t phase = 0;
