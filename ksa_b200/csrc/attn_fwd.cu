@@ -7,19 +7,29 @@
 // O += P V products and the two softmax warpgroups ping-pong against the tensor
 // pipe.  Key tiles come from a closed-form range (attn_common.cuh): summary-key
 // tiles first, then the text-key tiles of the window up to the diagonal.
-// The grid is persistent: one CTA per SM walks the items (longest first) with
-// barrier phases that run on across items, so the loads and the first S product
-// of the next item overlap the epilogue of the current one.
+// The grid is persistent: one CTA per SM walks the items (longest first), and for the tensor cores their tiles are one
+// sequence: a slot's first S product of an item follows its last P V product of the one before, while the epilogue
+// warpgroup still reads the finished O.
 //
-//   warps 0-3   softmax + correction + epilogue for slot 0 (thread = query row)
-//   warps 4-7   the same for slot 1
-//   warp 8      TMA producer (Q once, then K_j / V_j through a 5-stage ring)
-//   warp 9      MMA issuer (one elected thread);  warps 10-11 only give their registers away
-// The three warpgroups re-divide the register file at entry (setmaxnreg): 224 registers per softmax thread, which
-// holds a whole 128-column score row without spilling, 56 for the producer / issuer warpgroup.
+//   warps 0-3    softmax + correction for slot 0 (thread = query row)
+//   warps 4-7    the same for slot 1
+//   warps 8-11   epilogue: O / l through shared memory to global, in whole 128-byte lines; LSE
+//   warp 12      TMA producer (per item Q of both slots; V_j and K_{j+1} as a pair, two pairs in flight)
+//   warp 13      MMA issuer (one elected thread);  warps 14-15 only give their registers away
 //
 // TMEM: S0 @0, S1 @128 (fp32 scores; P, packed bf16, overwrites S in place and is
 // the A operand of the second product), O0 @256, O1 @256+HD.
+//
+// What bounds it: products of 64 cycles each, 2048 cycles a tile of both slots, against about 3100 from one tile to the next: a slot's chain
+// (S product, scores from TMEM, maximum, exponentials, P to TMEM, P V product) is longer than the other slot's work covers, and each
+// wait of the issuer returns only when its queue of some six products has nearly run dry.  Under sustained load the card's power
+// limit comes first: 1.45 GHz at 990 W (the products alone, waiting for nothing, take 1640 us of the 1960 of 16384 causal tokens there).
+// An epilogue of its own instead of one in the softmax warps, S of the next item ahead of it, and pairs of tiles
+// (one wait and one commit a tile instead of two of each): 32768 summary-attention tokens (32 heads) 776 -> 728 us, 8192 (16 heads)
+// 98.3 -> 96.1, causal 8192 (16 heads) 265 -> 263, 16384 (32 heads) 1980 -> 1967; a single item per SM (2 x 700 tokens, 16 heads) 16.4 -> 16.8.
+// Slower, all with the same or nearly the same bits: two threads a row (1960 -> 2050), an issuer per slot (2110), exponentials
+// taken with the previous maximum while the tile's own is being found (2550), a warp that waits for the operands in the issuer's place (equal on
+// causal, 735 on summary attention).
 //
 // Bar: FlashAttentionForwardSm100 + block-sparse lists in the reference wheel
 // (flash_attn/cute/flash_fwd_sm100.py:68 in the flash_attn_cute wheel, summary_attn/interface.py:77-82 in the
@@ -30,15 +40,20 @@
 
 namespace ksa {
 
-constexpr int kFwdThreads = 384;
-constexpr int kKvStages = 5;
+constexpr int kFwdThreads = 512;
+constexpr int kOutPitch = 144;                // bytes of a staged row of 64 output columns
+// Registers a thread after setmaxnreg: 184 * 256 + 64 * 128 + 80 * 128 = 128 * 512, what the block is launched with.  (A score row of
+// 128 columns fits 184 without spilling; with 192 + 64 + 64 the issuer spilled, and a reload costs more there than anywhere else.)
+constexpr int kSoftmaxRegs = 184, kEpilogueRegs = 64, kIssueRegs = 80;
 template <int HD>
 struct FwdSmem {
   static constexpr int kTile = 128 * HD * 2;  // bytes of one 128-row tile
   static constexpr int kQ = 2 * kTile;
-  static constexpr int kRing = kKvStages * kTile;
+  static constexpr int kRing = 4 * kTile;     // two pairs: V of a tile, K of the next
+  static constexpr int kStat = 2 * 2 * 128 * 8;          // (max, sum) of every row: two slots, two items
+  static constexpr int kOut = 128 * kOutPitch;
   static constexpr int kBar = 256;
-  static constexpr int kTotal = kQ + kRing + kBar + 1024;
+  static constexpr int kTotal = kQ + kRing + kStat + kOut + kBar + 1024;
 };
 
 struct FwdParams {
@@ -67,16 +82,19 @@ __device__ __forceinline__ void attn_fwd_body(const CUtensorMap& tmQ, const CUte
   uint8_t* smem = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~uintptr_t(1023));
   uint8_t* sQ = smem;
   uint8_t* sKV = smem + S::kQ;
-  uint64_t* bars = reinterpret_cast<uint64_t*>(smem + S::kQ + S::kRing);
-  uint64_t* q_full = bars;                 // Q of the current work item has landed
-  uint64_t* q_empty = bars + 1;            // every S product of the item has read Q
-  uint64_t* kv_full = bars + 2;            // kKvStages
-  uint64_t* kv_empty = kv_full + kKvStages;
-  uint64_t* s_full = kv_empty + kKvStages;  // 2
-  uint64_t* p_full = s_full + 2;            // 4: slot t, keys 0-63 and 64-127 of the tile
-  uint64_t* o_full = p_full + 4;            // 2
-  uint64_t* o_free = o_full + 2;            // 2: the epilogue has copied O of the finished item into registers
-  uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(o_free + 2);
+  float2* sStat = reinterpret_cast<float2*>(sKV + S::kRing);       // [slot][item & 1][row]
+  uint8_t* sOut = sKV + S::kRing + S::kStat;
+  uint64_t* bars = reinterpret_cast<uint64_t*>(sOut + S::kOut);
+  uint64_t* q_full = bars;                 // 2: Q of the slot's current work item has landed
+  uint64_t* q_empty = q_full + 2;          // 2: every S product of the item has read it
+  uint64_t* kv_full = q_empty + 2;          // 2: V of a tile and K of the next one have landed
+  uint64_t* kv_empty = kv_full + 2;         // 2: all products of the pair have read it
+  uint64_t* s_full = kv_empty + 2;          // 2
+  uint64_t* p_full = s_full + 2;            // 4: slot t, first and last keys of the tile
+  uint64_t* o_full = p_full + 4;            // 2: the item's last product has been added to O
+  uint64_t* o_free = o_full + 2;            // 2: the epilogue has read O
+  uint64_t* l_full = o_free + 2;            // 4: slot t, item & 1: the item's row maxima and sums are in shared memory
+  uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(l_full + 4);
   volatile int* abort_flag = reinterpret_cast<volatile int*>(tmem_slot + 1);
 
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
@@ -101,34 +119,50 @@ __device__ __forceinline__ void attn_fwd_body(const CUtensorMap& tmQ, const CUte
     b = r / n_groups;
     head0 = (r - b * n_groups) * heads_per_cta;
   };
+  // key tiles of the next item at or after round k that has any; 0 when there is none left
+  auto next_item = [&](int& k) {
+    for (; k < n_rounds; ++k) {
+      const int item = item_of_round(k);
+      if (item >= n_items) continue;
+      int q_tile, head0, b;
+      decode(item, q_tile, head0, b);
+      const int total = key_tiles_for_query_tile(sh, q_tile, b).total();
+      if (total > 0) return total;
+    }
+    return 0;
+  };
 
   if (threadIdx.x == 0) {
-    mbar_init(q_full, 1);
-    mbar_init(q_empty, 1);
-    for (int i = 0; i < kKvStages; ++i) { mbar_init(&kv_full[i], 1); mbar_init(&kv_empty[i], 1); }
+    for (int i = 0; i < 2; ++i) { mbar_init(&kv_full[i], 2); mbar_init(&kv_empty[i], 1); }
     for (int i = 0; i < 2; ++i) {
+      mbar_init(&q_full[i], 1);
+      mbar_init(&q_empty[i], 1);
       mbar_init(&s_full[i], 1);
       mbar_init(&p_full[2 * i], 128);
       mbar_init(&p_full[2 * i + 1], 128);
       mbar_init(&o_full[i], 1);
-      mbar_init(&o_free[i], 128);
+      mbar_init(&o_free[i], 4);
+      mbar_init(&l_full[2 * i], 4);
+      mbar_init(&l_full[2 * i + 1], 4);
     }
     *abort_flag = 0;
     fence_mbar_init();
   }
-  if (warp == 8) { tmem_alloc(tmem_slot, 512); tmem_relinquish(); }
+  if (warp == 12) { tmem_alloc(tmem_slot, 512); tmem_relinquish(); }
   tc_fence_before();
   __syncthreads();
   tc_fence_after();
   const uint32_t tmem_base = *tmem_slot;
   if (!kCp) grid_dependency_enter();     // the context-parallel form waits for other GPUs: see grid_dependency_enter
 
-  if (warp >= 8) {
-    asm volatile("setmaxnreg.dec.sync.aligned.u32 56;");
-    if (warp == 8) {
+  if (warp >= 12) {
+    asm volatile("setmaxnreg.dec.sync.aligned.u32 %0;" ::"n"(kIssueRegs));
+    if (warp == 12) {
       // -------------------------------------------------------------- TMA producer
       if (elect_one()) {
-        int n = 0, it = 0;
+        // Tiles travel in pairs, V of one with K of the next (of all items in one sequence); the first pair has only K.
+        int it = 0;
+        uint32_t pair = 0;
         bool ok = true;
         uint32_t waited = 0;   // context parallel: sources whose flag has been seen (bit s: text, bit 2 + s: summary)
         for (int k = 0; k < n_rounds && ok; ++k) {
@@ -139,21 +173,8 @@ __device__ __forceinline__ void attn_fwd_body(const CUtensorMap& tmQ, const CUte
           const int kv_head = head0 / (sh.Hq / sh.Hkv);
           const TileRange tr = key_tiles_for_query_tile(sh, q_tile, b);
           const int total = tr.total();
-          // Q can only be replaced once the previous item's last S product has read it; the first K / V tiles of
-          // this item do not have to wait for that, so they are requested first and cross the item boundary in flight
-          bool q_loaded = false;
-          auto load_q = [&]() {
-            if (it > 0 && !mbar_wait(q_empty, (it - 1) & 1, guard, kTimeoutStageEmpty)) return false;
-            ++it;
-            mbar_expect_tx(q_full, heads_per_cta * S::kTile);
-            for (int t = 0; t < heads_per_cta; ++t)
-              load_tile<HD>(sQ + t * S::kTile, &tmQ, q_tile * 128, head0 + t, b, q_full);
-            q_loaded = true;
-            return true;
-          };
-          if (it == 0 && !load_q()) break;
+          if (total == 0) continue;
           for (int j = 0; j < total && ok; ++j) {
-            if (!q_loaded && j == 2 && !load_q()) { ok = false; break; }
             const bool is_sum = j < tr.n_sum_tiles;
             const int kt = is_sum ? j : tr.text_first + (j - tr.n_sum_tiles);
             const CUtensorMap* mk = is_sum ? &tmKs : &tmK;
@@ -175,95 +196,177 @@ __device__ __forceinline__ void attn_fwd_body(const CUtensorMap& tmQ, const CUte
                 waited |= bit;
               }
             }
-            for (int kv = 0; kv < 2; ++kv, ++n) {
-              const int stage = n % kKvStages;
-              const uint32_t phase = (n / kKvStages) & 1;
-              if (!mbar_wait(&kv_empty[stage], phase ^ 1, guard, kTimeoutStageEmpty)) { ok = false; break; }
-              mbar_expect_tx(&kv_full[stage], S::kTile);
-              load_tile<HD>(sKV + stage * S::kTile, kv == 0 ? mk : mv, row, kv_head, b, &kv_full[stage]);
+            if (pair == 0) {
+              mbar_arrive(&kv_full[0]);
             }
+            mbar_expect_tx(&kv_full[pair & 1], S::kTile);
+            load_tile<HD>(sKV + ((pair & 1) * 2 + 1) * S::kTile, mk, row, kv_head, b, &kv_full[pair & 1]);
+            // a slot's Q is replaced once the previous item's last S product has read it
+            if (j == 0) {
+              for (int t = 0; t < heads_per_cta && ok; ++t) {
+                if (!mbar_wait(&q_empty[t], (it & 1) ^ 1, guard, kTimeoutStageEmpty)) { ok = false; break; }
+                mbar_expect_tx(&q_full[t], S::kTile);
+                load_tile<HD>(sQ + t * S::kTile, &tmQ, q_tile * 128, head0 + t, b, &q_full[t]);
+              }
+              if (!ok) break;
+            }
+            ++pair;
+            if (!mbar_wait(&kv_empty[pair & 1], ((pair >> 1) & 1) ^ 1, guard, kTimeoutStageEmpty)) { ok = false; break; }
+            mbar_expect_tx(&kv_full[pair & 1], S::kTile);
+            load_tile<HD>(sKV + (pair & 1) * 2 * S::kTile, mv, row, kv_head, b, &kv_full[pair & 1]);
           }
-          if (ok && !q_loaded && !load_q()) ok = false;
+          ++it;
         }
+        if (ok && it > 0) mbar_arrive(&kv_full[pair & 1]);      // the last pair has no K
       }
-    } else if (warp == 9) {
+    } else if (warp == 13) {
       // -------------------------------------------------------------- MMA issuer
       if (elect_one()) {
         constexpr uint32_t idesc_s = umma_idesc_bf16(128, 128, 0, 0);
         constexpr uint32_t idesc_o = umma_idesc_bf16(128, HD, 0, 1);
-        auto issue_s = [&](int t, int stage) {
-          const uint32_t qa = smem_u32(sQ + t * S::kTile), ka = smem_u32(sKV + stage * S::kTile);
+        const uint64_t q_desc = smem_desc_kmajor_sw128(smem_u32(sQ)), k_desc = smem_desc_kmajor_sw128(smem_u32(sKV) + S::kTile);
+        const uint64_t v_desc = smem_desc_mnmajor_sw128(smem_u32(sKV), 16384);
+        auto issue_s = [&](int t, uint32_t pair) {
+          const uint64_t qd = q_desc + t * (S::kTile >> 4), kd = k_desc + (pair & 1) * (S::kTile >> 3);
 #pragma unroll
           for (int kk = 0; kk < HD / 16; ++kk) {
-            const uint32_t off = (kk / 4) * 16384 + (kk % 4) * 32;
-            umma_ss(tmem_base + t * 128, smem_desc_kmajor_sw128(qa + off), smem_desc_kmajor_sw128(ka + off), idesc_s,
-                    kk != 0);
+            const uint32_t off = ((kk / 4) * 16384 + (kk % 4) * 32) >> 4;
+            umma_ss(tmem_base + t * 128, qd + off, kd + off, idesc_s, kk != 0);
           }
           umma_commit(&s_full[t]);
         };
-        int n0 = 0;    // ring slots used by earlier items
-        int g = 0;     // key tiles of earlier items (phase of s_full / p_full / o_full)
-        int it = 0, it_o = 0;   // items seen; items that produced an output tile
-        bool ok = true;
-        for (int k = 0; k < n_rounds && ok; ++k) {
-          const int item = item_of_round(k);
-          if (item >= n_items) continue;
-          int q_tile, head0, b;
-          decode(item, q_tile, head0, b);
-          const int total = key_tiles_for_query_tile(sh, q_tile, b).total();
-          ok = mbar_wait(q_full, it & 1, guard, kTimeoutTmaFull);
-          if (ok && total > 0) {
-            ok = mbar_wait(&kv_full[n0 % kKvStages], (n0 / kKvStages) & 1, guard, kTimeoutTmaFull);
-            if (ok) {
-              tc_fence_after();
-              for (int t = 0; t < heads_per_cta; ++t) issue_s(t, n0 % kKvStages);
-              umma_commit(&kv_empty[n0 % kKvStages]);
-            }
+        // One sequence of key tiles over all items: a slot's S product of tile i + 1 follows its P V product of tile i, whether
+        // both belong to one item or not.
+        int round = 0, total = next_item(round);
+        bool ok = total > 0;
+        if (ok) {
+          ok = mbar_wait(&kv_full[0], 0, guard, kTimeoutTmaFull);
+          for (int t = 0; t < heads_per_cta && ok; ++t) {
+            ok = mbar_wait(&q_full[t], 0, guard, kTimeoutTmaFull);
+            if (!ok) break;
+            tc_fence_after();
+            issue_s(t, 0);
+            if (total == 1) umma_commit(&q_empty[t]);
           }
-          for (int j = 0; j < total && ok; ++j) {
-            const int nv = n0 + 2 * j + 1, nk = n0 + 2 * j + 2;
-            const int st_v = nv % kKvStages, st_k = nk % kKvStages;
-            if (!mbar_wait(&kv_full[st_v], (nv / kKvStages) & 1, guard, kTimeoutTmaFull)) { ok = false; break; }
-            const bool more = (j + 1 < total);
-            for (int t = 0; t < heads_per_cta && ok; ++t) {
-              if (!mbar_wait(&p_full[2 * t], (g + j) & 1, guard, kTimeoutSoftmax)) { ok = false; break; }
-              // the first product of an item overwrites O: the previous item's epilogue must have read it
-              if (j == 0 && it_o > 0 && !mbar_wait(&o_free[t], (it_o - 1) & 1, guard, kTimeoutSoftmax)) { ok = false; break; }
-              tc_fence_after();
-              const uint32_t va = smem_u32(sKV + st_v * S::kTile);
+          if (ok) umma_commit(&kv_empty[0]);
+        }
+        bool first = true;
+        int j = 0;
+        uint32_t it = 0;
+        for (uint32_t step = 0; ok; ++step) {
+          const uint32_t pair = step + 1;
+          const bool last = j + 1 == total;
+          if (last) {
+            ++round;
+            total = next_item(round);
+            j = -1;
+          }
+          if (!mbar_wait(&kv_full[pair & 1], (pair >> 1) & 1, guard, kTimeoutTmaFull)) break;
+          for (int t = 0; t < heads_per_cta; ++t) {
+            // the next item's S product follows: its Q is there
+            if (last && total > 0 && !mbar_wait(&q_full[t], (it + 1) & 1, guard, kTimeoutTmaFull)) { ok = false; break; }
+            // the first product of an item overwrites O: the previous item's epilogue must have read it
+            if (first && it > 0 && !mbar_wait(&o_free[t], (it - 1) & 1, guard, kTimeoutSoftmax)) { ok = false; break; }
+            if (!mbar_wait(&p_full[2 * t], step & 1, guard, kTimeoutSoftmax)) { ok = false; break; }
+            tc_fence_after();
+            const uint64_t vd = v_desc + (pair & 1) * (S::kTile >> 3);
+            const uint32_t tS = tmem_base + t * 128, tO = tmem_base + 256 + t * HD;
 #pragma unroll
-              for (int kk = 0; kk < 8; ++kk) {
-                if (kk == 4) {
-                  if (!mbar_wait(&p_full[2 * t + 1], (g + j) & 1, guard, kTimeoutSoftmax)) { ok = false; break; }
-                  tc_fence_after();
-                }
-                umma_ts(tmem_base + 256 + t * HD, tmem_base + t * 128 + kk * 8,
-                        smem_desc_mnmajor_sw128(va + kk * 2048, 16384), idesc_o, (j | kk) != 0);
-              }
-              if (!ok) break;
-              umma_commit(&o_full[t]);
-              if (more) {
-                if (t == 0 && !mbar_wait(&kv_full[st_k], (nk / kKvStages) & 1, guard, kTimeoutTmaFull)) { ok = false; break; }
-                tc_fence_after();
-                issue_s(t, st_k);
-              }
-            }
-            if (ok) {
-              umma_commit(&kv_empty[st_v]);
-              if (more) umma_commit(&kv_empty[st_k]);
+            for (int kk = 0; kk < 4; ++kk) umma_ts(tO, tS + kk * 8, vd + kk * 128, idesc_o, !first || kk != 0);
+            if (!mbar_wait(&p_full[2 * t + 1], step & 1, guard, kTimeoutSoftmax)) { ok = false; break; }
+            tc_fence_after();
+#pragma unroll
+            for (int kk = 4; kk < 8; ++kk) umma_ts(tO, tS + kk * 8, vd + kk * 128, idesc_o, 1);
+            if (last) umma_commit(&o_full[t]);
+            if (total > 0) {
+              issue_s(t, pair);
+              if (j + 2 == total) umma_commit(&q_empty[t]);
             }
           }
-          if (ok) umma_commit(q_empty);   // fires when the S products issued so far have read Q
-          n0 += 2 * total;
-          g += total;
-          if (total > 0) ++it_o;
-          ++it;
+          if (!ok || total == 0) break;
+          umma_commit(&kv_empty[pair & 1]);
+          first = last;
+          if (last) ++it;
+          ++j;
         }
       }
     }
+  } else if (warp >= 8) {
+    asm volatile("setmaxnreg.dec.sync.aligned.u32 %0;" ::"n"(kEpilogueRegs));
+    // ---------------------------------------------------------------- epilogue: O / l -> global, LSE
+    const int quad = warp & 3;
+    const int r = quad * 32 + lane;
+    uint8_t* stage = sOut + quad * 32 * kOutPitch;
+    int it = 0;
+    bool ok = true;
+    for (int k = 0; k < n_rounds && ok; ++k) {
+      const int item = item_of_round(k);
+      if (item >= n_items) continue;
+      int q_tile, head0, b;
+      decode(item, q_tile, head0, b);
+      const int total = key_tiles_for_query_tile(sh, q_tile, b).total();
+      if (total > 0) {
+        int next = k + 1;
+        if (next_item(next) == 0) continue;        // the last one: see below
+      }
+      const int q0 = q_tile * 128 + quad * 32, rows = min(32, sh.Lq - q0);       // rows of this warp, <= 0 past the end
+      for (int t = 0; t < heads_per_cta; ++t) {
+        const int head = head0 + t;
+        bf16* dst = p.o + (long long)b * p.o_batch_stride + (long long)q0 * p.o_row_stride + (long long)head * HD;
+        float m = 0.f, l = 0.f;
+        if (total > 0) {
+          if (!mbar_wait(&l_full[2 * t + (it & 1)], (it >> 1) & 1, guard, kTimeoutSoftmax)) { ok = false; break; }
+          const float2 ml = sStat[(t * 2 + (it & 1)) * 128 + r];
+          m = ml.x;
+          l = ml.y;
+          if (!mbar_wait(&o_full[t], it & 1, guard, kTimeoutAccFull)) { ok = false; break; }
+          tc_fence_after();
+        }
+        const float inv = l > 0.f ? 1.f / l : 0.f;
+        const uint32_t tO = tmem_base + ((uint32_t)(quad * 32) << 16) + 256 + t * HD;
+#pragma unroll
+        for (int h = 0; h < HD / 64; ++h) {
+#pragma unroll
+          for (int c = 0; c < 4; ++c) {
+            uint32_t o[16];
+            if (total > 0) {
+              tmem_ld16(tO + h * 64 + c * 16, o);
+              tmem_wait_ld();
+            } else {
+#pragma unroll
+              for (int i = 0; i < 16; ++i) o[i] = 0;
+            }
+#pragma unroll
+            for (int i = 0; i < 16; i += 8) {
+              uint4 v;
+              v.x = pack_bf16x2(__uint_as_float(o[i]) * inv, __uint_as_float(o[i + 1]) * inv);
+              v.y = pack_bf16x2(__uint_as_float(o[i + 2]) * inv, __uint_as_float(o[i + 3]) * inv);
+              v.z = pack_bf16x2(__uint_as_float(o[i + 4]) * inv, __uint_as_float(o[i + 5]) * inv);
+              v.w = pack_bf16x2(__uint_as_float(o[i + 6]) * inv, __uint_as_float(o[i + 7]) * inv);
+              *reinterpret_cast<uint4*>(stage + lane * kOutPitch + c * 32 + i * 2) = v;
+            }
+          }
+          if (h == HD / 64 - 1) tc_fence_before();
+          __syncwarp();
+          if (h == HD / 64 - 1 && lane == 0 && total > 0) mbar_arrive(&o_free[t]);
+#pragma unroll 2
+          for (int i = 0; i < 8; ++i) {
+            const int row = i * 4 + (lane >> 3);
+            if (row < rows)
+              *reinterpret_cast<uint4*>(dst + row * p.o_row_stride + h * 64 + (lane & 7) * 8) =
+                  *reinterpret_cast<const uint4*>(stage + row * kOutPitch + (lane & 7) * 16);
+          }
+          __syncwarp();
+        }
+        if (lane < rows && p.lse)
+          p.lse[((long long)b * sh.Hq + head) * sh.Lq + q0 + lane] =
+              (l > 0.f) ? (m + log2f(l)) * 0.6931471805599453f : -INFINITY;
+      }
+      if (total > 0) ++it;
+    }
   } else {
-    asm volatile("setmaxnreg.inc.sync.aligned.u32 224;");
-    // ---------------------------------------------------------------- softmax / correction / epilogue
+    asm volatile("setmaxnreg.inc.sync.aligned.u32 %0;" ::"n"(kSoftmaxRegs));
+    // ---------------------------------------------------------------- softmax and rescaling
     const int t = warp >> 2;  // slot
     if (t < heads_per_cta) {
       const int quad = warp & 3;
@@ -271,7 +374,8 @@ __device__ __forceinline__ void attn_fwd_body(const CUtensorMap& tmQ, const CUte
       const uint32_t lane_addr = (uint32_t)(quad * 32) << 16;
       const uint32_t tS = tmem_base + lane_addr + t * 128;
       const uint32_t tO = tmem_base + lane_addr + 256 + t * HD;
-      int g = 0;
+      uint32_t step = 0;
+      int it = 0;
       bool ok = true;
       for (int k = 0; k < n_rounds && ok; ++k) {
         const int item = item_of_round(k);
@@ -280,18 +384,19 @@ __device__ __forceinline__ void attn_fwd_body(const CUtensorMap& tmQ, const CUte
         decode(item, q_tile, head0, b);
         const TileRange tr = key_tiles_for_query_tile(sh, q_tile, b);
         const int total = tr.total();
+        if (total == 0) continue;
         const int q_local = q_tile * 128 + r;
         const int t_glob = sh.q_off + q_local;
         float m_run = -INFINITY, l_run = 0.f;
         const int doc_start = (sh.q_doc_start && q_local < sh.Lq) ? sh.q_doc_start[(long long)b * sh.Lq + q_local] : 0;
-        for (int j = 0; j < total; ++j) {
+        for (int j = 0; j < total; ++j, ++step) {
           // what this row may see of the tile does not depend on the scores: worked out before they arrive
           const bool is_sum = j < tr.n_sum_tiles;
           const int kt = is_sum ? j : tr.text_first + (j - tr.n_sum_tiles);
           int lo, hi;
           allowed_columns(sh, t_glob, is_sum, kt, lo, hi, doc_start);
           const bool row_masked = lo > 0 || hi < 127;
-          if (!mbar_wait(&s_full[t], (g + j) & 1, guard, kTimeoutAccFull)) { ok = false; break; }
+          if (!mbar_wait(&s_full[t], step & 1, guard, kTimeoutAccFull)) { ok = false; break; }
           tc_fence_after();
           uint32_t sreg[4][32];
 #pragma unroll
@@ -306,32 +411,28 @@ __device__ __forceinline__ void attn_fwd_body(const CUtensorMap& tmQ, const CUte
                 if (col < lo || col > hi) sreg[c][i] = 0xff800000u;  // -inf; its exponential is an exact 0
               }
           }
-          float mx0 = -INFINITY, mx1 = -INFINITY;
+          float mx[4] = {-INFINITY, -INFINITY, -INFINITY, -INFINITY};
 #pragma unroll
-          for (int c = 0; c < 4; ++c)
+          for (int i = 0; i < 32; i += 2)
 #pragma unroll
-            for (int i = 0; i < 32; i += 4) {
-              mx0 = max3(mx0, __uint_as_float(sreg[c][i]), __uint_as_float(sreg[c][i + 1]));
-              mx1 = max3(mx1, __uint_as_float(sreg[c][i + 2]), __uint_as_float(sreg[c][i + 3]));
-            }
-          const float mx = fmaxf(mx0, mx1) * p.scale_log2;  // scale > 0
-          const float m_new = fmaxf(m_run, mx);
+            for (int c = 0; c < 4; ++c)
+              mx[c] = max3(mx[c], __uint_as_float(sreg[c][i]), __uint_as_float(sreg[c][i + 1]));
+          const float m_new = fmaxf(m_run, fmaxf(max3(mx[0], mx[1], mx[2]), mx[3]) * p.scale_log2);  // scale > 0
           if (j == 0) {
             m_run = m_new;
           } else {
+            // O is complete up to the previous tile: its product was issued before the S product that has just arrived
             const bool need = m_new > m_run + 8.f;
             if (__any_sync(0xffffffffu, need)) {
-              if (!mbar_wait(&o_full[t], (g + j - 1) & 1, guard, kTimeoutAccFull)) { ok = false; break; }
-              tc_fence_after();
               const float alpha = need ? fast_exp2(m_run - m_new) : 1.f;
-#pragma unroll
-              for (int c = 0; c < HD / 32; ++c) {
-                uint32_t o[32];
-                tmem_ld32(tO + c * 32, o);
+#pragma unroll 1
+              for (int c = 0; c < HD / 16; ++c) {
+                uint32_t o[16];
+                tmem_ld16(tO + c * 16, o);
                 tmem_wait_ld();
 #pragma unroll
-                for (int i = 0; i < 32; ++i) o[i] = __float_as_uint(__uint_as_float(o[i]) * alpha);
-                tmem_st32(tO + c * 32, o);
+                for (int i = 0; i < 16; ++i) o[i] = __float_as_uint(__uint_as_float(o[i]) * alpha);
+                tmem_st16(tO + c * 16, o);
               }
               tmem_wait_st();
               l_run *= alpha;
@@ -342,7 +443,7 @@ __device__ __forceinline__ void attn_fwd_body(const CUtensorMap& tmQ, const CUte
           const uint64_t sc2 = f2_pack(p.scale_log2, p.scale_log2), nm2 = f2_pack(-m_use, -m_use);
           uint64_t acc0 = f2_pack(0.f, 0.f), acc1 = acc0;
           // P = 2^(S * scale - m) -> bf16 over the first half of the columns of S; the product P V starts on the
-          // first 64 keys while the exponentials of the other 64 are still being computed
+          // first keys while the exponentials of the others are still being computed
 #pragma unroll
           for (int c = 0; c < 4; ++c) {
             uint32_t pk[16];
@@ -368,48 +469,47 @@ __device__ __forceinline__ void attn_fwd_body(const CUtensorMap& tmQ, const CUte
           l_run += lsum + l1;
         }
         if (!ok) break;
-        // epilogue: copy O into registers, hand the accumulator back, then O / l -> global and LSE
-        const bool valid = q_local < sh.Lq;
+        int next = k + 1;
+        if (next_item(next) > 0) {
+          sStat[(t * 2 + (it & 1)) * 128 + r] = make_float2(m_run, l_run);
+          __syncwarp();
+          if (lane == 0) mbar_arrive(&l_full[2 * t + (it & 1)]);
+          ++it;
+          continue;
+        }
+        // The last item: nothing is left to overlap the epilogue with, so both slots' warps write their rows at the same time.
+        if (!mbar_wait(&o_full[t], it & 1, guard, kTimeoutAccFull)) break;
+        tc_fence_after();
+        const float inv = l_run > 0.f ? 1.f / l_run : 0.f;
         const int head = head0 + t;
         bf16* dst = p.o + (long long)b * p.o_batch_stride + (long long)q_local * p.o_row_stride + (long long)head * HD;
-        if (total > 0) {
-          if (!mbar_wait(&o_full[t], (g + total - 1) & 1, guard, kTimeoutAccFull)) { ok = false; break; }
-          tc_fence_after();
-          uint32_t o[HD / 32][32];
+        uint32_t o[HD / 32][32];
 #pragma unroll
-          for (int c = 0; c < HD / 32; ++c) tmem_ld32(tO + c * 32, o[c]);
-          tmem_wait_ld();
-          tc_fence_before();
-          mbar_arrive(&o_free[t]);
-          const float inv = l_run > 0.f ? 1.f / l_run : 0.f;
-          if (valid) {
+        for (int c = 0; c < HD / 32; ++c) tmem_ld32(tO + c * 32, o[c]);
+        tmem_wait_ld();
+        if (q_local < sh.Lq) {
 #pragma unroll
-            for (int c = 0; c < HD / 32; ++c)
+          for (int c = 0; c < HD / 32; ++c)
 #pragma unroll
-              for (int i = 0; i < 32; i += 8) {
-                uint4 v;
-                v.x = pack_bf16x2(__uint_as_float(o[c][i]) * inv, __uint_as_float(o[c][i + 1]) * inv);
-                v.y = pack_bf16x2(__uint_as_float(o[c][i + 2]) * inv, __uint_as_float(o[c][i + 3]) * inv);
-                v.z = pack_bf16x2(__uint_as_float(o[c][i + 4]) * inv, __uint_as_float(o[c][i + 5]) * inv);
-                v.w = pack_bf16x2(__uint_as_float(o[c][i + 6]) * inv, __uint_as_float(o[c][i + 7]) * inv);
-                *reinterpret_cast<uint4*>(dst + c * 32 + i) = v;
-              }
-          }
-        } else if (valid) {
-#pragma unroll
-          for (int i = 0; i < HD; i += 8) *reinterpret_cast<uint4*>(dst + i) = make_uint4(0, 0, 0, 0);
+            for (int i = 0; i < 32; i += 8) {
+              uint4 v;
+              v.x = pack_bf16x2(__uint_as_float(o[c][i]) * inv, __uint_as_float(o[c][i + 1]) * inv);
+              v.y = pack_bf16x2(__uint_as_float(o[c][i + 2]) * inv, __uint_as_float(o[c][i + 3]) * inv);
+              v.z = pack_bf16x2(__uint_as_float(o[c][i + 4]) * inv, __uint_as_float(o[c][i + 5]) * inv);
+              v.w = pack_bf16x2(__uint_as_float(o[c][i + 6]) * inv, __uint_as_float(o[c][i + 7]) * inv);
+              *reinterpret_cast<uint4*>(dst + c * 32 + i) = v;
+            }
+          if (p.lse)
+            p.lse[((long long)b * sh.Hq + head) * sh.Lq + q_local] =
+                (l_run > 0.f) ? (m_run + log2f(l_run)) * 0.6931471805599453f : -INFINITY;
         }
-        if (valid && p.lse)
-          p.lse[((long long)b * sh.Hq + head) * sh.Lq + q_local] =
-              (l_run > 0.f) ? (m_run + log2f(l_run)) * 0.6931471805599453f : -INFINITY;
-        g += total;
       }
     }
   }
 
   tc_fence_before();
   __syncthreads();
-  if (warp == 8) {
+  if (warp == 12) {
     tc_fence_after();
     tmem_dealloc(tmem_base, 512);
   }
