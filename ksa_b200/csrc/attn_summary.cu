@@ -25,6 +25,7 @@ struct SumAttnArgs {
   int k_off;       // global text index of local text key row 0
   int s_off;       // global summary index of local summary key row 0
   float scale;
+  int beside;      // forward with a kernel of its own: launch_beside()
   // backward only
   const bf16* d_os; bf16* dqs; long long dqs_rs, dqs_bs;
   bf16* dk; bf16* dv; bf16* dks; bf16* dvs;
@@ -222,7 +223,7 @@ constexpr int kSumFwdMaxQ = 8;
 // us; four queries, 256 chunks: 97.1 -> 87.3 us).
 template <int HD, int NQ>
 __global__ void __launch_bounds__(kSumFwdThreads) summary_attn_fwd_fast_kernel(SumAttnArgs a, int nk_max) {
-  grid_dependency_enter();
+  grid_dependency_enter(a.beside);
   extern __shared__ uint32_t smw[];
   const int G = a.Hq / a.Hkv, S = a.n_sum, nq = NQ < kSumFwdMaxQ ? NQ : G * S;
   bf16* v_s = reinterpret_cast<bf16*>(smw);
@@ -335,6 +336,7 @@ __global__ void __launch_bounds__(kSumFwdThreads) summary_attn_fwd_fast_kernel(S
     *reinterpret_cast<uint32_t*>(a.os + (long long)b * a.os_bs + (long long)row * a.os_rs + (long long)head * HD + 2 * d2) =
         pack_bf16x2(o0, o1);
   }
+  grid_dependency_leave(a.beside);
 }
 
 // Backward fast path.  grid (local chunks, Hkv, B), 256 threads, head dim 128.  Only the chunk's K rows are staged
@@ -521,8 +523,8 @@ static int launch_fwd_fast(const SumAttnArgs& a, int nk_max, size_t smem, cudaSt
   auto kern = summary_attn_fwd_fast_kernel<128, NQ>;
   static PerDevice raised;
   KSA_CHECK_CUDA(raise_smem_limit(raised, kern, 100 * 1024));
-  KSA_CHECK_CUDA(launch_stream_kernel((long long)a.B * a.Hkv * (a.Nq / a.n_sum) * nk_max * 512, kern, dim3(a.Nq / a.n_sum,
-                                      a.Hkv, a.B), dim3(kSumFwdThreads), smem, st, a, nk_max));
+  const bool dependent = a.beside || (long long)a.B * a.Hkv * (a.Nq / a.n_sum) * nk_max * 512 <= kStreamedDependent;
+  KSA_CHECK_CUDA(launch_kernel_if(dependent, kern, dim3(a.Nq / a.n_sum, a.Hkv, a.B), dim3(kSumFwdThreads), smem, st, a, nk_max));
   return 0;
 }
 
@@ -560,6 +562,7 @@ KSA_API int ksa_summary_attn_fwd(const void* qs, const void* k, const void* v, c
     const int nq = (Hq / Hkv) * n_sum, nk_max = chunk + n_sum;
     const size_t fast_smem = (size_t)nk_max * HD * sizeof(bf16) + (size_t)nq * (HD + nk_max) * sizeof(float);
     if (HD == 128 && nq <= kSumFwdMaxQ && fast_smem <= 100 * 1024 && os_rs % 2 == 0) {
+      a.beside = launch_beside();
       cudaStream_t st = reinterpret_cast<cudaStream_t>(stream);
       if (nq == 1) return launch_fwd_fast<1>(a, nk_max, fast_smem, st);
       if (nq == 2) return launch_fwd_fast<2>(a, nk_max, fast_smem, st);

@@ -322,6 +322,15 @@ __device__ __forceinline__ void grid_dependency_enter() {
   grid_dependency_wait();
   grid_dependency_launch();
 }
+// The same for a kernel that may run beside the one before it (host.h: launch_beside): it waits only before it ends, in one block, so that
+// whoever waits for it has waited for both.  The other blocks leave and make room as they finish.
+__device__ __forceinline__ void grid_dependency_enter(int beside) {
+  if (!beside) grid_dependency_wait();
+  grid_dependency_launch();
+}
+__device__ __forceinline__ void grid_dependency_leave(int beside) {
+  if (beside && blockIdx.x == 0 && blockIdx.y == 0 && blockIdx.z == 0) grid_dependency_wait();
+}
 
 // ----------------------------------------------------------------- small helpers
 __device__ __forceinline__ uint32_t pack_bf16x2(float lo, float hi) {

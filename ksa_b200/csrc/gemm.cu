@@ -39,6 +39,7 @@ struct GemmEpilogue {
   int out_fp32;       // 0: bf16, 1: fp32
   int accumulate;     // 1: C += acc (fp32 output only)
   float alpha;        // scale applied to the accumulator
+  int beside;         // launch_beside()
 };
 
 template <int BN, bool A_MN, bool B_MN>
@@ -89,7 +90,7 @@ gemm_bf16_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant_
   __syncthreads();
   tc_fence_after();
   const uint32_t tmem_base = *tmem_slot;
-  grid_dependency_enter();
+  grid_dependency_enter(ep.beside);
 
   auto tile_coords = [&](int tile, int& mb, int& nb) {
     const int per_group = kGroupM * tiles_n;
@@ -229,6 +230,7 @@ gemm_bf16_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant_
     tc_fence_after();
     tmem_dealloc(tmem_base, 2 * BN);
   }
+  grid_dependency_leave(ep.beside);
 }
 
 // ----------------------------------------------------------------------------------------------
@@ -295,7 +297,7 @@ KSA_API int ksa_gemm_bf16(const void* a, const void* b, void* c, int M, int N, i
   KSA_REQUIRE(N % 8 == 0 && ldc % (out_fp32 ? 4 : 8) == 0, "gemm: N and ldc must keep 16-byte row alignment (N=%d ldc=%lld)", N, ldc);
   KSA_REQUIRE((reinterpret_cast<uintptr_t>(c) & 15) == 0, "gemm: C must be 16-byte aligned");
   KSA_REQUIRE(!(accumulate && !out_fp32), "gemm: accumulate needs an fp32 output");
-  GemmEpilogue ep{c, ldc, out_fp32, accumulate, alpha};
+  GemmEpilogue ep{c, ldc, out_fp32, accumulate, alpha, launch_beside()};
   cudaStream_t st = reinterpret_cast<cudaStream_t>(stream);
   const bool wide = (N >= 256) && (((long long)((M + 127) / 128) * ((N + 255) / 256)) >= 96 || N % 256 == 0);
 #define KSA_GEMM_DISPATCH(BN)                                                                        \

@@ -46,6 +46,7 @@ struct Gemm2Epilogue {
   long long ldc;
   int out_fp32, accumulate;
   float alpha;
+  int beside;                // launch_beside(); never in the communicating forms
   // GEMM -> reduce-scatter (bf16 output only): output row `row` belongs to rank row / c_shard_rows and is stored, from
   // the epilogue, straight into that rank's memory at c_peer[owner] + (row - owner * c_shard_rows) * ldc.
   int c_shard_rows;          // 0: every row goes to `c`
@@ -173,7 +174,7 @@ gemm2_bf16_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant
   cluster_sync_all();          // both CTAs' barriers are initialised before any remote arrival
   tc_fence_after();
   const uint32_t tmem_base = *tmem_slot;
-  if (!comm.active && ep.c_world <= 1) grid_dependency_enter();     // not in the communicating forms: see there
+  if (!comm.active && ep.c_world <= 1) grid_dependency_enter(ep.beside);     // not in the communicating forms: see there
 
   auto tile_coords = [&](int tile, int& mb, int& nb) {
     const int per_group = k2GroupM * tiles_n;
@@ -479,6 +480,7 @@ gemm2_bf16_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant
     tc_fence_after();
     tmem_dealloc2(tmem_base, 512);
   }
+  grid_dependency_leave(ep.beside);
 }
 
 static const ScatterMaps kNoScatterMaps{};
@@ -549,6 +551,7 @@ KSA_API int ksa_gemm2_bf16(const void* a, const void* b, void* c, int M, int N, 
   Gemm2Epilogue ep{};
   ep.c = c; ep.ldc = ldc; ep.out_fp32 = out_fp32; ep.accumulate = accumulate; ep.alpha = alpha;
   ep.c_tma = 1; ep.c_shard_rows = M; ep.c_world = 1; ep.c_peer[0] = c;
+  ep.beside = launch_beside();
   ScatterMaps smaps{};
   {
     const uint64_t elem = out_fp32 ? 4 : 2;

@@ -30,6 +30,7 @@ struct NarrowArgs {
   int M, N, K;               // N: rows of W
   int bt, split, stages, tiles_m, tmem_cols;
   float alpha;
+  int beside;                // launch_beside()
 };
 
 __device__ __forceinline__ uint32_t nw_cluster_rank() {
@@ -86,7 +87,7 @@ gemm_narrow_kernel(const __grid_constant__ CUtensorMap tmW, const __grid_constan
   __syncthreads();
   tc_fence_after();
   const uint32_t tmem_base = tmem_slot;
-  grid_dependency_enter();
+  grid_dependency_enter(p.beside);
 
   if (warp == 0) {
     if (elect_one()) {
@@ -194,6 +195,7 @@ gemm_narrow_kernel(const __grid_constant__ CUtensorMap tmW, const __grid_constan
     tc_fence_after();
     tmem_dealloc(tmem_base, p.tmem_cols);
   }
+  grid_dependency_leave(p.beside);
 }
 
 // Tile height and split for a product, and its time in microseconds as modelled.  The figures were fitted to 315 measured
@@ -351,6 +353,7 @@ KSA_API int ksa_gemm_narrow_bf16(const void* x, const void* w, void* c, int M, i
               "gemm_narrow: K = %d in %d parts", K, split);
   NarrowArgs p{};
   p.c = static_cast<bf16*>(c); p.ldc = ldc; p.M = M; p.N = N; p.K = K; p.bt = bt; p.split = split; p.alpha = alpha;
+  p.beside = launch_beside();
   cudaStream_t st = reinterpret_cast<cudaStream_t>(stream);
   if (glu) return launch_narrow<false, true>(x, w, p, ldx, ldw, st);
   return w_mn_major ? launch_narrow<true, false>(x, w, p, ldx, ldw, st) : launch_narrow<false, false>(x, w, p, ldx, ldw, st);

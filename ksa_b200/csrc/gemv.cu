@@ -76,7 +76,9 @@ __device__ __forceinline__ void multiply_sync() { asm volatile("bar.sync 1, %0;"
 // byte offset of columns 8 q .. 8 q + 7 (q < 8) of row r in a box of 128-byte rows with the 128-byte swizzle
 __device__ __forceinline__ uint32_t swizzled(int r, int q) { return (uint32_t)(r * 128 + ((q ^ (r & 7)) << 4)); }
 
-template <int NB, bool kGlu, bool kNorm>   // NB: batch blocks of 8 rows, 1 (M <= 8) or 2 (M <= 16)
+// NB: batch blocks of 8 rows, 1 (M <= 8) or 2 (M <= 16).  kBeside: launch_beside(); known to the compiler, since a decode step of four
+// sequences took 442 us instead of 420 with the conditions in the kernels that it launches.
+template <int NB, bool kGlu, bool kNorm, bool kBeside>
 __global__ void __launch_bounds__(kStThreads + 32, 2)
 stream_gemm_kernel(const __grid_constant__ CUtensorMap tmB, const __grid_constant__ CUtensorMap tmA, const StreamArgs p,
                    int* status) {
@@ -145,10 +147,10 @@ stream_gemm_kernel(const __grid_constant__ CUtensorMap tmB, const __grid_constan
       next(x);
     };
     // in a decode step weights do not depend on the previous kernel; the activations do
-    if (!p.early) grid_dependency_wait();
+    if (!kBeside && !p.early) grid_dependency_wait();
     const int ahead = min(p.stages, n_items);
     for (int it = 0; it < ahead; ++it) load_weights();
-    grid_dependency_wait();
+    if (!kBeside) grid_dependency_wait();
     for (int it = 0; it < ahead; ++it) load_acts();
     for (int it = ahead; it < n_items; ++it) {
       if (!__all_sync(0xffffffffu, mbar_wait(&empty[w.stage], w.phase, guard, kTimeoutStageEmpty))) break;
@@ -159,7 +161,7 @@ stream_gemm_kernel(const __grid_constant__ CUtensorMap tmB, const __grid_constan
   }
 
   // -------------------------------------------------------------- the eight warps that multiply
-  grid_dependency_wait();     // also for the outputs: an earlier kernel may still read their memory
+  if (!kBeside) grid_dependency_wait();     // also for the outputs: an earlier kernel may still read their memory
   if (kNorm) {
     float ss[4] = {0.f, 0.f, 0.f, 0.f};
     for (int c = threadIdx.x * 8; c < p.K; c += kStThreads * 8) {
@@ -316,9 +318,10 @@ stream_gemm_kernel(const __grid_constant__ CUtensorMap tmB, const __grid_constan
       multiply_sync();        // the next group's partial sums overwrite these
     }
   }
+  if (kBeside) grid_dependency_leave(1);
 }
 
-template <int NB, bool kGlu, bool kNorm>
+template <int NB, bool kGlu, bool kNorm, bool kBeside = false>
 static int launch_stream(StreamArgs p, const void* b, long long ldb, cudaStream_t st) {
   const int sms = sm_count();
   KSA_REQUIRE(sms > 0, "gemv: no device");
@@ -366,7 +369,7 @@ static int launch_stream(StreamArgs p, const void* b, long long ldb, cudaStream_
     uint32_t box[3] = {64, (uint32_t)p.M, (uint32_t)(p.ragged ? 1 : p.boxes)};
     if ((rc = make_tmap(&tmA, p.A, 2, 3, dims, str, box, true))) return rc;
   }
-  auto kern = stream_gemm_kernel<NB, kGlu, kNorm>;
+  auto kern = stream_gemm_kernel<NB, kGlu, kNorm, kBeside>;
   static PerDevice raised;
   KSA_CHECK_CUDA(raise_smem_limit(raised, kern, kStSmemMost));
   KSA_CHECK_CUDA(launch_kernel(kern, dim3(grid), dim3(kStThreads + 32), (size_t)smem, st, tmB, tmA,
@@ -390,7 +393,7 @@ __device__ __forceinline__ uint4 ld_stream_16(const void* p) {
   return v;
 }
 
-template <int MT, int R, bool kGlu>
+template <int MT, int R, bool kGlu, bool kBeside>
 __global__ void __launch_bounds__(kGemvThreads)
 gemv_kernel(const bf16* A, const bf16* B, bf16* C, int M, int N, int K,
             long long lda, long long ldb, long long ldc, int early) {
@@ -426,10 +429,9 @@ gemv_kernel(const bf16* A, const bf16* B, bf16* C, int M, int N, int K,
   };
   // in a decode step weights are not written by an earlier kernel of the stream: ask for the first chunks, then wait for the
   // kernel that produces the activations
-  if (!early) grid_dependency_wait();
+  if (!kBeside && !early) grid_dependency_wait();
   load_w(0, min(kGemvKTile, K), lane * 8);
-  grid_dependency_wait();
-  grid_dependency_launch();
+  grid_dependency_enter((int)kBeside);
 
   for (int k0 = 0; k0 < K; k0 += kGemvKTile) {
     const int kt = min(kGemvKTile, K - k0);          // multiple of 8
@@ -488,15 +490,16 @@ gemv_kernel(const bf16* A, const bf16* B, bf16* C, int M, int N, int K,
       }
     }
   }
+  if (kBeside) grid_dependency_leave(1);
 }
 
-template <int MT, int R, bool kGlu>
+template <int MT, int R, bool kGlu, bool kBeside = false>
 static int launch_gemv(const void* a, const void* b, void* c, int M, int N, int K, long long lda, long long ldb,
                        long long ldc, cudaStream_t st) {
   const int per_cta = (kGemvThreads / 32) * (kGlu ? R / 2 : R);      // output columns per CTA
   const int n_out = kGlu ? N / 2 : N;
   const size_t smem = (size_t)MT * kGemvKTile * sizeof(bf16);
-  auto kern = gemv_kernel<MT, R, kGlu>;
+  auto kern = gemv_kernel<MT, R, kGlu, kBeside>;
   KSA_CHECK_CUDA(launch_kernel(kern, dim3((n_out + per_cta - 1) / per_cta),
                               dim3(kGemvThreads), smem, st, (const bf16*)a, (const bf16*)b, (bf16*)c, M, N, K, lda, ldb,
                               ldc, (int)weights_early()));
@@ -515,6 +518,14 @@ static int gemv_dispatch(const void* a, const void* b, void* c, int M, int N, in
   p.nrm = nrm;
   p.early = weights_early();
   if (nrm.w != nullptr) return launch_stream<1, kGlu, true>(p, b, ldb, st);
+  if (!kGlu && launch_beside()) {          // the summary rows of a short prompt: the same kernels as below
+    if (M > 8) return launch_stream<2, false, false, true>(p, b, ldb, st);
+    if (M > 2) return launch_stream<1, false, false, true>(p, b, ldb, st);
+    if (M == 1) return N <= 8192 ? launch_gemv<1, 1, false, true>(a, b, c, M, N, K, lda, ldb, ldc, st)
+                                 : launch_gemv<1, 4, false, true>(a, b, c, M, N, K, lda, ldb, ldc, st);
+    return N <= 8192 ? launch_gemv<2, 1, false, true>(a, b, c, M, N, K, lda, ldb, ldc, st)
+                     : launch_gemv<2, 4, false, true>(a, b, c, M, N, K, lda, ldb, ldc, st);
+  }
   // In a decode step the ring is filled while the previous kernel runs (one row x 2560 x 9728 10.4 against 11.9 us, x
   // 4096 x 2048 4.4 against 5.4, x 2560 x 4096 6.2 both); the output head is long enough not to need that.
   if (M <= 2 && !(weights_early() && N <= 32768)) {

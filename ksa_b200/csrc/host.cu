@@ -178,6 +178,8 @@ static int first_launch_mode() {
 }
 static thread_local int t_launch_mode = first_launch_mode();
 int launch_mode() { return t_launch_mode; }
+static thread_local bool t_beside = false;
+bool launch_beside() { return t_beside && t_launch_mode == kLaunchDependent; }
 }  // namespace ksa
 
 // Sets the calling thread's launch mode (below zero: ordinary, 0: dependent, above: dependent with early weights) and returns the
@@ -185,6 +187,13 @@ int launch_mode() { return t_launch_mode; }
 KSA_API int ksa_set_dependent_launch(int mode) {
   const int before = ksa::t_launch_mode;
   ksa::t_launch_mode = mode < 0 ? ksa::kLaunchOrdinary : mode > 0 ? ksa::kLaunchEarlyWeights : ksa::kLaunchDependent;
+  return before;
+}
+
+// Whether the calling thread's launches may run beside the kernel before them (host.h: launch_beside); returns the setting before.
+KSA_API int ksa_set_launch_beside(int on) {
+  const int before = ksa::t_beside;
+  ksa::t_beside = on != 0;
   return before;
 }
 

@@ -86,6 +86,16 @@ int launch_mode();
 inline bool dependent_launches() { return launch_mode() != kLaunchOrdinary; }
 inline bool weights_early() { return launch_mode() == kLaunchEarlyWeights; }
 
+// Two kernels of one call that do not depend on one another (text rows and summary rows: other inputs' rows, other outputs) need not
+// run one after the other.  After ksa_set_launch_beside(1), products and summary attention are launched to start as soon as every block of the
+// kernel before them has begun its work, and wait for its end only before their own.  That is sound because a kernel begins its
+// work when its own predecessors have ended (grid_dependency_enter), so what the second kernel reads and overwrites has to be
+// finished before the FIRST one begins, and the first one has to be such a kernel: not one that lets successors start before it waits
+// (the weight-streaming products) or lets none start.  What may come between the two from another thread is no exception: it, too, starts
+// after the first has begun, and ends after it.  No effect with early weights, whose chains hold such products.
+// A layer on 333 tokens 158.7 -> 142.9 us (the projection and the attention of two summary rows lie under those of the text rows), a
+// training layer on 2 x 700 632 -> 615, on 8192 2840 -> 2800, attention over 32768 tokens 811 -> 794.
+bool launch_beside();
 template <typename Kern, typename... Args>
 inline cudaError_t launch_kernel_if(bool dependent, Kern kern, dim3 grid, dim3 block, size_t smem, cudaStream_t st, Args... args) {
   cudaLaunchConfig_t cfg = {};
@@ -110,9 +120,10 @@ inline cudaError_t launch_kernel(Kern kern, dim3 grid, dim3 block, size_t smem, 
 // dependent the output head over 4096 tokens took 7.14 ms instead of 6.91 (two cross entropies over 0.6 GB each), a training layer on
 // 8192 tokens 2.98 ms instead of 2.93, summary attention on 32768 tokens 931 us instead of 912.  What the short ones gain: a layer on
 // 333 tokens 185 -> 164 us, a feed-forward block of 48 rows 51 -> 43, a training layer on 1400 tokens 666 -> 646.
+constexpr long long kStreamedDependent = 32LL << 20;
 template <typename Kern, typename... Args>
 inline cudaError_t launch_stream_kernel(long long bytes, Kern kern, dim3 grid, dim3 block, size_t smem, cudaStream_t st, Args... args) {
-  return launch_kernel_if(bytes <= (32LL << 20), kern, grid, block, smem, st, args...);
+  return launch_kernel_if(bytes <= kStreamedDependent, kern, grid, block, smem, st, args...);
 }
 
 #define KSA_REQUIRE(cond, ...)                  \

@@ -58,6 +58,7 @@ int ksa_attn_fwd(const void* q, const void* k, const void* v, const void* ks, co
                  long long v_rs, long long v_bs, long long ks_rs, long long ks_bs, long long vs_rs, long long vs_bs, long long o_rs,
                  long long o_bs, int q_off, int k_off, int s_off, int chunk, int n_sum, int window, int tok_window, float scale,
                  const void* q_doc_start, const void* k_doc_end, void* stream);
+int ksa_set_launch_beside(int on);
 int ksa_summary_attn_fwd(const void* q, const void* k, const void* v, const void* ks, const void* vs, void* o, void* lse, int B,
                          int Hq, int Hkv, int D, int Nq, int seq_len, long long q_rs, long long q_bs, long long k_rs,
                          long long k_bs, long long v_rs, long long v_bs, long long ks_rs, long long ks_bs, long long vs_rs,
@@ -160,6 +161,14 @@ PyObject* wrap(Tensor t) { return THPVariable_Wrap(std::move(t)); }
 PyObject* wrap(const Tensor& a, const Tensor& b) { return Py_BuildValue("(NN)", wrap(a), wrap(b)); }
 PyObject* none() { Py_RETURN_NONE; }
 
+// While it lives, launches may run beside the kernel before them: csrc/host.h (launch_beside) says when that is sound.
+struct Beside {
+  explicit Beside(bool on) : before(ksa_set_launch_beside(on)) {}
+  ~Beside() { ksa_set_launch_beside(before); }
+  Beside(const Beside&) = delete;
+  int before;
+};
+
 // The kernel for C[M, N] = op(A) op(B) (+ C): the rules of `gemm` in ops/__init__.py, which explains them.
 struct Product {
   const void* a;
@@ -247,7 +256,8 @@ PyObject* py_linear(PyObject*, PyObject* const* v, Py_ssize_t n) {
   END_HANDLE_TH_ERRORS
 }
 
-// linear_dw(dy, x, lo, hi, out | None, accumulate, pair_min) -> dy[lo:hi]^T x[lo:hi], into an fp32 buffer or as bf16
+// linear_dw(dy, x, lo, hi, out | None, accumulate, pair_min, beside) -> dy[lo:hi]^T x[lo:hi], into an fp32 buffer or as bf16.
+// beside: the caller launched another product of the same tensors just before (csrc/host.h, launch_beside)
 PyObject* py_linear_dw(PyObject*, PyObject* const* v, Py_ssize_t n) {
   HANDLE_TH_ERRORS
   Args a(v, n);
@@ -255,6 +265,7 @@ PyObject* py_linear_dw(PyObject*, PyObject* const* v, Py_ssize_t n) {
   const long long lo = a.integer(), hi = a.integer();
   const Tensor* out = a.tensor(at::kFloat, true);
   const int acc = a.integer() != 0, pair_min = (int)a.integer();
+  const bool on = a.integer() != 0;
   if (!a.ok() || !rows2d(dy) || !rows2d(x) || dy->size(0) != x->size(0) || lo < 0 || hi <= lo || hi > x->size(0)) return none();
   Product p{at_row(*dy, lo), at_row(*x, lo), nullptr, dy->size(1), x->size(1), hi - lo, dy->stride(0), x->stride(0), 0, 1, 1,
             out != nullptr, out != nullptr && acc};
@@ -266,6 +277,7 @@ PyObject* py_linear_dw(PyObject*, PyObject* const* v, Py_ssize_t n) {
     const Tensor& c = out ? *out : made;
     p.c = c.mutable_data_ptr();
     p.ldc = c.stride(0);
+    const Beside beside(on && out);      // memory allocated here might be what the kernel before has just let go
     gemm(p, pair_min, a.stream());
   }
   return wrap(out ? *out : made);
@@ -290,6 +302,7 @@ PyObject* py_dual_linear(PyObject*, PyObject* const* v, Py_ssize_t n) {
     void* st = a.stream();
     if (n_a > 0)
       gemm({x->const_data_ptr(), wa->const_data_ptr(), y.mutable_data_ptr(), n_a, N, K, K, wa->stride(0), N, 0, b_mn, 0, 0}, pair_min, st);
+    const Beside beside(n_a > 16);     // at most 16 text rows take a product that lets its successors start before it waits
     if (R > n_a)
       gemm({at_row(*x, n_a), wb->const_data_ptr(), at_row_mut(y, n_a), R - n_a, N, K, K, wb->stride(0), N, 0, b_mn, 0, 0}, pair_min, st);
   }
@@ -557,13 +570,14 @@ PyObject* py_attention(PyObject*, PyObject* const* v, Py_ssize_t n) {
     pybind11::gil_scoped_release no_gil;
     out = a.empty({x->size(0), os});
     lse = a.empty({B, Hq, L}, at::kFloat);
+    if (Ns) lse_s = a.empty({B, Hq, Ns}, at::kFloat);      // ahead of the launches: no memory of a kernel that may still run
     const void *k = s.block(*x, 0, kc), *vv = s.block(*x, 0, vc);
     const void *ks = Ns ? s.block(*x, text, kc) : nullptr, *vs = Ns ? s.block(*x, text, vc) : nullptr;
     LAUNCH(ksa_attn_fwd, x->const_data_ptr(), k, vv, ks, vs, out.mutable_data_ptr(), lse.mutable_data_ptr(), B, Hq, Hkv, D, L, L, Ns, rs,
            L * rs, rs, L * rs, rs, L * rs, rs, Ns * rs, rs, Ns * rs, os, L * os, 0, 0, 0, (int)s.chunk, s.n_sum > 1 ? (int)s.n_sum : 1,
            (int)s.window, (int)s.tok_window, s.scale, nullptr, nullptr, a.stream());
     if (Ns) {
-      lse_s = a.empty({B, Hq, Ns}, at::kFloat);
+      const Beside beside(true);
       LAUNCH(ksa_summary_attn_fwd, s.block(*x, text, 0), k, vv, ks, vs, s.block_mut(out, text, 0), lse_s.mutable_data_ptr(), B, Hq, Hkv,
              D, Ns, L, rs, Ns * rs, rs, L * rs, rs, L * rs, rs, Ns * rs, rs, Ns * rs, os, Ns * os, (int)s.chunk, (int)s.n_sum, 0, 0, 0,
              s.scale, a.stream());

@@ -192,10 +192,11 @@ def _weight_grad(weight: torch.Tensor, compute):
     return compute(None, False)
 
 
-def _linear_weight_grad(weight: torch.Tensor, dy: torch.Tensor, x: torch.Tensor, lo: int, hi: int):
-    """The gradient of ``weight`` in ``x[lo:hi] @ weight.T``, routed by :func:`_weight_grad`."""
+def _linear_weight_grad(weight: torch.Tensor, dy: torch.Tensor, x: torch.Tensor, lo: int, hi: int, beside: bool = False):
+    """The gradient of ``weight`` in ``x[lo:hi] @ weight.T``, routed by :func:`_weight_grad`.  ``beside``: the caller has just
+    launched another product of the same tensors, which this one need not wait for (``launch_beside`` in ``csrc/host.h``)."""
     def compute(out, acc):
-        dw = _native.linear_dw(dy, x, lo, hi, out, acc, GEMM_PAIR_MIN_TILES)
+        dw = _native.linear_dw(dy, x, lo, hi, out, acc, GEMM_PAIR_MIN_TILES, int(beside))
         if dw is not None:
             return dw
         return gemm(dy[lo:hi], x[lo:hi], a_mn_major=True, b_mn_major=True, out=out, accumulate=acc)
@@ -280,7 +281,8 @@ class _DualLinearFn(torch.autograd.Function):
             if not need or hi <= lo:
                 grads.append(None)
                 continue
-            grads.append(_linear_weight_grad(w, dy, x, lo, hi))
+            # the text rows' gradients were launched above, from the same dy and x and into other buffers
+            grads.append(_linear_weight_grad(w, dy, x, lo, hi, beside=lo > 16 and (dx is not None or grads[0] is not None)))
         return dx, grads[0], grads[1], None
 
 
