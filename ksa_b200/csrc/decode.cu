@@ -19,6 +19,7 @@ namespace ksa {
 
 constexpr int kDecThreads = 128;
 constexpr int kDecTile = 64;       // keys per shared-memory tile
+constexpr int kDecKeys = 16;       // keys per iteration of a warp of the tensor-core variant
 constexpr int kDecMaxQ = 16;       // queries (G * Tq) served per CTA
 constexpr int kDecMaxSplits = 64;  // splits of the key range when the last split merges them itself
 
@@ -31,7 +32,7 @@ struct DecodeArgs {
   float* part_o;        // [B, Tq, Hq, splits, D]
   float* part_ml;       // [B, Tq, Hq, splits, 2]
   bf16* out;            // [B, Tq, Hq, D]
-  int B, Tq, Hq, Hkv, D, cap, splits, keys_per_split;
+  int B, Tq, Hq, Hkv, D, cap, splits, keys_per_split;   // keys_per_split 0: an even share of each slice
   float scale;
   long long q_rs;
   int* counters;        // [B * Hkv] zeros, or null: with counters the last split of a KV group to finish merges the
@@ -255,18 +256,14 @@ __device__ __forceinline__ void mma_qk(float (&c)[4], uint32_t a0, uint32_t a1, 
                : "r"(a0), "r"(a1), "r"(a2), "r"(a3), "r"(b0), "r"(b1));
 }
 
-template <int NQ>   // queries served per CTA, padded: 4, 8 or 16
-__global__ void __launch_bounds__(kDecThreads) decode_attn_mma_kernel(DecodeArgs a) {
-  grid_dependency_launch();   // the successor may start now: in a decode step it is a projection that reads its weights first
-  grid_dependency_wait();     // the previous kernel's results are complete from here on
-  constexpr int D = 128, KPI = 16;                 // keys per warp iteration
-  __shared__ __align__(16) float s_p[4][KPI][NQ];  // per warp: probabilities, [key][query]
-  __shared__ float s_m[4][NQ], s_l[4][NQ];
-  __shared__ __align__(16) float s_o[4][NQ][D];
-  const int split = blockIdx.x, kvh = blockIdx.y, b = blockIdx.z;
+// One warp's share of a split: sixteen keys at a time, W warps in turn.  Leaves the rows' maxima and sums (rows g and g + 8 of this lane's
+// group, log2 units, the sums complete over the four lanes of a row) and the unscaled outputs of its four head dimensions.
+template <int NQ, int W>
+__device__ __forceinline__ void decode_warp(const DecodeArgs& a, int split, int kvh, int b, int warp, int lane, float (*s_p)[NQ],
+                                            float (&acc)[NQ][4], float& m0, float& m1, float& l0, float& l1) {
+  constexpr int D = 128, KPI = kDecKeys;
   const int G = a.Hq / a.Hkv;
   const int nq = G * a.Tq;
-  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   const int g = lane >> 2, t = lane & 3;
   // per-row (g and g+8) slice bounds, and the CTA's key range
   int st0 = 0, en0 = 0, st1 = 0, en1 = 0, lo = a.cap, hi = 0;
@@ -276,8 +273,9 @@ __global__ void __launch_bounds__(kDecThreads) decode_attn_mma_kernel(DecodeArgs
     if (qi == g) { st0 = s; en0 = e; }
     if (qi == g + 8) { st1 = s; en1 = e; }
   }
-  const int k0 = lo + split * a.keys_per_split;
-  const int k1 = min(hi, k0 + a.keys_per_split);
+  const int per = a.keys_per_split > 0 ? a.keys_per_split : (max(hi - lo, 0) + a.splits * KPI - 1) / (a.splits * KPI) * KPI;
+  const int k0 = lo + split * per;
+  const int k1 = min(hi, k0 + per);
   // query fragments: row g and row g+8, 4 blocks of 32 head dimensions
   uint4 qa[4], qb[4];
 #pragma unroll
@@ -295,15 +293,15 @@ __global__ void __launch_bounds__(kDecThreads) decode_attn_mma_kernel(DecodeArgs
   }
   const bf16* kb = a.k_cache + ((long long)b * a.Hkv + kvh) * a.cap * D;
   const bf16* vb = a.v_cache + ((long long)b * a.Hkv + kvh) * a.cap * D;
-  float m0 = -INFINITY, m1 = -INFINITY, l0 = 0.f, l1 = 0.f;   // running max / partial sums of rows g and g+8
-  float acc[NQ][4];
+  m0 = m1 = -INFINITY;             // running max / partial sums of rows g and g+8
+  l0 = l1 = 0.f;
 #pragma unroll
   for (int q = 0; q < NQ; ++q)
 #pragma unroll
     for (int i = 0; i < 4; ++i) acc[q][i] = 0.f;
   const float sc = a.scale * 1.4426950408889634f;              // scores in log2 units
 
-  for (int kbase = k0 + warp * KPI; kbase < k1; kbase += 4 * KPI) {
+  for (int kbase = k0 + warp * KPI; kbase < k1; kbase += W * KPI) {
     // ---- scores of 16 keys
     float s[2][4];
 #pragma unroll
@@ -355,8 +353,8 @@ __global__ void __launch_bounds__(kDecThreads) decode_attn_mma_kernel(DecodeArgs
       for (int e = 0; e < 2; ++e) {
         const float p0 = exp2f(s[j][e] - u0), p1 = exp2f(s[j][2 + e] - u1);
         l0 += p0; l1 += p1;
-        if (g < NQ) s_p[warp][j * 8 + 2 * t + e][g] = p0;
-        if (NQ > 8) s_p[warp][j * 8 + 2 * t + e][g + 8] = p1;
+        if (g < NQ) s_p[j * 8 + 2 * t + e][g] = p0;
+        if (NQ > 8) s_p[j * 8 + 2 * t + e][g + 8] = p1;
       }
     // correction factors of all queries: row q lives in lanes 4*(q%8) .. +3
     float corr[NQ];
@@ -373,7 +371,7 @@ __global__ void __launch_bounds__(kDecThreads) decode_attn_mma_kernel(DecodeArgs
       const float2 v01 = unpack_bf16x2(vv[k].x), v23 = unpack_bf16x2(vv[k].y);
 #pragma unroll
       for (int q4 = 0; q4 < NQ / 4; ++q4) {
-        const float4 p = *reinterpret_cast<const float4*>(&s_p[warp][k][q4 * 4]);
+        const float4 p = *reinterpret_cast<const float4*>(&s_p[k][q4 * 4]);
         const float pq[4] = {p.x, p.y, p.z, p.w};
 #pragma unroll
         for (int i = 0; i < 4; ++i) {
@@ -385,9 +383,26 @@ __global__ void __launch_bounds__(kDecThreads) decode_attn_mma_kernel(DecodeArgs
       }
     }
   }
-  // ---- merge the four warps, write this split's partial result
   l0 += __shfl_xor_sync(0xffffffffu, l0, 1); l0 += __shfl_xor_sync(0xffffffffu, l0, 2);
   l1 += __shfl_xor_sync(0xffffffffu, l1, 1); l1 += __shfl_xor_sync(0xffffffffu, l1, 2);
+}
+
+template <int NQ>   // queries served per CTA, padded: 4, 8 or 16
+__global__ void __launch_bounds__(kDecThreads) decode_attn_mma_kernel(DecodeArgs a) {
+  grid_dependency_launch();   // the successor may start now: in a decode step it is a projection that reads its weights first
+  grid_dependency_wait();     // the previous kernel's results are complete from here on
+  constexpr int D = 128;
+  __shared__ __align__(16) float s_p[4][kDecKeys][NQ];  // per warp: probabilities, [key][query]
+  __shared__ float s_m[4][NQ], s_l[4][NQ];
+  __shared__ __align__(16) float s_o[4][NQ][D];
+  const int split = blockIdx.x, kvh = blockIdx.y, b = blockIdx.z;
+  const int G = a.Hq / a.Hkv;
+  const int nq = G * a.Tq;
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  const int g = lane >> 2, t = lane & 3;
+  float acc[NQ][4], m0, m1, l0, l1;
+  decode_warp<NQ, 4>(a, split, kvh, b, warp, lane, s_p[warp], acc, m0, m1, l0, l1);
+  // ---- merge the four warps, write this split's partial result
   if (t == 0) {
     if (g < NQ) { s_m[warp][g] = m0; s_l[warp][g] = l0; }
     if (NQ > 8) { s_m[warp][g + 8] = m1; s_l[warp][g + 8] = l1; }
@@ -416,6 +431,112 @@ __global__ void __launch_bounds__(kDecThreads) decode_attn_mma_kernel(DecodeArgs
     }
   }
   combine_if_last(a, b, kvh, nq, G);
+}
+
+// Slices of caches of up to kDecClusterKeys keys (the ring and summaries of a summary layer, short contexts): the splits of a KV group are a
+// cluster, which shares each slice evenly and merges through its shared memory.  What bounds such a slice is the chain of latencies,
+// and the merge by the split that finishes last (partial results to global memory, a counter, all of them read back) was half of
+// it: a decode step of four sequences of 1030 keys through four layers and the head 424 -> 408 us, of
+// one 367 -> 351, of two of 330 keys 375 -> 356.  While a cluster of every group fits beside the others: with six sequences (384 CTAs) both take 428 us, with
+// sixteen 530 and 570.
+// Four to eight warps a CTA are as good as one another; with twelve, which ask for all of a split's keys at once, the next projection finds no
+// room beside the CTAs and reads its weights late (448 us).  An L2 prefetch of the keys ahead of the wait changed nothing.
+constexpr int kDecClusterKeys = 2048;
+constexpr int kDecCluster = 8;
+template <int NQ>
+constexpr int dec_cluster_warps() { return NQ <= 8 ? 6 : 4; }      // sixteen queries' outputs of four warps take 32 KB of shared memory
+
+__device__ __forceinline__ float ld_cluster_f32(const float* local, uint32_t rank) {
+  float v;
+  asm volatile("{\n\t.reg .u32 a;\n\tmapa.shared::cluster.u32 a, %1, %2;\n\tld.shared::cluster.f32 %0, [a];\n\t}"
+               : "=f"(v) : "r"(smem_u32(local)), "r"(rank) : "memory");
+  return v;
+}
+__device__ __forceinline__ void cluster_barrier() {
+  asm volatile("barrier.cluster.arrive.release.aligned;\n\tbarrier.cluster.wait.acquire.aligned;" ::: "memory");
+}
+
+template <int NQ>
+__global__ void __launch_bounds__(dec_cluster_warps<NQ>() * 32) decode_attn_cluster_kernel(DecodeArgs a) {
+  constexpr int D = 128, W = dec_cluster_warps<NQ>();
+  __shared__ __align__(16) float s_p[W][kDecKeys][NQ];
+  __shared__ float s_m[W][NQ], s_l[W][NQ], s_cm[NQ], s_cl[NQ];
+  __shared__ __align__(16) float s_o[W][NQ][D];
+  const int split = blockIdx.x, kvh = blockIdx.y, b = blockIdx.z;
+  const int G = a.Hq / a.Hkv, nq = G * a.Tq;
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  grid_dependency_launch();   // the successor may start now: in a decode step it is a projection that reads its weights first
+  grid_dependency_wait();     // the previous kernel's results are complete from here on
+  float acc[NQ][4], m0, m1, l0, l1;
+  decode_warp<NQ, W>(a, split, kvh, b, warp, lane, s_p[warp], acc, m0, m1, l0, l1);
+  if ((lane & 3) == 0) {
+    const int g = lane >> 2;
+    if (g < NQ) { s_m[warp][g] = m0; s_l[warp][g] = l0; }
+    if (NQ > 8) { s_m[warp][g + 8] = m1; s_l[warp][g + 8] = l1; }
+  }
+#pragma unroll
+  for (int q = 0; q < NQ; ++q) *reinterpret_cast<float4*>(&s_o[warp][q][lane * 4]) = make_float4(acc[q][0], acc[q][1], acc[q][2], acc[q][3]);
+  __syncthreads();
+  // the warps' parts -> this split's, in the place of the first warp's
+  for (int i = threadIdx.x; i < nq * D; i += W * 32) {
+    const int q = i / D, d = i % D;
+    float m = -INFINITY;
+#pragma unroll
+    for (int w = 0; w < W; ++w) m = fmaxf(m, s_m[w][q]);
+    float o = 0.f, l = 0.f;
+#pragma unroll
+    for (int w = 0; w < W; ++w) {
+      const float f = s_m[w][q] == -INFINITY ? 0.f : exp2f(s_m[w][q] - m);
+      o += s_o[w][q][d] * f;
+      l += s_l[w][q] * f;
+    }
+    s_o[0][q][d] = o;
+    if (d == 0) { s_cm[q] = m; s_cl[q] = l; }
+  }
+  cluster_barrier();
+  // every split finishes its share of the outputs
+  const int share = (nq * D + kDecCluster - 1) / kDecCluster, end = min((split + 1) * share, nq * D);
+  for (int i = split * share + (int)threadIdx.x; i < end; i += W * 32) {
+    const int q = i / D, d = i % D;
+    float ms[kDecCluster], ls[kDecCluster], os[kDecCluster], m = -INFINITY;
+#pragma unroll
+    for (int r = 0; r < kDecCluster; ++r) {
+      ms[r] = ld_cluster_f32(&s_cm[q], r);
+      ls[r] = ld_cluster_f32(&s_cl[q], r);
+      os[r] = ld_cluster_f32(&s_o[0][q][d], r);
+      m = fmaxf(m, ms[r]);
+    }
+    float o = 0.f, l = 0.f;
+#pragma unroll
+    for (int r = 0; r < kDecCluster; ++r) {
+      const float f = ms[r] == -INFINITY ? 0.f : exp2f(ms[r] - m);
+      o = fmaf(os[r], f, o);
+      l = fmaf(ls[r], f, l);
+    }
+    a.out[(((long long)b * a.Tq + q / G) * a.Hq + kvh * G + q % G) * D + d] = __float2bfloat16(l > 0.f ? o / l : 0.f);
+  }
+  cluster_barrier();          // nobody leaves while its part may still be read
+}
+
+template <int NQ>
+static int launch_decode_cluster(DecodeArgs a, cudaStream_t st) {
+  a.splits = kDecCluster;
+  a.keys_per_split = 0;       // of the slice, not of the cache
+  cudaLaunchConfig_t cfg = {};
+  cfg.gridDim = dim3(a.splits, a.Hkv, a.B);
+  cfg.blockDim = dim3(dec_cluster_warps<NQ>() * 32);
+  cfg.stream = st;
+  cudaLaunchAttribute at[2];
+  at[0].id = cudaLaunchAttributeClusterDimension;
+  at[0].val.clusterDim.x = a.splits;
+  at[0].val.clusterDim.y = 1;
+  at[0].val.clusterDim.z = 1;
+  at[1].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+  at[1].val.programmaticStreamSerializationAllowed = 1;
+  cfg.attrs = at;
+  cfg.numAttrs = dependent_launches() ? 2 : 1;
+  KSA_CHECK_CUDA(cudaLaunchKernelEx(&cfg, decode_attn_cluster_kernel<NQ>, a));
+  return 0;
 }
 
 // one CTA per (b, t, head): merge the splits
@@ -507,6 +628,10 @@ KSA_API int ksa_decode_attn(const void* q, const void* k_cache, const void* v_ca
   dim3 grid(splits, Hkv, B);
   cudaStream_t st = reinterpret_cast<cudaStream_t>(stream);
   const int nq = (Hq / Hkv) * Tq;
+  if (D == 128 && cap <= kDecClusterKeys && counters != nullptr && kDecCluster * Hkv * B <= 2 * sm_count()) {
+    if (nq <= 4) return launch_decode_cluster<4>(a, st);
+    return nq <= 8 ? launch_decode_cluster<8>(a, st) : launch_decode_cluster<16>(a, st);
+  }
   if (D == 128 && nq <= 4) KSA_CHECK_CUDA(launch_kernel(decode_attn_mma_kernel<4>, grid, dim3(kDecThreads), 0, st, a));
   else if (D == 128 && nq <= 8) KSA_CHECK_CUDA(launch_kernel(decode_attn_mma_kernel<8>, grid, dim3(kDecThreads), 0, st, a));
   else if (D == 128) KSA_CHECK_CUDA(launch_kernel(decode_attn_mma_kernel<16>, grid, dim3(kDecThreads), 0, st, a));
