@@ -57,6 +57,18 @@ def _decode_attention(q, k_cache, v_cache, start, length, scale, counters=None):
     return out
 
 
+def _cache_fill(qkv, k_cache, v_cache, B, L, Ns, Hq, Hkv, D, spec) -> bool:
+    """A prompt's keys and values into the cache of one layer (``spec``: of a summary layer) in one launch; False where the rows or the
+    cache are not of the ordinary kind."""
+    if not (qkv.is_cuda and (spec is None or spec.n_sum > 0) and qkv.dtype == k_cache.dtype == torch.bfloat16 and D % 8 == 0 and qkv.stride(1) == 1
+            and qkv.stride(0) % 8 == 0 and qkv.data_ptr() % 16 == 0 and k_cache.is_contiguous() and v_cache.is_contiguous()):
+        return False
+    geometry = (spec.chunk, spec.n_sum, spec.window, spec.text0, spec.sum0) if spec is not None else (0, 0, 0, 0, 0)
+    _lib.call("ksa_kv_cache_fill", qkv[:, Hq * D:], qkv[:, (Hq + Hkv) * D:], k_cache, v_cache, B, L, Ns, Hkv, D, k_cache.shape[2],
+              qkv.stride(0), *geometry)
+    return True
+
+
 def _cache_append(k_new, v_new, k_cache, v_cache, slots):
     """``k_new``/``v_new`` ``[B, T, H, D]`` (views allowed) -> cache ``[B, H, cap, D]`` at ``slots[B, T]`` (< 0: skip)."""
     if not k_new.is_cuda:
@@ -188,6 +200,9 @@ class KsaInferenceEngine:
             for j in range(0, len(idx), step):
                 rows = idx[j:j + step]
                 logits = self._prefill_rows(tokens[rows, :L] if rows != list(range(B)) or L != Lmax else tokens, rows)
+                if rows == list(range(B)):
+                    out = logits
+                    continue
                 if out is None:
                     out = torch.empty(B, logits.shape[-1], dtype=torch.float32, device=logits.device)
                 out[rows] = logits
@@ -215,6 +230,9 @@ class KsaInferenceEngine:
 
         def sink(layer_idx, qkv, is_summary_layer):
             cache = self.layer_caches[layer_idx]
+            if contiguous and _cache_fill(qkv, cache.k[sel], cache.v[sel], B, L, Ns if is_summary_layer else 0, Hq, Hkv, Dh,
+                                          self.specs[layer_idx] if is_summary_layer else None):
+                return
             k_t = qkv[:B * L, Hq * Dh:(Hq + Hkv) * Dh].view(B, L, Hkv, Dh)
             v_t = qkv[:B * L, (Hq + Hkv) * Dh:].view(B, L, Hkv, Dh)
             if not is_summary_layer:

@@ -61,6 +61,7 @@ _SIGNATURES: Dict[str, Sequence] = {
     "ksa_decode_step_slices": [P, P, P, I, I, I, I, I, I, P],
     "ksa_decode_advance": [P, P, I, P],
     "ksa_kv_cache_append": [P] * 5 + [I] * 5 + [L, L, P],
+    "ksa_kv_cache_fill": [P, P, P, P, I, I, I, I, I, I, L, I, I, I, I, I, P],
     "ksa_kv_cache_move": [P] * 5 + [I] * 5 + [P],
     "ksa_peer_gather": [P, I, I, L, I, P, P, ctypes.c_uint, I, P],
     "ksa_peer_reduce_adamw": [P, I, I, L, L, P, P, P, P, P, F, F, F, F, F, P, P, P, ctypes.c_uint, I, P],
