@@ -56,7 +56,6 @@ struct StreamArgs {
   int ragged;            // K is no multiple of 64: one load per box, which fills the columns past K with zeros
   int w_rows, x_rows;    // rows of a box in shared memory (weights, activations): those loaded, for `ragged` in whole swizzle atoms
   int stages, stage_bytes;
-  int early;             // weights_early(): the weights are read before the previous kernel has ended
   GemvNorm nrm;
 };
 
@@ -76,9 +75,16 @@ __device__ __forceinline__ void multiply_sync() { asm volatile("bar.sync 1, %0;"
 // byte offset of columns 8 q .. 8 q + 7 (q < 8) of row r in a box of 128-byte rows with the 128-byte swizzle
 __device__ __forceinline__ uint32_t swizzled(int r, int q) { return (uint32_t)(r * 128 + ((q ^ (r & 7)) << 4)); }
 
-// NB: batch blocks of 8 rows, 1 (M <= 8) or 2 (M <= 16).  kBeside: launch_beside(); known to the compiler, since a decode step of four
-// sequences took 442 us instead of 420 with the conditions in the kernels that it launches.
-template <int NB, bool kGlu, bool kNorm, bool kBeside>
+// When the kernel waits for the one before it, and when it lets the one after it start.  Known to the compiler: with the conditions in the
+// kernels that a decode step launches, a step of four sequences took 442 us instead of 420.
+enum StreamMode {
+  kStWaits,      // before it reads anything; the successor of a block's first product (a norm, SwiGLU) starts behind that, and so may
+                 // take weights to be as they are for good (ops.linear_of_block: a feed-forward block of one row 32.3 -> 31.4 us)
+  kStEarly,      // weights_early(): the weights are read before the previous kernel has ended, and the successor starts at once
+  kStBeside,     // launch_beside(): before it ends
+};
+// NB: batch blocks of 8 rows, 1 (M <= 8) or 2 (M <= 16)
+template <int NB, bool kGlu, bool kNorm, StreamMode kMode>
 __global__ void __launch_bounds__(kStThreads + 32, 2)
 stream_gemm_kernel(const __grid_constant__ CUtensorMap tmB, const __grid_constant__ CUtensorMap tmA, const StreamArgs p,
                    int* status) {
@@ -112,7 +118,9 @@ stream_gemm_kernel(const __grid_constant__ CUtensorMap tmB, const __grid_constan
     if (!kNorm) tma_prefetch_desc(&tmA);
   }
   __syncthreads();
-  grid_dependency_launch();
+  // the plain product's successor starts at once in every mode (16 x 6144 x 2560 7.7 us in a row of them, 7.9 with the later start)
+  constexpr bool kAtOnce = kMode != kStWaits || (!kGlu && !kNorm);
+  if (kAtOnce) grid_dependency_launch();
 
   if (warp == kStWarps) {
     // ------------------------------------------------------------ producer: lane 0, or for `ragged` a lane per box
@@ -147,10 +155,11 @@ stream_gemm_kernel(const __grid_constant__ CUtensorMap tmB, const __grid_constan
       next(x);
     };
     // in a decode step weights do not depend on the previous kernel; the activations do
-    if (!kBeside && !p.early) grid_dependency_wait();
+    if (kMode == kStWaits) grid_dependency_wait();
+    if (!kAtOnce) grid_dependency_launch();
     const int ahead = min(p.stages, n_items);
     for (int it = 0; it < ahead; ++it) load_weights();
-    if (!kBeside) grid_dependency_wait();
+    if (kMode == kStEarly) grid_dependency_wait();
     for (int it = 0; it < ahead; ++it) load_acts();
     for (int it = ahead; it < n_items; ++it) {
       if (!__all_sync(0xffffffffu, mbar_wait(&empty[w.stage], w.phase, guard, kTimeoutStageEmpty))) break;
@@ -161,7 +170,7 @@ stream_gemm_kernel(const __grid_constant__ CUtensorMap tmB, const __grid_constan
   }
 
   // -------------------------------------------------------------- the eight warps that multiply
-  if (!kBeside) grid_dependency_wait();     // also for the outputs: an earlier kernel may still read their memory
+  if (kMode != kStBeside) grid_dependency_wait();     // also for the outputs: an earlier kernel may still read their memory
   if (kNorm) {
     float ss[4] = {0.f, 0.f, 0.f, 0.f};
     for (int c = threadIdx.x * 8; c < p.K; c += kStThreads * 8) {
@@ -318,10 +327,10 @@ stream_gemm_kernel(const __grid_constant__ CUtensorMap tmB, const __grid_constan
       multiply_sync();        // the next group's partial sums overwrite these
     }
   }
-  if (kBeside) grid_dependency_leave(1);
+  if (kMode == kStBeside) grid_dependency_leave(1);
 }
 
-template <int NB, bool kGlu, bool kNorm, bool kBeside = false>
+template <int NB, bool kGlu, bool kNorm, StreamMode kMode>
 static int launch_stream(StreamArgs p, const void* b, long long ldb, cudaStream_t st) {
   const int sms = sm_count();
   KSA_REQUIRE(sms > 0, "gemv: no device");
@@ -369,7 +378,7 @@ static int launch_stream(StreamArgs p, const void* b, long long ldb, cudaStream_
     uint32_t box[3] = {64, (uint32_t)p.M, (uint32_t)(p.ragged ? 1 : p.boxes)};
     if ((rc = make_tmap(&tmA, p.A, 2, 3, dims, str, box, true))) return rc;
   }
-  auto kern = stream_gemm_kernel<NB, kGlu, kNorm, kBeside>;
+  auto kern = stream_gemm_kernel<NB, kGlu, kNorm, kMode>;
   static PerDevice raised;
   KSA_CHECK_CUDA(raise_smem_limit(raised, kern, kStSmemMost));
   KSA_CHECK_CUDA(launch_kernel(kern, dim3(grid), dim3(kStThreads + 32), (size_t)smem, st, tmB, tmA,
@@ -516,11 +525,11 @@ static int gemv_dispatch(const void* a, const void* b, void* c, int M, int N, in
   p.A = (const bf16*)a; p.C = (bf16*)c;
   p.lda = lda; p.ldc = ldc; p.M = M; p.N = N; p.K = K;
   p.nrm = nrm;
-  p.early = weights_early();
-  if (nrm.w != nullptr) return launch_stream<1, kGlu, true>(p, b, ldb, st);
+  const bool early = weights_early();
+  if (nrm.w != nullptr) return early ? launch_stream<1, kGlu, true, kStEarly>(p, b, ldb, st) : launch_stream<1, kGlu, true, kStWaits>(p, b, ldb, st);
   if (!kGlu && launch_beside()) {          // the summary rows of a short prompt: the same kernels as below
-    if (M > 8) return launch_stream<2, false, false, true>(p, b, ldb, st);
-    if (M > 2) return launch_stream<1, false, false, true>(p, b, ldb, st);
+    if (M > 8) return launch_stream<2, false, false, kStBeside>(p, b, ldb, st);
+    if (M > 2) return launch_stream<1, false, false, kStBeside>(p, b, ldb, st);
     if (M == 1) return N <= 8192 ? launch_gemv<1, 1, false, true>(a, b, c, M, N, K, lda, ldb, ldc, st)
                                  : launch_gemv<1, 4, false, true>(a, b, c, M, N, K, lda, ldb, ldc, st);
     return N <= 8192 ? launch_gemv<2, 1, false, true>(a, b, c, M, N, K, lda, ldb, ldc, st)
@@ -528,7 +537,7 @@ static int gemv_dispatch(const void* a, const void* b, void* c, int M, int N, in
   }
   // In a decode step the ring is filled while the previous kernel runs (one row x 2560 x 9728 10.4 against 11.9 us, x
   // 4096 x 2048 4.4 against 5.4, x 2560 x 4096 6.2 both); the output head is long enough not to need that.
-  if (M <= 2 && !(weights_early() && N <= 32768)) {
+  if (M <= 2 && !(early && N <= 32768)) {
     // rows per warp: fewer for narrow outputs so that the grid still covers every SM a few times (with SwiGLU a warp
     // needs at least one gate row and one up row)
     constexpr int R1 = kGlu ? 2 : 1;
@@ -537,7 +546,8 @@ static int gemv_dispatch(const void* a, const void* b, void* c, int M, int N, in
     return N <= 8192 ? launch_gemv<2, R1, kGlu>(a, b, c, M, N, K, lda, ldb, ldc, st)
                      : launch_gemv<2, 4, kGlu>(a, b, c, M, N, K, lda, ldb, ldc, st);
   }
-  return M <= 8 ? launch_stream<1, kGlu, false>(p, b, ldb, st) : launch_stream<2, kGlu, false>(p, b, ldb, st);
+  if (early) return M <= 8 ? launch_stream<1, kGlu, false, kStEarly>(p, b, ldb, st) : launch_stream<2, kGlu, false, kStEarly>(p, b, ldb, st);
+  return M <= 8 ? launch_stream<1, kGlu, false, kStWaits>(p, b, ldb, st) : launch_stream<2, kGlu, false, kStWaits>(p, b, ldb, st);
 }
 }  // namespace ksa
 

@@ -59,6 +59,7 @@ int ksa_attn_fwd(const void* q, const void* k, const void* v, const void* ks, co
                  long long o_bs, int q_off, int k_off, int s_off, int chunk, int n_sum, int window, int tok_window, float scale,
                  const void* q_doc_start, const void* k_doc_end, void* stream);
 int ksa_set_launch_beside(int on);
+int ksa_set_dependent_launch(int mode);
 int ksa_summary_attn_fwd(const void* q, const void* k, const void* v, const void* ks, const void* vs, void* o, void* lse, int B,
                          int Hq, int Hkv, int D, int Nq, int seq_len, long long q_rs, long long q_bs, long long k_rs,
                          long long k_bs, long long v_rs, long long v_bs, long long ks_rs, long long ks_bs, long long vs_rs,
@@ -169,6 +170,17 @@ struct Beside {
   int before;
 };
 
+// While it lives, products of a thread that launches dependently read their weights early.
+struct EarlyWeights {
+  explicit EarlyWeights(bool on) : before(on ? ksa_set_dependent_launch(1) : 0), set(on) {
+    if (set && before != 0) ksa_set_dependent_launch(before);       // ordinary launches stay ordinary
+  }
+  ~EarlyWeights() { if (set) ksa_set_dependent_launch(before); }
+  EarlyWeights(const EarlyWeights&) = delete;
+  int before;
+  bool set;
+};
+
 // The kernel for C[M, N] = op(A) op(B) (+ C): the rules of `gemm` in ops/__init__.py, which explains them.
 struct Product {
   const void* a;
@@ -231,12 +243,14 @@ PyObject* py_gemm(PyObject*, PyObject* const* v, Py_ssize_t n) {
   END_HANDLE_TH_ERRORS
 }
 
-// linear(x, w, pair_min) -> y [..., N], for any x with contiguous rows
+// linear(x, w, pair_min, weights_ready) -> y [..., N], for any x with contiguous rows.  weights_ready: no kernel that may still run when
+// the one before this product has begun its work writes w (csrc/host.h, kLaunchEarlyWeights)
 PyObject* py_linear(PyObject*, PyObject* const* v, Py_ssize_t n) {
   HANDLE_TH_ERRORS
   Args a(v, n);
   const Tensor *x = a.tensor(), *w = a.tensor();
   const int pair_min = (int)a.integer();
+  const bool ready = a.integer() != 0;
   if (!a.ok() || !rows2d(w) || !(rows2d(x) || (x->dim() > 0 && x->is_contiguous())) || x->size(-1) != w->size(1)) return none();
   if (c10::GradMode::is_enabled() && (x->requires_grad() || w->requires_grad())) return none();
   const long long K = w->size(1), M = x->numel() / K;
@@ -250,6 +264,7 @@ PyObject* py_linear(PyObject*, PyObject* const* v, Py_ssize_t n) {
     sizes.back() = p.N;
     y = a.empty(sizes);
     p.c = y.mutable_data_ptr();
+    const EarlyWeights early(ready);
     gemm(p, pair_min, a.stream());
   }
   return wrap(y);

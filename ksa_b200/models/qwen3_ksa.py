@@ -122,7 +122,7 @@ class SwiGluMlp(nn.Module):
         """``res = x + delta``; the block on ``rms_norm(res)``.  Returns ``(res, block output)``.  For the few rows of a
         decode step the residual add, the norm, the gate/up projection and SwiGLU are one launch."""
         res, h = ops.norm_linear(x, delta, norm_scale, eps, self.w13.weight, glu=True)
-        return res, ops.linear(h, self.w2.weight)
+        return res, ops.linear_of_block(h, self.w2.weight)
 
     def forward(self, x, tp=None, residual_rows: Optional[int] = None):
         if tp is None or (x.dim() == 2 and x.shape[0] <= 16 and getattr(tp, "_pending", None) is None):

@@ -207,7 +207,7 @@ class _LinearFn(torch.autograd.Function):
     @staticmethod
     def forward(ctx, x, weight):
         ctx.x_shape = x.shape
-        y = None if _lib.pair_gather_pending() else _native.linear(x, weight, GEMM_PAIR_MIN_TILES)
+        y = None if _lib.pair_gather_pending() else _native.linear(x, weight, GEMM_PAIR_MIN_TILES, 0)
         if y is not None:
             ctx.save_for_backward(x if x.dim() == 2 else x.reshape(-1, x.shape[-1]), weight)
             return y
@@ -237,12 +237,23 @@ def linear(x: torch.Tensor, weight: torch.Tensor, bias: Optional[torch.Tensor] =
     if not _cuda(x):
         return ref.linear(x, weight, bias)
     if not _observed() and not _lib.pair_gather_pending():       # nobody differentiates it: one call
-        y = _native.linear(x, weight, GEMM_PAIR_MIN_TILES)
+        y = _native.linear(x, weight, GEMM_PAIR_MIN_TILES, 0)
         if y is not None:
             return y if bias is None else y + bias
     _require_bf16(x, weight)
     y = _run(_LinearFn, x, weight)
     return y if bias is None else y + bias
+
+
+def linear_of_block(x: torch.Tensor, weight: torch.Tensor) -> torch.Tensor:
+    """``linear(x, weight)`` for the second product of a block whose first one has just made ``x`` on the same stream.  That kernel began
+    its work behind everything that was launched before it, so whatever wrote ``weight`` has ended when this one starts, and a product of
+    a few rows reads its weights while the first is still at work."""
+    if x.dim() == 2 and x.shape[0] <= 16 and _cuda(x) and not _observed() and not _lib.pair_gather_pending():
+        y = _native.linear(x, weight, GEMM_PAIR_MIN_TILES, 1)
+        if y is not None:
+            return y
+    return linear(x, weight)
 
 
 class _DualLinearFn(torch.autograd.Function):
