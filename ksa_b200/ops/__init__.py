@@ -70,11 +70,14 @@ def _run(fn, *args):
     return fn.forward(_NoGrad(), *args)
 
 
-def _narrow_swiglu(x: torch.Tensor, w13: torch.Tensor):
-    """Plan of the split-K kernel for few rows with the activation, or None.  It takes feature counts in steps of 8; a
-    parameter gather that waits for a GEMM to ride in, and observed calls, are left to separate calls."""
+def _few_rows_swiglu(x: torch.Tensor, w13: torch.Tensor):
+    """Tile of the kernel for some hundred rows with the activation (an int), else the plan of the split-K kernel, or None.  They take
+    feature counts in steps of 8; a parameter gather that waits for a GEMM to ride in, and observed calls, are left to separate calls."""
     if w13.shape[0] % 16 != 0 or _lib.pair_gather_pending() or _observed():
         return None
+    columns = _lib.gemm_tall_plan(x.shape[0], w13.shape[0] // 2, x.shape[1], 1, x.stride(0) % 64 != 0 or w13.stride(0) % 64 != 0)
+    if columns:
+        return columns
     return _lib.gemm_narrow_plan(x.shape[0], w13.shape[0], x.shape[1], 1, GEMM_PAIR_MIN_TILES,
                                  (x.stride(0) % 64 != 0) + 2 * (w13.stride(0) % 64 != 0))
 
@@ -131,6 +134,13 @@ def gemm(a: torch.Tensor, b: torch.Tensor, *, a_mn_major: bool = False, b_mn_maj
         a, b = (t if t.stride(0) > 0 or t.shape[0] == 1 else t.contiguous() for t in (a, b))
         _lib.call("ksa_gemv_bf16", a, b, out, M, N, K, a.stride(0), b.stride(0), out.stride(0))
         return out
+    if (pair is None and sm_limit == 0 and alpha == 1.0 and not a_mn_major and not b_mn_major and out.dtype == torch.bfloat16
+            and not accumulate and out.data_ptr() % 16 == 0 and out.stride(0) % 8 == 0):
+        # some hundred rows and wide weights: all rows in one tile (csrc/gemm_tall.cu says when that is faster)
+        columns = _lib.gemm_tall_plan(M, N, K, 0, a.stride(0) % 64 != 0 or b.stride(0) % 64 != 0)
+        if columns:
+            _lib.call("ksa_gemm_tall_bf16", a, b, out, M, N, K, a.stride(0), b.stride(0), out.stride(0), 0, columns)
+            return out
     if pair is None and sm_limit == 0 and not a_mn_major and out.dtype == torch.bfloat16 and not accumulate:
         # too few tiles to occupy the chip: K is split as well (csrc/gemm_narrow.cu says when that is faster)
         lda, ldb = a.stride(0), b.stride(0)
@@ -661,7 +671,7 @@ class _LinearSwiGluFn(torch.autograd.Function):
 def linear_swiglu(x: torch.Tensor, w13: torch.Tensor) -> torch.Tensor:
     """``swiglu(x @ w13.T)`` with ``w13 = [gate rows | up rows]``.  Without autograd on a GPU the projection of few rows (a
     decode step, a short prompt) applies the activation itself: ``ksa_gemv_swiglu_bf16`` for at most 16 rows, the gated form of
-    ``ksa_gemm_narrow_bf16`` where ``gemm`` would take that kernel; in a differentiated call the CTA-pair kernel does so
+    ``ksa_gemm_tall_bf16`` or ``ksa_gemm_narrow_bf16`` where those are faster; in a differentiated call the CTA-pair kernel does so
     and leaves the projection for the backward pass (``ksa_gemm2_swiglu_bf16``).  Everything else is the projection followed by ``swiglu``."""
     if _cuda(x) and not _observed() and not _lib.pair_gather_pending():
         out = _native.linear_swiglu(x, w13, GEMM_PAIR_MIN_TILES)
@@ -674,11 +684,13 @@ def linear_swiglu(x: torch.Tensor, w13: torch.Tensor) -> torch.Tensor:
             and w13.stride(0) % 8 == 0 and min(x.stride(0), w13.stride(0)) > 0 and w13.shape[0] % 2 == 0):
         M, K = x.shape
         N = w13.shape[0]
-        plan = _narrow_swiglu(x, w13) if M > 16 else None
+        plan = _few_rows_swiglu(x, w13) if M > 16 else None
         if M <= 16 or plan is not None:
             out = torch.empty((M, N // 2), dtype=torch.bfloat16, device=x.device)
             if plan is None:
                 _lib.call("ksa_gemv_swiglu_bf16", x, w13, out, M, N, K, x.stride(0), w13.stride(0), out.stride(0))
+            elif isinstance(plan, int):
+                _lib.call("ksa_gemm_tall_bf16", x, w13, out, M, N // 2, K, x.stride(0), w13.stride(0), out.stride(0), 1, plan)
             else:
                 _lib.call("ksa_gemm_narrow_bf16", x, w13, out, M, N, K, x.stride(0), w13.stride(0), out.stride(0), 0, 1,
                           *plan, 1.0)

@@ -32,6 +32,7 @@ _SIGNATURES: Dict[str, Sequence] = {
     "ksa_gemm2_scatter_bf16": [P, P, I, I, I, L, L, L, P, I, I, P],
     "ksa_gemm2_swiglu_bf16": [P, P, P, P, I, I, I, L, L, L, L, P],
     "ksa_gemm_narrow_bf16": [P, P, P, I, I, I, L, L, L, I, I, I, I, F, P],
+    "ksa_gemm_tall_bf16": [P, P, P, I, I, I, L, L, L, I, I, P],
     "ksa_gemv_bf16": [P, P, P, I, I, I, L, L, L, P],
     "ksa_gemv_swiglu_bf16": [P, P, P, I, I, I, L, L, L, P],
     "ksa_gemv_norm_bf16": [P, P, P, P, P, P, I, I, I, L, L, L, L, L, F, I, I, P],
@@ -106,6 +107,8 @@ def load() -> ctypes.CDLL:
     lib.ksa_attn_bwd_num_segments.restype = I
     lib.ksa_gemm_on_pairs.argtypes = [I] * 3
     lib.ksa_gemm_on_pairs.restype = I
+    lib.ksa_gemm_tall_plan.argtypes = [I] * 5
+    lib.ksa_gemm_tall_plan.restype = I
     lib.ksa_gemm_narrow_plan.argtypes = [I] * 6
     lib.ksa_gemm_narrow_plan.restype = I
     lib.ksa_set_dependent_launch.argtypes = [I]
@@ -298,6 +301,11 @@ def gemm_on_pairs(M: int, N: int, pair_min_tiles: int) -> bool:
 
 
 @functools.lru_cache(maxsize=4096)
+def gemm_tall_plan(M: int, N: int, K: int, glu: int, ragged: bool) -> int:
+    """Weight rows of a tile for ``ksa_gemm_tall_bf16`` (``N``: columns of the result), or 0 where another kernel is taken."""
+    return load().ksa_gemm_tall_plan(M, N, K, glu, int(ragged))
+
+
 def gemm_narrow_plan(M: int, N: int, K: int, glu: int, pair_min_tiles: int, ragged: int = 0):
     """``(activation rows per tile, split of K)`` for ``ksa_gemm_narrow_bf16``, or None where a tiled kernel is faster.
     ``ragged``: bit 0 for activations, bit 1 for weights whose row pitch is no multiple of 64 elements."""
