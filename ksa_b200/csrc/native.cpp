@@ -26,7 +26,7 @@ int ksa_gemm_on_pairs(int M, int N, int pair_min_tiles);
 int ksa_gemm_narrow_plan(int M, int N, int K, int glu, int pair_min_tiles, int ragged);
 int ksa_gemm_tall_plan(int M, int N, int K, int glu, int ragged);
 int ksa_gemm_tall_bf16(const void* x, const void* w, void* c, int M, int N, int K, long long ldx, long long ldw, long long ldc, int glu,
-                       int columns, void* stream);
+                       int columns, int split, void* stream);
 int ksa_rmsnorm_bwd_parts(int rows);
 int ksa_attn_bwd_num_segments(int lq);
 int ksa_gemm_bf16(const void* a, const void* b, void* c, int M, int N, int K, long long lda, long long ldb, long long ldc,
@@ -200,9 +200,9 @@ void gemm(const Product& p, int pair_min, void* st) {
     return;
   }
   if (!p.a_mn && !p.b_mn && bf16_out && (reinterpret_cast<uintptr_t>(p.c) & 15) == 0 && p.ldc % 8 == 0) {
-    const int columns = ksa_gemm_tall_plan(M, N, K, 0, p.lda % 64 != 0 || p.ldb % 64 != 0);
-    if (columns != 0) {
-      LAUNCH(ksa_gemm_tall_bf16, p.a, p.b, p.c, M, N, K, p.lda, p.ldb, p.ldc, 0, columns, st);
+    const int plan = ksa_gemm_tall_plan(M, N, K, 0, p.lda % 64 != 0 || p.ldb % 64 != 0);
+    if (plan != 0) {
+      LAUNCH(ksa_gemm_tall_bf16, p.a, p.b, p.c, M, N, K, p.lda, p.ldb, p.ldc, 0, plan / 16, plan % 16, st);
       return;
     }
   }
@@ -483,11 +483,11 @@ PyObject* py_linear_swiglu(PyObject*, PyObject* const* v, Py_ssize_t n) {
     return none();
   if (c10::GradMode::is_enabled() && (x->requires_grad() || w->requires_grad())) return none();
   const int M = (int)x->size(0), N = (int)w->size(0), K = (int)x->size(1);
-  int plan = 0, columns = 0;
+  int plan = 0, tall = 0;
   if (M > 16) {
-    columns = ksa_gemm_tall_plan(M, N / 2, K, 1, x->stride(0) % 64 != 0 || w->stride(0) % 64 != 0);
-    if (columns == 0 && N % 16 == 0) plan = ksa_gemm_narrow_plan(M, N, K, 1, pair_min, (x->stride(0) % 64 != 0) + 2 * (w->stride(0) % 64 != 0));
-    if (plan == 0 && columns == 0) return none();
+    tall = ksa_gemm_tall_plan(M, N / 2, K, 1, x->stride(0) % 64 != 0 || w->stride(0) % 64 != 0);
+    if (tall == 0 && N % 16 == 0) plan = ksa_gemm_narrow_plan(M, N, K, 1, pair_min, (x->stride(0) % 64 != 0) + 2 * (w->stride(0) % 64 != 0));
+    if (plan == 0 && tall == 0) return none();
   }
   Tensor out;
   {
@@ -496,9 +496,9 @@ PyObject* py_linear_swiglu(PyObject*, PyObject* const* v, Py_ssize_t n) {
     if (M <= 16)
       LAUNCH(ksa_gemv_swiglu_bf16, x->const_data_ptr(), w->const_data_ptr(), out.mutable_data_ptr(), M, N, K, x->stride(0), w->stride(0),
              out.stride(0), a.stream());
-    else if (columns != 0)
+    else if (tall != 0)
       LAUNCH(ksa_gemm_tall_bf16, x->const_data_ptr(), w->const_data_ptr(), out.mutable_data_ptr(), M, N / 2, K, x->stride(0), w->stride(0),
-             out.stride(0), 1, columns, a.stream());
+             out.stride(0), 1, tall / 16, 1, a.stream());
     else
       LAUNCH(ksa_gemm_narrow_bf16, x->const_data_ptr(), w->const_data_ptr(), out.mutable_data_ptr(), M, N, K, x->stride(0), w->stride(0),
              out.stride(0), 0, 1, plan / 16, plan % 16, 1.f, a.stream());

@@ -71,15 +71,16 @@ def _run(fn, *args):
 
 
 def _few_rows_swiglu(x: torch.Tensor, w13: torch.Tensor):
-    """Tile of the kernel for some hundred rows with the activation (an int), else the plan of the split-K kernel, or None.  They take
-    feature counts in steps of 8; a parameter gather that waits for a GEMM to ride in, and observed calls, are left to separate calls."""
+    """Kernel for some hundred rows with the activation and its plan, or None.  They take feature counts in steps of 8; a
+    parameter gather that waits for a GEMM to ride in, and observed calls, are left to separate calls."""
     if w13.shape[0] % 16 != 0 or _lib.pair_gather_pending() or _observed():
         return None
-    columns = _lib.gemm_tall_plan(x.shape[0], w13.shape[0] // 2, x.shape[1], 1, x.stride(0) % 64 != 0 or w13.stride(0) % 64 != 0)
-    if columns:
-        return columns
-    return _lib.gemm_narrow_plan(x.shape[0], w13.shape[0], x.shape[1], 1, GEMM_PAIR_MIN_TILES,
-                                 (x.stride(0) % 64 != 0) + 2 * (w13.stride(0) % 64 != 0))
+    M, N, K, ragged = x.shape[0], w13.shape[0], x.shape[1], (x.stride(0) % 64 != 0) + 2 * (w13.stride(0) % 64 != 0)
+    plan = _lib.gemm_tall_plan(M, N // 2, K, 1, ragged != 0)
+    if plan is not None:
+        return "ksa_gemm_tall_bf16", plan
+    plan = _lib.gemm_narrow_plan(M, N, K, 1, GEMM_PAIR_MIN_TILES, ragged)
+    return None if plan is None else ("ksa_gemm_narrow_bf16", plan)
 
 
 def _require_bf16(*ts):
@@ -137,9 +138,9 @@ def gemm(a: torch.Tensor, b: torch.Tensor, *, a_mn_major: bool = False, b_mn_maj
     if (pair is None and sm_limit == 0 and alpha == 1.0 and not a_mn_major and not b_mn_major and out.dtype == torch.bfloat16
             and not accumulate and out.data_ptr() % 16 == 0 and out.stride(0) % 8 == 0):
         # some hundred rows and wide weights: all rows in one tile (csrc/gemm_tall.cu says when that is faster)
-        columns = _lib.gemm_tall_plan(M, N, K, 0, a.stride(0) % 64 != 0 or b.stride(0) % 64 != 0)
-        if columns:
-            _lib.call("ksa_gemm_tall_bf16", a, b, out, M, N, K, a.stride(0), b.stride(0), out.stride(0), 0, columns)
+        plan = _lib.gemm_tall_plan(M, N, K, 0, a.stride(0) % 64 != 0 or b.stride(0) % 64 != 0)
+        if plan is not None:
+            _lib.call("ksa_gemm_tall_bf16", a, b, out, M, N, K, a.stride(0), b.stride(0), out.stride(0), 0, *plan)
             return out
     if pair is None and sm_limit == 0 and not a_mn_major and out.dtype == torch.bfloat16 and not accumulate:
         # too few tiles to occupy the chip: K is split as well (csrc/gemm_narrow.cu says when that is faster)
@@ -684,16 +685,16 @@ def linear_swiglu(x: torch.Tensor, w13: torch.Tensor) -> torch.Tensor:
             and w13.stride(0) % 8 == 0 and min(x.stride(0), w13.stride(0)) > 0 and w13.shape[0] % 2 == 0):
         M, K = x.shape
         N = w13.shape[0]
-        plan = _few_rows_swiglu(x, w13) if M > 16 else None
-        if M <= 16 or plan is not None:
+        few = _few_rows_swiglu(x, w13) if M > 16 else None
+        if M <= 16 or few is not None:
             out = torch.empty((M, N // 2), dtype=torch.bfloat16, device=x.device)
-            if plan is None:
-                _lib.call("ksa_gemv_swiglu_bf16", x, w13, out, M, N, K, x.stride(0), w13.stride(0), out.stride(0))
-            elif isinstance(plan, int):
-                _lib.call("ksa_gemm_tall_bf16", x, w13, out, M, N // 2, K, x.stride(0), w13.stride(0), out.stride(0), 1, plan)
+            pitches = (x.stride(0), w13.stride(0), out.stride(0))
+            if few is None:
+                _lib.call("ksa_gemv_swiglu_bf16", x, w13, out, M, N, K, *pitches)
+            elif few[0] == "ksa_gemm_tall_bf16":
+                _lib.call(few[0], x, w13, out, M, N // 2, K, *pitches, 1, *few[1])
             else:
-                _lib.call("ksa_gemm_narrow_bf16", x, w13, out, M, N, K, x.stride(0), w13.stride(0), out.stride(0), 0, 1,
-                          *plan, 1.0)
+                _lib.call(few[0], x, w13, out, M, N, K, *pitches, 0, 1, *few[1], 1.0)
             return out
     if (_cuda(x) and x.dim() == 2 and w13.dim() == 2 and w13.shape[0] % 2 == 0 and torch.is_grad_enabled()
             and (x.requires_grad or w13.requires_grad)):

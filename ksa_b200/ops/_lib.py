@@ -32,7 +32,7 @@ _SIGNATURES: Dict[str, Sequence] = {
     "ksa_gemm2_scatter_bf16": [P, P, I, I, I, L, L, L, P, I, I, P],
     "ksa_gemm2_swiglu_bf16": [P, P, P, P, I, I, I, L, L, L, L, P],
     "ksa_gemm_narrow_bf16": [P, P, P, I, I, I, L, L, L, I, I, I, I, F, P],
-    "ksa_gemm_tall_bf16": [P, P, P, I, I, I, L, L, L, I, I, P],
+    "ksa_gemm_tall_bf16": [P, P, P, I, I, I, L, L, L, I, I, I, P],
     "ksa_gemv_bf16": [P, P, P, I, I, I, L, L, L, P],
     "ksa_gemv_swiglu_bf16": [P, P, P, I, I, I, L, L, L, P],
     "ksa_gemv_norm_bf16": [P, P, P, P, P, P, I, I, I, L, L, L, L, L, F, I, I, P],
@@ -301,9 +301,10 @@ def gemm_on_pairs(M: int, N: int, pair_min_tiles: int) -> bool:
 
 
 @functools.lru_cache(maxsize=4096)
-def gemm_tall_plan(M: int, N: int, K: int, glu: int, ragged: bool) -> int:
-    """Weight rows of a tile for ``ksa_gemm_tall_bf16`` (``N``: columns of the result), or 0 where another kernel is taken."""
-    return load().ksa_gemm_tall_plan(M, N, K, glu, int(ragged))
+def gemm_tall_plan(M: int, N: int, K: int, glu: int, ragged: bool):
+    """``(weight rows per tile, split of K)`` for ``ksa_gemm_tall_bf16`` (``N``: columns of the result), or None for the other kernels."""
+    plan = load().ksa_gemm_tall_plan(M, N, K, glu, int(ragged))
+    return divmod(plan, 16) if plan else None
 
 
 def gemm_narrow_plan(M: int, N: int, K: int, glu: int, pair_min_tiles: int, ragged: int = 0):
