@@ -198,23 +198,22 @@ gemm_narrow_kernel(const __grid_constant__ CUtensorMap tmW, const __grid_constan
   grid_dependency_leave(p.beside);
 }
 
-// Tile height and split for a product, and its time in microseconds as modelled.  The figures were fitted to 315 measured
-// (shape, height, split) triples of 17 to 1411 rows against 4096 x 2048 .. 19456 x 2560 weights, the last two items to 900 shapes of
+// Tile height and split for a product, and its time in microseconds as modelled.  The figures were fitted to 4176 measured (shape, height,
+// split) triples of 288 to 2048 rows against 512 x 4096 .. 9728 x 2560 weights in both layouts, the last two items to 900 shapes of
 // 17 to 2048 rows and 64 to 19456 x 64 to 12288 weights:
-//   * one 64-wide step of K takes a CTA that has an SM to itself 0.32 us (the latency of its loads) and two that share
-//     one 2 x (0.142 + 0.00044 bt), so a grid should fill both slots of every SM; a ring for more than 160 rows leaves
+//   * one 64-wide step of K takes a CTA that has an SM to itself 0.241 + 0.00054 bt us (the latency of its loads) and two that share
+//     one 2 x (0.093 + 0.00094 bt), so a grid should fill both slots of every SM; a ring for more than 160 rows leaves
 //     room for one CTA only;
-//   * the weights of all CTAs come through the L2 at 13.7 TB/s;
-//   * a launch costs 1.5 us, a wave of CTAs 4.6 us to start and drain, and 0.0126 + 0.0045 split per activation row to write
+//   * the weights of all CTAs come through the L2 at 16 TB/s, with the activations at 21.9;
+//   * a launch costs 1.4 us, a wave of CTAs 3.6 us to start and drain, and 0.013 + 0.0043 split per activation row to write
 //     and add up;
 //   * clusters of 4 and 8 do not fill every SM: narrow_first and narrow_slots below;
 //   * rows that do not start on a 128-byte line take a second line for every box row: weights and activations then come
 //     through the L2 at 21 TB/s as 1.86 and 1.55 times their bytes.
-// Measured on the widths of both model presets and their transposes (16 of them, 17 to 2048 rows, 808 products): the model's
-// standard deviation is 5 %, the choice 0.6 % above the best of the plans tried on average, and no product slower than on the
-// tiled kernels.  On 497 other shapes: 10 %, 0.7 %, one of the 244 that were chosen 6 % slower (1856 x 6144 x 9728).  Without the last
-// two items 8 of those were up to 23 % slower, and of the 900 shapes 21 up to 30 % (779 x 3552 x 6008: 62.5 us on tiles of 160 rows
-// in two parts, 42.9 on CTA pairs; 193 x 4256 x 3352 30.2 on 208 rows in four parts, 21.0).
+// The model's standard deviation is 8 %; over those 270 products the choice (tiled kernels included) is 1.2 % above the best on average,
+// against 3.3 % with the figures of before the issuing threads were elected, and 2 % faster: 333 x 2560 x 4096 19.8 -> 15.6 us, 576 x 2560 x 9728
+// 37.9 -> 31.2, 700 x 2048 x 12288 40.7 -> 34.9.  Without the last two items 21 of the 900 shapes were up to 30 % slower (779 x 3552 x 6008:
+// 62.5 us on tiles of 160 rows in two parts, 42.9 on CTA pairs; 193 x 4256 x 3352 30.2 on 208 rows in four parts, 21.0).
 constexpr int kNwSms = 148;
 constexpr int kNwMaxRows = 2048;   // the model holds near the range that it was fitted to (8000 x 128 x 2048: 27.4 against 15.3 us)
 static bool narrow_two_per_sm(int bt) { return 3 * (kNwWBytes + bt * kNwBK * 2) <= 110 * 1024; }
@@ -245,16 +244,18 @@ static double narrow_plan(int M, long long n_tiles, int K, bool ragged_x, bool r
         if (n == 0) return 0.0;
         const long long rounds = (n + first - 1) / first;
         const double per_sm = (double)(rounds < per_sm_most ? rounds : per_sm_most);
-        double step = per_sm * (0.142 + 0.00044 * bt);
-        if (step < 0.32 + 0.00027 * bt) step = 0.32 + 0.00027 * bt;
-        if (step < n * 0.00122) step = n * 0.00122;
+        double step = per_sm * (0.093 + 0.00094 * bt);
+        if (step < 0.241 + 0.00054 * bt) step = 0.241 + 0.00054 * bt;
+        if (step < n * 0.00102) step = n * 0.00102;
+        const double all = n * (kNwWBytes + bt * kNwBK * 2.0) / 21.9e6;
+        if (step < all) step = all;
         if (ragged_x || ragged_w) {
           const double bytes = kNwWBytes * (ragged_w ? 1.86 : 1.0) + bt * kNwBK * 2 * (ragged_x ? 1.55 : 1.0);
           if (step < n * bytes / 21e6) step = n * bytes / 21e6;
         }
-        return 4.6 + steps * step + per_sm * bt * (0.0126 + (split > 1 ? 0.0045 * split : 0.0)) + (split == 8 ? 0.26 : 0.0);
+        return 3.6 + steps * step + per_sm * bt * (0.013 + (split > 1 ? 0.0043 * split : 0.0)) + (split == 8 ? 0.26 : 0.0);
       };
-      const double t = 1.5 + (double)(ctas / slots) * wave(slots) + wave(ctas % slots);
+      const double t = 1.36 + (double)(ctas / slots) * wave(slots) + wave(ctas % slots);
       if (t < best) { best = t; *bt_out = bt; *split_out = split; }
     }
   }
@@ -269,20 +270,20 @@ static bool enough_for_pairs(int M, int N, int pair_min_tiles) {
 static bool on_pairs(int M, int N, int pair_min_tiles) {
   return enough_for_pairs(M, N, pair_min_tiles) && 2 * tiled_waves(M, N, 256, kNwSms / 2) < 3 * tiled_waves(M, N, 128, kNwSms);
 }
-// The time of the tiled kernel that serves the same product otherwise: 0.345 us a 64-wide step and wave of 74 CTA pairs with 256 x 256
-// tiles, 5 us around them.  Single CTAs with 128 x 256 tiles take 0.38 a step and wave and 5 around them where there are too few tiles for
-// pairs (17.5 us measured for 128 x 12288 x 2048, 55.3 for 1411 x 2560 x 9728, 61 for 48 to 700 x 2560 x 9728).  Where they are
-// taken for their fewer waves, most SMs have a tile: 6.5 us and, a step and wave, 0.38 and 0.05 for every megabyte of weights that the
-// step's tiles read: 1152 x 4096 x 2048 17.4 us (0.5 MB), 333 x 12288 x 2048 21.2 (1.6 MB), 128 x 19456 x 2560 26.2 (2.5 MB).
+// The time of the tiled kernel that serves the same product otherwise: 0.327 us a 64-wide step and wave of 74 CTA pairs with 256 x 256
+// tiles, 6.7 us around them.  Single CTAs with 128 x 256 tiles take 0.352 a step and wave and 5.6 around them where there are too few tiles for
+// pairs (16.4 us measured for 900 x 2048 x 2048, 60.5 for 576 x 2560 x 9728).  Where they are taken for their fewer waves, most SMs have a
+// tile: 5.7 us and, a step and wave, 0.364 and 0.057 for every megabyte of weights that the step's tiles read: 333 x 4096 x 2048 16.4 us
+// (0.5 MB), 333 x 12288 x 2048 21.2 (1.6 MB), 128 x 19456 x 2560 26.2 (2.5 MB).
 // glu: and of the separate activation kernel, 2 us and more, 2.8 to 3.7 behind the products of the last kind.
 static double tiled_time(int M, int N, int K, bool glu, int pair_min_tiles) {
   const long long num_kb = (K + 63) / 64;
   const double act = glu ? 2.0 : 0.0;
-  if (on_pairs(M, N, pair_min_tiles)) return act + 5.0 + 0.345 * num_kb * tiled_waves(M, N, 256, kNwSms / 2);
+  if (on_pairs(M, N, pair_min_tiles)) return act + 6.7 + 0.327 * num_kb * tiled_waves(M, N, 256, kNwSms / 2);
   const double steps = (double)(num_kb * tiled_waves(M, N, 128, kNwSms));
-  if (!enough_for_pairs(M, N, pair_min_tiles)) return act + 5.0 + 0.38 * steps;
+  if (!enough_for_pairs(M, N, pair_min_tiles)) return act + 5.6 + 0.352 * steps;
   const long long tm = (M + 127) / 128, tn = (N + 255) / 256, abreast = (kNwSms + tm - 1) / tm;      // tiles of a row in one wave
-  return (glu ? 3.5 : 0.0) + 6.5 + (0.38 + 0.05 * (tn < abreast ? tn : abreast) * 256 * kNwBK * 2 / 1e6) * steps;
+  return (glu ? 3.5 : 0.0) + 5.7 + (0.364 + 0.057 * (tn < abreast ? tn : abreast) * 256 * kNwBK * 2 / 1e6) * steps;
 }
 
 template <bool W_MN, bool kGlu>
@@ -372,13 +373,16 @@ KSA_API int ksa_gemm_on_pairs(int M, int N, int pair_min_tiles) {
 }
 
 // Whether this kernel is expected to beat the tiled ones (of which CTA pairs are taken from `pair_min_tiles` 256 x 256 tiles on, 0:
-// never), by more than the model's error: bt * 16 + split for ksa_gemm_narrow_bf16, or 0.  glu: the separate activation
-// kernel counts on the other side.  ragged: bit 0, the activations' rows do not all start on a 128-byte line (their
+// never), by more than 4 %, with K in one part by more than 8 (900 x 2048 x 2048 16.4 us on tiles and 17.5 here): bt * 16 + split for
+// ksa_gemm_narrow_bf16, or 0, as for weights of less than 64 KB, where nothing but the launch takes time.  glu: the separate activation
+// kernel counts on the other side; 2: it counts on this side, as CTA pairs apply it themselves.  ragged: bit 0, the activations' rows do not all start on a 128-byte line (their
 // pitch is no multiple of 64 elements); bit 1, those of the weights as they lie in memory.
 KSA_API int ksa_gemm_narrow_plan(int M, int N, int K, int glu, int pair_min_tiles, int ragged) {
   using namespace ksa;
-  if (M <= 0 || M > kNwMaxRows || N <= 0 || K <= 0) return 0;
+  if (M <= 0 || M > kNwMaxRows || N <= 0 || K <= 0 || (long long)N * K < 32768) return 0;
   int bt = 0, split = 0;
-  const double t = narrow_plan(M, glu ? (N / 2 + 63) / 64 : (N + 127) / 128, K, (ragged & 1) != 0, (ragged & 2) != 0, &bt, &split);
-  return t < 0.95 * tiled_time(M, N, K, glu != 0, pair_min_tiles) ? bt * 16 + split : 0;
+  const bool gated = glu == 1;
+  double t = narrow_plan(M, gated ? (N / 2 + 63) / 64 : (N + 127) / 128, K, (ragged & 1) != 0, (ragged & 2) != 0, &bt, &split);
+  if (glu == 2) t += 3.0;
+  return t < (split == 1 ? 0.92 : 0.96) * tiled_time(M, N, K, gated, pair_min_tiles) ? bt * 16 + split : 0;
 }

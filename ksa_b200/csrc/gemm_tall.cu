@@ -249,11 +249,13 @@ static int launch_tall(const void* x, const void* w, TallArgs p, long long ldx, 
   CUtensorMap tmX, tmXl, tmW;
   int rc;
   p.last_rows = (p.M - (MT - 1) * 128 + 7) / 8 * 8;
-  for (int last = 0; last < 2; ++last) {
+  for (int rows : {p.last_rows, 128}) {
     uint64_t dims[2] = {(uint64_t)p.K, (uint64_t)p.M};
     uint64_t str[2] = {2, (uint64_t)ldx * 2};
-    uint32_t box[2] = {kTlBK, (uint32_t)(last ? p.last_rows : 128)};
-    if ((rc = make_tmap(last ? &tmXl : &tmX, x, 2, 2, dims, str, box, true))) return rc;
+    uint32_t box[2] = {kTlBK, (uint32_t)rows};
+    if ((rc = make_tmap(&tmX, x, 2, 2, dims, str, box, true))) return rc;
+    if (rows == p.last_rows) tmXl = tmX;
+    if (MT == 1 || p.last_rows == 128) break;           // one map serves
   }
   {
     uint64_t dims[2] = {(uint64_t)p.K, (uint64_t)(kGlu ? 2 : 1) * p.N};

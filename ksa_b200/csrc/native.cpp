@@ -519,7 +519,7 @@ PyObject* py_gemm_swiglu(PyObject*, PyObject* const* v, Py_ssize_t n) {
     return none();
   const int M = (int)x->size(0), F = (int)(w->size(0) / 2), K = (int)x->size(1);
   if (!ksa_gemm_on_pairs(M, 2 * F, pair_min) ||
-      ksa_gemm_narrow_plan(M, 2 * F, K, 0, pair_min, (x->stride(0) % 64 != 0) + 2 * (w->stride(0) % 64 != 0)) != 0)
+      ksa_gemm_narrow_plan(M, 2 * F, K, 2, pair_min, (x->stride(0) % 64 != 0) + 2 * (w->stride(0) % 64 != 0)) != 0)
     return none();
   Tensor h, gu;
   {
