@@ -46,6 +46,7 @@ struct Gemm2Epilogue {
   long long ldc;
   int out_fp32, accumulate;
   float alpha;
+  int halves_from;           // tiles from here on are worked on as two halves of 128 columns (none: the number of tiles)
   int beside;                // launch_beside(); never in the communicating forms
   // GEMM -> reduce-scatter (bf16 output only): output row `row` belongs to rank row / c_shard_rows and is stored, from
   // the epilogue, straight into that rank's memory at c_peer[owner] + (row - owner * c_shard_rows) * ldc.
@@ -158,6 +159,7 @@ gemm2_bf16_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant
   const int tiles_m = (M + 2 * k2BM - 1) / (2 * k2BM);
   const int tiles_n = kGlu ? (N / 2 + k2BNh - 1) / k2BNh : (N + k2BN - 1) / k2BN;
   const int num_tiles = tiles_m * tiles_n;
+  const int units = kGlu ? num_tiles : 2 * num_tiles - ep.halves_from;
   const int num_kb = (K + k2BK - 1) / k2BK;
 
   if (threadIdx.x == 0) {
@@ -186,6 +188,13 @@ gemm2_bf16_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant
     if (mb >= tiles_m) mb -= tiles_m;
     nb = in_group / group_rows;
   };
+  // A unit is a tile, or one half of its columns: `side` is that half, -1 for the whole
+  auto unit_tile = [&](int unit, int& side) {
+    side = -1;
+    if (kGlu || unit < ep.halves_from) return unit;
+    side = (unit - ep.halves_from) & 1;
+    return ep.halves_from + ((unit - ep.halves_from) >> 1);
+  };
 
   if (warp == 0) {
     // ------------------------------------------------------------ TMA producer (both CTAs)
@@ -194,12 +203,14 @@ gemm2_bf16_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant
       uint32_t phase = 0;
       uint32_t segs_seen = 0;       // kMaxPeers x kBulkSegs = 32 segments
       bool ok = true;
-      for (int tile = pair; tile < num_tiles && ok; tile += n_pairs) {
-        int mb, nb;
-        tile_coords(tile, mb, nb);
+      for (int unit = pair; unit < units && ok; unit += n_pairs) {
+        int mb, nb, side;
+        tile_coords(unit_tile(unit, side), mb, nb);
         if (!KSA_DEV_CHECK(mb >= 0 && mb < tiles_m && nb >= 0 && nb < tiles_n && rank < 2 && stage < k2Stages, status)) break;
         const int row0 = mb * 2 * k2BM + (int)rank * k2BM;      // this CTA's rows of A
-        const int col0 = kGlu ? nb * k2BNh + (int)rank * (N / 2) : nb * k2BN + (int)rank * k2BNh;   // this CTA's rows of B
+        const int col0 = kGlu ? nb * k2BNh + (int)rank * (N / 2)                                    // this CTA's rows of B
+                         : side < 0 ? nb * k2BN + (int)rank * k2BNh : nb * k2BN + side * k2BNh + (int)rank * 64;
+        const int boxes = !kGlu && side >= 0 ? 1 : 2;                                               // of 64 rows
         if (comm.dep_operand != 0) {
           // the rows of this tile that live in the gathered buffer: wait for the segments of the shards that hold them
           const long long r_lo = comm.dep_operand == 1 ? row0 : col0;
@@ -238,18 +249,18 @@ gemm2_bf16_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant
           uint8_t* sa = smem + stage * k2StageBytes;
           uint8_t* sb = sa + k2ABytes;
           const uint32_t bar = map_to_cta(smem_u32(&full[stage]), 0);
-          if (rank == 0) mbar_expect_tx(&full[stage], 2 * k2StageBytes);
+          if (rank == 0) mbar_expect_tx(&full[stage], 2 * (k2ABytes + boxes * 8192));
           if (!A_MN) {
             tma_load_2d_pair(sa, &tmA, kb * k2BK, row0, bar);
           } else {
 #pragma unroll
             for (int a = 0; a < k2BM / 64; ++a) tma_load_2d_pair(sa + a * 8192, &tmA, row0 + a * 64, kb * k2BK, bar);
           }
-          if (!B_MN) {
-            tma_load_2d_pair(sb, &tmB, kb * k2BK, col0, bar);
-          } else {
 #pragma unroll
-            for (int a = 0; a < k2BNh / 64; ++a) tma_load_2d_pair(sb + a * 8192, &tmB, col0 + a * 64, kb * k2BK, bar);
+          for (int a = 0; a < 2; ++a) {
+            if (a >= boxes) break;
+            if (!B_MN) tma_load_2d_pair(sb + a * 8192, &tmB, kb * k2BK, col0 + a * 64, bar);
+            else tma_load_2d_pair(sb + a * 8192, &tmB, col0 + a * 64, kb * k2BK, bar);
           }
           if (++stage == k2Stages) { stage = 0; phase ^= 1; }
         }
@@ -258,12 +269,14 @@ gemm2_bf16_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant
   } else if (warp == 1) {
     // ------------------------------------------------------------ MMA issuer (leader CTA only)
     if (rank == 0 && elect_one()) {
-      constexpr uint32_t idesc = umma_idesc_bf16(2 * k2BM, k2BN, A_MN ? 1 : 0, B_MN ? 1 : 0);
+      constexpr uint32_t idesc_full = umma_idesc_bf16(2 * k2BM, k2BN, A_MN ? 1 : 0, B_MN ? 1 : 0);
+      constexpr uint32_t idesc_half = umma_idesc_bf16(2 * k2BM, k2BNh, A_MN ? 1 : 0, B_MN ? 1 : 0);
       int stage = 0;
       uint32_t phase = 0;
       int local = 0;
       bool ok = true;
-      for (int tile = pair; tile < num_tiles && ok; tile += n_pairs, ++local) {
+      for (int unit = pair; unit < units && ok; unit += n_pairs, ++local) {
+        const uint32_t idesc = kGlu || unit < ep.halves_from ? idesc_full : idesc_half;
         const int buf = local & 1;
         const uint32_t acc_phase = (local >> 1) & 1;
         if (!mbar_wait(&acc_empty[buf], acc_phase ^ 1, guard, kTimeoutAccEmpty)) { ok = false; break; }
@@ -298,9 +311,10 @@ gemm2_bf16_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant
     // Staging buffer of this warp's next store.  It flips with every store that is issued and is carried from tile to tile: pieces
     // past N issue none, so a tile may end on either buffer, and only the newest store may still be reading its own.
     int out_buf = 0;
-    for (int tile = pair; tile < num_tiles && ok; tile += n_pairs, ++local) {
-      int mb, nb;
-      tile_coords(tile, mb, nb);
+    for (int unit = pair; unit < units && ok; unit += n_pairs, ++local) {
+      int mb, nb, side;
+      tile_coords(unit_tile(unit, side), mb, nb);
+      const int col_base = nb * k2BN + (side > 0 ? k2BNh : 0), pieces = side < 0 ? k2BN / 32 : k2BNh / 32;
       const int buf = local & 1;
       const uint32_t acc_phase = (local >> 1) & 1;
       if (!mbar_wait(&acc_full[buf], acc_phase, guard, kTimeoutAccFull)) { ok = false; break; }
@@ -365,11 +379,11 @@ gemm2_bf16_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant
         }
       }
 #pragma unroll 1
-      for (int c = 0; c < (kGlu ? 0 : k2BN / 32); ++c) {
+      for (int c = 0; c < (kGlu ? 0 : pieces); ++c) {
         uint32_t r[32];
         tmem_ld32(t_row + c * 32, r);
         tmem_wait_ld();
-        const int col0 = nb * k2BN + c * 32;
+        const int col0 = col_base + c * 32;
         if (tma_block && ep.out_fp32) {
           uint8_t* stage = ring + ((warp - 2) * 2 + out_buf) * 4096;
           // this buffer was read by the last store but one; at most the newest store may be pending
@@ -395,7 +409,7 @@ gemm2_bf16_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant
         if (tma_block) {
           const int piece = c >> 1, half = c & 1;                   // 64-column piece, 32-column half of it
           uint8_t* stage = ring + ((warp - 2) * 2 + out_buf) * 4096;
-          const bool live = nb * k2BN + piece * 64 < N;             // columns past N are clipped by the map
+          const bool live = col_base + piece * 64 < N;             // columns past N are clipped by the map
           if (half == 0) {
             // this buffer was read by the last store but one; at most the newest store may be pending
             if (lane == 0) asm volatile("cp.async.bulk.wait_group.read 1;" ::: "memory");
@@ -417,7 +431,7 @@ gemm2_bf16_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant
             fence_proxy_async();
             __syncwarp();
             if (lane == 0 && live) {
-              tma_store_2d(&smaps.m[owner_w], stage, nb * k2BN + piece * 64, row_w - owner_w * ep.c_shard_rows);
+              tma_store_2d(&smaps.m[owner_w], stage, col_base + piece * 64, row_w - owner_w * ep.c_shard_rows);
               tma_store_commit();
             }
             if (live) out_buf ^= 1;
@@ -486,7 +500,7 @@ gemm2_bf16_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant
 static const ScatterMaps kNoScatterMaps{};
 
 template <bool A_MN, bool B_MN, bool kGlu = false>
-static int launch_gemm2(const void* a, const void* b, const Gemm2Epilogue& ep, int M, int N, int K, long long lda,
+static int launch_gemm2(const void* a, const void* b, Gemm2Epilogue ep, int M, int N, int K, long long lda,
                         long long ldb, cudaStream_t stream, const Comm2Work& comm,
                         const ScatterMaps& smaps = kNoScatterMaps) {
   CUtensorMap tmA, tmB;
@@ -506,7 +520,7 @@ static int launch_gemm2(const void* a, const void* b, const Gemm2Epilogue& ep, i
   if (!B_MN) {
     uint64_t dims[2] = {(uint64_t)K, (uint64_t)N};
     uint64_t str[2] = {2, (uint64_t)ldb * 2};
-    uint32_t box[2] = {k2BK, k2BNh};
+    uint32_t box[2] = {k2BK, 64};
     rc = make_tmap(&tmB, b, 2, 2, dims, str, box, true);
   } else {
     uint64_t dims[2] = {(uint64_t)N, (uint64_t)K};
@@ -522,7 +536,15 @@ static int launch_gemm2(const void* a, const void* b, const Gemm2Epilogue& ep, i
   KSA_CHECK_CUDA(raise_smem_limit(raised, kern, k2SmemTotal));
   const int tiles = ((M + 2 * k2BM - 1) / (2 * k2BM)) * (kGlu ? (N / 2 + k2BNh - 1) / k2BNh : (N + k2BN - 1) / k2BN);
   int pairs = num_sms / 2;
-  if (tiles < pairs) pairs = tiles;
+  // A last wave of at most half as many tiles as pairs is worked on as halves of 128 columns: it takes some 0.6 of a wave, as a half
+  // reads its 128 rows of A too (24 KB an SM for 256 cycles of products; quarters would read 20 for 128).  8192 x 2048 (256 tiles on 74
+  // pairs) at K = 2048 57.0 -> 55.4 us, 6144 167 -> 162, 12288 337 -> 325, 12288 x 2048 x 8192 into fp32 343 -> 335 under the power cap; a layer of full
+  // attention forward and backward on 8192 tokens 3416 -> 3376, one of the sliding window, whose summary rows fill the wave anyway, the same;
+  // from more than half as many tiles on, two waves of halves would take longer than one of whole tiles.
+  const int last = tiles % pairs;
+  ep.halves_from = !kGlu && !comm.active && ep.c_world <= 1 && 2 * last <= pairs ? tiles - last : tiles;
+  const int units = 2 * tiles - ep.halves_from;
+  if (units < pairs) pairs = units;
   int* status = status_word();
   KSA_REQUIRE(status != nullptr, "could not allocate the status word");
   if (comm.active || ep.c_world > 1) {
