@@ -8,7 +8,8 @@
 //     memory, each CTA a share of the rows: no workspace, no atomics, no second launch.
 // Measured against 128 x 256 tiles on single CTAs (weights from memory): 48 rows x 2560 x 9728 58.5 -> 18.1 us, 333 rows 61.1 ->
 // 28.9, 48 rows x 6144 x 2560 20.1 -> 14.1; with the activation, 48 rows x 19456 x 2560 36.2 -> 23.1 (two launches -> one).
-// The weights alone take 7.6, 7.6, 4.8 and 15.2 us at the copy bandwidth.
+// The weights alone take 7.6, 7.6, 4.8 and 15.2 us at the copy bandwidth.  Row-major weights of up to 256 rows go to csrc/gemm_tall.cu now (13.2
+// us for the first of these), which reads the activations again for every tile; from there on this one has the better balance.
 // Roles per CTA (192 threads): warp 0 TMA producer, warp 1 MMA issuer, warps 2..5 move the accumulator to shared
 // memory, and all of them write the result.  One tile per CTA.  No TMA load uses multicast; every wait is bounded.
 //

@@ -130,7 +130,7 @@ def gemm(a: torch.Tensor, b: torch.Tensor, *, a_mn_major: bool = False, b_mn_maj
             and alpha == 1.0 and K % 8 == 0):
         # decoding: a few activation rows against a whole weight matrix is a stream of the weights, served by the
         # bandwidth-shaped kernel instead of 128-row tensor-core tiles: at 16 rows, where it ends, 6144 x 2560 take 9.3 us there and
-        # 11.9 on the split-K kernel below, 2560 x 9728 12.3 and 15.4
+        # 9.7 on the kernel below that takes all rows as a tile, 2560 x 9728 12.3 and 13.2
         # (its tensor maps take no pitch of zero: expanded rows are written out first)
         a, b = (t if t.stride(0) > 0 or t.shape[0] == 1 else t.contiguous() for t in (a, b))
         _lib.call("ksa_gemv_bf16", a, b, out, M, N, K, a.stride(0), b.stride(0), out.stride(0))
