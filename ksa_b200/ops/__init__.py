@@ -203,6 +203,16 @@ def _weight_grad(weight: torch.Tensor, compute):
     return compute(None, False)
 
 
+def _share_memory(a: Optional[torch.Tensor], b: Optional[torch.Tensor]) -> bool:
+    """Whether the address ranges of two tensors overlap (rows that only interleave count as well)."""
+    def span(t):
+        return t.data_ptr(), t.data_ptr() + (1 + sum((n - 1) * s for n, s in zip(t.shape, t.stride()))) * t.element_size()
+    if a is None or b is None or a.numel() == 0 or b.numel() == 0:
+        return False
+    (a0, a1), (b0, b1) = span(a), span(b)
+    return a0 < b1 and b0 < a1
+
+
 def _linear_weight_grad(weight: torch.Tensor, dy: torch.Tensor, x: torch.Tensor, lo: int, hi: int, beside: bool = False):
     """The gradient of ``weight`` in ``x[lo:hi] @ weight.T``, routed by :func:`_weight_grad`.  ``beside``: the caller has just
     launched another product of the same tensors, which this one need not wait for (``launch_beside`` in ``csrc/host.h``)."""
@@ -303,8 +313,11 @@ class _DualLinearFn(torch.autograd.Function):
             if not need or hi <= lo:
                 grads.append(None)
                 continue
-            # the text rows' gradients were launched above, from the same dy and x and into other buffers
-            grads.append(_linear_weight_grad(w, dy, x, lo, hi, beside=lo > 16 and (dx is not None or grads[0] is not None)))
+            # the text rows' gradients were launched above, from the same dy and x; the summary rows' need not wait for them where they go
+            # into another buffer.  One weight for both kinds of rows, or two whose gradients share memory: the second adds to the first.
+            beside = lo > 16 and (dx is not None or grads[0] is not None) and not _share_memory(
+                getattr(w_a, "main_grad", None), getattr(w, "main_grad", None))
+            grads.append(_linear_weight_grad(w, dy, x, lo, hi, beside=beside))
         return dx, grads[0], grads[1], None
 
 
