@@ -322,10 +322,17 @@ __device__ __forceinline__ void grid_dependency_enter() {
   grid_dependency_wait();
   grid_dependency_launch();
 }
+// In place of the wait, for a kernel that runs beside the one before it: what that kernel's own predecessors wrote is complete, but this grid
+// has not waited for it, so nothing has told this SM to forget older copies.  The first fence keeps loads that follow from lines that the
+// SM held before, the second orders TMA loads behind it.
+__device__ __forceinline__ void grid_dependency_observe() {
+  asm volatile("fence.acq_rel.gpu;\n\tfence.proxy.async.global;" ::: "memory");
+}
 // The same for a kernel that may run beside the one before it (host.h: launch_beside): it waits only before it ends, in one block, so that
 // whoever waits for it has waited for both.  The other blocks leave and make room as they finish.
 __device__ __forceinline__ void grid_dependency_enter(int beside) {
-  if (!beside) grid_dependency_wait();
+  if (beside) grid_dependency_observe();
+  else grid_dependency_wait();
   grid_dependency_launch();
 }
 __device__ __forceinline__ void grid_dependency_leave(int beside) {

@@ -81,7 +81,7 @@ enum StreamMode {
   kStWaits,      // before it reads anything; the successor of a block's first product (a norm, SwiGLU) starts behind that, and so may
                  // take weights to be as they are for good (ops.linear_of_block: a feed-forward block of one row 32.3 -> 31.4 us)
   kStEarly,      // weights_early(): the weights are read before the previous kernel has ended, and the successor starts at once
-  kStBeside,     // launch_beside(): before it ends
+  kStBeside,     // launch_beside(): before it ends; all that it reads of global memory goes through the producer
 };
 // NB: batch blocks of 8 rows, 1 (M <= 8) or 2 (M <= 16)
 template <int NB, bool kGlu, bool kNorm, StreamMode kMode>
@@ -156,6 +156,7 @@ stream_gemm_kernel(const __grid_constant__ CUtensorMap tmB, const __grid_constan
     };
     // in a decode step weights do not depend on the previous kernel; the activations do
     if (kMode == kStWaits) grid_dependency_wait();
+    if (kMode == kStBeside) grid_dependency_observe();
     if (!kAtOnce) grid_dependency_launch();
     const int ahead = min(p.stages, n_items);
     for (int it = 0; it < ahead; ++it) load_weights();
@@ -438,9 +439,10 @@ gemv_kernel(const bf16* A, const bf16* B, bf16* C, int M, int N, int K,
   };
   // in a decode step weights are not written by an earlier kernel of the stream: ask for the first chunks, then wait for the
   // kernel that produces the activations
-  if (!kBeside && !early) grid_dependency_wait();
+  if (kBeside) grid_dependency_enter(1);
+  else if (!early) grid_dependency_wait();
   load_w(0, min(kGemvKTile, K), lane * 8);
-  grid_dependency_enter((int)kBeside);
+  if (!kBeside) grid_dependency_enter();
 
   for (int k0 = 0; k0 < K; k0 += kGemvKTile) {
     const int kt = min(kGemvKTile, K - k0);          // multiple of 8

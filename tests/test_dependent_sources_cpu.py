@@ -38,3 +38,20 @@ def test_kernels_that_start_early_promise_nothing_about_their_memory():
     kernels = [(n, h) for n, h, body in SOURCES if "__global__" in h and "grid_dependency_" in body]
     assert len(kernels) >= 25
     assert not [(n, h) for n, h in kernels if "__restrict__" in h]
+
+
+def test_kernels_that_run_beside_another_read_nothing_that_an_sm_kept_from_before():
+    """They have not waited when they read, so the fences that stand in for the wait come before anything else they do with memory."""
+    common = [body for header, body in _functions((CSRC / "common.cuh").read_text()) if "grid_dependency_enter(int beside)" in header]
+    assert len(common) == 1 and re.match(r"\s*if \(beside\) grid_dependency_observe\(\);\s*else grid_dependency_wait\(\);", common[0])
+    checked = 0
+    for name, header, body in SOURCES:
+        if "grid_dependency_leave(" not in body:
+            continue
+        checked += 1
+        at = re.search(r"grid_dependency_observe\(\)|grid_dependency_enter\([^)]+\)", body)
+        assert at, (name, header[-120:])
+        reads = re.finditer(r"\bload_w(?:eights)?\(|\bload_acts\(|tma_load_2d(?:_pair)?\(|const uint4\*>\((?:A |key_row)", body)
+        reads = [m.start() for m in reads]
+        assert reads and min(reads) > at.start(), (name, header[-120:])
+    assert checked >= 6
