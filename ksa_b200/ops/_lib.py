@@ -307,6 +307,7 @@ def gemm_tall_plan(M: int, N: int, K: int, glu: int, ragged: bool):
     return divmod(plan, 16) if plan else None
 
 
+@functools.lru_cache(maxsize=4096)
 def gemm_narrow_plan(M: int, N: int, K: int, glu: int, pair_min_tiles: int, ragged: int = 0):
     """``(activation rows per tile, split of K)`` for ``ksa_gemm_narrow_bf16``, or None where a tiled kernel is faster.
     ``ragged``: bit 0 for activations, bit 1 for weights whose row pitch is no multiple of 64 elements."""

@@ -12,3 +12,9 @@ from ksa_b200.ops import _lib
     (576, 4096, 9728, 2, (144, 2))])
 def test_plan(M, N, K, glu, plan):
     assert _lib.gemm_narrow_plan(M, N, K, glu, 32) == plan
+
+
+@pytest.mark.parametrize("plan,args", [(_lib.gemm_narrow_plan, (333, 2560, 4096, 0, 32)), (_lib.gemm_tall_plan, (48, 2560, 4096, 0, False))])
+def test_a_plan_is_searched_once(plan, args):
+    plan.cache_clear()
+    assert plan(*args) == plan(*args) and plan.cache_info()[:2] == (1, 1)         # hits, misses
