@@ -40,6 +40,7 @@ constexpr int k2BarrierBytes = 256;
 constexpr int k2SmemTotal = k2Stages * k2StageBytes + k2BarrierBytes + kBulkRingBytes + 1024;
 static_assert(kMaxPeers * kBulkSegs <= 32, "one bit per segment in the producers' bookkeeping");
 static_assert(k2SmemTotal <= 232448, "the operand ring, the barriers and the copy ring must fit 227 KB");
+static_assert(k2SmemTotal >= kTmemClusterAlone, "a pair holds all tensor memory: no block of another cluster beside it (host.h)");
 
 struct Gemm2Epilogue {
   void* c;

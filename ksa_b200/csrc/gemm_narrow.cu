@@ -217,11 +217,22 @@ gemm_narrow_kernel(const __grid_constant__ CUtensorMap tmW, const __grid_constan
 // 62.5 us on tiles of 160 rows in two parts, 42.9 on CTA pairs; 193 x 4256 x 3352 30.2 on 208 rows in four parts, 21.0).
 constexpr int kNwSms = 148;
 constexpr int kNwMaxRows = 2048;   // the model holds near the range that it was fitted to (8000 x 128 x 2048: 27.4 against 15.3 us)
-static bool narrow_two_per_sm(int bt) { return 3 * (kNwWBytes + bt * kNwBK * 2) <= 110 * 1024; }
-static int narrow_stages(int bt) {
+static constexpr bool narrow_two_per_sm(int bt) { return 3 * (kNwWBytes + bt * kNwBK * 2) <= 110 * 1024; }
+static constexpr int narrow_stages(int bt) {
   const int stages = (narrow_two_per_sm(bt) ? 110 : 220) * 1024 / (kNwWBytes + bt * kNwBK * 2);
   return stages < kNwMaxStages ? stages : kNwMaxStages;
 }
+// the ring, or the partial tile that takes its place
+static constexpr int narrow_smem(int bt) {
+  const int ring = narrow_stages(bt) * (kNwWBytes + bt * kNwBK * 2), part = bt * 128 * 4;
+  return (ring > part ? ring : part) + 1024;
+}
+static constexpr int narrow_least_smem() {
+  int least = narrow_smem(16);
+  for (int bt = 32; bt <= 256; bt += 16) least = narrow_smem(bt) < least ? narrow_smem(bt) : least;
+  return least;
+}
+static_assert(narrow_least_smem() >= kTmemClusterLeast, "a smaller block would share an SM with clusters that count on its size");
 // CTAs that run with an SM to themselves, and CTAs resident at once.  A cluster stays within one group of SMs, and the groups' sizes
 // are no multiples of 4 and 8: 33 clusters of 4 and 15 of 8 with one CTA per SM (the occupancy query's answer and the
 // grids at which the time jumps), 70 and 33 with two (the grids at which it jumps).
@@ -305,9 +316,7 @@ static int launch_narrow(const void* x, const void* w, NarrowArgs p, long long l
   }
   // two CTAs per SM while a ring of three stages fits half of its shared memory, else one with a deeper ring
   p.stages = narrow_stages(p.bt);
-  const int part_bytes = p.bt * 128 * 4;
-  const int ring = p.stages * (kNwWBytes + p.bt * kNwBK * 2);
-  const int smem = (ring > part_bytes ? ring : part_bytes) + 1024;
+  const int smem = narrow_smem(p.bt);
   p.tmem_cols = 32;
   while (p.tmem_cols < p.bt) p.tmem_cols *= 2;
   p.tiles_m = (p.M + p.bt - 1) / p.bt;

@@ -285,10 +285,10 @@ static int launch_tall(const void* x, const void* w, TallArgs p, long long ldx, 
   cudaLaunchConfig_t cfg = {};
   cfg.gridDim = dim3(tiles * p.split);
   cfg.blockDim = dim3(kTlThreads);
-  // No room for a block of another cluster that holds tensor memory: each might wait for what the other's peer holds, for good.  The least
-  // such block is 85 KB (split-K kernel, tiles of 96 rows).
-  const int least = 150 * 1024, held = ring > parts ? ring : parts;
-  cfg.dynamicSmemBytes = (size_t)((held > least ? held : least) + 1024);
+  // all of the tensor memory: no room for a block of another cluster that holds some (host.h)
+  const int held = (ring > parts ? ring : parts) + 1024;
+  cfg.dynamicSmemBytes = (size_t)(held > kTmemClusterAlone ? held : kTmemClusterAlone);
+  static_assert(kTlRing + 1024 >= kTmemClusterAlone, "the limit raised above covers it");
   cfg.stream = st;
   cudaLaunchAttribute at[2];
   at[0].id = cudaLaunchAttributeClusterDimension;

@@ -86,6 +86,17 @@ int launch_mode();
 inline bool dependent_launches() { return launch_mode() != kLaunchOrdinary; }
 inline bool weights_early() { return launch_mode() == kLaunchEarlyWeights; }
 
+// Clusters whose blocks hold tensor memory: a block that finds none left on its SM waits without a limit, while the rest of its cluster waits
+// for it.  Two clusters from two streams could so wait for one another's blocks, for good, unless no two blocks of theirs
+// that might want more tensor memory than there is find room in an SM's shared memory.  So every such block takes at least kTmemClusterLeast
+// (the least is split-K, csrc/gemm_narrow.cu: tiles of 96 rows), which leaves room for two, and one that takes more than half of the
+// tensor memory also takes kTmemClusterAlone, which leaves none for another.
+constexpr int kSmSharedBytes = 228 * 1024;           // of which every block costs 1024 besides its own
+constexpr int kTmemClusterLeast = 85 * 1024;
+constexpr int kTmemClusterAlone = kSmSharedBytes - kTmemClusterLeast;
+static_assert(3 * (kTmemClusterLeast + 1024) > kSmSharedBytes && kTmemClusterLeast + kTmemClusterAlone + 2 * 1024 > kSmSharedBytes,
+              "two blocks of half the tensor memory each, or one alone");
+
 // Two kernels of one call that do not depend on one another (text rows and summary rows: other inputs' rows, other outputs) need not
 // run one after the other.  After ksa_set_launch_beside(1), products and summary attention are launched to start as soon as every block of the
 // kernel before them has begun its work, and wait for its end only before their own.  That is sound because a kernel begins its

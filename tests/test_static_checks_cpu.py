@@ -1,8 +1,10 @@
 """Static checks of the Python sources that guard the branches only a GPU run reaches: every kernel entry point is
-called with as many arguments as its prototype takes, and no function reads a global name that nothing defines."""
+called with as many arguments as its prototype takes, and no function reads a global name that nothing defines; and of a size that kernels
+in several files have to agree on."""
 import ast
 import builtins
 import pathlib
+import re
 import symtable
 
 from ksa_b200.ops import _lib
@@ -82,3 +84,13 @@ def test_no_function_reads_a_name_that_nothing_defines():
     for f in SOURCES + sorted((ROOT / "tests").glob("*.py")):
         problems += _undefined(f, f.read_text())
     assert not problems, problems
+
+
+def test_clusters_that_hold_tensor_memory_keep_to_the_shared_memory_rule():
+    """Two such clusters may wait for one another's blocks for good unless host.h's sizes hold; each file is checked against them when it is built."""
+    csrc = ROOT / "ksa_b200" / "csrc"
+    clusters = {f.name: f.read_text() for f in csrc.glob("*.cu")
+                if "tmem_alloc" in f.read_text() and ("ClusterDimension" in f.read_text() or "__cluster_dims__" in f.read_text())}
+    assert len(clusters) >= 3
+    for name, text in clusters.items():
+        assert re.search(r"static_assert\([^;]*>= kTmemCluster(Least|Alone)", text), name
