@@ -299,7 +299,7 @@ KSA_API int ksa_gemm_bf16(const void* a, const void* b, void* c, int M, int N, i
   KSA_REQUIRE(!(accumulate && !out_fp32), "gemm: accumulate needs an fp32 output");
   GemmEpilogue ep{c, ldc, out_fp32, accumulate, alpha, launch_beside()};
   cudaStream_t st = reinterpret_cast<cudaStream_t>(stream);
-  const bool wide = (N >= 256) && (((long long)((M + 127) / 128) * ((N + 255) / 256)) >= 96 || N % 256 == 0);
+  const bool wide = gemm_wide_tiles(M, N);
 #define KSA_GEMM_DISPATCH(BN)                                                                        \
   if (!a_mn_major && !b_mn_major) return launch_gemm<BN, false, false>(a, b, ep, M, N, K, lda, ldb, sm_limit, st); \
   if (!a_mn_major && b_mn_major) return launch_gemm<BN, false, true>(a, b, ep, M, N, K, lda, ldb, sm_limit, st);   \

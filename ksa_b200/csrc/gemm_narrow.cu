@@ -8,8 +8,9 @@
 //     memory, each CTA a share of the rows: no workspace, no atomics, no second launch.
 // Measured against 128 x 256 tiles on single CTAs (weights from memory): 48 rows x 2560 x 9728 58.5 -> 18.1 us, 333 rows 61.1 ->
 // 28.9, 48 rows x 6144 x 2560 20.1 -> 14.1; with the activation, 48 rows x 19456 x 2560 36.2 -> 23.1 (two launches -> one).
-// The weights alone take 7.6, 7.6, 4.8 and 15.2 us at the copy bandwidth.  Row-major weights of up to 256 rows go to csrc/gemm_tall.cu now (13.2
-// us for the first of these), which reads the activations again for every tile; from there on this one has the better balance.
+// The weights alone take 7.6, 7.6, 4.8 and 15.2 us at the copy bandwidth.  Row-major weights whose rows start on 128-byte lines go to
+// csrc/gemm_tall.cu where that gives no CTA too many of them (13.2 us for the first of these; ksa_gemm_tall_plan), [K, N] weights of any number of rows
+// and the rest stay here, most from 257 rows on, as that kernel reads the activations again for every tile.
 // Roles per CTA (192 threads): warp 0 TMA producer, warp 1 MMA issuer, warps 2..5 move the accumulator to shared
 // memory, and all of them write the result.  One tile per CTA.  No TMA load uses multicast; every wait is bounded.
 //
@@ -199,22 +200,23 @@ gemm_narrow_kernel(const __grid_constant__ CUtensorMap tmW, const __grid_constan
   grid_dependency_leave(p.beside);
 }
 
-// Tile height and split for a product, and its time in microseconds as modelled.  The figures were fitted to 4176 measured (shape, height,
-// split) triples of 288 to 2048 rows against 512 x 4096 .. 9728 x 2560 weights in both layouts, the last two items to 900 shapes of
-// 17 to 2048 rows and 64 to 19456 x 64 to 12288 weights:
-//   * one 64-wide step of K takes a CTA that has an SM to itself 0.241 + 0.00054 bt us (the latency of its loads) and two that share
-//     one 2 x (0.093 + 0.00094 bt), so a grid should fill both slots of every SM; a ring for more than 160 rows leaves
-//     room for one CTA only;
-//   * the weights of all CTAs come through the L2 at 16 TB/s, with the activations at 21.9;
-//   * a launch costs 1.4 us, a wave of CTAs 3.6 us to start and drain, and 0.013 + 0.0043 split per activation row to write
-//     and add up;
+// Tile height and split for a product, and its time in microseconds as modelled.  The figures were fitted to 10551 measured (shape, height,
+// split) triples of 1650 products of 2 to 2048 rows with 64 to 24000 x 64 to 12288 weights in both layouts, 74 % of them with
+// rows off the 128-byte lines:
+//   * one 64-wide step of K takes a CTA that has an SM to itself 1.05 us over the stages of its ring (the latency of its loads), and CTAs
+//     that share an SM 0.078 + 0.00102 bt each, so a grid should fill both slots of every SM; a ring for more than 160 rows leaves room for
+//     one CTA only, but has five stages again;
+//   * operands of all CTAs come through the L2 at 23 TB/s, the weights from memory at 5, at 5.7 in a single wave;
+//   * a wave of CTAs costs 3.2 us to start and drain, and 0.0175 + 0.0035 split per activation row to write and add up;
 //   * clusters of 4 and 8 do not fill every SM: narrow_first and narrow_slots below;
-//   * rows that do not start on a 128-byte line take a second line for every box row: weights and activations then come
-//     through the L2 at 21 TB/s as 1.86 and 1.55 times their bytes.
-// The model's standard deviation is 8 %; over those 270 products the choice (tiled kernels included) is 1.2 % above the best on average,
-// against 3.3 % with the figures of before the issuing threads were elected, and 2 % faster: 333 x 2560 x 4096 19.8 -> 15.6 us, 576 x 2560 x 9728
-// 37.9 -> 31.2, 700 x 2048 x 12288 40.7 -> 34.9.  Without the last two items 21 of the 900 shapes were up to 30 % slower (779 x 3552 x 6008:
-// 62.5 us on tiles of 160 rows in two parts, 42.9 on CTA pairs; 193 x 4256 x 3352 30.2 on 208 rows in four parts, 21.0).
+//   * less than eight steps are not split from 65 rows on, so that their sums are those of the tiled kernels whatever the number of rows (512
+//     x 512 x 256 5.7 us on tiles, 5.0 here, 4.5 in two parts);
+//   * rows that do not start on a 128-byte line take a second line for every box row, weights and activations 1.82 and 1.87 times their
+//     bytes: in full through the L2, for three quarters of it in what CTAs that share an SM take, for a fifth in the latency.
+// The model's standard deviation is 9 %; over the 1650 products the choice (tiled kernels included) is 1.0 % above the best on average, 4 % faster
+// than the first one, fitted to 17 to 1411 rows of the presets' widths, and one product in a hundred more than 5 % slower than that; figures fitted to
+// 288 to 2048 rows alone, with the tiled kernels at 128 x 256 throughout, were 2.7 % above the best and slower in one of twenty-two: 62 x
+// 1704 x 416 4.3 us on tiles and 5.4 here, 1151 x 1184 x 8472 39.5 with 192 rows and 45.7 with 240, 310 x 3840 x 4096 17.4 and 19.4.
 constexpr int kNwSms = 148;
 constexpr int kNwMaxRows = 2048;   // the model holds near the range that it was fitted to (8000 x 128 x 2048: 27.4 against 15.3 us)
 static constexpr bool narrow_two_per_sm(int bt) { return 3 * (kNwWBytes + bt * kNwBK * 2) <= 110 * 1024; }
@@ -241,14 +243,18 @@ static int narrow_slots(int bt, int split) {
   if (!narrow_two_per_sm(bt)) return narrow_first(split);
   return split <= 2 ? 2 * kNwSms : split == 4 ? 280 : 264;
 }
-static double narrow_plan(int M, long long n_tiles, int K, bool ragged_x, bool ragged_w, int* bt_out, int* split_out) {
+static double narrow_plan(int M, int N, long long n_tiles, int K, bool ragged_x, bool ragged_w, int* bt_out, int* split_out) {
   const int num_kb = (K + kNwBK - 1) / kNwBK, fewest = (M + 255) / 256;
-  double best = 1e30;
+  const double weights = (double)N * K * 2e-6;
+  double best = 1e30, best_t = 1e30;
   for (int tm = fewest; tm < fewest + 9; ++tm) {
     const int bt = ((M + tm - 1) / tm + 15) / 16 * 16;
     if (tm > fewest && bt < 48) break;
     const int per_sm_most = narrow_two_per_sm(bt) ? 2 : 1;
+    const double bytes = kNwWBytes + bt * kNwBK * 2;
+    const double lines = (kNwWBytes * (ragged_w ? 1.82 : 1.0) + bt * kNwBK * 2 * (ragged_x ? 1.87 : 1.0)) / bytes - 1.0;
     for (int split = 1; split <= 8 && split <= num_kb; split *= 2) {
+      if (split > 1 && M > 64 && num_kb < 8) break;
       const long long ctas = (long long)((M + bt - 1) / bt) * n_tiles * split;
       const double steps = (num_kb + split - 1) / split;
       const int slots = narrow_slots(bt, split), first = narrow_first(split);
@@ -256,19 +262,14 @@ static double narrow_plan(int M, long long n_tiles, int K, bool ragged_x, bool r
         if (n == 0) return 0.0;
         const long long rounds = (n + first - 1) / first;
         const double per_sm = (double)(rounds < per_sm_most ? rounds : per_sm_most);
-        double step = per_sm * (0.093 + 0.00094 * bt);
-        if (step < 0.241 + 0.00054 * bt) step = 0.241 + 0.00054 * bt;
-        if (step < n * 0.00102) step = n * 0.00102;
-        const double all = n * (kNwWBytes + bt * kNwBK * 2.0) / 21.9e6;
-        if (step < all) step = all;
-        if (ragged_x || ragged_w) {
-          const double bytes = kNwWBytes * (ragged_w ? 1.86 : 1.0) + bt * kNwBK * 2 * (ragged_x ? 1.55 : 1.0);
-          if (step < n * bytes / 21e6) step = n * bytes / 21e6;
-        }
-        return 3.6 + steps * step + per_sm * bt * (0.013 + (split > 1 ? 0.0043 * split : 0.0)) + (split == 8 ? 0.26 : 0.0);
+        const double shared = per_sm * (0.078 + 0.00102 * bt) * (1 + 0.76 * lines), alone = 1.05 / narrow_stages(bt) * (1 + 0.21 * lines);
+        const double l2 = n * bytes * (1 + lines) / 23.2e6;
+        const double step = shared > alone ? (shared > l2 ? shared : l2) : (alone > l2 ? alone : l2);
+        return 3.2 + steps * step + per_sm * bt * (0.0175 + (split > 1 ? 0.0035 * split : 0.0));
       };
-      const double t = 1.36 + (double)(ctas / slots) * wave(slots) + wave(ctas % slots);
-      if (t < best) { best = t; *bt_out = bt; *split_out = split; }
+      const double t = (double)(ctas / slots) * wave(slots) + wave(ctas % slots), memory = 4.0 + weights / (ctas <= slots ? 5.7 : 5.0);
+      const double all = t > memory ? t : memory;
+      if (all < best || (all == best && t < best_t)) { best = all; best_t = t; *bt_out = bt; *split_out = split; }
     }
   }
   return best;
@@ -282,20 +283,32 @@ static bool enough_for_pairs(int M, int N, int pair_min_tiles) {
 static bool on_pairs(int M, int N, int pair_min_tiles) {
   return enough_for_pairs(M, N, pair_min_tiles) && 2 * tiled_waves(M, N, 256, kNwSms / 2) < 3 * tiled_waves(M, N, 128, kNwSms);
 }
-// The time of the tiled kernel that serves the same product otherwise: 0.327 us a 64-wide step and wave of 74 CTA pairs with 256 x 256
-// tiles, 6.7 us around them.  Single CTAs with 128 x 256 tiles take 0.352 a step and wave and 5.6 around them where there are too few tiles for
-// pairs (16.4 us measured for 900 x 2048 x 2048, 60.5 for 576 x 2560 x 9728).  Where they are taken for their fewer waves, most SMs have a
-// tile: 5.7 us and, a step and wave, 0.364 and 0.057 for every megabyte of weights that the step's tiles read: 333 x 4096 x 2048 16.4 us
-// (0.5 MB), 333 x 12288 x 2048 21.2 (1.6 MB), 128 x 19456 x 2560 26.2 (2.5 MB).
-// glu: and of the separate activation kernel, 2 us and more, 2.8 to 3.7 behind the products of the last kind.
-static double tiled_time(int M, int N, int K, bool glu, int pair_min_tiles) {
-  const long long num_kb = (K + 63) / 64;
-  const double act = glu ? 2.0 : 0.0;
-  if (on_pairs(M, N, pair_min_tiles)) return act + 6.7 + 0.327 * num_kb * tiled_waves(M, N, 256, kNwSms / 2);
-  const double steps = (double)(num_kb * tiled_waves(M, N, 128, kNwSms));
-  if (!enough_for_pairs(M, N, pair_min_tiles)) return act + 5.6 + 0.352 * steps;
-  const long long tm = (M + 127) / 128, tn = (N + 255) / 256, abreast = (kNwSms + tm - 1) / tm;      // tiles of a row in one wave
-  return (glu ? 3.5 : 0.0) + 5.7 + (0.364 + 0.057 * (tn < abreast ? tn : abreast) * 256 * kNwBK * 2 / 1e6) * steps;
+// The time of the tiled kernel that serves the same product otherwise, fitted to the same products (12 %).  74 CTA pairs with 256 x 256 tiles take
+// 0.3 us a 64-wide step, 2.1 a wave and 3.6 around them, a last wave of halves 0.7 of that.  Single CTAs with 128 x 256 tiles take 0.31 to 0.47 a
+// step, the more of the SMs have a tile, 4.5 around them and 2.4 between waves, those with 128 x 128 tiles 0.18 to 0.26, 3.1 and 1.2.
+// Weights come from memory at 5.2 and 5 TB/s.
+// glu: 1, and of the separate activation kernel, 3 us and the way of what it reads; 2, on pairs that apply it themselves, a microsecond more a wave and no halves.
+static double tiled_time(int M, int N, int K, int glu, int pair_min_tiles, bool ragged_x, bool ragged_w) {
+  const double num_kb = (double)((K + 63) / 64), weights = (double)N * K * 2e-6, act = glu == 1 ? 3.0 + 2.5e-7 * M * N : 0.0;
+  if (on_pairs(M, N, pair_min_tiles)) {
+    const long long tiles = (long long)((M + 255) / 256) * ((N + 255) / 256), last = tiles % (kNwSms / 2);
+    const double waves = (double)(tiles / (kNwSms / 2)) + (last == 0 ? 0.0 : 2 * last <= kNwSms / 2 && glu != 2 ? 0.7 : 1.0);
+    const double step = 0.3 * (1 + (ragged_x ? 0.1 : 0.0) + (ragged_w ? 0.04 : 0.0));
+    const double t = 3.6 + waves * (step * num_kb + (glu == 2 ? 3.1 : 2.1));
+    return act + (t > weights / 5.2 ? t : weights / 5.2);
+  }
+  const bool wide = gemm_wide_tiles(M, N);
+  const int bn = wide ? 256 : 128;
+  const long long tiles = (long long)((M + 127) / 128) * ((N + bn - 1) / bn);
+  const double waves = (double)((tiles + kNwSms - 1) / kNwSms), busy = tiles < kNwSms ? tiles / (double)kNwSms : 1.0;
+  const double step = (wide ? 0.31 + 0.16 * busy : 0.18 + 0.083 * busy) * (1 + (ragged_x ? 0.16 : 0.0) + (ragged_w ? 0.34 : 0.0));
+  const double t = (wide ? 4.5 : 3.1) + waves * step * num_kb + (waves - 1) * (wide ? 2.4 : 1.2), memory = 3.5 + weights / 5.0;
+  return act + (t > memory ? t : memory);
+}
+double few_rows_time(int M, int N, int K) {
+  int bt = 0, split = 0;
+  const double narrow = narrow_plan(M, N, (N + 127) / 128, K, false, false, &bt, &split), tiled = tiled_time(M, N, K, 0, 0, false, false);
+  return narrow < tiled ? narrow : tiled;
 }
 
 template <bool W_MN, bool kGlu>
@@ -383,16 +396,20 @@ KSA_API int ksa_gemm_on_pairs(int M, int N, int pair_min_tiles) {
 }
 
 // Whether this kernel is expected to beat the tiled ones (of which CTA pairs are taken from `pair_min_tiles` 256 x 256 tiles on, 0:
-// never), by more than 4 %, with K in one part by more than 8 (900 x 2048 x 2048 16.4 us on tiles and 17.5 here): bt * 16 + split for
-// ksa_gemm_narrow_bf16, or 0, as for weights of less than 64 KB, where nothing but the launch takes time.  glu: the separate activation
-// kernel counts on the other side; 2: it counts on this side, as CTA pairs apply it themselves.  ragged: bit 0, the activations' rows do not all start on a 128-byte line (their
-// pitch is no multiple of 64 elements); bit 1, those of the weights as they lie in memory.
+// never): bt * 16 + split for ksa_gemm_narrow_bf16, or 0, as for weights of less than 64 KB, where nothing but the launch takes time.  By 5 % at
+// least, but up to 64 rows with weights wide enough for pairs, whose tiled kernels take the longer the fewer of a tile's rows are there, which the
+// model does not know, also where it is modelled slower (112 such products: always faster here; 32 x 15856 x 9728 49.5 us and 56.3 on
+// pairs, 5 x 18408 x 6144 35.3 and 55.6, 4 x 19456 x 1024 10.3 and 15.2 on single CTAs, with the activation 18 x 2 x 9472 x 2560 21.3 and 29.0).
+// glu: 1, the gated form, one launch against the tiled kernels' two (then small weights of more than one step are worth it as well: 96 x 2 x 88 x 168 4.8 us and 5.5);
+// 2, the plain form and a separate activation, 2 us, against CTA pairs, which apply it themselves (77 x 2 x 4864 x 2048 15.2 us and 16.8, 429 x 2 x
+// 4864 x 4096 39.4 and 45.7; over 118 products the choice is 2.5 % above the better of both on average, always pairs 9 %, never pairs 16 %).
+// ragged: bit 0, the activations' rows do not all start on a 128-byte line (their pitch is no multiple of 64 elements); bit 1, those of
+// the weights as they lie in memory.
 KSA_API int ksa_gemm_narrow_plan(int M, int N, int K, int glu, int pair_min_tiles, int ragged) {
   using namespace ksa;
-  if (M <= 0 || M > kNwMaxRows || N <= 0 || K <= 0 || (long long)N * K < 32768) return 0;
+  if (M <= 0 || M > kNwMaxRows || N <= 0 || K <= 0 || (glu == 1 ? K <= kNwBK : (long long)N * K < 32768)) return 0;
   int bt = 0, split = 0;
-  const bool gated = glu == 1;
-  double t = narrow_plan(M, gated ? (N / 2 + 63) / 64 : (N + 127) / 128, K, (ragged & 1) != 0, (ragged & 2) != 0, &bt, &split);
-  if (glu == 2) t += 3.0;
-  return t < (split == 1 ? 0.92 : 0.96) * tiled_time(M, N, K, gated, pair_min_tiles) ? bt * 16 + split : 0;
+  const bool rx = (ragged & 1) != 0, rw = (ragged & 2) != 0;
+  const double t = narrow_plan(M, N, glu == 1 ? (N / 2 + 63) / 64 : (N + 127) / 128, K, rx, rw, &bt, &split) + (glu == 2 ? 2.0 : 0.0);
+  return t < (M <= 64 && enough_for_pairs(M, N, pair_min_tiles) ? 1.4 : 0.95) * tiled_time(M, N, K, glu, pair_min_tiles, rx, rw) ? bt * 16 + split : 0;
 }

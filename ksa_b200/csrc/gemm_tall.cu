@@ -345,7 +345,7 @@ static double tall_time(int rows, int blocks, int steps, int columns, int split,
   for (double t : terms) step = t > step ? t : step;
   return 2.1 + steps * step + (split > 1 ? 1.7 + 2.2e-4 * rows * columns : 2.6e-4 * rows * columns);
 }
-static int tall_split_plan(int M, int N, int K) {
+static int tall_split_plan(int M, int N, int K, double* time) {
   const int blocks = (M + 127) / 128, rows = (M + 7) / 8 * 8, num_kb = (K + kTlBK - 1) / kTlBK;
   double best = 1e30;
   int plan = 0;
@@ -356,6 +356,7 @@ static int tall_split_plan(int M, int N, int K) {
     const double t = tall_time(rows, blocks, (num_kb + split - 1) / split, columns, split, tiles * split);
     if (t < best) { best = t; plan = columns * 16 + split; }
   }
+  *time = best;
   return plan;
 }
 }  // namespace ksa
@@ -365,13 +366,18 @@ static int tall_split_plan(int M, int N, int K) {
 //   * plain, up to 128 rows: always (2560 x 9728 48 rows 17.7 -> 13.3, 128 rows 19.6 -> 14.5; 2560 x 4096 48 rows 10.7 -> 8.7; 6144 x 2560 48 rows
 //     13.2 -> 10.0; 128 x 2560 7.5 -> 6.8; 10240 x 2560 128 rows 19.8 -> 13.1) to 96 columns a CTA without a split, and the output head, several
 //     tiles to an SM from 160 columns on, as nothing covers the time between them (151936 x 2560 128 rows 195 -> 154; with 128 columns, 2 x 18944 x
-//     3584 48 rows 47.3 -> 48.3).  What lies between is gate and up rows, which come with SwiGLU.
+//     3584 48 rows 47.3 -> 48.3).  What lies between stays where it was, gate and up rows without SwiGLU for the most part, though it would
+//     gain here too: 22 x 15080 x 2560 15.9 -> 14.3, 40 x 19456 x 3840 27.5 -> 25.8, 84 x 19456 x 1280 14.7 -> 11.0, 81 x 19456 x 9728 76 -> 62.
 //   * plain, up to 256 rows: to 80 columns (2560 x 9728 256 rows 26.7 -> 19.5; 10240 x 2560 19.8 -> 18.2; 12288 x 2048 17.9 -> 18.0)
-//   * plain, up to 384 rows: a long K and few columns (2560 x 9728 333 rows 28.8 -> 24.5, 2048 x 6144 17.8 -> 16.8, but 4096 x 12288 40.0 ->
-//     43.5), or very few (1024 x 2560 11.1 -> 9.1); 2048 x 2048 384 rows 11.0 -> 11.1.  Weights of fewer than eight tiles of 16 are nobody's case.
+//   * plain, up to 384 rows: to 112 columns a CTA with K in four parts, where the model above is at most 8 % over those of the other kernels, from
+//     300 columns and a longer K on up to 20 %, as it is itself high there, the more the longer K (9 % over 233 such products of up to 6000 x
+//     12288): 333 x 2560 x 9728 28.8 -> 24.5, 328 x 2048 x 6144 16.9 -> 16.0, 290 x 640 x 4096 10.0 -> 9.2; but 357 x 152 x 512 4.5 -> 5.8,
+//     334 x 152 x 12288 11.2 -> 13.5, 346 x 1024 x 1024 6.2 -> 6.8, 333 x 2560 x 4096 14.2 -> 15.7.  3.6 % above the best on average, one in forty
+//     more than 5 % slower than without this kernel.  Weights of fewer than eight tiles of 16 are nobody's case.
 //   * SwiGLU: the smallest tile that gives no SM more tiles than another, from 48 columns on (2 x 3072 x 1024, 48: 48 rows 8.5 -> 7.2, 256 rows 18.9 ->
-//     9.3; 2 x 1536 x 2048, 32: 130 rows 9.7 -> 11.5); with fewer than 64 rows and a long K from 80 on (2 x 4608 x 4096, 64: 48 rows 17.5 -> 17.8); up
-//     to 224, with 256 there are too few stages (2 x 18944 x 3584 17 rows 46.1 -> 48.0, 2 x 14336 x 4096, 208: 48 rows 44.6 -> 43.5); above 128 rows up
+//     9.3; 2 x 1536 x 2048, 32: 130 rows 9.7 -> 11.5); with fewer than 64 rows and a long K from 80 on (2 x 4608 x 4096, 64: 48 rows 17.5 -> 17.8),
+//     as with more than 128 rows and K above 2560 (2 x 3072 x 4096, 48: 132 rows 16.1 -> 19.7, 256 rows x 6144 27.9 -> 29.3; 2 x 3072 x 2048 200 rows
+//     13.4 -> 11.9; 2 x 5920 x 4096, 80: 132 rows 25.3 -> 24.1); up to 224, with 256 there are too few stages (2 x 18944 x 3584 17 rows 46.1 -> 48.0, 2 x 14336 x 4096, 208: 48 rows 44.6 -> 43.5); above 128 rows up
 //     to 160 (2 x 14336 x 4096, 208: 130 rows 54.1 -> 61.4), up to 384 rows from 144 (2 x 9728 x 2560 384 rows 48.4 -> 39.5; 2 x 8960 x 1536, 128: 264
 //     rows 21.6 -> 23.0); four blocks of rows never (2 x 9728 x 2560 479 rows 55.7 -> 66.0).
 // ragged: rows off the 128-byte lines, which the split-K kernel's model knows about.
@@ -382,10 +388,13 @@ KSA_API int ksa_gemm_tall_plan(int M, int N, int K, int glu, int ragged) {
   const long long rows = (glu ? 2LL : 1LL) * N, waves = (rows + (long long)kTlSms * most - 1) / ((long long)kTlSms * most);
   const int columns = (int)(((rows + kTlSms * waves - 1) / (kTlSms * waves) + 15) / 16 * 16);
   if (!glu && waves == 1) {
-    const bool taken = blocks == 1 ? columns <= 96 : blocks == 2 ? columns <= 80 : N <= 1056 || (N <= 33 * 112 && K >= 6144);
-    return taken ? tall_split_plan(M, N, K) : 0;
+    if (blocks == 1 ? columns > 96 : blocks == 2 ? columns > 80 : N > 33 * 112) return 0;
+    double time = 0;
+    const int plan = tall_split_plan(M, N, K, &time);
+    const double over = 1.08 + (N < 300 || K <= 3456 ? 0.0 : 4.3e-5 * ((K < 6144 ? K : 6144) - 3456));
+    return blocks <= 2 || time < over * few_rows_time(M, N, K) ? plan : 0;
   }
   if (waves > 1 && blocks > 1) return 0;
-  const int least = blocks == 3 ? 144 : waves > 1 ? 160 : M < 64 && K > 3072 ? 80 : 48;
+  const int least = blocks == 3 ? 144 : waves > 1 ? 160 : (M < 64 && K > 3072) || (blocks == 2 && K > 2560) ? 80 : 48;
   return columns >= least ? columns * 16 + 1 : 0;
 }

@@ -142,6 +142,13 @@ inline cudaError_t launch_stream_kernel(long long bytes, Kern kern, dim3 grid, d
   return launch_kernel_if(bytes <= kStreamedDependent, kern, grid, block, smem, st, args...);
 }
 
+// Whether the single-CTA kernel (csrc/gemm.cu) takes tiles of 128 x 256 for an M x N product, or of 128 x 128.
+inline bool gemm_wide_tiles(int M, int N) {
+  return N >= 256 && ((long long)((M + 127) / 128) * ((N + 255) / 256) >= 96 || N % 256 == 0);
+}
+// Modelled time in us of a row-major product on the split-K kernel or the single-CTA kernel, whichever is the faster (csrc/gemm_narrow.cu).
+double few_rows_time(int M, int N, int K);
+
 #define KSA_REQUIRE(cond, ...)                  \
   do {                                          \
     if (!(cond)) {                              \
