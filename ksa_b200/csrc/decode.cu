@@ -132,8 +132,8 @@ __global__ void __launch_bounds__(kDecThreads) decode_attn_kernel(DecodeArgs a) 
   if (tid < nq) {
     const int t = tid / G;
     const int st = a.start[b * a.Tq + t];
-    s_start[tid] = st;
-    s_end[tid] = st + a.len[b * a.Tq + t];
+    s_start[tid] = max(st, 0);
+    s_end[tid] = min(st + a.len[b * a.Tq + t], a.cap);     // whatever the device holds as slices: never past the cache
     m_s[tid] = -INFINITY;
     l_s[tid] = 0.f;
   }
@@ -268,7 +268,9 @@ __device__ __forceinline__ void decode_warp(const DecodeArgs& a, int split, int 
   // per-row (g and g+8) slice bounds, and the CTA's key range
   int st0 = 0, en0 = 0, st1 = 0, en1 = 0, lo = a.cap, hi = 0;
   for (int qi = 0; qi < nq; ++qi) {
-    const int s = a.start[b * a.Tq + qi / G], e = s + a.len[b * a.Tq + qi / G];
+    int s = a.start[b * a.Tq + qi / G];
+    const int e = min(s + a.len[b * a.Tq + qi / G], a.cap);      // whatever the device holds as slices: never past the cache
+    s = max(s, 0);
     lo = min(lo, s); hi = max(hi, e);
     if (qi == g) { st0 = s; en0 = e; }
     if (qi == g + 8) { st1 = s; en1 = e; }

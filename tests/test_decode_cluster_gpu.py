@@ -35,3 +35,19 @@ def test_slices(B, Tq, Hq, Hkv, cap):
         assert torch.equal(got, _decode_attention(q, k, v, start, length, D ** -0.5, counters))
     assert (counters == 0).all()
     _lib.check_status()
+
+
+@pytest.mark.parametrize("cap", [40, 1200, 2049])
+@pytest.mark.parametrize("D", [64, 128])
+def test_slices_end_with_the_cache(D, cap):
+    """A slice that a device value makes too long, or start too early, is cut: nothing outside the cache is read."""
+    torch.manual_seed(cap)
+    B, Hq, Hkv = 2, 8, 2
+    k, v = [torch.randn(B, Hkv, cap, D, device="cuda").bfloat16() for _ in range(2)]
+    q = torch.randn(B, 1, Hq, D, device="cuda").bfloat16()
+    at = lambda *x: torch.tensor(x, device="cuda").view(B, 1).int()
+    want = _decode_attention(q, k, v, at(0, cap - 10), at(cap, 10), D ** -0.5)
+    for far in (17, 100000, 2 ** 31 - 1 - cap):
+        assert torch.equal(want, _decode_attention(q, k, v, at(0, cap - 10), at(cap + far, 10 + far), D ** -0.5))
+    assert torch.equal(want, _decode_attention(q, k, v, at(-50, cap - 10), at(cap + 50, 10), D ** -0.5))
+    _lib.check_status()
