@@ -435,15 +435,21 @@ __global__ void __launch_bounds__(kDecThreads) decode_attn_mma_kernel(DecodeArgs
   combine_if_last(a, b, kvh, nq, G);
 }
 
-// Slices of caches of up to kDecClusterKeys keys (the ring and summaries of a summary layer, short contexts): the splits of a KV group are a
-// cluster, which shares each slice evenly and merges through its shared memory.  What bounds such a slice is the chain of latencies,
-// and the merge by the split that finishes last (partial results to global memory, a counter, all of them read back) was half of
-// it: a decode step of four sequences of 1030 keys through four layers and the head 424 -> 408 us, of
-// one 367 -> 351, of two of 330 keys 375 -> 356.  While a cluster of every group fits beside the others: with six sequences (384 CTAs) both take 428 us, with
-// sixteen 530 and 570.
+// Slices of short caches (the ring and summaries of a summary layer, short contexts): the splits of a KV group are a cluster, which shares
+// each slice evenly and merges through its shared memory.  What bounds such a slice is the chain of latencies, and the merge by the split
+// that finishes last (partial results to global memory, a counter, all of them read back) was half of it: a decode step of four
+// sequences of 1030 keys through four layers and the head 424 -> 408 us, of one 367 -> 351, of two of 330 keys 375 -> 356.
 // Four to eight warps a CTA are as good as one another; with twelve, which ask for all of a split's keys at once, the next projection finds no
 // room beside the CTAs and reads its weights late (448 us).  An L2 prefetch of the keys ahead of the wait changed nothing.
-constexpr int kDecClusterKeys = 2048;
+// Where the lines lie, in us of attention (32 heads) and the projection behind it, by the grid of splits and here:
+//   * a cluster of every group fits beside the others: of 8 groups a sequence, four sequences of 330 keys 17.9 -> 15.9, of 1130 20.7 -> 21.0, but five
+//     18.8 -> 19.2 and 20.8 -> 24.0, eight 19.3 -> 22.0 and 23.7 -> 27.4;
+//   * up to 2048 slots: one sequence of 2000 keys 18.9 -> 15.8, two 20.3 -> 17.0, three of 2018 20.7 -> 17.6, eight of four groups 34.5 -> 27.6.  What
+//     is in the cache is not known here, and the grid has as many splits as the cache takes: a long cache that is not full
+//     would gain as well (8192 slots, 1030 keys, four sequences 38.8 -> 20.4; 8000 keys 57.2 -> 51.8, but one 27.9 -> 30.4);
+//   * with more clusters' blocks than SMs and at most four queries a group to 1536, two rounds of a warp's keys: four sequences of 1506 keys 20.8 ->
+//     21.8, of 1634 21.5 -> 24.0, of 2018 21.9 -> 24.7.
+constexpr int kDecClusterKeys = 2048, kDecClusterKeysCrowded = 1536;
 constexpr int kDecCluster = 8;
 template <int NQ>
 constexpr int dec_cluster_warps() { return NQ <= 8 ? 6 : 4; }      // sixteen queries' outputs of four warps take 32 KB of shared memory
@@ -669,7 +675,9 @@ KSA_API int ksa_decode_attn(const void* q, const void* k_cache, const void* v_ca
   dim3 grid(splits, Hkv, B);
   cudaStream_t st = reinterpret_cast<cudaStream_t>(stream);
   const int nq = (Hq / Hkv) * Tq;
-  if (D == 128 && cap <= kDecClusterKeys && counters != nullptr && kDecCluster * Hkv * B <= 2 * sm_count()) {
+  const int blocks = kDecCluster * Hkv * B, sms = sm_count();
+  const bool crowded = blocks > sms && nq <= 4;
+  if (D == 128 && counters != nullptr && blocks <= 2 * sms && cap <= (crowded ? kDecClusterKeysCrowded : kDecClusterKeys)) {
     if (nq <= 4) return launch_decode_cluster<4>(a, st);
     return nq <= 8 ? launch_decode_cluster<8>(a, st) : launch_decode_cluster<16>(a, st);
   }

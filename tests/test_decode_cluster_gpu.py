@@ -51,3 +51,9 @@ def test_slices_end_with_the_cache(D, cap):
         assert torch.equal(want, _decode_attention(q, k, v, at(0, cap - 10), at(cap + far, 10 + far), D ** -0.5))
     assert torch.equal(want, _decode_attention(q, k, v, at(-50, cap - 10), at(cap + 50, 10), D ** -0.5))
     _lib.check_status()
+
+
+@pytest.mark.parametrize("cap", [1536, 1537])                 # by clusters and by the splits of a grid
+def test_more_blocks_than_multiprocessors(cap):
+    test_slices(4, 1, 32, 8, cap)
+    test_slices(3, 1, 64, 8, cap)                              # eight queries a group: clusters either way
