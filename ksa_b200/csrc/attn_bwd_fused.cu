@@ -26,9 +26,11 @@
 // What bounds it: the compute warps, 5200 cycles a step (probabilities 1600, dS^T 900, dQ^T to shared memory 1700 with the waits for the
 // reductions that read it), next to 4350 of shared memory at 128 bytes a cycle (operands of five products, both copies of dQ^T)
 // and 2560 of the tensor cores.  An SM's TMA engine reduces 26 bytes a cycle, 2500 cycles for a step's dQ^T, and without the reductions a
-// step takes 4700.  Against the form that waited for S^T and dP^T together and staged dQ^T in one buffer of 4 KB a warp: causal 8192 tokens
-// (16 heads) 960 -> 921 us, summary attention 8192 308 -> 301, 2 x 700 52.3 -> 49.3.  Slower: 16 compute warps (1065 us), dQ^T
-// added with plain reductions from registers (1004; half of it so 999).
+// step takes 4700.  Against the form that waited for S^T and dP^T together and staged dQ^T in one buffer of 4 KB a warp, one kernel between
+// those of a forward and backward pass, both with a grid head by head: causal 8192 tokens (16 heads) 947 -> 807 us (with the order of
+// grid_order() below 667), 2048 x 4 287 -> 262, summary attention 8192 (window of eight chunks) 264 -> 240, 32768 1049 -> 921, 2 x 700 46.5 -> 41.4.
+// Launched back to back for seconds, at the power limit: causal 8192 960 -> 921 (842), summary 8192 308 -> 301, 2 x 700 52.3 -> 49.3; there were
+// slower, against the 921: 16 compute warps (1065 us), dQ^T added with plain reductions from registers (1004; half of it so 999).
 //
 // Two small kernels surround it: a preparation pass (delta = rowsum(O * dO), scaled LSE, zeroing of the fp32
 // dQ buffer) and a conversion pass (dQ fp32 -> bf16, times the softmax scale).  The key-stationary order,
@@ -652,8 +654,8 @@ __global__ void attn_bwd_dq_convert_kernel(const float* dq32, bf16* dq, long lon
 
 // Blocks start in the order of their index, key tiles by ascending position.  Without a window, or with one that reaches over more than
 // a quarter of the sequence, a tile's number of queries falls with its position: all heads of the first tiles go first, so that
-// the longest blocks do not start last (causal 8192 tokens, 16 heads: 921 -> 842 us; 2048 x 4 308 -> 281; summary attention 2048 x 4
-// 260 -> 251, 4096 x 2 292 -> 287, 1111 x 3 105 -> 80).  Under a shorter window all blocks are as long as one another, and neighbouring
+// the longest blocks do not start last (causal 8192 tokens, 16 heads: 807 -> 667 us, 32 heads 1592 -> 1338, 2048 x 4 262 -> 211, summary
+// attention 2048 x 4 201 -> 181; back to back at the power limit 921 -> 842, 308 -> 281, 260 -> 251, summary 4096 x 2 292 -> 287, 1111 x 3 105 -> 80).  Under a shorter window all blocks are as long as one another, and neighbouring
 // tiles of one head share their queries in L2 while they run side by side (8192 tokens 305 against 301 us, 32768 1309 against 1249).
 static dim3 grid_order(FbParams& p, int text_tiles, int sum_blocks, bool one_shard) {
   const long long heads = (long long)p.s.Hkv * p.s.B, tiles = (long long)text_tiles + sum_blocks;

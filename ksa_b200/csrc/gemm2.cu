@@ -257,6 +257,8 @@ gemm2_bf16_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant
 #pragma unroll
             for (int a = 0; a < k2BM / 64; ++a) tma_load_2d_pair(sa + a * 8192, &tmA, row0 + a * 64, kb * k2BK, bar);
           }
+          // a box of 64 rows for halves, two for whole tiles: one of 128 there is no faster (8192 x 12288 x 2048 312.2 against 311.2 us, 8192 x
+          // 4096 x 2048 104.2 against 103.8, with SwiGLU 328.4 against 330.5, 1400 rows 64.4 against 64.5; the runs of one side differ by 1 %)
 #pragma unroll
           for (int a = 0; a < 2; ++a) {
             if (a >= boxes) break;
