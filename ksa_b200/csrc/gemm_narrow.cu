@@ -207,7 +207,9 @@ gemm_narrow_kernel(const __grid_constant__ CUtensorMap tmW, const __grid_constan
 //     that share an SM 0.078 + 0.00102 bt each, so a grid should fill both slots of every SM; a ring for more than 160 rows leaves room for
 //     one CTA only, but has five stages again;
 //   * operands of all CTAs come through the L2 at 23 TB/s, the weights from memory at 5, at 5.7 in a single wave;
-//   * a wave of CTAs costs 3.2 us to start and drain, and 0.0175 + 0.0035 split per activation row to write and add up;
+//   * a wave of CTAs costs 3.2 us to start and drain, and 0.0175 + 0.0035 split per activation row to write and add up; with the activation
+//     0.012 more where nothing else on the SM covers it and 0.002 split (3200 measured triples, 8 %; 471 x 2 x 3888 x 2048 18.3 us in two
+//     launches, 20.6 with 240 rows a tile);
 //   * clusters of 4 and 8 do not fill every SM: narrow_first and narrow_slots below;
 //   * less than eight steps are not split from 65 rows on, so that their sums are those of the tiled kernels whatever the number of rows (512
 //     x 512 x 256 5.7 us on tiles, 5.0 here, 4.5 in two parts);
@@ -243,7 +245,7 @@ static int narrow_slots(int bt, int split) {
   if (!narrow_two_per_sm(bt)) return narrow_first(split);
   return split <= 2 ? 2 * kNwSms : split == 4 ? 280 : 264;
 }
-static double narrow_plan(int M, int N, long long n_tiles, int K, bool ragged_x, bool ragged_w, int* bt_out, int* split_out) {
+static double narrow_plan(int M, int N, long long n_tiles, int K, bool gated, bool ragged_x, bool ragged_w, int* bt_out, int* split_out) {
   const int num_kb = (K + kNwBK - 1) / kNwBK, fewest = (M + 255) / 256;
   const double weights = (double)N * K * 2e-6;
   double best = 1e30, best_t = 1e30;
@@ -257,6 +259,7 @@ static double narrow_plan(int M, int N, long long n_tiles, int K, bool ragged_x,
       if (split > 1 && M > 64 && num_kb < 8) break;
       const long long ctas = (long long)((M + bt - 1) / bt) * n_tiles * split;
       const double steps = (num_kb + split - 1) / split;
+      const double row = 0.0175 + (gated && per_sm_most == 1 ? 0.012 : 0.0) + (split > 1 ? (gated ? 0.0055 : 0.0035) * split : 0.0);
       const int slots = narrow_slots(bt, split), first = narrow_first(split);
       auto wave = [&](long long n) {
         if (n == 0) return 0.0;
@@ -265,7 +268,7 @@ static double narrow_plan(int M, int N, long long n_tiles, int K, bool ragged_x,
         const double shared = per_sm * (0.078 + 0.00102 * bt) * (1 + 0.76 * lines), alone = 1.05 / narrow_stages(bt) * (1 + 0.21 * lines);
         const double l2 = n * bytes * (1 + lines) / 23.2e6;
         const double step = shared > alone ? (shared > l2 ? shared : l2) : (alone > l2 ? alone : l2);
-        return 3.2 + steps * step + per_sm * bt * (0.0175 + (split > 1 ? 0.0035 * split : 0.0));
+        return 3.2 + steps * step + per_sm * bt * row;
       };
       const double t = (double)(ctas / slots) * wave(slots) + wave(ctas % slots), memory = 4.0 + weights / (ctas <= slots ? 5.7 : 5.0);
       const double all = t > memory ? t : memory;
@@ -307,7 +310,7 @@ static double tiled_time(int M, int N, int K, int glu, int pair_min_tiles, bool 
 }
 double few_rows_time(int M, int N, int K) {
   int bt = 0, split = 0;
-  const double narrow = narrow_plan(M, N, (N + 127) / 128, K, false, false, &bt, &split), tiled = tiled_time(M, N, K, 0, 0, false, false);
+  const double narrow = narrow_plan(M, N, (N + 127) / 128, K, false, false, false, &bt, &split), tiled = tiled_time(M, N, K, 0, 0, false, false);
   return narrow < tiled ? narrow : tiled;
 }
 
@@ -410,6 +413,6 @@ KSA_API int ksa_gemm_narrow_plan(int M, int N, int K, int glu, int pair_min_tile
   if (M <= 0 || M > kNwMaxRows || N <= 0 || K <= 0 || (glu == 1 ? K <= kNwBK : (long long)N * K < 32768)) return 0;
   int bt = 0, split = 0;
   const bool rx = (ragged & 1) != 0, rw = (ragged & 2) != 0;
-  const double t = narrow_plan(M, N, glu == 1 ? (N / 2 + 63) / 64 : (N + 127) / 128, K, rx, rw, &bt, &split) + (glu == 2 ? 2.0 : 0.0);
+  const double t = narrow_plan(M, N, glu == 1 ? (N / 2 + 63) / 64 : (N + 127) / 128, K, glu == 1, rx, rw, &bt, &split) + (glu == 2 ? 2.0 : 0.0);
   return t < (M <= 64 && enough_for_pairs(M, N, pair_min_tiles) ? 1.4 : 0.95) * tiled_time(M, N, K, glu, pair_min_tiles, rx, rw) ? bt * 16 + split : 0;
 }

@@ -31,6 +31,24 @@ MEASURED = [
     ((5, 18408, 6144, 2), 55.4, {(16, 1): 35.3, (16, 2): 38.5}),
 ]
 
+GATED = [
+    ((471, 7776, 2048), 18.5, {(128, 1): 20.6, (240, 1): 20.6}),
+    ((675, 6144, 1024), 13.9, {(128, 1): 14.1, (144, 1): 14.6, (240, 1): 15.1}),
+    ((1193, 3504, 2048), 18.4, {(128, 1): 20.1, (144, 1): 21.2, (240, 1): 20.2}),
+    ((471, 9728, 2048), 24.8, {(160, 1): 23.1}),
+    ((48, 19456, 2560), 22.5, {(48, 1): 20.2}),
+    ((333, 1040, 1024), 8.1, {(48, 1): 7.6, (48, 2): 6.4, (64, 2): 7.4, (80, 2): 7.6}),
+    ((129, 272, 2048), 6.7, {(48, 2): 7.3, (48, 4): 6.5, (48, 8): 7.1, (80, 4): 7.6}),
+    ((200, 7680, 6144), 27.2, {(112, 2): 29.5, (208, 2): 25.8}),
+    ((132, 6144, 4096), 17.3, {(48, 2): 15.9, (80, 2): 18.3}),
+    ((280, 6144, 2560), 17.3, {(48, 1): 15.7, (64, 1): 17.2, (80, 1): 18.8, (96, 2): 16.0}),
+    ((700, 3072, 4096), 21.0, {(64, 1): 24.0, (128, 2): 22.4, (144, 2): 23.6, (176, 1): 24.5, (240, 2): 21.3}),
+    ((1024, 12288, 2048), 44.0, {}),
+    ((1306, 3072, 1024), 13.8, {(112, 1): 13.1, (128, 1): 13.8, (144, 1): 14.4, (160, 1): 15.1, (224, 1): 14.3}),
+    ((64, 2048, 1024), 6.7, {(64, 2): 7.5, (64, 4): 7.1}),
+    ((381, 12288, 256), 11.7, {(128, 1): 9.6}),
+]
+
 
 @pytest.mark.parametrize("shape,tiled,plans", MEASURED, ids=lambda v: "x".join(map(str, v)) if isinstance(v, tuple) else "")
 def test_the_choice_is_near_the_best(shape, tiled, plans):
@@ -47,6 +65,15 @@ def test_the_choice_is_near_the_best(shape, tiled, plans):
 def test_a_separate_activation_counts_against_the_split(shape, fused, split):
     M, N, K = shape
     assert (_lib.gemm_narrow_plan(M, N, K, 2, 32) is not None) == (split < fused)
+
+
+# (rows, gate and up rows, K), us of the product and the activation in two launches, and of the gated plans that come within a fifth of the best
+@pytest.mark.parametrize("shape,two,gated", GATED, ids=lambda v: "x".join(map(str, v)) if isinstance(v, tuple) else "")
+def test_the_gated_choice_is_near_the_best(shape, two, gated):
+    M, N, K = shape
+    plan = _lib.gemm_narrow_plan(M, N, K, 1, 32)
+    time = two if plan is None else gated.get(plan, float("inf"))
+    assert time <= 1.1 * min([two, *gated.values()]), (plan, time)
 
 
 # (rows, columns, K, gated), us of the kernels that serve it otherwise, and with all rows in one tile
