@@ -52,7 +52,7 @@ GATED = [
 
 @pytest.mark.parametrize("shape,tiled,plans", MEASURED, ids=lambda v: "x".join(map(str, v)) if isinstance(v, tuple) else "")
 def test_the_choice_is_near_the_best(shape, tiled, plans):
-    """Within a tenth, twice the model's share of what it chooses wrongly at all."""
+    """Within a tenth, about the standard deviation of the modelled times."""
     M, N, K, ragged = shape
     plan = _lib.gemm_narrow_plan(M, N, K, 0, 32, ragged)
     time = tiled if plan is None else plans.get(plan, float("inf"))
